@@ -19,8 +19,8 @@ import numpy as np
 import torch
 
 from .base import CudaAugBase
-from ..ops.cuda_fun_tools import (affine_2d, affine_3d, affine_label_2d, affine_label_3d, apply_offset_2d,
-                                  apply_offset_3d)
+from .. import _C
+from ..ops.cuda_fun_tools import affine_2d, affine_3d, apply_offset_2d, apply_offset_3d
 
 
 def _one_roi(dim, center, shape, shifts, scales, rotate):
@@ -32,21 +32,17 @@ def _one_roi(dim, center, shape, shifts, scales, rotate):
 
 def _resample_sample(result, dim, rois, out_size, sampling_ratio, order):
     """Resamples every image field (order ``order``) and label field (nearest) of one sample."""
-    out_size = tuple(int(v) for v in out_size)
-    fn, label_fn = (affine_2d, affine_label_2d) if dim == 2 else (affine_3d, affine_label_3d)
-    for key in result.get('img_fields', []):
-        image = result[key]
-        assert image.is_cuda, 'image should be cuda'
-        assert image.ndim == dim + 1, 'image should be channel, **dim'
-        img = fn(image.unsqueeze(0), rois.to(image.device), out_size, 1.0, sampling_ratio, True, order).squeeze(0)
-        result[key] = img
-        if key == 'img':
-            result['img_shape'] = tuple(img.shape)
-    for key in result.get('seg_fields', []):
-        seg = result[key]
-        assert seg.is_cuda, 'seg should be cuda'
-        assert seg.ndim == dim + 1, 'seg should be channel, **dim'
-        result[key] = label_fn(seg.unsqueeze(0), rois.to(seg.device), out_size, 1.0, True).squeeze(0)
+    img_keys, seg_keys = list(result.get('img_fields', ())), list(result.get('seg_fields', ()))
+    for key in img_keys + seg_keys:
+        assert result[key].is_cuda, 'image should be cuda'
+        assert result[key].ndim == dim + 1, 'image should be channel, **dim'
+    images, labels = _C._native.resample_fields(dim, [result[k].unsqueeze(0) for k in img_keys],
+                                                [result[k].unsqueeze(0) for k in seg_keys], rois,
+                                                tuple(int(v) for v in out_size), sampling_ratio, order)
+    for key, t in zip(img_keys + seg_keys, images + labels):
+        result[key] = t.squeeze(0)
+    if 'img' in img_keys:
+        result['img_shape'] = tuple(result['img'].shape)
     for _ in result.get('det_fields', []):
         raise NotImplementedError('detection boxes are not transformed by this implementation')
 

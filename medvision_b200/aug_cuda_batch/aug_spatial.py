@@ -17,61 +17,37 @@ import numpy as np
 import torch
 
 from .base import BatchCudaAugBase
-from ..ops.cuda_fun_tools import (affine_2d, affine_3d, affine_fields_3d, affine_label_2d, affine_label_3d,
-                                  apply_offset_2d, apply_offset_3d)
-from ..ops.roi_stage import stage_rois
+from .. import _C
+from ..ops.cuda_fun_tools import affine_2d, affine_3d, apply_offset_2d, apply_offset_3d
 
 
 def _resample_fields(result, dim, rois, out_size, sampling_ratio, order):
-    """All image and label fields of ``result`` through the rois of this call (CPU float32).  The rois go to the
-    device once (one asynchronous copy, float32 and float16 at once); in 3D an image field and a label field are
-    resampled by one fused call whose label work rides along with the image's launches."""
-    out_size = tuple(int(v) for v in out_size)
+    """All image and label fields of ``result`` through the rois of this call (CPU float32), in one native call: the rois
+    go to the device once (one asynchronous copy, float32 and float16 at once); in 3D an image field and a label field are
+    resampled by one fused launch pair whose label work rides along with the image's."""
     assert not result.get('det_fields'), 'detection boxes are not handled by the resampling transforms'
-    img_keys, seg_keys = list(result.get('img_fields', [])), list(result.get('seg_fields', []))
-    fields = [result[k] for k in img_keys + seg_keys]
-    if not fields:
-        return
-    for image in fields:
-        assert image.is_cuda, 'image should be cuda'
-        assert image.ndim == dim + 2, 'image should be batch, channel, **dim'
-    device = fields[0].device
-    rois_f32, rois_f16, release = stage_rois(rois, device)
-
-    def rois_for(t):
-        r = rois_f16 if t.dtype == torch.float16 else rois_f32
-        return r if t.device == device else r.to(t.device, non_blocking=True)
-
-    fn = affine_2d if dim == 2 else affine_3d
-    label_fn = affine_label_2d if dim == 2 else affine_label_3d
-    fused = 0
-    if dim == 3 and sampling_ratio == 1 and order in (0, 1):  # pairs of (image field, label field): one call each
-        for ik, sk in zip(img_keys, seg_keys):
-            image, seg = result[ik], result[sk]
-            if image.device != device or seg.device != device or image.shape[0] != seg.shape[0] \
-                    or image.shape[2:] != seg.shape[2:] or image.dtype not in (torch.float16, torch.float32):
-                break
-            result[ik], result[sk] = affine_fields_3d(image, seg, rois_f32, out_size, 1.0, True, order,
-                                                      rois_image=rois_for(image))
-            fused += 1
-    for key in img_keys[fused:]:
-        image = result[key]
-        result[key] = fn(image, rois_for(image), out_size, 1.0, sampling_ratio, True, order)
-    for key in seg_keys[fused:]:
-        image = result[key]
-        # = fn(image.float(), rois, out_size, 1.0, 1, True, 0).int() of the reference, on the integers themselves
-        r = rois_f32 if image.device == device else rois_f32.to(image.device, non_blocking=True)
-        result[key] = label_fn(image, r, out_size, 1.0, True)
-    release()
+    img_keys, seg_keys = result.get('img_fields', ()), result.get('seg_fields', ())
+    images, labels = _C._native.resample_fields(dim, [result[k] for k in img_keys], [result[k] for k in seg_keys], rois,
+                                                tuple(int(v) for v in out_size), sampling_ratio, order)
+    result.update(zip(img_keys, images))
+    result.update(zip(seg_keys, labels))
 
 
 def _affine_rois(index, center, shape, shifts, scales, rotate, dim):
-    """[index, center - shape * shifts / scales, shape / scales, angles]; rotation about z in 3D."""
-    if dim == 2:
-        angles = rotate
-    else:
-        angles = torch.cat([torch.zeros_like(rotate), torch.zeros_like(rotate), rotate], dim=1)
-    return torch.cat([index, center - shape * shifts / scales, shape / scales, angles], dim=-1)
+    """[index, center - shape * shifts / scales, shape / scales, angles] in float32; rotation about z in 3D."""
+    scales = scales.astype(np.float32)
+    rois = np.zeros((len(scales), 2 * dim + (2 if dim == 2 else 4)), dtype=np.float32)
+    rois[:, 0] = index
+    rois[:, 1:1 + dim] = center - shape * shifts.astype(np.float32) / scales
+    rois[:, 1 + dim:1 + 2 * dim] = shape / scales
+    rois[:, -1:] = rotate
+    return torch.from_numpy(rois)
+
+
+def _whole_image(image_shape):
+    """Centre and extent (float32, xyz) of a (d,) h, w shape."""
+    shape = np.array(image_shape[::-1], dtype=np.float32)
+    return shape / 2, shape
 
 
 class BatchCudaResize(BatchCudaAugBase):
@@ -117,12 +93,10 @@ class BatchCudaResize(BatchCudaAugBase):
             self.params = tuple(1 / np.array(params))
 
     def _rois(self):
-        index = torch.arange(self.batch, dtype=torch.float32).unsqueeze(-1)
-        center = torch.tensor([i / 2 for i in self.image_shape[::-1]], dtype=torch.float32)  # dhw => xyz
-        shape = torch.tensor(list(self.image_shape[::-1]), dtype=torch.float32)
-        angles = torch.zeros(1 if self.dim == 2 else 3)
-        boxes = torch.cat([center, shape, angles]).unsqueeze(0).repeat(self.batch, 1)
-        return torch.cat([index, boxes], dim=-1)
+        rois = np.zeros((self.batch, 2 * self.dim + (2 if self.dim == 2 else 4)), dtype=np.float32)
+        rois[:, 0] = np.arange(self.batch)
+        rois[:, 1:1 + self.dim], rois[:, 1 + self.dim:1 + 2 * self.dim] = _whole_image(self.image_shape)
+        return torch.from_numpy(rois)
 
     def apply_to_img(self, result):
         # the whole image is one roi; image and label fields share it
@@ -152,12 +126,8 @@ class BatchCudaRandomAffine(BatchCudaAugBase):
 
     def _forward_params(self, result):
         self._init_params(result)
-        scales, shifts, rotate = [], [], []
-        for _ in range(self.batch):
-            scales.append([self.get_range(self.scale, 1), ] * self.dim)
-            shifts.append([self.get_range(self.shift, 0) for _ in range(self.dim)])
-            rotate.append([math.pi * self.get_range(self.rotate, 0) / 180])
-        self.params = {"scales": np.array(scales), "shifts": np.array(shifts), "rotate": np.array(rotate)}
+        scales, shifts, rotate = self._draw_affine(self.batch)
+        self.params = {"scales": scales, "shifts": shifts, "rotate": rotate}
         result[self.key_name] = self.params
 
     def _backward_params(self, result: dict):
@@ -167,13 +137,9 @@ class BatchCudaRandomAffine(BatchCudaAugBase):
             self.params = {"scales": 1 / params["scales"], "shifts": -params["shifts"], "rotate": -params["rotate"]}
 
     def _rois(self):
-        scales = torch.FloatTensor(self.params["scales"])
-        shifts = torch.FloatTensor(self.params["shifts"])
-        rotate = torch.FloatTensor(self.params["rotate"])
-        index = torch.arange(self.batch, dtype=torch.float32).unsqueeze(-1)
-        center = torch.tensor([i / 2 for i in self.image_shape[::-1]], dtype=torch.float32)
-        shape = torch.tensor(list(self.image_shape[::-1]), dtype=torch.float32)
-        return _affine_rois(index, center, shape, shifts, scales, rotate, self.dim)
+        center, shape = _whole_image(self.image_shape)
+        return _affine_rois(np.arange(self.batch), center, shape, self.params["shifts"], self.params["scales"],
+                            self.params["rotate"], self.dim)
 
     def apply_to_img(self, result: dict):
         _resample_fields(result, self.dim, self._rois(), self.image_shape, self.sampling_ratio, self.order)
@@ -325,12 +291,7 @@ class BatchCudaCropRandomWithAffine(BatchCudaAugBase):
         result[self.key_name] = self.params
 
     def _forward_affine_params(self, result: dict):
-        scales, shifts, rotate = [], [], []
-        for _ in range(self.batch):
-            scales.append([self.get_range(self.scale, 1), ] * self.dim)
-            shifts.append([self.get_range(self.shift, 0) for _ in range(self.dim)])
-            rotate.append([math.pi * self.get_range(self.rotate, 0) / 180])
-        return np.array(scales), np.array(shifts), np.array(rotate)
+        return self._draw_affine(self.batch)
 
     def _random_start(self):
         return tuple(map(lambda a, da: np.random.randint(0, a - da + 1), self.image_shape, self.patch_size))
@@ -349,17 +310,16 @@ class BatchCudaCropRandomWithAffine(BatchCudaAugBase):
         return np.array(batch_start), np.array(batch_end)
 
     def _forward_crop_params(self, result: dict):
-        return self._collect([self._random_start() for _ in range(self.batch)])
+        # one draw per patch and axis (d, h, w), as _random_start() makes them
+        start = np.random.randint(0, np.tile(np.subtract(self.image_shape, self.patch_size) + 1, (self.batch, 1)))
+        return start[:, ::-1], (start + np.array(self.patch_size))[:, ::-1]
 
     def _rois(self):
-        start = torch.FloatTensor(self.params["start"])
-        end = torch.FloatTensor(self.params["end"])
-        scales = torch.FloatTensor(self.params["scales"])
-        shifts = torch.FloatTensor(self.params["shifts"])
-        rotate = torch.FloatTensor(self.params["rotate"])
+        start = self.params["start"].astype(np.float32)
+        end = self.params["end"].astype(np.float32)
         # patch r*B + b is cut from image b
-        index = (torch.arange(self.batch) % self.n_images).float().unsqueeze(-1)
-        return _affine_rois(index, (start + end) / 2, end - start, shifts, scales, rotate, self.dim)
+        return _affine_rois(np.arange(self.batch) % self.n_images, (start + end) / 2, end - start, self.params["shifts"],
+                            self.params["scales"], self.params["rotate"], self.dim)
 
     def apply_to_img(self, result: dict):
         _resample_fields(result, self.dim, self._rois(), self.patch_size, self.sampling_ratio, self.order)

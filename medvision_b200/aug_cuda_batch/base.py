@@ -12,6 +12,7 @@ of the random draws are the interface a pipeline relies on; the bodies are this 
 * ``backward`` pops that log entry and, for a transform with ``canBackward``, applies the inverse
   parameters (``_backward_params``) through the same ``apply_to_*`` hooks.
 """
+import math
 import random
 import time
 from datetime import datetime
@@ -19,6 +20,8 @@ from typing import Iterable, List, Tuple, Union
 
 import numpy as np
 import torch
+
+from .. import _C
 
 # field families, in the order the hooks run
 _HOOKS = ('apply_to_img', 'apply_to_cls', 'apply_to_seg', 'apply_to_det')
@@ -52,15 +55,34 @@ class BatchCudaAugBase(object):
 
     # ---- parameter helpers ------------------------------------------------------------------
     @staticmethod
-    def get_range(val_range, bias=0, always_pos=False):
-        """One uniform draw: a number r stands for [-r, r] (or [0, r] with ``always_pos``), a pair is
-        taken as it is; ``bias`` is added to the draw."""
+    def _bounds(val_range, always_pos=False):
         if not isinstance(val_range, (list, tuple)):
             assert isinstance(val_range, (int, float))
             val_range = (0 if always_pos else -val_range, val_range)
         lo, hi = val_range  # a pair, nothing else
         assert hi >= lo
+        return lo, hi
+
+    @staticmethod
+    def get_range(val_range, bias=0, always_pos=False):
+        """One uniform draw: a number r stands for [-r, r] (or [0, r] with ``always_pos``), a pair is
+        taken as it is; ``bias`` is added to the draw."""
+        lo, hi = BatchCudaAugBase._bounds(val_range, always_pos)
         return bias + np.random.uniform(lo, hi)
+
+    def _draw_affine(self, n):
+        """Scale, shifts and rotation (radians) of ``n`` samples: the values that :meth:`get_range` draws sample by sample
+        -- scale, one shift per axis, rotation -- from one array of uniform numbers (numpy's ``uniform(lo, hi)`` is
+        ``lo + (hi - lo) * random_sample()``, one number per draw).  Returns (n, dim), (n, dim) and (n, 1) arrays."""
+        dim = self.dim
+        u = np.random.random_sample((n, dim + 2))
+        lo, hi = self._bounds(self.scale)
+        scales = np.empty((n, dim))
+        scales[:] = 1 + (lo + (hi - lo) * u[:, :1])
+        lo, hi = self._bounds(self.shift)
+        shifts = 0 + (lo + (hi - lo) * u[:, 1:-1])
+        lo, hi = self._bounds(self.rotate)
+        return scales, shifts, math.pi * (0 + (lo + (hi - lo) * u[:, -1:])) / 180
 
     @staticmethod
     def to_tuple(value: Union[int, float, Iterable[int], Iterable[float]], length: int = 1) \
@@ -130,7 +152,7 @@ class BatchCudaAugBase(object):
         took = time.time() - self._tic_
         began = datetime.fromtimestamp(self._tic_).strftime('%H:%M:%S.%f')
         # the reference logs the allocator's peak divided by 1024 * 1024 * 8 under the label "MB"; kept as is
-        peak = torch.cuda.max_memory_allocated() / (1024 * 1024 * 8) if torch.cuda.is_available() else 0.0
+        peak = _C._native.peak_allocated() / (1024 * 1024 * 8) if torch.cuda.is_initialized() else 0.0
         result['history'].append(self.name)
         result['time'].append(f"{self.name}-{began}-{took:.03f}s")
         result['memory'].append(f"{self.name}-{peak:.02f}MB")

@@ -5,25 +5,9 @@ Same signatures as ``affine_2d`` / ``affine_3d`` of medvision/ops/cuda_fun_tools
 import torch
 
 from .. import _C
-from ._common import parse_output_size
 
-
-
-def _affine(ndim, features, rois, out_size, spatial_scale, sampling_ratio, aligned, order):
-    out = parse_output_size(out_size, ndim, name="out_size")
-    assert features.dtype in [torch.float32, torch.float16], \
-        f'input must be float16 or float32 but got {features.dtype}'
-    assert order in [0, 1, 3], f'order {order} is not supported!'
-    if order == 0:
-        # one sample per output voxel: averaging would blend labels
-        sampling_ratio = 1
-    assert features.dim() == ndim + 2
-    output = features.new_empty((rois.size(0), features.size(1)) + tuple(out))
-    # the rois take the dtype (and device) of the image, as rois.type(features.type()) does
-    rois = rois.to(device=features.device, dtype=features.dtype)
-    fn = _C.affine_2d if ndim == 2 else _C.affine_3d
-    fn(features, rois, output, *out, spatial_scale, sampling_ratio, aligned, order)
-    return output
+_affine = _C._native.affine
+_affine_label = _C._native.affine_label
 
 
 def affine_2d(features, rois, out_size, spatial_scale, sampling_ratio=0, aligned=True, order=1):
@@ -63,17 +47,6 @@ def apply_offset_3d(img, offset, order=1):
     return _apply_offset(3, img, offset, order)
 
 
-def _affine_label(ndim, seg, rois, out_size, spatial_scale, aligned):
-    assert seg.dim() == ndim + 2 and len(out_size) == ndim
-    rois = rois.to(device=seg.device, dtype=torch.float32)
-    if seg.dtype in _C._LABEL_DTYPES:
-        out = torch.empty((rois.shape[0], seg.shape[1], *out_size), dtype=torch.int32, device=seg.device)
-        if _C.affine_label(seg, rois, out, tuple(int(v) for v in out_size), spatial_scale, aligned):
-            return out
-    fn = affine_2d if ndim == 2 else affine_3d
-    return fn(seg.float(), rois, out_size, spatial_scale, 1, aligned, 0).int()
-
-
 def affine_fields_3d(image, seg, rois, out_size, spatial_scale=1.0, aligned=True, order=1, rois_image=None):
     """An image field and a label field over the same volumes, resampled with the same rois in one go:
     returns ``(affine_3d(image, rois, out_size, spatial_scale, 1, aligned, order),
@@ -98,9 +71,9 @@ def affine_label_2d(seg, rois, out_size, spatial_scale=1.0, aligned=True):
     """Label map (N, C, H, W) of an integer dtype -> int32 (R, C, oh, ow): what the reference's
     augmentations compute as ``affine_2d(seg.float(), rois, out_size, spatial_scale, 1, aligned,
     0).int()`` (medvision/aug_cuda_batch/aug_spatial.py:158-194), in one kernel on the integers."""
-    return _affine_label(2, seg, rois, out_size, spatial_scale, aligned)
+    return _affine_label(2, seg, rois, tuple(int(v) for v in out_size), spatial_scale, aligned)
 
 
 def affine_label_3d(seg, rois, out_size, spatial_scale=1.0, aligned=True):
     """3D: (N, C, D, H, W) -> int32 (R, C, od, oh, ow)."""
-    return _affine_label(3, seg, rois, out_size, spatial_scale, aligned)
+    return _affine_label(3, seg, rois, tuple(int(v) for v in out_size), spatial_scale, aligned)

@@ -6,51 +6,22 @@ Same public surface as medvision/ops/roi_align_rotated_nd.py: ``RoIAlignRotated2
 (``RoIAlignRotated(output_size, spatial_scale, sampling_ratio=-1, aligned=True)(features, rois, order=1)``).
 """
 import torch.nn as nn
-from torch.autograd import Function
 
 from .. import _C
-from ._common import parse_output_size
+
+# features, rois, output_size, spatial_scale, sampling_ratio=0, aligned=True, order=1; differentiable in the features
+roi_align_rotated_2d = _C._native.roi_align_rotated_2d
+roi_align_rotated_3d = _C._native.roi_align_rotated_3d
 
 
-def _make_function(ndim):
-    fwd = _C.roi_align_rotated_2d_forward if ndim == 2 else _C.roi_align_rotated_3d_forward
-    bwd = _C.roi_align_rotated_2d_backward if ndim == 2 else _C.roi_align_rotated_3d_backward
-
-    class _RoIAlignRotatedFunction(Function):
-        @staticmethod
-        def forward(ctx, features, rois, output_size, spatial_scale, sampling_ratio=0, aligned=True, order=1):
-            out = parse_output_size(output_size, ndim)
-            ctx.spatial_scale = spatial_scale
-            ctx.sampling_ratio = sampling_ratio
-            ctx.aligned = aligned
-            ctx.order = order
-            ctx.save_for_backward(rois)
-            ctx.feature_size = features.size()
-            assert features.dim() == ndim + 2
-            output = features.new_empty((rois.size(0), features.size(1)) + tuple(out))
-            fwd(features, rois, output, *out, spatial_scale, sampling_ratio, aligned, order)
-            return output
-
-        @staticmethod
-        def backward(ctx, grad_output):
-            rois = ctx.saved_tensors[0]
-            assert ctx.feature_size is not None
-            grad_input = None
-            if ctx.needs_input_grad[0]:
-                grad_input = rois.new_zeros(ctx.feature_size)
-                bwd(grad_output.contiguous(), rois, grad_input, *grad_output.shape[2:],
-                    ctx.spatial_scale, ctx.sampling_ratio, ctx.aligned, ctx.order)
-            return grad_input, None, None, None, None, None, None
-
-    _RoIAlignRotatedFunction.__name__ = f"RoIAlignRotated{ndim}DFunction"
-    _RoIAlignRotatedFunction.__qualname__ = _RoIAlignRotatedFunction.__name__
-    return _RoIAlignRotatedFunction
+class RoIAlignRotated2DFunction:
+    """``apply`` is the differentiable operation; its autograd node is native (csrc/mvr_torch.cpp)."""
+    apply = staticmethod(roi_align_rotated_2d)
 
 
-RoIAlignRotated2DFunction = _make_function(2)
-RoIAlignRotated3DFunction = _make_function(3)
-roi_align_rotated_2d = RoIAlignRotated2DFunction.apply
-roi_align_rotated_3d = RoIAlignRotated3DFunction.apply
+class RoIAlignRotated3DFunction:
+    """See :class:`RoIAlignRotated2DFunction`."""
+    apply = staticmethod(roi_align_rotated_3d)
 
 
 class RoIAlignRotated(nn.Module):

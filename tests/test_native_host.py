@@ -1,0 +1,60 @@
+"""The native host path: draws made from one array equal the draws made one by one; the ring through which a transform's
+rois are uploaded gives every call its own rois, whatever the number of calls in flight, threads and streams."""
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+from medvision_b200.aug_cuda_batch import BatchCudaCropRandomWithAffine, BatchCudaRandomAffine
+
+
+@pytest.mark.parametrize("shape,patch", [((3, 1, 8, 10, 12), (4, 10, 6)), ((2, 1, 33, 17), (33, 5))])
+def test_draws_equal_the_scalar_draws_bit_for_bit(shape, patch):
+    dim = len(patch)
+    res = {"img_dim": dim, "img": torch.zeros(shape), "img_fields": ["img"], "seg_fields": []}
+    t = BatchCudaCropRandomWithAffine(patch, scale=(-0.05, 0.3), shift=0.1, rotate=(5, 5), times=7)
+    np.random.seed(3)
+    t._forward_params(dict(res))
+    state = np.random.get_state()[2]
+    np.random.seed(3)
+    starts = [t._random_start() for _ in range(7 * shape[0])]
+    affine = [([t.get_range(t.scale, 1)] * dim, [t.get_range(t.shift, 0) for _ in range(dim)],
+               [np.pi * t.get_range(t.rotate, 0) / 180]) for _ in range(7 * shape[0])]
+    assert np.random.get_state()[2] == state
+    assert np.array_equal(t.params["start"], np.array([s[::-1] for s in starts]))
+    assert np.array_equal(t.params["end"] - t.params["start"], np.broadcast_to(patch[::-1], (7 * shape[0], dim)))
+    for k, key in enumerate(("scales", "shifts", "rotate")):
+        assert np.array_equal(t.params[key], np.array([a[k] for a in affine]))
+
+
+@pytest.mark.gpu
+def test_roi_uploads_from_several_threads_and_streams_do_not_mix():
+    from medvision_b200 import _C
+    from medvision_b200.ops import affine_3d
+    img = torch.rand(2, 1, 20, 24, 32, generator=torch.Generator().manual_seed(1)).cuda()
+    t = BatchCudaRandomAffine(1.0, scale=0.2, shift=0.1, rotate=25)
+    sets = []
+    for k in range(24):  # three times the ring's slots; one set larger than what the ring was made for
+        t._forward_params({"img_dim": 3, "img": img})
+        rois = t._rois()
+        sets.append(rois.repeat(150, 1) if k == 11 else rois)
+    want = [affine_3d(img, r.cuda(), (16, 16, 20), 1.0, 1, True, 1) for r in sets]
+    torch.cuda.synchronize()
+    got = [None] * len(sets)
+
+    def work(lane):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for rep in range(3):
+                for k in range(lane, len(sets), 2):
+                    got[k] = _C._native.resample_fields(3, [img], [], sets[k], (16, 16, 20), 1, 1)[0][0]
+
+    threads = [threading.Thread(target=work, args=(lane,)) for lane in (0, 1)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    _C.release_cached_memory()  # the ring goes away and comes back
+    assert torch.equal(_C._native.resample_fields(3, [img], [], sets[0], (16, 16, 20), 1, 1)[0][0], want[0])
