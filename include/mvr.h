@@ -270,6 +270,20 @@ int mvr_apply_offset_2d(const void* img, const void* offset, void* out, int dtyp
 int mvr_apply_offset_3d(const void* img, const void* offset, void* out, int dtype, int offset_dtype, int64_t B,
                         int64_t C, int64_t D, int64_t H, int64_t W, int order, void* stream);
 
+/* Elastic deformation from the coarse grid of control points, without a dense field in memory: what
+ *     field = affine_*(coarse, roi of the inner control points, (D, H, W), 1, 1, aligned, order = 3)
+ *     image_out = apply_offset_*(image, field, order = 1)
+ *     label_out = apply_offset_*(labels cast to dtype, field, order = 0) cast to int32
+ * compute (medvision/aug_cuda_batch/aug_spatial.py:204-313).  coarse is FLOAT32 (B, ndim, [gd,] gh, gw) with the
+ * displacement along [d,] h, w in voxels; `border` control points are locked on every side, so the roi is centred on the
+ * grid and 2 * border - 1 cells narrower than it.  image (B, C_image, [D,] H, W) of dtype and labels (B, C_label, ...) of
+ * label_dtype may each be null; dtype is also the type the sample positions are formed in.  With `field` given, only the
+ * dense field, float32 (B, ndim, [D,] H, W), is written.  Returns MVR_ERR_UNSUPPORTED for grids whose tables exceed a
+ * CTA's shared memory or of fewer than 2 * border points (use the two-step form). */
+int mvr_elastic(const float* coarse, int ndim, int gd, int gh, int gw, int border, const void* image, int dtype,
+                void* image_out, int64_t C_image, const void* labels, int label_dtype, int32_t* label_out, int64_t C_label,
+                float* field, int64_t B, int64_t D, int64_t H, int64_t W, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

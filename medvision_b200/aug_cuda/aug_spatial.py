@@ -20,7 +20,7 @@ import torch
 
 from .base import CudaAugBase
 from .. import _C
-from ..ops.cuda_fun_tools import affine_2d, affine_3d, apply_offset_2d, apply_offset_3d
+from ..aug_cuda_batch.elastic_field import ElasticField
 
 
 def _one_roi(dim, center, shape, shifts, scales, rotate):
@@ -169,10 +169,11 @@ class CudaRandomRotate(CudaRandomAffine):
         super().__init__(p, scale=0, shift=0, rotate=rotate, sampling_ratio=sampling_ratio)
 
 
-class CudaRandomElasticDeformation(CudaAugBase):
+class CudaRandomElasticDeformation(ElasticField, CudaAugBase):
     """Random smooth warp: a coarse grid of random displacements (two outermost control points of
-    every axis locked) is blown up to a dense field by one Catmull-Rom ``affine_*`` resample and
-    applied with ``apply_offset_*`` -- linear for images, nearest for labels."""
+    every axis locked), interpolated to every voxel with Catmull-Rom and applied -- linear for images,
+    nearest for labels.  ``dense_field`` / ``tmp_params`` is the field itself, made when it is asked for."""
+    _field_order = 3
 
     def __init__(self, p, num_control_points=8, max_displacement: float = 0.8):
         super().__init__()
@@ -182,7 +183,6 @@ class CudaRandomElasticDeformation(CudaAugBase):
         self.SPLINE_ORDER = 3
         self.num_locked_borders = 2
         assert max_displacement <= 1.0
-        self.tmp_params = None
 
     def __repr__(self):
         return self.__class__.__name__ + "(p={}, num_control_points={}, max_displacement={})".format(
@@ -195,17 +195,7 @@ class CudaRandomElasticDeformation(CudaAugBase):
     def _forward_params(self, result):
         self.tmp_params = None
         self._init_params(result)
-        grid_shape = self.to_tuple(self.num_control_points, self.dim)
-        reach = self.max_displacement * (np.array(self.image_shape) / (np.array(grid_shape) - 1)) / 2
-        coarse = 2 * np.random.rand(*grid_shape, self.dim).astype(np.float32) - 1  # [-1, 1)
-        coarse *= reach.astype(np.float32)
-        for axis in range(self.dim):
-            locked = [slice(None)] * self.dim
-            for i in range(self.num_locked_borders):
-                for pos in (i, -1 - i):
-                    locked[axis] = pos
-                    coarse[tuple(locked)] = 0
-        self.params = coarse
+        self.params = self._draw_coarse()
         result[self.key_name] = self.params
 
     def _backward_params(self, result):
@@ -215,38 +205,38 @@ class CudaRandomElasticDeformation(CudaAugBase):
         if params is not None:
             self.params = -params
 
+    def _blow_up(self, device):
+        return super()._blow_up(device).squeeze(0)
+
+    def _warp_with_dense_field(self, image, field, order):
+        return super()._warp_with_dense_field(image.unsqueeze(0), field.unsqueeze(0), order).squeeze(0)
+
     def dense_field(self, device):
         """(dim, *image_shape) float32 displacement field on ``device``."""
-        if self.tmp_params is None:
-            coarse = torch.from_numpy(self.params).permute(self.dim, *range(self.dim)) / 2  # halved to smooth
-            grid = coarse.shape[1:]
-            center = torch.tensor([i / 2 for i in grid[::-1]], dtype=torch.float32)
-            shape = torch.tensor(list(grid[::-1]), dtype=torch.float32) - (2 * self.num_locked_borders - 1)
-            rois = _one_roi(self.dim, center, shape, torch.zeros(self.dim), torch.ones(self.dim), 0.0).to(device)
-            fn = affine_2d if self.dim == 2 else affine_3d
-            self.tmp_params = fn(coarse.contiguous().to(device).unsqueeze(0), rois, tuple(self.image_shape), 1, 1,
-                                 True, self.SPLINE_ORDER).squeeze(0)
-        return self.tmp_params
+        if self._dense is None:
+            self._dense = self._blow_up(device)
+        return self._dense
 
     def elastic_transform(self, image: torch.Tensor, order=1):
-        field = self.dense_field(image.device)
-        if order == 0:
-            image = image.to(self.img_type)
-        fn = apply_offset_2d if self.dim == 2 else apply_offset_3d
-        image = fn(image.unsqueeze(0), field.unsqueeze(0), order=order).squeeze(0)
-        return image.int() if order == 0 else image
+        return self._warp_with_dense_field(image, self.dense_field(image.device), order)
 
     def apply_to_img(self, result):
-        for key in result.get('img_fields', []):
-            result[key] = self.elastic_transform(result[key])
+        # image and label fields together
+        img_keys, seg_keys = list(result.get('img_fields', ())), list(result.get('seg_fields', ()))
+        images, labels = self._warp_fields([result[k] for k in img_keys], [result[k] for k in seg_keys])
+        result.update(zip(img_keys, images))
+        result.update(zip(seg_keys, labels))
 
     def apply_to_seg(self, result):
-        for key in result.get('seg_fields', []):
-            result[key] = self.elastic_transform(result[key], order=0)
+        pass  # done together with the images
 
     def apply_to_det(self, result):
         for _ in result.get('det_fields', []):
             raise NotImplementedError
+
+    def _warp_coarse(self, images, labels):
+        both = super()._warp_coarse([t.unsqueeze(0) for t in images], [t.unsqueeze(0) for t in labels])
+        return both and tuple([t.squeeze(0) for t in v] for v in both)
 
 
 class CudaCropRandomWithAffine(CudaAugBase):

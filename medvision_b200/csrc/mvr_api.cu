@@ -14,6 +14,7 @@
 #include "mvr_flat.cuh"
 #include "mvr_label.cuh"
 #include "mvr_plane2d.cuh"
+#include "mvr_elastic.cuh"
 
 // ---- scratch of the entry point that allocates nothing ------------------------------------
 // Lives in the library image: every GPU that loads the library holds these 16 MiB until the
@@ -365,6 +366,39 @@ int mvr_apply_offset_2d(const void* img, const void* offset, void* out, int dtyp
 int mvr_apply_offset_3d(const void* img, const void* offset, void* out, int dtype, int offset_dtype, int64_t B,
                         int64_t C, int64_t D, int64_t H, int64_t W, int order, void* stream) {
   return apply_offset_impl(img, offset, out, dtype, offset_dtype, 3, B, C, D, H, W, order, stream);
+}
+
+int mvr_elastic(const float* coarse, int ndim, int gd, int gh, int gw, int border, const void* image, int dtype,
+                void* image_out, int64_t C_image, const void* labels, int label_dtype, int32_t* label_out, int64_t C_label,
+                float* field, int64_t B, int64_t D, int64_t H, int64_t W, void* stream) {
+  if (dtype != MVR_F32 && dtype != MVR_F16) return MVR_ERR_DTYPE;
+  if (labels && (label_dtype < MVR_LABEL_U8 || label_dtype > MVR_LABEL_I64)) return MVR_ERR_DTYPE;
+  if (ndim != 2 && ndim != 3) return MVR_ERR_NDIM;
+  if (B < 0 || C_image < 0 || C_label < 0 || D < 1 || H < 1 || W < 1 || border < 1 || (ndim == 2 && (D != 1 || gd != 1)))
+    return MVR_ERR_SHAPE;
+  if (B > INT32_MAX || C_image > INT32_MAX || C_label > INT32_MAX || D * H * W >= 0x7fffffffLL) return MVR_ERR_TOO_LARGE;
+  if (!coarse || (image && !image_out) || (labels && !label_out)) return MVR_ERR_NULL;
+  const int g[3] = {gw, gh, gd}, size[3] = {(int)W, (int)H, (int)D};
+  ElasticParams p = {};
+  p.coarse = coarse; p.gw = gw; p.gh = gh; p.gd = gd;
+  for (int a = 0; a < ndim; ++a) {
+    if (g[a] < 2 * border) return MVR_ERR_UNSUPPORTED;
+    // the decode of an aligned roi: centre - 0.5, start = -size / 2, bin = size / output size
+    const float extent = (float)(g[a] - (2 * border - 1));
+    p.centre[a] = (float)g[a] / 2 - 0.5f;
+    p.bin[a] = extent / (float)size[a];
+    p.start[a] = -extent * 0.5f;
+  }
+  p.img = image; p.out = image_out; p.C = (int)C_image;
+  p.lab = labels; p.lab_out = label_out; p.CL = (int)C_label;
+  p.field = field;
+  p.B = (int)B; p.D = (int)D; p.H = (int)H; p.W = (int)W;
+  const bool even = (W & 1) == 0;
+  p.vec_img = even && (uintptr_t)image_out % (dtype == MVR_F32 ? 8 : 4) == 0;
+  p.vec_lab = even && (uintptr_t)label_out % 8 == 0;
+  p.vec_field = even && (uintptr_t)field % 8 == 0;
+  const int rc = launch_elastic(p, ndim, dtype, label_dtype, (cudaStream_t)stream);
+  return rc == 0 ? MVR_OK : (rc == 1 ? MVR_ERR_UNSUPPORTED : MVR_ERR_LAUNCH);
 }
 
 // ---- the reference's extension surface --------------------------------------------------

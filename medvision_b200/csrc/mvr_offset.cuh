@@ -48,6 +48,94 @@ __device__ __forceinline__ __half2 load_offset_pair<__half>(const OffsetParams& 
   return __halves2half2(f[0], has_b ? f[1] : __float2half_rn(0.0f));
 }
 
+// Taps of the two voxels of a pair at (T)index + offset (mvr_elastic.cuh uses them too): base offsets inside a channel's
+// volume, steps to the upper neighbours (0 where clamped), weights (order 1) or the one-hot choice (order 0) per axis,
+// and which lane lies strictly inside (-1, size) on every axis.
+template <typename T, int NDIM>
+struct WarpTaps {
+  typedef typename P2<T>::V V;
+  AxisTap2<T> t[3];  // w, h, d
+  int ba, bb, xa1, xb1, ya1, yb1, za1, zb1;
+  bool ina, inb;
+};
+
+// o2: displacement of the two voxels per axis (index 0 = w, 1 = h, 2 = d), in the image's element type
+template <typename T, int NDIM>
+__device__ __forceinline__ void warp_positions(int w0, int h, int d, const typename P2<T>::V* o2, typename P2<T>::V* c) {
+  typedef Ar<T> A;
+  typedef P2<T> Q;
+  c[0] = Q::add(Q::make(A::fi(w0), A::fi(w0 + 1)), o2[0]);
+  c[1] = Q::add(Q::dup(A::fi(h)), o2[1]);
+  c[2] = (NDIM == 3) ? Q::add(Q::dup(A::fi(d)), o2[2]) : Q::dup(A::fi(0));
+}
+template <typename T, int NDIM>
+__device__ __forceinline__ void warp_inside(const typename P2<T>::V* c, int W, int H, int D, bool has_b, bool& ina, bool& inb) {
+  typedef Ar<T> A;
+  typedef P2<T> Q;
+  const int size[3] = {W, H, D};
+  ina = true;
+  inb = has_b;
+#pragma unroll
+  for (int a = 0; a < NDIM; ++a) {
+    ina = ina && A::tof(Q::lo(c[a])) > -1.0f && A::tof(Q::lo(c[a])) < (float)size[a];
+    inb = inb && A::tof(Q::hi(c[a])) > -1.0f && A::tof(Q::hi(c[a])) < (float)size[a];
+  }
+}
+template <typename T, int NDIM>
+__device__ __forceinline__ void warp_taps(const typename P2<T>::V* c, int W, int H, int D, int order, bool has_b, WarpTaps<T, NDIM>& t) {
+  warp_inside<T, NDIM>(c, W, H, D, has_b, t.ina, t.inb);
+  axis_tap2<T>(c[0], W, order, t.t[0]);
+  axis_tap2<T>(c[1], H, order, t.t[1]);
+  if (NDIM == 3) axis_tap2<T>(c[2], D, order, t.t[2]);
+  const AxisTap2<T>&tx = t.t[0], &ty = t.t[1], &tz = t.t[2];
+  const int HW = H * W;
+  t.ba = t.ina ? (((NDIM == 3 ? tz.i0a * H : 0) + ty.i0a) * W + tx.i0a) : 0;
+  t.bb = t.inb ? (((NDIM == 3 ? tz.i0b * H : 0) + ty.i0b) * W + tx.i0b) : 0;
+  t.xa1 = t.ina ? tx.da : 0;
+  t.xb1 = t.inb ? tx.db : 0;
+  t.ya1 = (t.ina && ty.da) ? W : 0;
+  t.yb1 = (t.inb && ty.db) ? W : 0;
+  t.za1 = (NDIM == 3 && t.ina && tz.da) ? HW : 0;
+  t.zb1 = (NDIM == 3 && t.inb && tz.db) ? HW : 0;
+}
+template <typename T, int NDIM>
+__device__ __forceinline__ void warp_weights(const WarpTaps<T, NDIM>& t, typename P2<T>::V* w) {
+  typedef P2<T> Q;
+  typedef typename Q::V V;
+  const AxisTap2<T>&tx = t.t[0], &ty = t.t[1], &tz = t.t[2];
+  if (NDIM == 3) {
+    const V hzhy = Q::mul(tz.h, ty.h), hzly = Q::mul(tz.h, ty.l);
+    const V lzhy = Q::mul(tz.l, ty.h), lzly = Q::mul(tz.l, ty.l);
+    w[0] = Q::mul(hzhy, tx.h); w[1] = Q::mul(hzhy, tx.l); w[2] = Q::mul(hzly, tx.h); w[3] = Q::mul(hzly, tx.l);
+    w[4] = Q::mul(lzhy, tx.h); w[5] = Q::mul(lzhy, tx.l); w[6] = Q::mul(lzly, tx.h); w[7] = Q::mul(lzly, tx.l);
+  } else {
+    w[0] = Q::mul(ty.h, tx.h); w[1] = Q::mul(ty.h, tx.l); w[2] = Q::mul(ty.l, tx.h); w[3] = Q::mul(ty.l, tx.l);
+  }
+}
+// one channel: the reference's tap sum, 0 for a lane outside
+template <typename T, int NDIM>
+__device__ __forceinline__ typename P2<T>::V warp_channel(const WarpTaps<T, NDIM>& t, const typename P2<T>::V* w, const T* img) {
+  typedef P2<T> Q;
+  typedef typename Q::V V;
+  const T* pa = img + t.ba;
+  const T* pb = img + t.bb;
+  V v[1 << NDIM];
+  v[0] = Q::make(__ldg(pa), __ldg(pb));
+  v[1] = Q::make(__ldg(pa + t.xa1), __ldg(pb + t.xb1));
+  v[2] = Q::make(__ldg(pa + t.ya1), __ldg(pb + t.yb1));
+  v[3] = Q::make(__ldg(pa + t.ya1 + t.xa1), __ldg(pb + t.yb1 + t.xb1));
+  if (NDIM == 3) {
+    v[4] = Q::make(__ldg(pa + t.za1), __ldg(pb + t.zb1));
+    v[5] = Q::make(__ldg(pa + t.za1 + t.xa1), __ldg(pb + t.zb1 + t.xb1));
+    v[6] = Q::make(__ldg(pa + t.za1 + t.ya1), __ldg(pb + t.zb1 + t.yb1));
+    v[7] = Q::make(__ldg(pa + t.za1 + t.ya1 + t.xa1), __ldg(pb + t.zb1 + t.yb1 + t.xb1));
+  }
+  V acc = Q::tap_first(w[0], v[0], w[1], v[1]);
+#pragma unroll
+  for (int k = 2; k < (1 << NDIM); ++k) acc = Q::tap_next(acc, w[k], v[k]);
+  return Q::apply(acc, Q::make_mask(t.ina, t.inb));
+}
+
 template <typename T, int NDIM, bool CUBIC>
 __device__ __forceinline__ void apply_offset_pair(const OffsetParams& p, int b, int d, int h, int wp) {
   typedef Ar<T> A;
@@ -60,39 +148,27 @@ __device__ __forceinline__ void apply_offset_pair(const OffsetParams& p, int b, 
   const long long off0 = (long long)b * NDIM * vol + s0;
   const T zero = A::fi(0);
 
-  // displacement of the two voxels per axis (index 0 = w, 1 = h, 2 = d)
-  V o2[3];
+  V o2[3], c[3];
 #pragma unroll
   for (int a = 0; a < NDIM; ++a) {
     const long long q = off0 + (long long)(NDIM - 1 - a) * vol;  // channel order of the field: d, h, w
     o2[a] = load_offset_pair<T>(p, q, has_b);
   }
-  // sample positions: (T)index + offset
-  const V cx = Q::add(Q::make(A::fi(w0), A::fi(w0 + 1)), o2[0]);
-  const V cy = Q::add(Q::dup(A::fi(h)), o2[1]);
-  const V cz = (NDIM == 3) ? Q::add(Q::dup(A::fi(d)), o2[2]) : Q::dup(zero);
-  // strictly inside (-1, size) on every axis, else the result is 0
-  bool ina = A::tof(Q::lo(cx)) > -1.0f && A::tof(Q::lo(cx)) < (float)p.W && A::tof(Q::lo(cy)) > -1.0f &&
-             A::tof(Q::lo(cy)) < (float)p.H;
-  bool inb = has_b && A::tof(Q::hi(cx)) > -1.0f && A::tof(Q::hi(cx)) < (float)p.W && A::tof(Q::hi(cy)) > -1.0f &&
-             A::tof(Q::hi(cy)) < (float)p.H;
-  if (NDIM == 3) {
-    ina = ina && A::tof(Q::lo(cz)) > -1.0f && A::tof(Q::lo(cz)) < (float)p.D;
-    inb = inb && A::tof(Q::hi(cz)) > -1.0f && A::tof(Q::hi(cz)) < (float)p.D;
-  }
+  warp_positions<T, NDIM>(w0, h, d, o2, c);
   const T* img = (const T*)p.img + (long long)b * p.C * vol;
   T* out = (T*)p.out + (long long)b * p.C * vol + s0;
-  const V zero2 = Q::dup(zero);
 
   if (CUBIC) {  // Catmull-Rom: per voxel
-    for (int c = 0; c < p.C; ++c, img += vol, out += vol) {
+    bool ina, inb;
+    warp_inside<T, NDIM>(c, p.W, p.H, p.D, has_b, ina, inb);
+    for (int ch = 0; ch < p.C; ++ch, img += vol, out += vol) {
       T va = zero, vb = zero;
       if (NDIM == 3) {
-        if (ina) va = hermite_3d<T>(img, p.D, p.H, p.W, Q::lo(cz), Q::lo(cy), Q::lo(cx), p.fm);
-        if (inb) vb = hermite_3d<T>(img, p.D, p.H, p.W, Q::hi(cz), Q::hi(cy), Q::hi(cx), p.fm);
+        if (ina) va = hermite_3d<T>(img, p.D, p.H, p.W, Q::lo(c[2]), Q::lo(c[1]), Q::lo(c[0]), p.fm);
+        if (inb) vb = hermite_3d<T>(img, p.D, p.H, p.W, Q::hi(c[2]), Q::hi(c[1]), Q::hi(c[0]), p.fm);
       } else {
-        if (ina) va = hermite_2d<T>(img, p.H, p.W, Q::lo(cy), Q::lo(cx), p.fm);
-        if (inb) vb = hermite_2d<T>(img, p.H, p.W, Q::hi(cy), Q::hi(cx), p.fm);
+        if (ina) va = hermite_2d<T>(img, p.H, p.W, Q::lo(c[1]), Q::lo(c[0]), p.fm);
+        if (inb) vb = hermite_2d<T>(img, p.H, p.W, Q::hi(c[1]), Q::hi(c[0]), p.fm);
       }
       out[0] = va;
       if (has_b) out[1] = vb;
@@ -100,46 +176,13 @@ __device__ __forceinline__ void apply_offset_pair(const OffsetParams& p, int b, 
     return;
   }
 
-  AxisTap2<T> tx, ty, tz;
-  axis_tap2<T>(cx, p.W, p.order, tx);
-  axis_tap2<T>(cy, p.H, p.order, ty);
-  if (NDIM == 3) axis_tap2<T>(cz, p.D, p.order, tz);
-  const int W = p.W, HW = p.H * p.W;
-  const int ba = ina ? (((NDIM == 3 ? tz.i0a * p.H : 0) + ty.i0a) * W + tx.i0a) : 0;
-  const int bb = inb ? (((NDIM == 3 ? tz.i0b * p.H : 0) + ty.i0b) * W + tx.i0b) : 0;
-  const int xa1 = ina ? tx.da : 0, xb1 = inb ? tx.db : 0;
-  const int ya1 = (ina && ty.da) ? W : 0, yb1 = (inb && ty.db) ? W : 0;
-  const int za1 = (NDIM == 3 && ina && tz.da) ? HW : 0, zb1 = (NDIM == 3 && inb && tz.db) ? HW : 0;
-  const typename Q::M mask = Q::make_mask(ina, inb);
+  WarpTaps<T, NDIM> t;
+  warp_taps<T, NDIM>(c, p.W, p.H, p.D, p.order, has_b, t);
   V w[1 << NDIM];
-  if (NDIM == 3) {
-    const V hzhy = Q::mul(tz.h, ty.h), hzly = Q::mul(tz.h, ty.l);
-    const V lzhy = Q::mul(tz.l, ty.h), lzly = Q::mul(tz.l, ty.l);
-    w[0] = Q::mul(hzhy, tx.h); w[1] = Q::mul(hzhy, tx.l); w[2] = Q::mul(hzly, tx.h); w[3] = Q::mul(hzly, tx.l);
-    w[4] = Q::mul(lzhy, tx.h); w[5] = Q::mul(lzhy, tx.l); w[6] = Q::mul(lzly, tx.h); w[7] = Q::mul(lzly, tx.l);
-  } else {
-    w[0] = Q::mul(ty.h, tx.h); w[1] = Q::mul(ty.h, tx.l); w[2] = Q::mul(ty.l, tx.h); w[3] = Q::mul(ty.l, tx.l);
-  }
+  warp_weights<T, NDIM>(t, w);
 #pragma unroll 1
-  for (int c = 0; c < p.C; ++c, img += vol, out += vol) {
-    const T* pa = img + ba;
-    const T* pb = img + bb;
-    V v[1 << NDIM];
-    v[0] = Q::make(__ldg(pa), __ldg(pb));
-    v[1] = Q::make(__ldg(pa + xa1), __ldg(pb + xb1));
-    v[2] = Q::make(__ldg(pa + ya1), __ldg(pb + yb1));
-    v[3] = Q::make(__ldg(pa + ya1 + xa1), __ldg(pb + yb1 + xb1));
-    if (NDIM == 3) {
-      v[4] = Q::make(__ldg(pa + za1), __ldg(pb + zb1));
-      v[5] = Q::make(__ldg(pa + za1 + xa1), __ldg(pb + zb1 + xb1));
-      v[6] = Q::make(__ldg(pa + za1 + ya1), __ldg(pb + zb1 + yb1));
-      v[7] = Q::make(__ldg(pa + za1 + ya1 + xa1), __ldg(pb + zb1 + yb1 + xb1));
-    }
-    V acc = Q::tap_first(w[0], v[0], w[1], v[1]);
-#pragma unroll
-    for (int k = 2; k < (1 << NDIM); ++k) acc = Q::tap_next(acc, w[k], v[k]);
-    // a sample outside the image gives the literal 0; inside, the reference returns the sum as it is
-    const V val = Q::apply(acc, mask);
+  for (int ch = 0; ch < p.C; ++ch, img += vol, out += vol) {
+    const V val = warp_channel<T, NDIM>(t, w, img);
     if (p.vec_ok) {
       Q::store2(out, val);
     } else {
@@ -147,7 +190,6 @@ __device__ __forceinline__ void apply_offset_pair(const OffsetParams& p, int b, 
       if (has_b) out[1] = Q::hi(val);
     }
   }
-  (void)zero2;
 }
 
 template <typename T, int NDIM, bool CUBIC>

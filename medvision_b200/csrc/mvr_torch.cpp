@@ -266,47 +266,40 @@ void fields_into(const RoiOp& op, const at::Tensor& image, const at::Tensor& ima
                                 (int)op.out[2], op.scale, op.aligned, op.order, status_ptr(index), stream));
 }
 
-// ---- upload of a call's rois ------------------------------------------------------------------------
+// ---- upload of a call's parameters ------------------------------------------------------------------
 // The parameters of a transform are drawn on the host, so one small upload per call is inherent.  It is ONE asynchronous
-// copy from pinned memory into a device buffer kept across calls, carrying the rois in float32 (label fields) and, rounded
-// on the host exactly as the device cast rounds, in float16 (half images).  A ring of kSlots such pairs per device: a slot
-// is used again when the kernels that read it last are done (an event recorded behind them), so up to kSlots calls can be
-// in flight; the ring is locked for the whole call, so any number of threads and streams may use it.  It holds kSlots
-// times the largest call (a few KB each) and goes away with release_staging().
+// copy from pinned memory into a device buffer kept across calls.  A ring of kSlots such pairs per device: a slot is used
+// again when the kernels that read it last are done (an event recorded behind them), so up to kSlots calls can be in
+// flight; the ring is locked for the whole call, so any number of threads and streams may use it.  It holds kSlots times
+// twice the largest call (some KB each) and goes away with release_staging().
 constexpr int kSlots = 8;
 
 struct Stage {
   std::mutex mutex;
-  int64_t capacity = 0;  // roi values per slot
+  int64_t capacity = 0;  // bytes per slot
   void* host[kSlots] = {};
   at::Tensor dev[kSlots];
   cudaEvent_t event[kSlots] = {};
   bool recorded[kSlots] = {};
   int next = 0;
 
-  void wait_all() {
-    for (int k = 0; k < kSlots; ++k)
-      if (recorded[k]) {
-        C10_CUDA_CHECK(cudaEventSynchronize(event[k]));
-        recorded[k] = false;
-      }
-  }
   void release() {
-    wait_all();
     for (int k = 0; k < kSlots; ++k) {
+      if (recorded[k]) C10_CUDA_CHECK(cudaEventSynchronize(event[k]));
+      recorded[k] = false;
       if (host[k]) C10_CUDA_CHECK(cudaFreeHost(host[k]));
       host[k] = nullptr;
       dev[k] = at::Tensor();
     }
     capacity = 0;
   }
-  void reserve(int64_t values, at::Device device) {
-    if (values <= capacity) return;
+  void reserve(int64_t bytes, at::Device device) {
+    if (bytes <= capacity) return;
     release();
-    const int64_t want = std::max<int64_t>(1024, 2 * values);
+    const int64_t want = std::max<int64_t>(8192, 2 * bytes);
     for (int k = 0; k < kSlots; ++k) {
-      C10_CUDA_CHECK(cudaHostAlloc(&host[k], (size_t)want * 6, cudaHostAllocDefault));
-      dev[k] = at::empty({want * 6}, at::TensorOptions().dtype(at::kByte).device(device));
+      C10_CUDA_CHECK(cudaHostAlloc(&host[k], (size_t)want, cudaHostAllocDefault));
+      dev[k] = at::empty({want}, at::TensorOptions().dtype(at::kByte).device(device));
       if (!event[k]) C10_CUDA_CHECK(cudaEventCreateWithFlags(&event[k], cudaEventDisableTiming));
     }
     capacity = want;
@@ -322,46 +315,58 @@ Stage& stage_of(int index) {
   return *g_stage[index];
 }
 
-// Rois of one call on the device, while the ring is locked.
-struct StagedRois {
+// A slot of the ring for one call: fill host(), send(), launch the kernels that read device(); the destructor marks the
+// slot free behind them.
+struct Upload {
   Stage& stage;
   std::lock_guard<std::mutex> lock;
   cudaStream_t stream;
   bool capturing;
   int slot;
-  at::Tensor f32, f16;
 
-  StagedRois(const at::Tensor& rois, at::Device device)
+  Upload(int64_t bytes, at::Device device)
       : stage(stage_of(device.index())), lock(stage.mutex), stream(c10::cuda::getCurrentCUDAStream(device.index()).stream()) {
-    const int64_t n = rois.numel(), R = rois.size(0), K = rois.size(1);
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     C10_CUDA_CHECK(cudaStreamIsCapturing(stream, &cs));
     capturing = cs != cudaStreamCaptureStatusNone;
-    stage.reserve(n, device);
+    stage.reserve(bytes, device);
     slot = stage.next;
     stage.next = (slot + 1) % kSlots;
     if (stage.recorded[slot] && !capturing) {
       C10_CUDA_CHECK(cudaEventSynchronize(stage.event[slot]));
       stage.recorded[slot] = false;
     }
-    const float* src = (const float*)rois.data_ptr();
-    float* h32 = (float*)stage.host[slot];
-    at::Half* h16 = (at::Half*)(h32 + n);
-    for (int64_t i = 0; i < n; ++i) {
-      h32[i] = src[i];
-      h16[i] = at::Half(src[i]);  // round to nearest even, as the device cast
-    }
-    const at::Tensor& d = stage.dev[slot];
-    C10_CUDA_CHECK(cudaMemcpyAsync(d.data_ptr(), h32, (size_t)n * 6, cudaMemcpyHostToDevice, stream));
-    // views by pointer: the ring keeps the memory
-    auto none = [](void*) {};
-    f32 = at::from_blob(d.data_ptr(), {R, K}, none, at::TensorOptions().dtype(at::kFloat).device(device));
-    f16 = at::from_blob((char*)d.data_ptr() + 4 * n, {R, K}, none, at::TensorOptions().dtype(at::kHalf).device(device));
   }
-  ~StagedRois() {
+  void* host() { return stage.host[slot]; }
+  void* device() { return stage.dev[slot].data_ptr(); }
+  void send(int64_t bytes) { C10_CUDA_CHECK(cudaMemcpyAsync(device(), host(), (size_t)bytes, cudaMemcpyHostToDevice, stream)); }
+  ~Upload() {
     if (capturing) return;
     if (cudaEventRecord(stage.event[slot], stream) == cudaSuccess) stage.recorded[slot] = true;
     else cudaStreamSynchronize(stream);
+  }
+};
+
+// Rois of one call on the device, in float32 (label fields) and, rounded on the host exactly as the device cast rounds, in
+// float16 (half images).
+struct StagedRois {
+  Upload up;
+  at::Tensor f32, f16;
+
+  StagedRois(const at::Tensor& rois, at::Device device) : up(rois.numel() * 6, device) {
+    const int64_t n = rois.numel(), R = rois.size(0), K = rois.size(1);
+    const float* src = (const float*)rois.data_ptr();
+    float* h32 = (float*)up.host();
+    at::Half* h16 = (at::Half*)(h32 + n);
+    for (int64_t i = 0; i < n; ++i) {
+      h32[i] = src[i];
+      h16[i] = at::Half(src[i]);  // round to nearest even
+    }
+    up.send(n * 6);
+    // views by pointer: the ring keeps the memory
+    auto none = [](void*) {};
+    f32 = at::from_blob(up.device(), {R, K}, none, at::TensorOptions().dtype(at::kFloat).device(device));
+    f16 = at::from_blob((char*)up.device() + 4 * n, {R, K}, none, at::TensorOptions().dtype(at::kHalf).device(device));
   }
 };
 
@@ -428,6 +433,65 @@ at::Tensor apply_offset(const at::Tensor& input, const at::Tensor& offset_any, i
                      : mvr_apply_offset_3d(input.data_ptr(), offset.data_ptr(), out.data_ptr(), dtype_code(t), dtype_code(ot),
                                            input.size(0), input.size(1), input.size(2), input.size(3), input.size(4), order, stream));
   return out;
+}
+
+// ---- elastic deformation ------------------------------------------------------------------------------
+
+// coarse (B, *grid, ndim) float32 on the host, halved as it goes up ("to smooth"); every image field and label field of one
+// call, or the dense field.  False: no kernel for the grid.
+bool elastic(const at::Tensor& coarse, int border, const std::vector<int64_t>& shape, at::ScalarType position_type,
+             const Tensors& images, const Tensors& labels, at::Tensor* field, at::Device device, Tensors& images_out,
+             Tensors& labels_out) {
+  at::NoGradGuard no_grad;
+  const int ndim = (int)shape.size();
+  const int64_t B = coarse.size(0);
+  const int gd = ndim == 3 ? (int)coarse.size(1) : 1, gh = (int)coarse.size(ndim - 1), gw = (int)coarse.size(ndim);
+  const int64_t points = (int64_t)gd * gh * gw, D = ndim == 3 ? shape[0] : 1, H = shape[ndim - 2], W = shape[ndim - 1];
+  c10::cuda::CUDAGuard guard(device);
+  Upload up(coarse.numel() * 4, device);
+  const float* src = (const float*)coarse.data_ptr();
+  float* dst = (float*)up.host();
+  for (int64_t b = 0; b < B; ++b)
+    for (int64_t i = 0; i < points; ++i)
+      for (int c = 0; c < ndim; ++c) dst[(b * ndim + c) * points + i] = src[(b * points + i) * ndim + c] / 2;
+  up.send(coarse.numel() * 4);
+  auto call = [&](const at::Tensor* im, const at::Tensor* lb, float* f) {
+    at::Tensor i, l, io, lo;
+    if (im) {
+      i = im->contiguous();
+      io = at::empty(i.sizes(), i.options().requires_grad(false));
+    }
+    if (lb) {
+      l = lb->contiguous();
+      lo = at::empty(l.sizes(), l.options().dtype(at::kInt));
+    }
+    const int rc = mvr_elastic((const float*)up.device(), ndim, gd, gh, gw, border, im ? i.data_ptr() : nullptr,
+                               dtype_code(im ? i.scalar_type() : position_type), im ? io.data_ptr() : nullptr, im ? i.size(1) : 0,
+                               lb ? l.data_ptr() : nullptr, lb ? label_code(l.scalar_type()) : 0,
+                               lb ? (int32_t*)lo.data_ptr() : nullptr, lb ? l.size(1) : 0, f, B, D, H, W, (void*)up.stream);
+    if (rc == MVR_ERR_UNSUPPORTED) return false;
+    check_rc(rc);
+    if (im) images_out.push_back(io);
+    if (lb) labels_out.push_back(lo);
+    return true;
+  };
+  if (field) {
+    std::vector<int64_t> size{B, ndim};
+    size.insert(size.end(), shape.begin(), shape.end());
+    *field = at::empty(size, at::TensorOptions().dtype(at::kFloat).device(device));
+    return call(nullptr, nullptr, (float*)field->data_ptr());
+  }
+  const size_t n = std::max(images.size(), labels.size());
+  for (size_t k = 0; k < n; ++k) {
+    const at::Tensor* im = k < images.size() ? &images[k] : nullptr;
+    const at::Tensor* lb = k < labels.size() ? &labels[k] : nullptr;
+    if (im && lb && im->scalar_type() == position_type) {
+      if (!call(im, lb, nullptr)) return false;
+    } else if ((im && !call(im, nullptr, nullptr)) || (lb && !call(nullptr, lb, nullptr))) {
+      return false;
+    }
+  }
+  return true;
 }
 
 // ---- Python bindings ----------------------------------------------------------------------------------
@@ -735,6 +799,58 @@ PyObject* py_apply_offset(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// elastic(coarse, border, shape, like, images, labels) -> (images, labels), or None where the two-step form is needed;
+// elastic(coarse, border, shape, device, None, None) -> the dense field, or None.  `like`: a tensor of the type in which the
+// sample positions are formed.
+PyObject* py_elastic(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  need(n, 6, 6);
+  const at::Tensor& coarse = tensor_arg(a[0], "coarse");
+  const int border = (int)int_arg(a[1]);
+  std::vector<int64_t> shape;
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(a[2]); ++i) shape.push_back(int_arg(PyTuple_GET_ITEM(a[2], i)));
+  const int ndim = (int)shape.size();
+  TORCH_CHECK((ndim == 2 || ndim == 3) && coarse.dim() == ndim + 2 && coarse.size(ndim + 1) == ndim && !coarse.is_cuda() &&
+                  coarse.scalar_type() == at::kFloat && coarse.is_contiguous(),
+              "coarse: expected a contiguous float32 CPU tensor (B, *grid, dim)");
+  const at::Tensor& like = tensor_arg(a[3], "like");
+  TORCH_CHECK(like.is_cuda(), "Not implemented on the CPU");
+  if (a[4] == Py_None) {
+    at::Tensor field;
+    Tensors none;
+    bool done;
+    {
+      pybind11::gil_scoped_release nogil;
+      done = elastic(coarse, border, shape, at::kFloat, none, none, &field, like.device(), none, none);
+    }
+    if (!done) Py_RETURN_NONE;
+    return THPVariable_Wrap(std::move(field));
+  }
+  Tensors images = tensor_list(a[4], "images"), labels = tensor_list(a[5], "labels");
+  for (const Tensors* v : {&images, &labels})
+    for (const at::Tensor& t : *v) {
+      if (t.dim() != ndim + 2 || t.size(0) != coarse.size(0) || t.sizes().slice(2) != at::IntArrayRef(shape))
+        raise(PyExc_AssertionError, "the fields of an elastic deformation must be (B, C, *image_shape)");
+      if (t.device() != like.device() || (v == &images ? t.scalar_type() != at::kHalf && t.scalar_type() != at::kFloat : label_code(t.scalar_type()) < 0))
+        Py_RETURN_NONE;
+    }
+  if (like.scalar_type() != at::kHalf && like.scalar_type() != at::kFloat) Py_RETURN_NONE;
+  Tensors images_out, labels_out;
+  bool done;
+  {
+    pybind11::gil_scoped_release nogil;
+    done = elastic(coarse, border, shape, like.scalar_type(), images, labels, nullptr, like.device(), images_out, labels_out);
+  }
+  if (!done) Py_RETURN_NONE;
+  PyObject* io = wrap_list(images_out);
+  PyObject* lo = wrap_list(labels_out);
+  PyObject* both = PyTuple_Pack(2, io, lo);
+  Py_DECREF(io);
+  Py_DECREF(lo);
+  return both;
+  END_HANDLE_TH_ERRORS
+}
+
 // status_word(index): the int32 tensor the kernels of that device OR their status bits into
 PyObject* py_status_word(PyObject*, PyObject* index) {
   HANDLE_TH_ERRORS
@@ -775,6 +891,7 @@ PyMethodDef methods[] = {
     {"label_call", FAST(py_label_call), nullptr},
     {"fields_call", FAST(py_fields_call), nullptr},
     {"resample_fields", FAST(py_resample_fields), nullptr},
+    {"elastic", FAST(py_elastic), nullptr},
     {"apply_offset", FAST(py_apply_offset), nullptr},
     {"status_word", py_status_word, METH_O, nullptr},
     {"peak_allocated", py_peak_allocated, METH_NOARGS, nullptr},
