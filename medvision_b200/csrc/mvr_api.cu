@@ -15,6 +15,7 @@
 #include "mvr_label.cuh"
 #include "mvr_plane2d.cuh"
 #include "mvr_elastic.cuh"
+#include "mvr_head.cuh"
 
 // ---- scratch of the entry point that allocates nothing ------------------------------------
 // Lives in the library image: every GPU that loads the library holds these 16 MiB until the
@@ -116,6 +117,10 @@ int launch_mark(const Params& p, cudaStream_t st) {
 // The kernels that need neither the streaming shape nor any memory beyond inputs and outputs:
 // the flat kernel where it applies, else the one-CTA-per-tile kernel.
 int dispatch_flat_or_generic(const Params& p, int dtype, bool fwd, cudaStream_t st) {
+  if (dtype != MVR_F64) {
+    const int rc = dtype == MVR_F32 ? launch_box_head<float>(p, fwd, st) : launch_box_head<__half>(p, fwd, st);
+    if (rc == 0) return cudaGetLastError() == cudaSuccess ? MVR_OK : MVR_ERR_LAUNCH;
+  }
   {
     int rc;
     switch (dtype) {

@@ -1,0 +1,76 @@
+"""The box-head kernels (csrc/mvr_head.cuh) at the sizes where their dispatch and their tables change: adaptive and three-sample
+grids, boxes from below one voxel to beyond the tables, boxes over the border and outside, channel groups, row widths, odd
+maps, unaligned gradient tensors.  Forward bit for bit, backward against the wide-accumulator restatement."""
+import pytest
+import torch
+
+import cases
+from oracle import port
+from util import BWD_TOL, assert_close, n_mismatch
+
+pytestmark = pytest.mark.gpu
+REF_FM = 1 | (1 << 1) | (1 << 2) | (1 << 3) | (1 << 5) | (1 << 7) | (1 << 10) | (1 << 13) | \
+    (1 << 16) | (1 << 18) | (2 << 20) | (1 << 22)
+
+CASES = [
+    # spatial,        channels, rois, output,    sampling, order, dtype
+    ((37, 41),        5, 12, (7, 7),    0, 1, torch.float32),
+    ((600, 530),      1, 9,  (7, 5),    0, 1, torch.float32),   # boxes wider than the tables of positions and of taps
+    ((64, 97),        2, 40, (14, 14),  3, 1, torch.float32),   # groups of two
+    ((50, 63),        3, 9,  (3, 33),   0, 1, torch.float32),   # rows wider than a warp
+    ((37, 41),        4, 12, (7, 7),    0, 0, torch.float32),   # nearest
+    ((33, 27),        3, 60, (7, 7),    0, 1, torch.float16),
+    ((64, 97),        6, 90, (14, 14),  2, 1, torch.float16),
+    ((19, 23, 29),    7, 80, (7, 6, 5), 3, 1, torch.float32),
+    ((19, 23, 29),    9, 60, (7, 6, 5), 0, 1, torch.float32),   # enough outputs for the 3D tables
+    ((12, 40, 170),   2, 30, (5, 5, 5), 0, 1, torch.float16),   # an axis beyond the tables of positions
+    ((19, 23, 29),    3, 40, (7, 7, 7), 2, 0, torch.float16),
+]
+
+
+def _rois(spatial, R, g):
+    nd = len(spatial)
+    ext = torch.tensor(spatial[::-1], dtype=torch.float32)
+    b = torch.randint(0, 2, (R, 1), generator=g).float()
+    c = torch.rand(R, nd, generator=g) * ext * 1.1 - 0.05 * ext
+    s = torch.rand(R, nd, generator=g) * ext * 0.5 + 0.5
+    s[0] = 0.2                        # below one voxel
+    s[1] = ext * 2.5                  # the whole map and beyond
+    c[1] = ext / 2
+    c[2] = ext * 3                    # outside
+    c[3], s[3] = ext - 0.5, 3.0       # the last voxels
+    c[4], s[4] = torch.zeros(nd), 4.0
+    s[5], c[5] = 2.0, ext / 3         # far fewer voxels than bins
+    return torch.cat([b, c - s / 2, c + s / 2], 1)
+
+
+@pytest.mark.parametrize("spatial,C,R,out,sr,order,dtype", CASES,
+                         ids=["%s-%s-s%d-o%d-%s" % ("x".join(map(str, c[0])), "x".join(map(str, c[3])), c[4], c[5], str(c[6])[6:]) for c in CASES])
+def test_box_heads_match_the_restatement(spatial, C, R, out, sr, order, dtype):
+    from medvision_b200 import _C
+    nd = len(spatial)
+    g = torch.Generator().manual_seed(sum(spatial) + R)
+    feat = (torch.rand((2, C) + spatial, generator=g) * 2 - 0.5).to(dtype)
+    rois = _rois(spatial, R, g).to(dtype)
+    bad = rois.clone()
+    bad[6, 0] = 5                     # batch index outside the batch
+    fwd = _C.roi_align_2d_forward if nd == 2 else _C.roi_align_3d_forward
+    bwd = _C.roi_align_2d_backward if nd == 2 else _C.roi_align_3d_backward
+    kw = dict(spatial_scale=1.0, sampling_ratio=sr, aligned=True, order=order, fma_mode=REF_FM if dtype == torch.float32 else 0)
+    keep = [i for i in range(R) if i != 6]
+    got = torch.full((R, C) + out, float("nan"), dtype=dtype, device="cuda")
+    fwd(feat.cuda(), bad.cuda(), got, *out, 1.0, sr, order)
+    assert not bool(got[6].any())
+    assert n_mismatch(got[keep], port.forward(feat, rois[keep], out, cases.KIND_BOX, **kw)) == 0
+    grad = torch.randn((R, C) + out, generator=g).to(dtype)
+    want = port.backward(grad[keep], rois[keep], feat.shape, cases.KIND_BOX, wide_acc=True, **kw)
+    n = feat.numel()
+    for offset in (0, 3):             # a gradient tensor at an unaligned place inside a buffer
+        buf = torch.full((n + 32,), -0.0, dtype=dtype, device="cuda")
+        gin = buf[16 + offset:16 + offset + n].view(feat.shape)
+        gin.zero_()
+        bwd(grad.cuda(), bad.cuda(), gin, *out, 1.0, sr, order)
+        assert_close(gin, want, 1e-5 if dtype == torch.float32 else BWD_TOL[dtype], "gradient")
+        around = torch.cat([buf[:16 + offset], buf[16 + offset + n:]])
+        assert bool((torch.signbit(around) & (around == 0)).all()), "something was added outside the gradient tensor"
+    _C.last_status()
