@@ -251,6 +251,12 @@ int mvr_affine_fields_3d(const void* image, int dtype, const void* image_rois, v
                          int64_t C_label, int64_t N, int64_t D, int64_t H, int64_t W, int64_t R, int roi_width, int od,
                          int oh, int ow, float spatial_scale, int aligned, int order, int* status, void* stream);
 
+/* 2D: one launch for both where the output is dense; a float image and its labels share their sample positions. */
+int mvr_affine_fields_2d(const void* image, int dtype, const void* image_rois, void* image_out, int64_t C_image,
+                         const void* labels, int label_dtype, const float* label_rois, int32_t* label_out,
+                         int64_t C_label, int64_t N, int64_t H, int64_t W, int64_t R, int roi_width, int oh, int ow,
+                         float spatial_scale, int aligned, int order, int* status, void* stream);
+
 /* ---- elastic warp ---------------------------------------------------------------------- */
 
 /* out[b, c, p] = interp(img[b, c], p + offset[b, :, p]) for every voxel p; float32 / float16;

@@ -48,6 +48,8 @@ PROTOTYPES = {
                             _i32, _vp, _vp],
     "mvr_affine_fields_3d": [_vp, _i32, _vp, _vp, _i64, _vp, _i32, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i64, _i32,
                              _i32, _i32, _i32, _f32, _i32, _i32, _vp, _vp],
+    "mvr_affine_fields_2d": [_vp, _i32, _vp, _vp, _i64, _vp, _i32, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i32, _i32, _i32,
+                             _f32, _i32, _i32, _vp, _vp],
     "mvr_elastic": [_vp, _i32, _i32, _i32, _i32, _i32, _vp, _i32, _vp, _i64, _vp, _i32, _vp, _i64, _vp, _i64, _i64, _i64,
                     _i64, _vp],
     "mvr_affine_2d": _ROT2D,

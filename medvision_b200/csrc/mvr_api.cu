@@ -287,6 +287,17 @@ int mvr_roi_resample_bwd_noalloc(const void* grad_out, const void* rois, void* g
   return dispatch_flat_or_generic(p, dtype, false, st);
 }
 
+// the label job of a 2D call, from its parameters (in = labels, rois = float32 rois, out = int32 result)
+static Plane2dLabel plane2d_label_of(const Params& p) {
+  Plane2dLabel lab;
+  lab.in = p.in;
+  lab.rois = (const float*)p.rois;
+  lab.out = (int*)p.out;
+  lab.C = p.C;
+  lab.vec = (p.ow & 1) == 0 && (uintptr_t)p.out % 8 == 0;
+  return lab;
+}
+
 static int affine_label_impl(const void* labels, int label_dtype, const float* rois, int32_t* output, int ndim,
                              int64_t N, int64_t C, int64_t D, int64_t H, int64_t W, int64_t R, int roi_width, int od,
                              int oh, int ow, float spatial_scale, int aligned, int* status, void* stream) {
@@ -295,6 +306,14 @@ static int affine_label_impl(const void* labels, int label_dtype, const float* r
   if (rc != MVR_OK) return rc;
   Params p = make_params(labels, rois, output, ndim, MVR_ROI_ROTATED, N, C, D, H, W, R, od, oh, ow, spatial_scale, 1,
                          aligned, 0, status);
+  if (ndim == 2 && p.R > 0 && p.C > 0) {  // dense outputs
+    const Plane2dLabel lab = plane2d_label_of(p);
+    Params none = p;
+    none.in = nullptr;
+    none.out = nullptr;
+    if (try_launch_plane2d(none, MVR_F32, (cudaStream_t)stream, &lab, label_dtype) == 0)
+      return cudaGetLastError() == cudaSuccess ? MVR_OK : MVR_ERR_LAUNCH;
+  }
   rc = launch_label(p, label_dtype, (cudaStream_t)stream);
   return rc == 0 ? MVR_OK : (rc == -9 ? MVR_ERR_UNSUPPORTED : MVR_ERR_LAUNCH);
 }
@@ -341,6 +360,31 @@ int mvr_affine_fields_3d(const void* image, int dtype, const void* image_rois, v
     if (rc != 0) return rc == -9 ? MVR_ERR_UNSUPPORTED : MVR_ERR_LAUNCH;
   }
   return MVR_OK;
+}
+
+int mvr_affine_fields_2d(const void* image, int dtype, const void* image_rois, void* image_out, int64_t C_image,
+                         const void* labels, int label_dtype, const float* label_rois, int32_t* label_out,
+                         int64_t C_label, int64_t N, int64_t H, int64_t W, int64_t R, int roi_width, int oh, int ow,
+                         float spatial_scale, int aligned, int order, int* status, void* stream) {
+  if (label_dtype < MVR_LABEL_U8 || label_dtype > MVR_LABEL_I64) return MVR_ERR_DTYPE;
+  int rc = check_common(image, image_rois, image_out, dtype, 2, MVR_ROI_ROTATED, N, C_image, 1, H, W, R, roi_width, 1, oh, ow, order);
+  if (rc != MVR_OK) return rc;
+  rc = check_common(labels, label_rois, label_out, MVR_F32, 2, MVR_ROI_ROTATED, N, C_label, 1, H, W, R, roi_width, 1, oh, ow, 0);
+  if (rc != MVR_OK) return rc;
+  cudaStream_t st = (cudaStream_t)stream;
+  const Params pi = make_params(image, image_rois, image_out, 2, MVR_ROI_ROTATED, N, C_image, 1, H, W, R, 1, oh, ow, spatial_scale, 1,
+                                aligned, order, status);
+  const Params pl = make_params(labels, label_rois, label_out, 2, MVR_ROI_ROTATED, N, C_label, 1, H, W, R, 1, oh, ow, spatial_scale, 1,
+                                aligned, 0, status);
+  if (R > 0 && C_image > 0 && C_label > 0) {
+    const Plane2dLabel lab = plane2d_label_of(pl);
+    if (try_launch_plane2d(pi, dtype, st, &lab, label_dtype) == 0) return cudaGetLastError() == cudaSuccess ? MVR_OK : MVR_ERR_LAUNCH;
+  }
+  // small outputs and the like: one launch each
+  rc = dispatch(pi, dtype, true, st);
+  if (rc != MVR_OK) return rc;
+  rc = launch_label(pl, label_dtype, st);
+  return rc == 0 ? MVR_OK : (rc == -9 ? MVR_ERR_UNSUPPORTED : MVR_ERR_LAUNCH);
 }
 
 static int apply_offset_impl(const void* img, const void* offset, void* out, int dtype, int offset_dtype, int ndim,

@@ -96,10 +96,10 @@ resample_bwd_stream3d(const Params p, const S3Launch L, typename BwdAcc<T>::type
     float acc0[8], acc1[8];  // [0..3] voxel a, [4..7] voxel b; taps x0y0, x1y0, x0y1, x1y1
 #pragma unroll
     for (int t = 0; t < 8; ++t) acc0[t] = acc1[t] = 0.0f;
-    long long held0 = -1, held1 = -1;  // plane offsets of acc0 / acc1, -1: nothing held
-    auto flush = [&](const float* a, long long plane) {
+    int held0 = -1, held1 = -1;  // planes of acc0 / acc1, -1: nothing held
+    auto flush = [&](const float* a, int plane) {
       if (plane < 0) return;
-      Acc* pl = acc + plane;
+      Acc* pl = acc + plane * HW;
       if (ina) {
         bwd_red_row(pl + oa[0], pl + oa[1], a[0], a[1], acc_lo, acc_hi);
         bwd_red_row(pl + oa[2], pl + oa[3], a[2], a[3], acc_lo, acc_hi);
@@ -111,7 +111,7 @@ resample_bwd_stream3d(const Params p, const S3Launch L, typename BwdAcc<T>::type
     };
     for (int i = 0; i < k.npd; ++i) {
       const S3ZTap<T> e = sh.zt[i];
-      if (!e.inside) continue;
+      if (e.z0 < 0) continue;
       const T ga = go[i * plane_o];
       const T gb = has_b ? go[i * plane_o + 1] : A::fi(0);
       const V g2 = Q::make(ga, gb);
@@ -128,22 +128,22 @@ resample_bwd_stream3d(const Params p, const S3Launch L, typename BwdAcc<T>::type
         c0[t] = A::tof(Q::lo(lo)); c0[4 + t] = A::tof(Q::hi(lo));
         c1[t] = A::tof(Q::lo(hi)); c1[4 + t] = A::tof(Q::hi(hi));
       }
-      if (e.o0 == held0 && e.o1 == held1) {  // CTA-uniform
+      if (e.z0 == held0 && e.z1 == held1) {  // CTA-uniform
 #pragma unroll
         for (int t = 0; t < 8; ++t) { acc0[t] += c0[t]; acc1[t] += c1[t]; }
-      } else if (e.o0 == held1) {
+      } else if (e.z0 == held1) {
         flush(acc0, held0);
 #pragma unroll
         for (int t = 0; t < 8; ++t) { acc0[t] = acc1[t] + c0[t]; acc1[t] = c1[t]; }
         held0 = held1;
-        held1 = e.o1;
+        held1 = e.z1;
       } else {
         flush(acc0, held0);
         flush(acc1, held1);
 #pragma unroll
         for (int t = 0; t < 8; ++t) { acc0[t] = c0[t]; acc1[t] = c1[t]; }
-        held0 = e.o0;
-        held1 = e.o1;
+        held0 = e.z0;
+        held1 = e.z1;
       }
     }
     flush(acc0, held0);
@@ -176,7 +176,6 @@ resample_bwd_stream3d(const Params p, const S3Launch L, typename BwdAcc<T>::type
                     acc_hi);
     }
   }
-  (void)HW;
 }
 
 // grad_in (half) += scratch (float), rounded once

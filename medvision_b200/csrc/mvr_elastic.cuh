@@ -30,6 +30,7 @@ struct ElasticParams {
   int* lab_out;
   float* field;                        // dense-field kernel only: (B, NDIM, [D,] H, W)
   int B, C, CL, D, H, W;
+  PairConst pair;
   int rows, blocks_h;                  // rows per CTA, row blocks per plane
   int vec_img, vec_lab, vec_field;     // two-element vector stores are aligned
 };
@@ -204,16 +205,20 @@ elastic_warp_kernel(const ElasticParams p) {
       for (int a = 0; a < NDIM; ++a)  // axis w, h, d <- channel d, h, w; rounded to the image's type
         o2[a] = Q::make(Ar<T>::ff(da[NDIM - 1 - a]), Ar<T>::ff(db[NDIM - 1 - a]));
       warp_positions<T, NDIM>(w0, h, k.d, o2, c);
-      WarpTaps<T, NDIM> t;
-      warp_taps<T, NDIM>(c, p.W, p.H, p.D, 1, has_b, t);
+      AxisTap2<T> t[3];
+      warp_taps<T, NDIM>(c, p.pair, 1, t);
+      const typename Q::M mask = warp_inside<T, NDIM>(c, p.pair, has_b);
+      const PairTaps<T, NDIM> taps(t[0], t[1], t[2], p.pair);
       if (img0) {
         V w[1 << NDIM];
-        warp_weights<T, NDIM>(t, w);
+        pair_weights<T, NDIM>(t[0], t[1], t[2], w);
         const T* img = img0;
         T* out = (T*)p.out + (long long)k.b * p.C * vol + row + w0;
 #pragma unroll 1
         for (int ch = 0; ch < p.C; ++ch, img += vol, out += vol) {
-          const V val = warp_channel<T, NDIM>(t, w, img);
+          V v[1 << NDIM];
+          taps.load(img, p.pair, v);
+          const V val = Q::apply(pair_sum<T, (1 << NDIM)>(w, v), mask);
           if (p.vec_img) {
             Q::store2(out, val);
           } else {
@@ -224,20 +229,20 @@ elastic_warp_kernel(const ElasticParams p) {
       }
       if (lab0) {
         // nearest: the lower tap of an axis where its weight is at least one half, else the upper one
-        int ia = t.ba, ib = t.bb;
-        if (!Ar<T>::ge_half(Q::lo(t.t[0].h))) ia += t.xa1;
-        if (!Ar<T>::ge_half(Q::hi(t.t[0].h))) ib += t.xb1;
-        if (!Ar<T>::ge_half(Q::lo(t.t[1].h))) ia += t.ya1;
-        if (!Ar<T>::ge_half(Q::hi(t.t[1].h))) ib += t.yb1;
-        if (NDIM == 3) {
-          if (!Ar<T>::ge_half(Q::lo(t.t[2].h))) ia += t.za1;
-          if (!Ar<T>::ge_half(Q::hi(t.t[2].h))) ib += t.zb1;
+        unsigned oa = taps.a, ob = taps.b;
+#pragma unroll
+        for (int a = 0; a < NDIM; ++a) {
+          const unsigned step = a == 0 ? (unsigned)sizeof(T) : a == 1 ? p.pair.sy : p.pair.sz;
+          if (t[a].ca || !Ar<T>::ge_half(Q::lo(t[a].h))) oa += step;
+          if (t[a].cb || !Ar<T>::ge_half(Q::hi(t[a].h))) ob += step;
         }
+        const unsigned ia = oa / (unsigned)sizeof(T), ib = ob / (unsigned)sizeof(T);
+        const bool ina = Q::lane_a(mask), inb = Q::lane_b(mask);
         const IT* lab = lab0;
         int* out = p.lab_out + (long long)k.b * p.CL * vol + row + w0;
 #pragma unroll 1
         for (int ch = 0; ch < p.CL; ++ch, lab += vol, out += vol) {
-          const int va = t.ina ? elastic_label<T, IT>(lab + ia) : 0, vb = t.inb ? elastic_label<T, IT>(lab + ib) : 0;
+          const int va = ina ? elastic_label<T, IT>(lab + ia) : 0, vb = inb ? elastic_label<T, IT>(lab + ib) : 0;
           if (p.vec_lab) {
             *reinterpret_cast<int2*>(out) = make_int2(va, vb);
           } else {
@@ -250,10 +255,11 @@ elastic_warp_kernel(const ElasticParams p) {
   }
 }
 
-// 0 launched, 1 not applicable (grid too large for the tables, volume too large for 32-bit offsets), -8 launch failed
+// 0 launched, 1 not applicable (grid too large for the tables, a single voxel along an axis, volume too large for 32-bit offsets), -8 launch failed
 inline int launch_elastic(ElasticParams p, int ndim, int dtype, int label_dtype, cudaStream_t st) {
-  if ((long long)p.D * p.H * p.W >= 0x7fffffffLL || elastic_smem(ndim, p.gw, p.gh) > (size_t)kElasticMaxSmem) return 1;
+  if (!pair_taps_applicable(ndim, p.D, p.H, p.W, (long long)p.D * p.H * p.W, dtype == 0 ? 4 : 2) || elastic_smem(ndim, p.gw, p.gh) > (size_t)kElasticMaxSmem) return 1;
   if (p.B == 0) return 0;
+  p.pair = make_pair_const(ndim, p.D, p.H, p.W, dtype == 0 ? 4 : 2);
   // A CTA's contraction along z costs about as much as a row: as many rows per CTA as leave six CTAs per SM.
   p.rows = 64;
   while (p.rows > 8 && (long long)p.B * p.D * ((p.H + p.rows - 1) / p.rows) < 148LL * 6) p.rows >>= 1;

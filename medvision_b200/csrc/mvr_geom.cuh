@@ -106,6 +106,75 @@ __device__ void decode_roi(const T* __restrict__ rois, long long n, int ndim, in
   g.count_bwd = (ndim == 2) ? A::fi(prod) : A::fi(max(prod, 1));
 }
 
+// decode_roi for one sample per bin, by the 32 lanes of one warp: a lane per axis, a lane per sine and cosine (one thread
+// doing six of them and three divisions in a row is 1-2 us in which the rest of a dense kernel's CTA waits).  Same values.
+// Lanes below ndim return whether their axis's lattice and centre are finite, the others true.
+template <typename T>
+__device__ __forceinline__ bool decode_roi_warp(const T* __restrict__ rois, long long n, int ndim, int kind, int ow, int oh, int od,
+                                                float spatial_scale, int aligned, int fm, RoiGeom<T>& g) {
+  typedef Ar<T> A;
+  const int lane = threadIdx.x & 31;
+  const int width = (kind == KIND_BOX) ? (ndim == 2 ? 5 : 7) : (ndim == 2 ? 6 : 10);
+  const T* r = rois + n * width;
+  const T scale = A::ff(spatial_scale), one = A::fi(1), zero = A::fi(0);
+  const int a = lane < ndim ? lane : 0;
+  const int osz = a == 0 ? ow : a == 1 ? oh : od;
+  T size, start, centre = zero;
+  if (kind == KIND_BOX) {
+    const T hi = r[1 + ndim + a];
+    start = A::mul(r[1 + a], scale);
+    size = (A::kCanFuse && Fm::boxsize(fm)) ? A::fma_(hi, scale, A::neg(start)) : A::sub(A::mul(hi, scale), start);
+    if (!A::ge_one(size)) size = one;
+  } else {
+    const T off = aligned ? A::ff(0.5f) : zero;
+    centre = (A::kCanFuse && Fm::centre(fm)) ? A::fma_(r[1 + a], scale, A::neg(off)) : A::sub(A::mul(r[1 + a], scale), off);
+    size = A::mul(r[1 + ndim + a], scale);
+    if (!aligned && !A::ge_one(size)) size = one;
+    start = A::halve_neg(size);
+    const int na = ndim == 2 ? 1 : 3, k = (lane - 8) >> 1;
+    T v = zero;
+    if (k >= 0 && k < na) v = (lane & 1) ? A::sinT(r[1 + 2 * ndim + k]) : A::cosT(r[1 + 2 * ndim + k]);
+    const T c0 = __shfl_sync(0xffffffffu, v, 8), s0 = __shfl_sync(0xffffffffu, v, 9);
+    if (ndim == 2) {
+      if (lane == 0) {
+        g.rot[0] = c0;
+        g.rot[1] = s0;
+      }
+    } else {
+      const T cg = c0, sg = s0;
+      const T cb = __shfl_sync(0xffffffffu, v, 10), sb = __shfl_sync(0xffffffffu, v, 11);
+      const T ca = __shfl_sync(0xffffffffu, v, 12), sa = __shfl_sync(0xffffffffu, v, 13);
+      if (lane == 0) {
+        g.rot[0] = A::mul(ca, cb);
+        g.rot[1] = rot_entry<T>(ca, sb, sg, sa, cg, true, Fm::entry(fm, 0));
+        g.rot[2] = rot_entry<T>(ca, sb, cg, sa, sg, false, Fm::entry(fm, 1));
+        g.rot[3] = A::mul(sa, cb);
+        g.rot[4] = rot_entry<T>(sa, sb, sg, ca, cg, false, Fm::entry(fm, 2));
+        g.rot[5] = rot_entry<T>(sa, sb, cg, ca, sg, true, Fm::entry(fm, 3));
+        g.rot[6] = A::neg(sb);
+        g.rot[7] = A::mul(cb, sg);
+        g.rot[8] = A::mul(cb, cg);
+      }
+    }
+  }
+  const T bin = A::div(size, A::fi(osz));
+  if (lane < 3) {
+    g.grid[lane] = 1;
+    g.start[lane] = lane < ndim ? start : zero;
+    g.bin[lane] = lane < ndim ? bin : zero;
+    g.centre[lane] = lane < ndim ? centre : zero;
+  }
+  if (lane == 0) {
+    g.batch = A::toi(r[0]);
+    g.count_fwd = g.count_bwd = one;
+  }
+  const T sub = A::mul(A::ff(0.5f), bin);
+  const T first = (A::kCanFuse && Fm::lattice(fm)) ? A::fma_(A::fi(0), bin, start) : A::add(start, A::mul(A::fi(0), bin));
+  const T last = (A::kCanFuse && Fm::lattice(fm)) ? A::fma_(A::fi(osz - 1), bin, start) : A::add(start, A::mul(A::fi(osz - 1), bin));
+  __syncwarp();
+  return lane >= ndim || (A::finite(A::add(first, sub)) && A::finite(A::add(last, sub)) && A::finite(centre));
+}
+
 // in-bin offset of sub-sample i:  ((i + .5) * bin) / g
 template <typename T>
 __device__ __forceinline__ T lattice_sub(T bin, int i, int g) {

@@ -30,14 +30,61 @@ __device__ __forceinline__ int label_axis_pick(float c, int size, bool& outside)
   return t.h == 1.0f ? t.i0 : (t.l == 1.0f ? t.i1 : -1);
 }
 
+// The same choice in few instructions (sizes up to kTapMaxSize; see axis_tap2): kTapMagic + the picked index, always valid;
+// `in` stays true for a coordinate inside the band only (a NaN is not: its weights do not qualify).  The upper tap is taken
+// when its weight l exceeds one half (h = 1 - l is then below it).
+__device__ __forceinline__ unsigned label_pick(float c, float size, float last, bool& in) {
+  const float magic = 8388608.0f;
+  in = in && c >= -1.0f && c <= size;
+  const float f = fminf(fmaxf(c, 0.0f), last);
+  const float m = __fadd_rz(f, magic);
+  return __float_as_uint(m) + (__fsub_rn(f, __fsub_rn(m, magic)) > 0.5f ? 1u : 0u);
+}
+
+struct LabelShared {
+  RoiGeom<float> g;
+  int zsep;
+  union {
+    int plane[kS3MaxChunk];             // z-separable: element offset of the picked plane, -1: none
+    S3ZProd<float> zp[kS3MaxChunk];     // general rotation: the products R_i3 * z
+  };
+};
+
 // One work item (32 x 16 tile x depth chunk of one (roi, channel)) of the dense 3D label path.
 template <typename IT>
-__device__ __forceinline__ void label_item_stream3d(const Params& p, const S3Launch& L, const S3Cta& k, S3Shared<float>& sh) {
+__device__ __forceinline__ void label_item_stream3d(const Params& p, const S3Launch& L, const S3Cta& k, LabelShared& sh) {
   typedef Ar<float> A;
-  s3_prologue<float>(p, k, sh);  // p.order == 0: the per-depth weights in the table are one-hot
-  const RoiGeom<float>& g = sh.g;
   const int fm = kS3FloatPattern;
+  if (threadIdx.x < 32) {
+    const bool finite = decode_roi_warp<float>((const float*)p.rois, k.n, 3, p.kind, p.ow, p.oh, p.od, p.spatial_scale, p.aligned, fm, sh.g);
+    const RoiGeom<float>& g = sh.g;
+    const bool zsep = p.kind != KIND_ROTATED || (g.rot[2] == 0.0f && g.rot[5] == 0.0f && g.rot[6] == 0.0f && g.rot[7] == 0.0f && g.rot[8] == 1.0f);
+    const bool all = __all_sync(0xffffffffu, finite && zsep);
+    if (threadIdx.x == 0) sh.zsep = all;
+  }
+  __syncthreads();
+  const RoiGeom<float>& g = sh.g;
   const bool rotated = (p.kind == KIND_ROTATED);
+  const bool zsep = sh.zsep != 0;
+  const int npd = k.npd;
+  const int HW = p.H * p.W;
+  const float sx = (float)p.W, sy = (float)p.H, sz = (float)p.D, lx = sx - 1.0f, ly = sy - 1.0f, lz = sz - 1.0f;
+  if ((int)threadIdx.x < npd) {
+    const int i = threadIdx.x;
+    const float z = A::add(lattice_base<float>(g.start[2], k.pd0 + i, g.bin[2], fm), lattice_sub<float>(g.bin[2], 0, 1));
+    if (zsep) {
+      bool in = true;
+      const unsigned raw = label_pick(rotated ? A::add(z, g.centre[2]) : z, sz, lz, in);
+      sh.plane[i] = in ? (int)(raw - kTapMagic) * HW : -1;
+    } else {
+      S3ZProd<float> e;
+      e.p[0] = A::mul(g.rot[2], z);
+      e.p[1] = A::mul(g.rot[5], z);
+      e.p[2] = A::mul(g.rot[8], z);
+      sh.zp[i] = e;
+    }
+  }
+  __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int pw0 = k.tw * kS3TileW + (warp & 1) * 16 + (lane & 7) * 2;
   const int ph = k.th * kS3TileH + (warp >> 1) * 4 + (lane >> 3);
@@ -46,7 +93,6 @@ __device__ __forceinline__ void label_item_stream3d(const Params& p, const S3Lau
   const long long plane_o = (long long)p.oh * p.ow;
   int* out = (int*)p.out + k.nc * p.ovol + (long long)k.pd0 * plane_o + (long long)ph * p.ow + pw0;
   const bool vec = L.vec_store && has_b;
-  const int npd = k.npd;
 
   if (g.batch < 0 || g.batch >= p.N) {
     if (p.status && threadIdx.x == 0 && k.tw == 0 && k.th == 0 && k.ck == 0) atomicOr(p.status, STATUS_BAD_BATCH_INDEX);
@@ -62,8 +108,9 @@ __device__ __forceinline__ void label_item_stream3d(const Params& p, const S3Lau
                       A::add(lattice_base<float>(g.start[0], has_b ? pw0 + 1 : pw0, g.bin[0], fm), sub_x)};
   const float y = A::add(lattice_base<float>(g.start[1], ph, g.bin[1], fm), sub_y);
 
-  if (sh.zsep) {
-    int off[2];  // in-plane offset of the picked tap, -1: the voxel is 0 at every depth
+  if (zsep) {
+    const IT* at[2];  // the picked tap in plane 0
+    bool in[2] = {true, has_b};
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
       float rx = x[s], ry = y;
@@ -71,20 +118,16 @@ __device__ __forceinline__ void label_item_stream3d(const Params& p, const S3Lau
         rx = A::add(__fmaf_rn(g.rot[0], x[s], A::mul(g.rot[1], y)), g.centre[0]);
         ry = A::add(__fmaf_rn(g.rot[3], x[s], A::mul(g.rot[4], y)), g.centre[1]);
       }
-      bool ox, oy;
-      const int ix = label_axis_pick(rx, p.W, ox), iy = label_axis_pick(ry, p.H, oy);
-      off[s] = (ox || oy || ix < 0 || iy < 0 || (s == 1 && !has_b)) ? -1 : iy * p.W + ix;
+      const unsigned ix = label_pick(rx, sx, lx, in[s]), iy = label_pick(ry, sy, ly, in[s]);
+      at[s] = vol + (iy * (unsigned)p.W + ix - kTapMagic * ((unsigned)p.W + 1u));
     }
-#pragma unroll 4
-    for (int i = 0; i < npd; ++i, out += plane_o) {  // unrolled: several depths' loads in flight
-      const S3ZTap<float> e = sh.zt[i];
+    // eight depths' loads in flight: the kernel waits for memory, not for instructions
+#pragma unroll 8
+    for (int i = 0; i < npd; ++i, out += plane_o) {
+      const int pl = sh.plane[i];
       int va = 0, vb = 0;
-      const bool take0 = e.h == 1.0f, take1 = e.l == 1.0f;
-      if (e.inside && (take0 || take1)) {
-        const IT* pl = vol + (take0 ? e.o0 : e.o1);
-        if (off[0] >= 0) va = label_value<IT>(pl + off[0]);
-        if (off[1] >= 0) vb = label_value<IT>(pl + off[1]);
-      }
+      if (pl >= 0 && in[0]) va = label_value<IT>(at[0] + pl);
+      if (pl >= 0 && in[1]) vb = label_value<IT>(at[1] + pl);
       if (vec) {
         *reinterpret_cast<int2*>(out) = make_int2(va, vb);
       } else {
@@ -101,19 +144,18 @@ __device__ __forceinline__ void label_item_stream3d(const Params& p, const S3Lau
   for (int s = 0; s < 2; ++s)
 #pragma unroll
     for (int r = 0; r < 3; ++r) sxy[s][r] = __fmaf_rn(g.rot[3 * r], x[s], A::mul(g.rot[3 * r + 1], y));
-  const long long HW = (long long)p.H * p.W;
+  const unsigned bias = kTapMagic * ((unsigned)HW + (unsigned)p.W + 1u);
+#pragma unroll 4
   for (int i = 0; i < npd; ++i, out += plane_o) {
     const S3ZProd<float> e = sh.zp[i];
     int val[2] = {0, 0};
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
-      if (s == 1 && !has_b) continue;
-      const float rx = A::add(A::add(sxy[s][0], e.p[0]), g.centre[0]);
-      const float ry = A::add(A::add(sxy[s][1], e.p[1]), g.centre[1]);
-      const float rz = A::add(A::add(sxy[s][2], e.p[2]), g.centre[2]);
-      bool ox, oy, oz;
-      const int ix = label_axis_pick(rx, p.W, ox), iy = label_axis_pick(ry, p.H, oy), iz = label_axis_pick(rz, p.D, oz);
-      if (!(ox || oy || oz || ix < 0 || iy < 0 || iz < 0)) val[s] = label_value<IT>(vol + iz * HW + (long long)iy * p.W + ix);
+      bool in = s == 0 || has_b;
+      const unsigned ix = label_pick(A::add(A::add(sxy[s][0], e.p[0]), g.centre[0]), sx, lx, in);
+      const unsigned iy = label_pick(A::add(A::add(sxy[s][1], e.p[1]), g.centre[1]), sy, ly, in);
+      const unsigned iz = label_pick(A::add(A::add(sxy[s][2], e.p[2]), g.centre[2]), sz, lz, in);
+      if (in) val[s] = label_value<IT>(vol + (iz * (unsigned)HW + (iy * (unsigned)p.W + ix) - bias));
     }
     if (vec) {
       *reinterpret_cast<int2*>(out) = make_int2(val[0], val[1]);
@@ -127,7 +169,7 @@ __device__ __forceinline__ void label_item_stream3d(const Params& p, const S3Lau
 template <typename IT>
 __global__ void __launch_bounds__(kS3Threads)
 resample_label_stream3d(const Params p, const S3Launch L) {
-  __shared__ S3Shared<float> sh;
+  __shared__ LabelShared sh;
   label_item_stream3d<IT>(p, L, s3_cta(p, L), sh);
 }
 
@@ -137,12 +179,12 @@ resample_label_stream3d(const Params p, const S3Launch L) {
 // image field and its label field thus cost the two overlapped launches of the image alone.
 // p / L / items: the image (element type T); pl / Ll / items_l: the label job (float32 rois, int32 result).
 template <typename T, typename IT>
-__global__ void __launch_bounds__(kS3Threads)
+__global__ void __launch_bounds__(kS3Threads, 4)
 resample_fwd_stream3d_rest_label(const Params p, const S3Launch L, long long items, const Params pl, const S3Launch Ll,
                                  long long items_l) {
   __shared__ union Tables {
     S3Shared<T> img;
-    S3Shared<float> lab;
+    LabelShared lab;
   } sh;
   __shared__ unsigned general[kS3RestMaxRois / 32];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -158,8 +200,8 @@ resample_fwd_stream3d_rest_label(const Params p, const S3Launch L, long long ite
     for (long long item = blockIdx.x; item < items; item += gridDim.x) {
       const S3Cta k = s3_cta(p, L, item);
       if (!((general[k.n >> 5] >> (k.n & 31)) & 1u)) continue;  // CTA-uniform
-      s3_prologue<T>(p, k, sh.img);
-      s3_body_l1<T>(p, L, k, sh.img);
+      s3_prologue<T, true>(p, k, sh.img);
+      s3_body_l1<T, true>(p, L, k, sh.img);
       __syncthreads();  // the next item's prologue overwrites the tables
     }
   for (long long item = blockIdx.x; item < items_l; item += gridDim.x) {
@@ -224,13 +266,13 @@ enum { LABEL_U8 = 0, LABEL_I16 = 1, LABEL_I32 = 2, LABEL_I64 = 3 };
 
 // Work items of the dense 3D label path; false: the call has not its shape.
 inline bool label_stream3d_geometry(const Params& p, S3Launch& L, long long& items) {
-  if (!(p.ndim == 3 && p.ovol >= 4096 && p.ow >= 8 && p.vol < 0x7fffffffLL && p.fm == kS3FloatPattern)) return false;
+  if (!(p.ndim == 3 && p.ovol >= 4096 && p.ow >= 8 && p.vol < 0x7fffffffLL && p.fm == kS3FloatPattern &&
+        p.D <= kTapMaxSize && p.H <= kTapMaxSize && p.W <= kTapMaxSize))
+    return false;
   L.tiles_w = (p.ow + kS3TileW - 1) / kS3TileW;
   L.tiles_h = (p.oh + kS3TileH - 1) / kS3TileH;
   const long long per_depth = (long long)p.R * p.C * L.tiles_w * L.tiles_h;
-  int chunk = kS3MaxChunk;
-  while (chunk > 8 && per_depth * ((p.od + chunk - 1) / chunk) < 148LL * 16) chunk >>= 1;
-  L.chunk = min(chunk, p.od);
+  L.chunk = s3_pick_chunk(per_depth, p.od, 148 * 4, 12);
   L.chunks = (p.od + L.chunk - 1) / L.chunk;
   L.vec_store = ((p.ow & 1) == 0) && (((uintptr_t)p.out) % 8 == 0);
   L.filter = 0;

@@ -23,6 +23,7 @@ struct OffsetParams {
   const void* off;   // (B, NDIM, [D,] H, W): displacement along d, h, w (3D) or h, w (2D), in voxels
   void* out;         // (B, C, [D,] H, W)
   int B, C, D, H, W, order, fm, vec_ok;
+  PairConst pair;
   int off_f32;       // the field is float32 although the image is half: rounded to half on load (= offset.half())
 };
 
@@ -48,17 +49,7 @@ __device__ __forceinline__ __half2 load_offset_pair<__half>(const OffsetParams& 
   return __halves2half2(f[0], has_b ? f[1] : __float2half_rn(0.0f));
 }
 
-// Taps of the two voxels of a pair at (T)index + offset (mvr_elastic.cuh uses them too): base offsets inside a channel's
-// volume, steps to the upper neighbours (0 where clamped), weights (order 1) or the one-hot choice (order 0) per axis,
-// and which lane lies strictly inside (-1, size) on every axis.
-template <typename T, int NDIM>
-struct WarpTaps {
-  typedef typename P2<T>::V V;
-  AxisTap2<T> t[3];  // w, h, d
-  int ba, bb, xa1, xb1, ya1, yb1, za1, zb1;
-  bool ina, inb;
-};
-
+// Sample positions (T)index + offset of a pair (mvr_elastic.cuh uses them too).
 // o2: displacement of the two voxels per axis (index 0 = w, 1 = h, 2 = d), in the image's element type
 template <typename T, int NDIM>
 __device__ __forceinline__ void warp_positions(int w0, int h, int d, const typename P2<T>::V* o2, typename P2<T>::V* c) {
@@ -68,75 +59,23 @@ __device__ __forceinline__ void warp_positions(int w0, int h, int d, const typen
   c[1] = Q::add(Q::dup(A::fi(h)), o2[1]);
   c[2] = (NDIM == 3) ? Q::add(Q::dup(A::fi(d)), o2[2]) : Q::dup(A::fi(0));
 }
+// lanes strictly inside (-1, size) on every axis
 template <typename T, int NDIM>
-__device__ __forceinline__ void warp_inside(const typename P2<T>::V* c, int W, int H, int D, bool has_b, bool& ina, bool& inb) {
-  typedef Ar<T> A;
+__device__ __forceinline__ typename P2<T>::M warp_inside(const typename P2<T>::V* c, const PairConst& k, bool has_b) {
   typedef P2<T> Q;
-  const int size[3] = {W, H, D};
-  ina = true;
-  inb = has_b;
-#pragma unroll
-  for (int a = 0; a < NDIM; ++a) {
-    ina = ina && A::tof(Q::lo(c[a])) > -1.0f && A::tof(Q::lo(c[a])) < (float)size[a];
-    inb = inb && A::tof(Q::hi(c[a])) > -1.0f && A::tof(Q::hi(c[a])) < (float)size[a];
-  }
+  typename Q::M m = Q::make_mask(true, has_b) & Q::strictly_inside(c[0], k, 0) & Q::strictly_inside(c[1], k, 1);
+  if (NDIM == 3) m &= Q::strictly_inside(c[2], k, 2);
+  return m;
 }
 template <typename T, int NDIM>
-__device__ __forceinline__ void warp_taps(const typename P2<T>::V* c, int W, int H, int D, int order, bool has_b, WarpTaps<T, NDIM>& t) {
-  warp_inside<T, NDIM>(c, W, H, D, has_b, t.ina, t.inb);
-  axis_tap2<T>(c[0], W, order, t.t[0]);
-  axis_tap2<T>(c[1], H, order, t.t[1]);
-  if (NDIM == 3) axis_tap2<T>(c[2], D, order, t.t[2]);
-  const AxisTap2<T>&tx = t.t[0], &ty = t.t[1], &tz = t.t[2];
-  const int HW = H * W;
-  t.ba = t.ina ? (((NDIM == 3 ? tz.i0a * H : 0) + ty.i0a) * W + tx.i0a) : 0;
-  t.bb = t.inb ? (((NDIM == 3 ? tz.i0b * H : 0) + ty.i0b) * W + tx.i0b) : 0;
-  t.xa1 = t.ina ? tx.da : 0;
-  t.xb1 = t.inb ? tx.db : 0;
-  t.ya1 = (t.ina && ty.da) ? W : 0;
-  t.yb1 = (t.inb && ty.db) ? W : 0;
-  t.za1 = (NDIM == 3 && t.ina && tz.da) ? HW : 0;
-  t.zb1 = (NDIM == 3 && t.inb && tz.db) ? HW : 0;
-}
-template <typename T, int NDIM>
-__device__ __forceinline__ void warp_weights(const WarpTaps<T, NDIM>& t, typename P2<T>::V* w) {
-  typedef P2<T> Q;
-  typedef typename Q::V V;
-  const AxisTap2<T>&tx = t.t[0], &ty = t.t[1], &tz = t.t[2];
-  if (NDIM == 3) {
-    const V hzhy = Q::mul(tz.h, ty.h), hzly = Q::mul(tz.h, ty.l);
-    const V lzhy = Q::mul(tz.l, ty.h), lzly = Q::mul(tz.l, ty.l);
-    w[0] = Q::mul(hzhy, tx.h); w[1] = Q::mul(hzhy, tx.l); w[2] = Q::mul(hzly, tx.h); w[3] = Q::mul(hzly, tx.l);
-    w[4] = Q::mul(lzhy, tx.h); w[5] = Q::mul(lzhy, tx.l); w[6] = Q::mul(lzly, tx.h); w[7] = Q::mul(lzly, tx.l);
-  } else {
-    w[0] = Q::mul(ty.h, tx.h); w[1] = Q::mul(ty.h, tx.l); w[2] = Q::mul(ty.l, tx.h); w[3] = Q::mul(ty.l, tx.l);
-  }
-}
-// one channel: the reference's tap sum, 0 for a lane outside
-template <typename T, int NDIM>
-__device__ __forceinline__ typename P2<T>::V warp_channel(const WarpTaps<T, NDIM>& t, const typename P2<T>::V* w, const T* img) {
-  typedef P2<T> Q;
-  typedef typename Q::V V;
-  const T* pa = img + t.ba;
-  const T* pb = img + t.bb;
-  V v[1 << NDIM];
-  v[0] = Q::make(__ldg(pa), __ldg(pb));
-  v[1] = Q::make(__ldg(pa + t.xa1), __ldg(pb + t.xb1));
-  v[2] = Q::make(__ldg(pa + t.ya1), __ldg(pb + t.yb1));
-  v[3] = Q::make(__ldg(pa + t.ya1 + t.xa1), __ldg(pb + t.yb1 + t.xb1));
-  if (NDIM == 3) {
-    v[4] = Q::make(__ldg(pa + t.za1), __ldg(pb + t.zb1));
-    v[5] = Q::make(__ldg(pa + t.za1 + t.xa1), __ldg(pb + t.zb1 + t.xb1));
-    v[6] = Q::make(__ldg(pa + t.za1 + t.ya1), __ldg(pb + t.zb1 + t.yb1));
-    v[7] = Q::make(__ldg(pa + t.za1 + t.ya1 + t.xa1), __ldg(pb + t.zb1 + t.yb1 + t.xb1));
-  }
-  V acc = Q::tap_first(w[0], v[0], w[1], v[1]);
-#pragma unroll
-  for (int k = 2; k < (1 << NDIM); ++k) acc = Q::tap_next(acc, w[k], v[k]);
-  return Q::apply(acc, Q::make_mask(t.ina, t.inb));
+__device__ __forceinline__ void warp_taps(const typename P2<T>::V* c, const PairConst& k, int order, AxisTap2<T>* t) {
+  axis_tap2<T, 0>(c[0], k, order, t[0]);
+  axis_tap2<T, 1>(c[1], k, order, t[1]);
+  if (NDIM == 3) axis_tap2<T, 2>(c[2], k, order, t[2]);
+  else t[2] = t[1];  // not read
 }
 
-template <typename T, int NDIM, bool CUBIC>
+template <typename T, int NDIM, bool VOXELS>
 __device__ __forceinline__ void apply_offset_pair(const OffsetParams& p, int b, int d, int h, int wp) {
   typedef Ar<T> A;
   typedef P2<T> Q;
@@ -158,17 +97,33 @@ __device__ __forceinline__ void apply_offset_pair(const OffsetParams& p, int b, 
   const T* img = (const T*)p.img + (long long)b * p.C * vol;
   T* out = (T*)p.out + (long long)b * p.C * vol + s0;
 
-  if (CUBIC) {  // Catmull-Rom: per voxel
-    bool ina, inb;
-    warp_inside<T, NDIM>(c, p.W, p.H, p.D, has_b, ina, inb);
+  if (VOXELS) {  // Catmull-Rom, and volumes too large for the pair form's 32-bit offsets: voxel by voxel
+    const int lim[3] = {p.W, p.H, p.D};  // in float: any size
+    bool ina = true, inb = has_b;
+#pragma unroll
+    for (int a = 0; a < NDIM; ++a) {
+      ina = ina && A::tof(Q::lo(c[a])) > -1.0f && A::tof(Q::lo(c[a])) < (float)lim[a];
+      inb = inb && A::tof(Q::hi(c[a])) > -1.0f && A::tof(Q::hi(c[a])) < (float)lim[a];
+    }
     for (int ch = 0; ch < p.C; ++ch, img += vol, out += vol) {
       T va = zero, vb = zero;
-      if (NDIM == 3) {
-        if (ina) va = hermite_3d<T>(img, p.D, p.H, p.W, Q::lo(c[2]), Q::lo(c[1]), Q::lo(c[0]), p.fm);
-        if (inb) vb = hermite_3d<T>(img, p.D, p.H, p.W, Q::hi(c[2]), Q::hi(c[1]), Q::hi(c[0]), p.fm);
-      } else {
-        if (ina) va = hermite_2d<T>(img, p.H, p.W, Q::lo(c[1]), Q::lo(c[0]), p.fm);
-        if (inb) vb = hermite_2d<T>(img, p.H, p.W, Q::hi(c[1]), Q::hi(c[0]), p.fm);
+#pragma unroll 1
+      for (int s = 0; s < 2; ++s) {
+        if (!(s ? inb : ina)) continue;
+        const T x = s ? Q::hi(c[0]) : Q::lo(c[0]), y = s ? Q::hi(c[1]) : Q::lo(c[1]), z = s ? Q::hi(c[2]) : Q::lo(c[2]);
+        T val;
+        if (p.order == 3) {
+          val = NDIM == 3 ? hermite_3d<T>(img, p.D, p.H, p.W, z, y, x, p.fm) : hermite_2d<T>(img, p.H, p.W, y, x, p.fm);
+        } else {
+          T w[1 << NDIM], v[1 << NDIM];
+          long long off[1 << NDIM];
+          make_taps<T, NDIM>(p.D, p.H, p.W, z, y, x, p.order, w, off);
+#pragma unroll
+          for (int k = 0; k < (1 << NDIM); ++k) v[k] = __ldg(img + off[k]);
+          val = tap_sum<T, (1 << NDIM)>(w, v, p.fm);
+        }
+        if (s) vb = val;
+        else va = val;
       }
       out[0] = va;
       if (has_b) out[1] = vb;
@@ -176,13 +131,21 @@ __device__ __forceinline__ void apply_offset_pair(const OffsetParams& p, int b, 
     return;
   }
 
-  WarpTaps<T, NDIM> t;
-  warp_taps<T, NDIM>(c, p.W, p.H, p.D, p.order, has_b, t);
+  AxisTap2<T> t[3];
+  warp_taps<T, NDIM>(c, p.pair, p.order, t);
+  const typename Q::M mask = warp_inside<T, NDIM>(c, p.pair, has_b);
+  const PairTaps<T, NDIM> taps(t[0], t[1], t[2], p.pair);
   V w[1 << NDIM];
-  warp_weights<T, NDIM>(t, w);
+  pair_weights<T, NDIM>(t[0], t[1], t[2], w);
 #pragma unroll 1
   for (int ch = 0; ch < p.C; ++ch, img += vol, out += vol) {
-    const V val = warp_channel<T, NDIM>(t, w, img);
+    V val = Q::dup(zero);
+    if (mask) {
+      V v[1 << NDIM];
+      taps.load(img, p.pair, v);
+      // a sample outside the image gives the literal 0; inside, the reference returns the sum as it is
+      val = Q::apply(pair_sum<T, (1 << NDIM)>(w, v), mask);
+    }
     if (p.vec_ok) {
       Q::store2(out, val);
     } else {
@@ -192,8 +155,8 @@ __device__ __forceinline__ void apply_offset_pair(const OffsetParams& p, int b, 
   }
 }
 
-template <typename T, int NDIM, bool CUBIC>
-__global__ void __launch_bounds__(kOffsetThreads, CUBIC ? 1 : 4)
+template <typename T, int NDIM, bool VOXELS>
+__global__ void __launch_bounds__(kOffsetThreads, VOXELS ? 1 : 4)
 apply_offset_kernel(const OffsetParams p) {
   typedef Ar<T> A;
   typedef P2<T> Q;
@@ -207,20 +170,21 @@ apply_offset_kernel(const OffsetParams p) {
   const unsigned row = idx / pairs_w;
   const int h = (int)(row % (unsigned)p.H);
   const int d = (int)(row / (unsigned)p.H);
-  for (int b = blockIdx.y; b < p.B; b += gridDim.y) apply_offset_pair<T, NDIM, CUBIC>(p, b, d, h, wp);
+  for (int b = blockIdx.y; b < p.B; b += gridDim.y) apply_offset_pair<T, NDIM, VOXELS>(p, b, d, h, wp);
 }
 
 template <int NDIM>
-inline int launch_apply_offset(const OffsetParams& p, int dtype, cudaStream_t st) {
+inline int launch_apply_offset(OffsetParams p, int dtype, cudaStream_t st) {
   const long long per_sample = (long long)p.D * p.H * ((p.W + 1) / 2);
   if (per_sample == 0 || p.B == 0 || p.C == 0) return 0;
   const dim3 grid((unsigned)((per_sample + kOffsetThreads - 1) / kOffsetThreads), (unsigned)min(p.B, 65535));
-  const bool cubic = p.order == 3;
+  p.pair = make_pair_const(NDIM, p.D, p.H, p.W, dtype == 0 ? 4 : 2);
+  const bool voxels = p.order == 3 || !pair_taps_applicable(NDIM, p.D, p.H, p.W, (long long)p.D * p.H * p.W, dtype == 0 ? 4 : 2);
   if (dtype == 0) {
-    if (cubic) apply_offset_kernel<float, NDIM, true><<<grid, kOffsetThreads, 0, st>>>(p);
+    if (voxels) apply_offset_kernel<float, NDIM, true><<<grid, kOffsetThreads, 0, st>>>(p);
     else apply_offset_kernel<float, NDIM, false><<<grid, kOffsetThreads, 0, st>>>(p);
   } else {
-    if (cubic) apply_offset_kernel<__half, NDIM, true><<<grid, kOffsetThreads, 0, st>>>(p);
+    if (voxels) apply_offset_kernel<__half, NDIM, true><<<grid, kOffsetThreads, 0, st>>>(p);
     else apply_offset_kernel<__half, NDIM, false><<<grid, kOffsetThreads, 0, st>>>(p);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -8;

@@ -1,108 +1,166 @@
 // Dense 2D forward (one sample per output pixel: every 2D augmentation call): the 2D counterpart
-// of the 3D gather path.  A thread owns two w-adjacent pixels (the two lanes of half2
-// arithmetic), walks down a column of row blocks of its 32 x (16 * kP2Blocks) tile and applies
+// of the 3D gather path, for an image field, an integer label field, or both at once.  A thread owns two w-adjacent pixels
+// (the two lanes of half2 arithmetic), walks down a column of row blocks of its tile and applies
 // the taps and weights of a pixel pair to every channel; the roi is decoded once per CTA; stores
 // are 2-element vectors, consecutive along w within a warp row.  The arithmetic is the
 // reference's (medvision/csrc/cuda/roi_align_rotated_2d_cuda_kernel.cuh:15-90,
 // roi_align_2d_cuda_kernel.cuh:11-74, interpolation_helpers_2d.h), one rounded operation at a
 // time: only the x products of the rotation, which do not change down a column, are hoisted.
+//
+// Labels: affine_2d(labels.float(), rois, ..., order 0).int() on the integers, as mvr_label.cuh does it; the geometry is
+// float32 and is the image's own for a float image.
+//
+// Bound by the latency of position -> loads -> sum (issue slots half busy): two channels' loads are in flight per thread.
 #pragma once
-#include "mvr_stream3d.cuh"
+#include "mvr_label.cuh"
 
 namespace mvr {
 
-constexpr int kP2Blocks = 8;  // row blocks of kS3TileH rows per CTA
+// Label part of a call: same rois (in float32), same spatial sizes as the image.
+struct Plane2dLabel {
+  const void* in;      // (N, C, H, W) of IT
+  const float* rois;
+  int* out;            // (R, C, oh, ow)
+  int C, vec;
+};
 
-template <typename T, int ORDER>
-__global__ void __launch_bounds__(kS3Threads)
-resample_fwd_plane2d(const Params p, int tiles_w, int tiles_h, int vec_store) {
+template <typename T, int ORDER, typename IT, bool IMG, bool LAB>
+__global__ void __launch_bounds__(kS3Threads, 5)
+resample_fwd_plane2d(const Params p, const PairConst pc, const Plane2dLabel lab, int tiles_w, int tiles_h, int blocks, int vec_store) {
   typedef Ar<T> A;
   typedef P2<T> Q;
   typedef typename Q::V V;
+  constexpr bool kOwnLabelGeometry = LAB && (!IMG || sizeof(T) != 4);
   __shared__ RoiGeom<T> g_sh;
+  __shared__ RoiGeom<float> gl_sh;
   const int fm = kS3FloatPattern;
   long long cta = blockIdx.x;
   const int tw = (int)(cta % tiles_w); cta /= tiles_w;
   const int th = (int)(cta % tiles_h); cta /= tiles_h;
   const long long n = cta;
-  if (threadIdx.x == 0) {
-    const int osz[3] = {p.ow, p.oh, 1};
-    decode_roi<T>((const T*)p.rois, n, 2, p.kind, osz, p.spatial_scale, 1, p.aligned, fm, g_sh);
-  }
+  if (IMG && threadIdx.x < 32)
+    decode_roi_warp<T>((const T*)p.rois, n, 2, p.kind, p.ow, p.oh, 1, p.spatial_scale, p.aligned, fm, g_sh);
+  if (kOwnLabelGeometry && threadIdx.x >= 32 && threadIdx.x < 64)
+    decode_roi_warp<float>(lab.rois, n, 2, p.kind, p.ow, p.oh, 1, p.spatial_scale, p.aligned, fm, gl_sh);
   __syncthreads();
   const RoiGeom<T>& g = g_sh;
+  const int batch = IMG ? g_sh.batch : gl_sh.batch;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int pw0 = tw * kS3TileW + (warp & 1) * 16 + (lane & 7) * 2;
-  const int row0 = th * (kS3TileH * kP2Blocks) + (warp >> 1) * 4 + (lane >> 3);
+  const int row0 = th * (kS3TileH * blocks) + (warp >> 1) * 4 + (lane >> 3);
   if (pw0 >= p.ow || row0 >= p.oh) return;
   const bool has_b = (pw0 + 1 < p.ow);
-  const bool vec = vec_store && has_b;
+  const bool vec = vec_store && has_b, vec_l = LAB && lab.vec && has_b;
   const long long ovol = p.ovol, vol_e = p.vol;
-  T* out = (T*)p.out + n * p.C * ovol + pw0;
+  T* out = IMG ? (T*)p.out + n * p.C * ovol + pw0 : nullptr;
+  int* out_l = LAB ? lab.out + n * lab.C * ovol + pw0 : nullptr;
   const T zero = A::fi(0);
   const V zero2 = Q::dup(zero);
 
-  if (g.batch < 0 || g.batch >= p.N) {
+  if (batch < 0 || batch >= p.N) {
     if (p.status && threadIdx.x == 0 && tw == 0 && th == 0) atomicOr(p.status, STATUS_BAD_BATCH_INDEX);
-    for (int b = 0; b < kP2Blocks; ++b) {
+    for (int b = 0; b < blocks; ++b) {
       const int ph = row0 + b * kS3TileH;
       if (ph >= p.oh) break;
-      for (int c = 0; c < p.C; ++c) {
+      for (int c = 0; IMG && c < p.C; ++c) {
         T* o = out + c * ovol + (long long)ph * p.ow;
         o[0] = zero;
         if (has_b) o[1] = zero;
       }
+      for (int c = 0; LAB && c < lab.C; ++c) {
+        int* o = out_l + c * ovol + (long long)ph * p.ow;
+        o[0] = 0;
+        if (has_b) o[1] = 0;
+      }
     }
     return;
   }
-  const T* vol = (const T*)p.in + (long long)g.batch * p.C * vol_e;
+  const T* vol = IMG ? (const T*)p.in + (long long)batch * p.C * vol_e : nullptr;
+  const IT* vol_l = LAB ? (const IT*)lab.in + (long long)batch * lab.C * vol_e : nullptr;
   const bool rotated = (p.kind == KIND_ROTATED);
-  const T sub_x = lattice_sub<T>(g.bin[0], 0, 1), sub_y = lattice_sub<T>(g.bin[1], 0, 1);
-  const T xa = A::add(lattice_base<T>(g.start[0], pw0, g.bin[0], fm), sub_x);
-  const T xb = A::add(lattice_base<T>(g.start[0], has_b ? pw0 + 1 : pw0, g.bin[0], fm), sub_x);
-  const V x2 = Q::make(xa, xb);
-  const V cos2 = Q::dup(g.rot[0]), sin2 = Q::dup(g.rot[1]);
-  const V cx2 = Q::dup(g.centre[0]), cy2 = Q::dup(g.centre[1]);
-  const int W = p.W, H = p.H, C = p.C, oh = p.oh;
+  V x2 = zero2;
+  if (IMG) {
+    const T sub_x = lattice_sub<T>(g.bin[0], 0, 1);
+    x2 = Q::make(A::add(lattice_base<T>(g.start[0], pw0, g.bin[0], fm), sub_x),
+                 A::add(lattice_base<T>(g.start[0], has_b ? pw0 + 1 : pw0, g.bin[0], fm), sub_x));
+  }
+  Float2Lanes xl = {0.0f, 0.0f};
+  if (kOwnLabelGeometry) {
+    const float sub = lattice_sub<float>(gl_sh.bin[0], 0, 1);
+    xl.a = __fadd_rn(lattice_base<float>(gl_sh.start[0], pw0, gl_sh.bin[0], fm), sub);
+    xl.b = __fadd_rn(lattice_base<float>(gl_sh.start[0], has_b ? pw0 + 1 : pw0, gl_sh.bin[0], fm), sub);
+  }
+  const typename Q::M lanes = Q::make_mask(true, has_b);
+  const unsigned row_l = (unsigned)p.W, bias_l = kTapMagic * ((unsigned)p.W + 1u);
+  const int C = p.C, oh = p.oh;
   const long long row_step = (long long)kS3TileH * p.ow;
-  T* orow = out + (long long)row0 * p.ow;
+  long long row_o = (long long)row0 * p.ow;
 
 #pragma unroll 1
-  for (int b = 0, ph = row0; b < kP2Blocks && ph < oh; ++b, ph += kS3TileH, orow += row_step) {
-    const T y = A::add(lattice_base<T>(g.start[1], ph, g.bin[1], fm), sub_y);
-    V rx2, ry2;
-    if (rotated) {
-      // rx = (x*cos - y*sin) + cx ; ry = (x*sin + y*cos) + cy
-      rx2 = Q::add(Q::row_xy(cos2, x2, Q::dup(A::neg(A::mul(y, g.rot[1])))), cx2);
-      ry2 = Q::add(Q::row_xy(sin2, x2, Q::dup(A::mul(y, g.rot[0]))), cy2);
-    } else {
-      rx2 = x2;
-      ry2 = Q::dup(y);
+  for (int b = 0, ph = row0; b < blocks && ph < oh; ++b, ph += kS3TileH, row_o += row_step) {
+    V rx2 = zero2, ry2 = zero2;
+    if (IMG) {
+      const T y = A::add(lattice_base<T>(g.start[1], ph, g.bin[1], fm), lattice_sub<T>(g.bin[1], 0, 1));
+      if (rotated) {
+        // rx = (x*cos - y*sin) + cx ; ry = (x*sin + y*cos) + cy
+        rx2 = Q::add(Q::row_xy(Q::dup(g.rot[0]), x2, Q::dup(A::neg(A::mul(y, g.rot[1])))), Q::dup(g.centre[0]));
+        ry2 = Q::add(Q::row_xy(Q::dup(g.rot[1]), x2, Q::dup(A::mul(y, g.rot[0]))), Q::dup(g.centre[1]));
+      } else {
+        rx2 = x2;
+        ry2 = Q::dup(y);
+      }
     }
+    if (LAB) {
+      float rx[2], ry[2];
+      if (kOwnLabelGeometry) {
+        const float y = __fadd_rn(lattice_base<float>(gl_sh.start[1], ph, gl_sh.bin[1], fm), lattice_sub<float>(gl_sh.bin[1], 0, 1));
+        const float c = gl_sh.rot[0], s = gl_sh.rot[1], ys = -__fmul_rn(y, s), yc = __fmul_rn(y, c);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const float x = k ? xl.b : xl.a;
+          rx[k] = rotated ? __fadd_rn(__fmaf_rn(c, x, ys), gl_sh.centre[0]) : x;
+          ry[k] = rotated ? __fadd_rn(__fmaf_rn(s, x, yc), gl_sh.centre[1]) : y;
+        }
+      } else {
+        rx[0] = A::tof(Q::lo(rx2)); rx[1] = A::tof(Q::hi(rx2));
+        ry[0] = A::tof(Q::lo(ry2)); ry[1] = A::tof(Q::hi(ry2));
+      }
+      bool in[2] = {true, has_b};
+      unsigned at[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        at[k] = label_pick(ry[k], pc.size[1], pc.last[1], in[k]) * row_l + label_pick(rx[k], pc.size[0], pc.last[0], in[k]) - bias_l;
+      const IT* v = vol_l;
+      int* o = out_l + row_o;
+      for (int c = 0; c < lab.C; ++c, v += vol_e, o += ovol) {
+        const int va = in[0] ? label_value<IT>(v + at[0]) : 0, vb = in[1] ? label_value<IT>(v + at[1]) : 0;
+        if (vec_l) {
+          *reinterpret_cast<int2*>(o) = make_int2(va, vb);
+        } else {
+          o[0] = va;
+          if (has_b) o[1] = vb;
+        }
+      }
+    }
+    if (!IMG) continue;
     AxisTap2<T> tx, ty;
-    axis_tap2<T>(rx2, W, ORDER, tx);
-    axis_tap2<T>(ry2, H, ORDER, ty);
-    const bool ina = !(tx.outa || ty.outa), inb = has_b && !(tx.outb || ty.outb);
-    // 32-bit offsets of the four taps of either pixel inside a channel's plane
-    const int a0 = ty.i0a * W + tx.i0a, b0 = ty.i0b * W + tx.i0b;
-    const int a1 = a0 + tx.da, b1 = b0 + tx.db;
-    const int a2 = a0 + (ty.da ? W : 0), b2 = b0 + (ty.db ? W : 0);
-    const int a3 = a2 + tx.da, b3 = b2 + tx.db;
-    const V w0 = Q::mul(ty.h, tx.h), w1 = Q::mul(ty.h, tx.l), w2 = Q::mul(ty.l, tx.h), w3 = Q::mul(ty.l, tx.l);
-    const typename Q::M mask = Q::make_mask(ina, inb);
+    axis_tap2<T, 0>(rx2, pc, ORDER, tx);
+    axis_tap2<T, 1>(ry2, pc, ORDER, ty);
+    const typename Q::M mask = lanes & ~(Q::outside(rx2, pc, 0) | Q::outside(ry2, pc, 1));
+    const PairTaps<T, 2> taps(tx, ty, ty, pc);
+    V w[4];
+    pair_weights<T, 2>(tx, ty, ty, w);
     const T* plane = vol;
-    T* o = orow;
-#pragma unroll 1
+    T* o = out + row_o;
+#pragma unroll 2
     for (int c = 0; c < C; ++c, plane += vol_e, o += ovol) {
-      const V v0 = Q::make(__ldg(plane + a0), __ldg(plane + b0));
-      const V v1 = Q::make(__ldg(plane + a1), __ldg(plane + b1));
-      const V v2 = Q::make(__ldg(plane + a2), __ldg(plane + b2));
-      const V v3 = Q::make(__ldg(plane + a3), __ldg(plane + b3));
-      V acc = Q::tap_first(w0, v0, w1, v1);
-      acc = Q::tap_next(acc, w2, v2);
-      acc = Q::tap_next(acc, w3, v3);
-      // output_val = 0 + val (normalises -0), then / count with count == 1
-      const V val = Q::apply(Q::add(zero2, acc), mask);
+      V val = zero2;
+      if (mask) {
+        V v[4];
+        taps.load(plane, pc, v);
+        // output_val = 0 + val (normalises -0), then / count with count == 1
+        val = Q::apply(Q::add(zero2, pair_sum<T, 4>(w, v)), mask);
+      }
       if (vec) {
         Q::store2(o, val);
       } else {
@@ -113,28 +171,51 @@ resample_fwd_plane2d(const Params p, int tiles_w, int tiles_h, int vec_store) {
   }
 }
 
-// 0 launched, 1 not applicable
-inline int try_launch_plane2d(const Params& p, int dtype, cudaStream_t st) {
+// An image (`p`, orders 0 and 1; null input: none), labels (`lab`; null input: none), or both.  0 launched, 1 not applicable.
+inline int try_launch_plane2d(const Params& p, int dtype, cudaStream_t st, const Plane2dLabel* label = nullptr, int label_dtype = 0) {
   if (p.ndim != 2 || p.sampling_ratio != 1 || p.order > 1) return 1;
   if (dtype != 0 && dtype != 1) return 1;
-  if (dtype == 0 && p.fm != kS3FloatPattern) return 1;
+  if ((dtype == 0 || label) && p.fm != kS3FloatPattern) return 1;
   if (p.ovol < 4096 || p.ow < 8) return 1;
-  if (p.vol >= 0x7fffffffLL) return 1;                       // 32-bit offsets inside a plane
-  if (dtype == 1 && (p.H > 2048 || p.W > 2048)) return 1;    // sizes as half values
-  const int tiles_w = (p.ow + kS3TileW - 1) / kS3TileW;
-  const int tiles_h = (p.oh + kS3TileH * kP2Blocks - 1) / (kS3TileH * kP2Blocks);
+  const size_t esz = dtype == 0 ? 4 : 2;
+  if (!pair_taps_applicable(2, 1, p.H, p.W, p.vol, esz) || p.vol >= 0x7fffffffLL) return 1;
+  const int tiles_w = (p.ow + kS3TileW - 1) / kS3TileW, row_blocks = (p.oh + kS3TileH - 1) / kS3TileH;
+  // a CTA's set-up costs about two row blocks; five CTAs per SM
+  const int blocks = s3_pick_chunk((long long)p.R * tiles_w, std::min(row_blocks, 4096), 148 * 5, 2);
+  const int tiles_h = (row_blocks + blocks - 1) / blocks;
   const long long ctas = (long long)p.R * tiles_w * tiles_h;
   if (ctas > 0x7fffffffLL) return 1;
-  const size_t esz = dtype == 0 ? 4 : 2;
   const int vec_store = ((p.ow & 1) == 0) && (((uintptr_t)p.out) % (2 * esz) == 0);
   const unsigned grid = (unsigned)ctas;
-  if (dtype == 0) {
-    if (p.order == 0) resample_fwd_plane2d<float, 0><<<grid, kS3Threads, 0, st>>>(p, tiles_w, tiles_h, vec_store);
-    else resample_fwd_plane2d<float, 1><<<grid, kS3Threads, 0, st>>>(p, tiles_w, tiles_h, vec_store);
-  } else {
-    if (p.order == 0) resample_fwd_plane2d<__half, 0><<<grid, kS3Threads, 0, st>>>(p, tiles_w, tiles_h, vec_store);
-    else resample_fwd_plane2d<__half, 1><<<grid, kS3Threads, 0, st>>>(p, tiles_w, tiles_h, vec_store);
+  const PairConst pc = make_pair_const(2, 1, p.H, p.W, esz);
+  Plane2dLabel lab = {};
+  if (label) lab = *label;
+#define MVR_PLANE(T, ORDER, IT, IMG, LAB) \
+  resample_fwd_plane2d<T, ORDER, IT, IMG, LAB><<<grid, kS3Threads, 0, st>>>(p, pc, lab, tiles_w, tiles_h, blocks, vec_store)
+#define MVR_PLANE_IT(T, ORDER, IMG)                                        \
+  switch (label_dtype) {                                                   \
+    case LABEL_U8: MVR_PLANE(T, ORDER, unsigned char, IMG, true); break;   \
+    case LABEL_I16: MVR_PLANE(T, ORDER, short, IMG, true); break;          \
+    case LABEL_I32: MVR_PLANE(T, ORDER, int, IMG, true); break;            \
+    default: MVR_PLANE(T, ORDER, long long, IMG, true); break;             \
   }
+  if (!p.in) {
+    MVR_PLANE_IT(float, 0, false)
+  } else if (label) {
+    if (dtype == 0) {
+      if (p.order == 0) MVR_PLANE_IT(float, 0, true) else MVR_PLANE_IT(float, 1, true)
+    } else {
+      if (p.order == 0) MVR_PLANE_IT(__half, 0, true) else MVR_PLANE_IT(__half, 1, true)
+    }
+  } else if (dtype == 0) {
+    if (p.order == 0) MVR_PLANE(float, 0, int, true, false);
+    else MVR_PLANE(float, 1, int, true, false);
+  } else {
+    if (p.order == 0) MVR_PLANE(__half, 0, int, true, false);
+    else MVR_PLANE(__half, 1, int, true, false);
+  }
+#undef MVR_PLANE_IT
+#undef MVR_PLANE
   return 0;
 }
 

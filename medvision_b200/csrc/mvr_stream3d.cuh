@@ -28,6 +28,8 @@
 // Gathers go through L1/L2 (__ldg): neighbouring threads and consecutive depths hit the same
 // lines, and the per-thread register reuse above removes about half of the loads outright.
 #pragma once
+#include <algorithm>
+
 #include "mvr_generic.cuh"
 
 namespace mvr {
@@ -73,6 +75,36 @@ template <> struct P2<__half> {
     unsigned u = *reinterpret_cast<unsigned*>(&v) & m;
     return *reinterpret_cast<V*>(&u);
   }
+  __device__ __forceinline__ static bool lane_a(M m) { return (m & 0xffffu) != 0; }
+  __device__ __forceinline__ static bool lane_b(M m) { return (m >> 16) != 0; }
+  // lanes of m from w, the others from v
+  __device__ __forceinline__ static V blend(V v, V w, M m) {
+    const unsigned u = (*reinterpret_cast<unsigned*>(&v) & ~m) | (*reinterpret_cast<unsigned*>(&w) & m);
+    return *reinterpret_cast<const V*>(&u);
+  }
+  // lanes whose coordinate lies outside [-1, size]; a NaN does not.  A half is above `size` exactly when it is above the
+  // largest half value not above it, and below `size` exactly when it is below the smallest half value not below it.
+  template <typename K> __device__ __forceinline__ static M outside(V c, const K& k, int axis) {
+    return __hlt2_mask(c, __float2half2_rn(-1.0f)) | __hgt2_mask(c, *reinterpret_cast<const V*>(&k.size_floor2[axis]));
+  }
+  // lanes whose coordinate lies strictly inside (-1, size)
+  template <typename K> __device__ __forceinline__ static M strictly_inside(V c, const K& k, int axis) {
+    return __hgt2_mask(c, __float2half2_rn(-1.0f)) & __hlt2_mask(c, *reinterpret_cast<const V*>(&k.size_ceil2[axis]));
+  }
+  __device__ __forceinline__ static V from_floats(float a, float b) { return __floats2half2_rn(a, b); }
+  __device__ __forceinline__ static V sub(V a, V b) { return __hsub2_rn(a, b); }
+  // one-hot choice of an axis: prefer the lower index when h >= .5
+  __device__ __forceinline__ static void nearest(V& l, V& h) {
+    const __half2 half_ = __float2half2_rn(0.5f), one = __float2half2_rn(1.0f);
+    const unsigned hh = __hge2_mask(h, half_);
+    const unsigned ll = __hge2_mask(l, half_) & ~hh;
+    const unsigned ou = *reinterpret_cast<const unsigned*>(&one);
+    const unsigned hu = ou & hh, lu = ou & ll;
+    h = *reinterpret_cast<const __half2*>(&hu);
+    l = *reinterpret_cast<const __half2*>(&lu);
+  }
+  __device__ __forceinline__ static float lo_float(V v) { return __low2float(v); }
+  __device__ __forceinline__ static float hi_float(V v) { return __high2float(v); }
 };
 
 struct Float2Lanes { float a, b; };
@@ -101,6 +133,24 @@ template <> struct P2<float> {
   typedef unsigned M;
   __device__ __forceinline__ static M make_mask(bool keep_a, bool keep_b) { return (keep_a ? 1u : 0u) | (keep_b ? 2u : 0u); }
   __device__ __forceinline__ static V apply(V v, M m) { return make((m & 1u) ? v.a : 0.0f, (m & 2u) ? v.b : 0.0f); }
+  __device__ __forceinline__ static bool lane_a(M m) { return (m & 1u) != 0; }
+  __device__ __forceinline__ static bool lane_b(M m) { return (m & 2u) != 0; }
+  __device__ __forceinline__ static V blend(V v, V w, M m) { return make((m & 1u) ? w.a : v.a, (m & 2u) ? w.b : v.b); }
+  template <typename K> __device__ __forceinline__ static M outside(V c, const K& k, int axis) {
+    return make_mask(c.a < -1.0f || c.a > k.size[axis], c.b < -1.0f || c.b > k.size[axis]);
+  }
+  template <typename K> __device__ __forceinline__ static M strictly_inside(V c, const K& k, int axis) {
+    return make_mask(c.a > -1.0f && c.a < k.size[axis], c.b > -1.0f && c.b < k.size[axis]);
+  }
+  __device__ __forceinline__ static V from_floats(float a, float b) { return make(a, b); }
+  __device__ __forceinline__ static V sub(V a, V b) { return make(__fsub_rn(a.a, b.a), __fsub_rn(a.b, b.b)); }
+  __device__ __forceinline__ static void nearest(V& l, V& h) {
+    const bool ha = h.a >= 0.5f, hb = h.b >= 0.5f, la = l.a >= 0.5f, lb = l.b >= 0.5f;
+    h = make(ha ? 1.0f : 0.0f, hb ? 1.0f : 0.0f);
+    l = make(!ha && la ? 1.0f : 0.0f, !hb && lb ? 1.0f : 0.0f);
+  }
+  __device__ __forceinline__ static float lo_float(V v) { return v.a; }
+  __device__ __forceinline__ static float hi_float(V v) { return v.b; }
 };
 
 // per-axis (l, h) of one sample; order 0 replaces them by the one-hot choice that the
@@ -113,73 +163,155 @@ __device__ __forceinline__ void nearest_axis(T& l, T& h) {
   l = (!hh && ll) ? A::fi(1) : A::fi(0);
 }
 
-// One interpolation axis for the two voxels of a pair at once (same results as axis_tap /
-// axis_outside / nearest_axis applied to each lane; `size` must be at most 2048 for half so that
-// it is a half value).
+// ---- taps of the two voxels of a pair ------------------------------------------------------------------------------
+// Same taps, weights and sums as axis_tap / make_taps / tap_sum applied to each lane, arranged so that a pair costs few
+// instructions (these kernels are bound by instruction issue):
+//   * the truncation c -> i0 is one addition: for 0 <= c <= size - 1 < 2^22, c + 2^23 rounded towards zero carries i0 in
+//     its low mantissa bits (conversion instructions run at a sixteenth of the rate of an addition); the bias of the raw
+//     bits is part of the address constant;
+//   * the eight taps are read at FIXED distances from one address per lane: the lower tap of an axis is taken from
+//     [0, size - 2], and in the rare case that a coordinate sits on the last index (where the reference clamps the upper
+//     tap onto the lower one and the upper weight is 0) the values are put right afterwards, behind a branch;
+//   * everything that depends on the sizes only comes from the host, in the kernel's parameters.
+// Sizes of at least 2 on every axis; byte offsets inside a channel's volume below 2^32.
+constexpr unsigned kTapMagic = 0x4B000000u;   // bits of 2^23
+constexpr int kTapMaxSize = 1 << 22;
+
+struct PairConst {
+  float last[3];          // size - 1                                  (axis 0 = w, 1 = h, 2 = d)
+  unsigned base_max[3];   // kTapMagic + size - 2
+  float size[3];
+  unsigned size_floor2[3], size_ceil2[3];  // half2 of the largest half <= size and of the smallest half >= size
+  unsigned sy, sz, bias;  // byte strides, and -kTapMagic * (sx + sy + sz) modulo 2^32
+};
+inline PairConst make_pair_const(int ndim, int D, int H, int W, size_t esz) {
+  PairConst k;
+  const int size[3] = {W, H, D};
+  for (int a = 0; a < 3; ++a) {
+    k.last[a] = (float)(size[a] - 1);
+    k.base_max[a] = kTapMagic + (unsigned)(size[a] - 2);
+    k.size[a] = (float)size[a];
+    const unsigned lo = __half_as_ushort(__float2half_rd(k.size[a])), hi = __half_as_ushort(__float2half_ru(k.size[a]));
+    k.size_floor2[a] = lo | (lo << 16);
+    k.size_ceil2[a] = hi | (hi << 16);
+  }
+  k.sy = (unsigned)((size_t)W * esz);
+  k.sz = ndim == 3 ? (unsigned)((size_t)H * W * esz) : 0u;
+  k.bias = 0u - kTapMagic * ((unsigned)esz + k.sy + k.sz);
+  return k;
+}
+inline bool pair_taps_applicable(int ndim, int D, int H, int W, long long vol, size_t esz) {
+  return D <= kTapMaxSize && H <= kTapMaxSize && W <= kTapMaxSize && H >= 2 && W >= 2 && (ndim == 2 || D >= 2) &&
+         (unsigned long long)vol * esz <= 0xffffffffull;
+}
+
 template <typename T>
 struct AxisTap2 {
-  int i0a, i0b;        // lower tap index per lane
-  int da, db;          // 1 when the upper tap is i0 + 1, 0 when it is clamped onto i0
+  unsigned ra, rb;             // kTapMagic + index of the lower of the two taps read, per lane
+  bool ca, cb;                 // coordinate on the last index: both taps are the upper one
   typename P2<T>::V l, h;
-  bool outa, outb;     // coordinate outside [-1, size]: the sample contributes nothing
 };
 
-template <typename T>
-__device__ __forceinline__ void axis_tap2(typename P2<T>::V c, int size, int order, AxisTap2<T>& t);
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float min_nan(float a, float b) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
 
-template <>
-__device__ __forceinline__ void axis_tap2<__half>(__half2 c, int size, int order, AxisTap2<__half>& t) {
-  const __half2 zero = __float2half2_rn(0.0f), one = __float2half2_rn(1.0f);
-  const unsigned out = __hlt2_mask(c, __float2half2_rn(-1.0f)) | __hgt2_mask(c, __float2half2_rn((float)size));
-  t.outa = (out & 0xffffu) != 0;
-  t.outb = (out >> 16) != 0;
-  // `if (c <= 0) c = 0`: a NaN stays a NaN
-  c = __hmax2_nan(c, zero);
-  int ia = __half2int_rz(__low2half(c)), ib = __half2int_rz(__high2half(c));
-  const bool ca = ia >= size - 1, cb = ib >= size - 1;  // upper neighbour clamped onto the last index
-  ia = ca ? size - 1 : ia;
-  ib = cb ? size - 1 : ib;
-  t.i0a = ia; t.i0b = ib;
-  t.da = ca ? 0 : 1; t.db = cb ? 0 : 1;
-  // l = c - (T)i0: i0 = floor(c) for c >= 0; a clamped lane has c := (T)i0, hence l = +0
-  __half2 l = __hsub2_rn(c, h2floor(c));
-  const unsigned keep = (ca ? 0u : 0x0000ffffu) | (cb ? 0u : 0xffff0000u);
-  unsigned lu = *reinterpret_cast<unsigned*>(&l) & keep;
-  l = *reinterpret_cast<__half2*>(&lu);
-  __half2 h = __hsub2_rn(one, l);
-  if (order == 0) {  // one-hot choice per axis: prefer the lower index when h >= .5
-    const __half2 half_ = __float2half2_rn(0.5f);
-    const unsigned hh = __hge2_mask(h, half_);
-    const unsigned ll = __hge2_mask(l, half_) & ~hh;
-    unsigned ou = *reinterpret_cast<const unsigned*>(&one);
-    unsigned hu = ou & hh, l2 = ou & ll;
-    h = *reinterpret_cast<__half2*>(&hu);
-    l = *reinterpret_cast<__half2*>(&l2);
+// A NaN coordinate keeps a NaN weight and a valid index.
+template <typename T, int AXIS>
+__device__ __forceinline__ void axis_tap2(typename P2<T>::V c, const PairConst& k, int order, AxisTap2<T>& t) {
+  typedef P2<T> Q;
+  typedef Ar<T> A;
+  const float magic = 8388608.0f;
+  // `if (c <= 0) c = 0`; at and beyond the last index: c = last, hence l = 0
+  const float fa = min_nan(max_nan(Q::lo_float(c), 0.0f), k.last[AXIS]), fb = min_nan(max_nan(Q::hi_float(c), 0.0f), k.last[AXIS]);
+  const float ma = __fadd_rz(fa, magic), mb = __fadd_rz(fb, magic);
+  t.ra = min(__float_as_uint(ma), k.base_max[AXIS]);
+  t.rb = min(__float_as_uint(mb), k.base_max[AXIS]);
+  t.ca = fa >= k.last[AXIS];
+  t.cb = fb >= k.last[AXIS];
+  // c - i0 is exact in the element type, so forming it in float and narrowing it changes nothing
+  t.l = Q::from_floats(__fsub_rn(fa, __fsub_rn(ma, magic)), __fsub_rn(fb, __fsub_rn(mb, magic)));
+  t.h = Q::sub(Q::dup(A::fi(1)), t.l);
+  if (order == 0) Q::nearest(t.l, t.h);
+}
+
+// The 2^NDIM tap values of both lanes from one channel's volume, in the reference's tap order.
+template <typename T, int NDIM>
+struct PairTaps {
+  typedef typename P2<T>::V V;
+  unsigned a, b;               // byte offsets of the lowest taps
+  bool ca[3], cb[3], any;
+  __device__ __forceinline__ PairTaps(const AxisTap2<T>& tx, const AxisTap2<T>& ty, const AxisTap2<T>& tz, const PairConst& k) {
+    a = tx.ra * (unsigned)sizeof(T) + (ty.ra * k.sy + k.bias);
+    b = tx.rb * (unsigned)sizeof(T) + (ty.rb * k.sy + k.bias);
+    ca[0] = tx.ca; cb[0] = tx.cb;
+    ca[1] = ty.ca; cb[1] = ty.cb;
+    any = tx.ca || tx.cb || ty.ca || ty.cb;
+    if (NDIM == 3) {
+      a += tz.ra * k.sz;
+      b += tz.rb * k.sz;
+      ca[2] = tz.ca; cb[2] = tz.cb;
+      any = any || tz.ca || tz.cb;
+    }
   }
-  t.l = l;
-  t.h = h;
-}
+  __device__ __forceinline__ void load(const T* vol, const PairConst& k, V* v) const {
+    typedef P2<T> Q;
+    const char* pa = reinterpret_cast<const char*>(vol) + a;
+    const char* pb = reinterpret_cast<const char*>(vol) + b;
+#pragma unroll
+    for (int r = 0; r < (NDIM == 3 ? 4 : 2); ++r) {
+      const size_t step = (r & 1 ? k.sy : 0u) + (size_t)(r & 2 ? k.sz : 0u);
+      const T* ra = reinterpret_cast<const T*>(pa + step);
+      const T* rb = reinterpret_cast<const T*>(pb + step);
+      v[2 * r] = Q::make(__ldg(ra), __ldg(rb));
+      v[2 * r + 1] = Q::make(__ldg(ra + 1), __ldg(rb + 1));
+    }
+    if (any) {
+#pragma unroll
+      for (int ax = 0; ax < NDIM; ++ax) {
+        const typename Q::M m = Q::make_mask(ca[ax], cb[ax]);
+#pragma unroll
+        for (int t = 0; t < (1 << NDIM); ++t)
+          if (!((t >> ax) & 1)) v[t] = Q::blend(v[t], v[t | (1 << ax)], m);
+      }
+    }
+  }
+};
 
-template <>
-__device__ __forceinline__ void axis_tap2<float>(Float2Lanes c, int size, int order, AxisTap2<float>& t) {
-  AxisTap<float> a, b;
-  t.outa = axis_outside<float>(c.a, size);
-  t.outb = axis_outside<float>(c.b, size);
-  axis_tap<float>(c.a, size, a);
-  axis_tap<float>(c.b, size, b);
-  if (order == 0) { nearest_axis<float>(a.l, a.h); nearest_axis<float>(b.l, b.h); }
-  t.i0a = a.i0; t.i0b = b.i0;
-  t.da = a.i1 - a.i0; t.db = b.i1 - b.i0;
-  t.l = P2<float>::make(a.l, b.l);
-  t.h = P2<float>::make(a.h, b.h);
+// the products of the axis weights, in tap order
+template <typename T, int NDIM>
+__device__ __forceinline__ void pair_weights(const AxisTap2<T>& tx, const AxisTap2<T>& ty, const AxisTap2<T>& tz, typename P2<T>::V* w) {
+  typedef P2<T> Q;
+  typedef typename Q::V V;
+  if (NDIM == 3) {
+    const V hzhy = Q::mul(tz.h, ty.h), hzly = Q::mul(tz.h, ty.l);
+    const V lzhy = Q::mul(tz.l, ty.h), lzly = Q::mul(tz.l, ty.l);
+    w[0] = Q::mul(hzhy, tx.h); w[1] = Q::mul(hzhy, tx.l); w[2] = Q::mul(hzly, tx.h); w[3] = Q::mul(hzly, tx.l);
+    w[4] = Q::mul(lzhy, tx.h); w[5] = Q::mul(lzhy, tx.l); w[6] = Q::mul(lzly, tx.h); w[7] = Q::mul(lzly, tx.l);
+  } else {
+    w[0] = Q::mul(ty.h, tx.h); w[1] = Q::mul(ty.h, tx.l); w[2] = Q::mul(ty.l, tx.h); w[3] = Q::mul(ty.l, tx.l);
+  }
+}
+// the reference's tap sum, left to right
+template <typename T, int NT>
+__device__ __forceinline__ typename P2<T>::V pair_sum(const typename P2<T>::V* w, const typename P2<T>::V* v) {
+  typename P2<T>::V acc = P2<T>::tap_first(w[0], v[0], w[1], v[1]);
+#pragma unroll
+  for (int k = 2; k < NT; ++k) acc = P2<T>::tap_next(acc, w[k], v[k]);
+  return acc;
 }
 
 template <typename T>
-struct S3ZTap {        // z-separable: per output depth
-  long long o0, o1;    // element offsets of the two source planes inside the volume
+struct __align__(16) S3ZTap {  // z-separable: per output depth
   T l, h;
-  int inside;
-  int z0, z1;          // the two source planes' indices
+  int z0, z1;                  // the two source planes' indices; z0 = -1: the depth lies outside
 };
 template <typename T>
 struct S3ZProd {       // general rotation: per output depth, the rounded products R_i3 * z
@@ -200,6 +332,7 @@ struct S3Launch {
   int tiles_w, tiles_h, chunks, chunk;  // chunk = output depths per CTA
   int vec_store;                        // 1: two-element vector stores are aligned
   int filter;                           // 0: every roi; 1: only rois that turn about z at most; 2: only the others
+  PairConst pair;                       // gather kernels: constants of the pair taps
   // plane-streaming kernel only: limits of its bounded waits, and the self-test's left-out plane (-1: none)
   int skip_plane = -1;
   unsigned wait_tries = 1u << 20;       // tries of a bounded wait on a ring slot's barrier (each may be suspended by the hardware)
@@ -210,7 +343,7 @@ struct S3Launch {
 // the x- and y-products of the rotation are formed once per thread, the z-products once per
 // depth and CTA (S3ZProd table).  Both lanes of a pair go through the same instructions.
 template <typename T, int NP>
-__device__ __forceinline__ void s3_full_depth_loop(const Params& p, const S3Shared<T>& sh, int npd, int c,
+__device__ __forceinline__ void s3_full_depth_loop(const Params& p, const S3Launch& L, const S3Shared<T>& sh, int npd, int c,
                                                    int pw0, int ph0, int row_step, bool vec_store, T* out0) {
   typedef Ar<T> A;
   typedef P2<T> Q;
@@ -236,7 +369,8 @@ __device__ __forceinline__ void s3_full_depth_loop(const Params& p, const S3Shar
       sxy[q][r] = Q::row_xy(Q::dup(g.rot[3 * r]), x2, Q::dup(A::mul(g.rot[3 * r + 1], y)));
   }
   const V c2[3] = {Q::dup(g.centre[0]), Q::dup(g.centre[1]), Q::dup(g.centre[2])};
-  const int W = p.W, HW = p.H * p.W;
+  const PairConst& pc = L.pair;
+  const typename Q::M lanes = Q::make_mask(true, has_b);
   const long long plane_o = (long long)p.oh * p.ow;
   const long long sub_o = (long long)row_step * p.ow;
   T* o = out0;
@@ -249,38 +383,17 @@ __device__ __forceinline__ void s3_full_depth_loop(const Params& p, const S3Shar
       const V ry2 = Q::add(Q::add(sxy[q][1], Q::dup(e.p[1])), c2[1]);
       const V rz2 = Q::add(Q::add(sxy[q][2], Q::dup(e.p[2])), c2[2]);
       AxisTap2<T> tx, ty, tz;
-      axis_tap2<T>(rx2, p.W, p.order, tx);
-      axis_tap2<T>(ry2, p.H, p.order, ty);
-      axis_tap2<T>(rz2, p.D, p.order, tz);
-      const bool ina = !(tx.outa || ty.outa || tz.outa);
-      const bool inb = has_b && !(tx.outb || ty.outb || tz.outb);
-      // element offsets of the eight taps inside the volume, per lane
-      const int ba = (tz.i0a * p.H + ty.i0a) * W + tx.i0a;
-      const int bb = (tz.i0b * p.H + ty.i0b) * W + tx.i0b;
-      const int dya = ty.da ? W : 0, dyb = ty.db ? W : 0, dza = tz.da ? HW : 0, dzb = tz.db ? HW : 0;
-      const T* pa = vol + (ina ? ba : 0);
-      const T* pb = vol + (inb ? bb : 0);
-      const int xa1 = ina ? tx.da : 0, xb1 = inb ? tx.db : 0;
-      const int ya1 = ina ? dya : 0, yb1 = inb ? dyb : 0, za1 = ina ? dza : 0, zb1 = inb ? dzb : 0;
-      V v[8];
-      v[0] = Q::make(__ldg(pa), __ldg(pb));
-      v[1] = Q::make(__ldg(pa + xa1), __ldg(pb + xb1));
-      v[2] = Q::make(__ldg(pa + ya1), __ldg(pb + yb1));
-      v[3] = Q::make(__ldg(pa + ya1 + xa1), __ldg(pb + yb1 + xb1));
-      v[4] = Q::make(__ldg(pa + za1), __ldg(pb + zb1));
-      v[5] = Q::make(__ldg(pa + za1 + xa1), __ldg(pb + zb1 + xb1));
-      v[6] = Q::make(__ldg(pa + za1 + ya1), __ldg(pb + zb1 + yb1));
-      v[7] = Q::make(__ldg(pa + za1 + ya1 + xa1), __ldg(pb + zb1 + yb1 + xb1));
-      const V hzhy = Q::mul(tz.h, ty.h), hzly = Q::mul(tz.h, ty.l);
-      const V lzhy = Q::mul(tz.l, ty.h), lzly = Q::mul(tz.l, ty.l);
-      V acc = Q::tap_first(Q::mul(hzhy, tx.h), v[0], Q::mul(hzhy, tx.l), v[1]);
-      acc = Q::tap_next(acc, Q::mul(hzly, tx.h), v[2]);
-      acc = Q::tap_next(acc, Q::mul(hzly, tx.l), v[3]);
-      acc = Q::tap_next(acc, Q::mul(lzhy, tx.h), v[4]);
-      acc = Q::tap_next(acc, Q::mul(lzhy, tx.l), v[5]);
-      acc = Q::tap_next(acc, Q::mul(lzly, tx.h), v[6]);
-      acc = Q::tap_next(acc, Q::mul(lzly, tx.l), v[7]);
-      const V val = Q::apply(Q::add(zero2, acc), Q::make_mask(ina, inb));
+      axis_tap2<T, 0>(rx2, pc, p.order, tx);
+      axis_tap2<T, 1>(ry2, pc, p.order, ty);
+      axis_tap2<T, 2>(rz2, pc, p.order, tz);
+      const typename Q::M mask = lanes & ~(Q::outside(rx2, pc, 0) | Q::outside(ry2, pc, 1) | Q::outside(rz2, pc, 2));
+      V val = zero2;
+      if (mask) {  // a lane outside keeps valid (clamped) addresses; its value is dropped
+        V v[8], w[8];
+        PairTaps<T, 3>(tx, ty, tz, pc).load(vol, pc, v);
+        pair_weights<T, 3>(tx, ty, tz, w);
+        val = Q::apply(Q::add(zero2, pair_sum<T, 8>(w, v)), mask);
+      }
       T* oq = o + q * sub_o;
       if (vec_store && has_b) {
         Q::store2(oq, val);
@@ -311,6 +424,25 @@ __device__ __forceinline__ S3Cta s3_cta(const Params& p, const S3Launch& L, long
 }
 __device__ __forceinline__ S3Cta s3_cta(const Params& p, const S3Launch& L) { return s3_cta(p, L, blockIdx.x); }
 
+// Output depths per CTA: a CTA's set-up costs as much as `setup` depths and `resident` CTAs run at a time, so the launch takes
+// about waves * (setup + chunk); the fewest-waves split with long chunks wins over many short ones except where a wave would
+// be nearly empty.
+inline int s3_pick_chunk(long long per_depth, int od, int resident, int setup) {
+  int best = std::min(od, kS3MaxChunk);
+  double best_cost = 1e300;
+  for (int chunks = (od + kS3MaxChunk - 1) / kS3MaxChunk; chunks <= od; ++chunks) {
+    const int chunk = (od + chunks - 1) / chunks;
+    const long long ctas = per_depth * ((od + chunk - 1) / chunk);
+    const double cost = (double)((ctas + resident - 1) / resident) * (setup + chunk);
+    if (cost < best_cost * 0.999) {
+      best_cost = cost;
+      best = chunk;
+    }
+    if (chunk <= 2) break;
+  }
+  return best;
+}
+
 // The forward runs as two launches when the rois may be rotated: rois that turn about z at most
 // stream whole source planes through shared memory and want few, long CTAs (their set-up costs
 // as much as five depths); rois under a general rotation gather through L1, are bound by load
@@ -329,38 +461,27 @@ __device__ __forceinline__ bool s3_filtered_out(const Params& p, const S3Launch&
 }
 
 // Decode the roi, classify it, and fill the per-depth table.  Ends with a __syncthreads().
-template <typename T>
+// GENERAL: every roi is treated as one under a general rotation (which is right for all of them).
+template <typename T, bool GENERAL = false>
 __device__ __forceinline__ void s3_prologue(const Params& p, const S3Cta& k, S3Shared<T>& sh) {
   typedef Ar<T> A;
   const long long n = k.n;
   const int pd0 = k.pd0, npd = k.npd;
   const int fm = kS3FloatPattern;
-  if (threadIdx.x == 0) {
-    const int osz[3] = {p.ow, p.oh, p.od};
-    decode_roi<T>((const T*)p.rois, n, 3, p.kind, osz, p.spatial_scale, 1, p.aligned, fm, sh.g);
+  if (threadIdx.x < 32) {
+    // the z-separable shortcut drops terms of the form 0*coordinate: every lattice coordinate must be finite
+    const bool finite = decode_roi_warp<T>((const T*)p.rois, n, 3, p.kind, p.ow, p.oh, p.od, p.spatial_scale, p.aligned, fm, sh.g);
     const RoiGeom<T>& g = sh.g;
-    int zsep = 1;
-    if (p.kind == KIND_ROTATED) {
-      const float one = 1.0f;
-      zsep = (A::tof(g.rot[2]) == 0.0f) && (A::tof(g.rot[5]) == 0.0f) && (A::tof(g.rot[6]) == 0.0f) &&
-             (A::tof(g.rot[7]) == 0.0f) && (A::tof(g.rot[8]) == one);
-    }
-    // the shortcut drops terms of the form 0*coordinate: every lattice coordinate must be finite
-    const int last[3] = {p.ow - 1, p.oh - 1, p.od - 1};
-    for (int a = 0; a < 3; ++a) {
-      const T sub = lattice_sub<T>(g.bin[a], 0, 1);
-      const T c0 = A::add(lattice_base<T>(g.start[a], 0, g.bin[a], fm), sub);
-      const T c1 = A::add(lattice_base<T>(g.start[a], last[a], g.bin[a], fm), sub);
-      zsep = zsep && A::finite(c0) && A::finite(c1) && A::finite(g.centre[a]);
-    }
-    sh.zsep = zsep;
+    const bool zsep = p.kind != KIND_ROTATED || (A::tof(g.rot[2]) == 0.0f && A::tof(g.rot[5]) == 0.0f && A::tof(g.rot[6]) == 0.0f &&
+                                                 A::tof(g.rot[7]) == 0.0f && A::tof(g.rot[8]) == 1.0f);
+    const bool all = __all_sync(0xffffffffu, finite && zsep);
+    if (threadIdx.x == 0) sh.zsep = all && !GENERAL;
   }
   __syncthreads();
   const RoiGeom<T>& g = sh.g;
-  const bool zsep = sh.zsep != 0;
+  const bool zsep = !GENERAL && sh.zsep != 0;
   const bool rotated = (p.kind == KIND_ROTATED);
   const bool bad_batch = (g.batch < 0 || g.batch >= p.N);
-  const long long HW = (long long)p.H * p.W;
 
   // ---- per-depth table
   if (!bad_batch && (int)threadIdx.x < npd) {
@@ -369,13 +490,10 @@ __device__ __forceinline__ void s3_prologue(const Params& p, const S3Cta& k, S3S
     if (zsep) {
       const T rz = rotated ? A::add(z, g.centre[2]) : z;
       S3ZTap<T> e;
-      e.inside = !axis_outside<T>(rz, p.D);
       AxisTap<T> t;
       axis_tap<T>(rz, p.D, t);
       if (p.order == 0) nearest_axis<T>(t.l, t.h);
-      e.o0 = t.i0 * HW;
-      e.o1 = t.i1 * HW;
-      e.z0 = t.i0;
+      e.z0 = axis_outside<T>(rz, p.D) ? -1 : t.i0;
       e.z1 = t.i1;
       e.l = t.l;
       e.h = t.h;
@@ -393,7 +511,7 @@ __device__ __forceinline__ void s3_prologue(const Params& p, const S3Cta& k, S3S
 }
 
 // Everything after the prologue, gathering through L1/L2 with plain loads.
-template <typename T>
+template <typename T, bool GENERAL = false>
 __device__ void s3_body_l1(const Params& p, const S3Launch& L, const S3Cta& k, S3Shared<T>& sh) {
   typedef Ar<T> A;
   typedef P2<T> Q;
@@ -402,7 +520,7 @@ __device__ void s3_body_l1(const Params& p, const S3Launch& L, const S3Cta& k, S
   const long long nc = k.nc;
   const int fm = kS3FloatPattern;
   const RoiGeom<T>& g = sh.g;
-  const bool zsep = sh.zsep != 0;
+  const bool zsep = !GENERAL && sh.zsep != 0;
   const bool rotated = (p.kind == KIND_ROTATED);
   const bool bad_batch = (g.batch < 0 || g.batch >= p.N);
   // ---- this thread's two output columns
@@ -443,54 +561,58 @@ __device__ void s3_body_l1(const Params& p, const S3Launch& L, const S3Cta& k, S
       rx2 = x2;
       ry2 = Q::dup(y);
     }
-    const T rx[2] = {Q::lo(rx2), Q::hi(rx2)}, ry[2] = {Q::lo(ry2), Q::hi(ry2)};
-    int o00[2], o01[2], o10[2], o11[2];
-    T lx[2], hx[2], ly[2], hy[2];
-    bool in[2];
-#pragma unroll
-    for (int v = 0; v < 2; ++v) {
-      in[v] = !(axis_outside<T>(ry[v], p.H) || axis_outside<T>(rx[v], p.W));
-      AxisTap<T> tx, ty;
-      axis_tap<T>(rx[v], p.W, tx);
-      axis_tap<T>(ry[v], p.H, ty);
-      if (p.order == 0) { nearest_axis<T>(tx.l, tx.h); nearest_axis<T>(ty.l, ty.h); }
-      o00[v] = ty.i0 * p.W + tx.i0;
-      o01[v] = ty.i0 * p.W + tx.i1;
-      o10[v] = ty.i1 * p.W + tx.i0;
-      o11[v] = ty.i1 * p.W + tx.i1;
-      lx[v] = tx.l; hx[v] = tx.h; ly[v] = ty.l; hy[v] = ty.h;
-    }
-    in[1] = in[1] && has_b;
-    const V lx2 = Q::make(lx[0], lx[1]), hx2 = Q::make(hx[0], hx[1]);
-    const V ly2 = Q::make(ly[0], ly[1]), hy2 = Q::make(hy[0], hy[1]);
+    AxisTap2<T> tx, ty;
+    axis_tap2<T, 0>(rx2, L.pair, p.order, tx);
+    axis_tap2<T, 1>(ry2, L.pair, p.order, ty);
+    const typename Q::M mask = Q::make_mask(true, has_b) & ~(Q::outside(rx2, L.pair, 0) | Q::outside(ry2, L.pair, 1));
+    // the pair's in-plane taps; the plane is added per depth (the z stride of the bias belongs to it)
+    PairTaps<T, 2> taps(tx, ty, ty, L.pair);
+    taps.a += kTapMagic * L.pair.sz;
+    taps.b += kTapMagic * L.pair.sz;
+    const V lx2 = tx.l, hx2 = tx.h, ly2 = ty.l, hy2 = ty.h;
 
-    V q0[4], q1[4];          // tap values of the two source planes, lanes = the two voxels
-    long long have1 = -1;    // plane offset whose values sit in q1
-    for (int i = 0; i < npd; ++i) {
-      const S3ZTap<T> e = sh.zt[i];
+    // Tap values of the depth's two source planes and, on its way while a depth is computed, of the plane the next depth adds
+    // (every test below is CTA-uniform); *_at: which plane a set holds.
+    V q0[4], q1[4], qn[4];
+    int at0 = -1, at1 = -1, atn = -1;
+    const int HW = p.H * p.W;
+    auto load = [&](V* q, int plane) { taps.load(vol + (long long)plane * HW, L.pair, q); };
+    auto prefetch = [&](const S3ZTap<T>& e) {
+      if (e.z0 >= 0 && e.z1 != at1 && e.z1 != atn) {
+        load(qn, e.z1);
+        atn = e.z1;
+      }
+    };
+    S3ZTap<T> next = sh.zt[0];
+    prefetch(next);
+    T* o = out;
+    for (int i = 0; i < npd; ++i, o += plane_o) {
+      const S3ZTap<T> e = next;
+      if (i + 1 < npd) next = sh.zt[i + 1];
       V val = zero2;
-      if (e.inside) {
-        if (e.o0 == have1) {
+      if (e.z0 >= 0) {
+        if (e.z0 != at0) {
+          if (e.z0 == at1) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) q0[k] = q1[k];
-        } else {
-          const T* pl = vol + e.o0;
-          q0[0] = Q::make(__ldg(pl + o00[0]), __ldg(pl + o00[1]));
-          q0[1] = Q::make(__ldg(pl + o01[0]), __ldg(pl + o01[1]));
-          q0[2] = Q::make(__ldg(pl + o10[0]), __ldg(pl + o10[1]));
-          q0[3] = Q::make(__ldg(pl + o11[0]), __ldg(pl + o11[1]));
+            for (int k = 0; k < 4; ++k) q0[k] = q1[k];
+          } else {
+            load(q0, e.z0);
+          }
+          at0 = e.z0;
         }
-        if (e.o1 == e.o0) {
+        if (e.z1 != at1) {
+          if (e.z1 == e.z0) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) q1[k] = q0[k];
-        } else {
-          const T* pl = vol + e.o1;
-          q1[0] = Q::make(__ldg(pl + o00[0]), __ldg(pl + o00[1]));
-          q1[1] = Q::make(__ldg(pl + o01[0]), __ldg(pl + o01[1]));
-          q1[2] = Q::make(__ldg(pl + o10[0]), __ldg(pl + o10[1]));
-          q1[3] = Q::make(__ldg(pl + o11[0]), __ldg(pl + o11[1]));
+            for (int k = 0; k < 4; ++k) q1[k] = q0[k];
+          } else if (e.z1 == atn) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) q1[k] = qn[k];
+          } else {
+            load(q1, e.z1);
+          }
+          at1 = e.z1;
         }
-        have1 = e.o1;
+        prefetch(next);
         const V hz2 = Q::dup(e.h), lz2 = Q::dup(e.l);
         const V hzhy = Q::mul(hz2, hy2), hzly = Q::mul(hz2, ly2);
         const V lzhy = Q::mul(lz2, hy2), lzly = Q::mul(lz2, ly2);
@@ -501,10 +623,11 @@ __device__ void s3_body_l1(const Params& p, const S3Launch& L, const S3Cta& k, S
         acc = Q::tap_next(acc, Q::mul(lzhy, lx2), q1[1]);
         acc = Q::tap_next(acc, Q::mul(lzly, hx2), q1[2]);
         acc = Q::tap_next(acc, Q::mul(lzly, lx2), q1[3]);
-        // output_val = 0 + val (normalises -0), then /count with count == 1
-        val = Q::select(Q::add(zero2, acc), in[0], in[1]);
+        // output_val = 0 + val (normalises -0), then / count with count == 1
+        val = Q::apply(Q::add(zero2, acc), mask);
+      } else {
+        prefetch(next);
       }
-      T* o = out + i * plane_o;
       if (vec) {
         Q::store2(o, val);
       } else {
@@ -516,17 +639,22 @@ __device__ void s3_body_l1(const Params& p, const S3Launch& L, const S3Cta& k, S
   }
 
   // ---- general rotation: positions change with depth
-  s3_full_depth_loop<T, 1>(p, sh, npd, c, pw0, ph, kS3TileH, L.vec_store != 0, out);
+  s3_full_depth_loop<T, 1>(p, L, sh, npd, c, pw0, ph, kS3TileH, L.vec_store != 0, out);
 }
 
+// The plane walk of the rows that no tensor map can describe (row pitch not a multiple of 16 bytes), and every roi of calls
+// with more rois than the gather launch can mark.  Like the plane-streaming kernel it may have been started before the gather
+// launch ahead of it is finished; one thread waits for that before the grid ends.
 template <typename T>
-__global__ void __launch_bounds__(kS3Threads)
+__global__ void __launch_bounds__(kS3Threads, sizeof(T) == 2 ? 4 : 3)
 resample_fwd_stream3d(const Params p, const S3Launch L) {
   __shared__ S3Shared<T> sh;
   const S3Cta k = s3_cta(p, L);
-  if (s3_filtered_out<T>(p, L, k)) return;
-  s3_prologue<T>(p, k, sh);
-  s3_body_l1<T>(p, L, k, sh);
+  if (!s3_filtered_out<T>(p, L, k)) {
+    s3_prologue<T>(p, k, sh);
+    s3_body_l1<T>(p, L, k, sh);
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // The second launch of a rotated forward: the rois under a general rotation, which the
@@ -536,7 +664,7 @@ resample_fwd_stream3d(const Params p, const S3Launch L) {
 // work items of the marked rois.
 constexpr int kS3RestMaxRois = 16384;
 template <typename T>
-__global__ void __launch_bounds__(kS3Threads)
+__global__ void __launch_bounds__(kS3Threads, 4)
 resample_fwd_stream3d_rest(const Params p, const S3Launch L, long long items) {
   __shared__ S3Shared<T> sh;
   __shared__ unsigned general[kS3RestMaxRois / 32];
@@ -555,8 +683,8 @@ resample_fwd_stream3d_rest(const Params p, const S3Launch L, long long items) {
   for (long long item = blockIdx.x; item < items; item += gridDim.x) {
     const S3Cta k = s3_cta(p, L, item);
     if (!((general[k.n >> 5] >> (k.n & 31)) & 1u)) continue;  // CTA-uniform
-    s3_prologue<T>(p, k, sh);
-    s3_body_l1<T>(p, L, k, sh);
+    s3_prologue<T, true>(p, k, sh);
+    s3_body_l1<T, true>(p, L, k, sh);
     __syncthreads();  // the next item's prologue overwrites the tables
   }
 }

@@ -288,9 +288,9 @@ __device__ __forceinline__ void t3_body(const Params& p, const S3Launch& L, cons
       const S3ZTap<T> e = sh.s3.zt[i];
       T3Ent<T> t;
       t.h = e.h; t.l = e.l; t.flags = 0;
-      if (e.inside) {
+      if (e.z0 >= 0) {
         adv = 2;
-        if (i > 0 && sh.s3.zt[i - 1].inside) {
+        if (i > 0 && sh.s3.zt[i - 1].z0 >= 0) {
           const int pz0 = sh.s3.zt[i - 1].z0, pz1 = sh.s3.zt[i - 1].z1;
           if (e.z0 == pz0 && e.z1 == pz1) adv = 0;
           else if (e.z0 == pz1) adv = 1;
@@ -564,8 +564,8 @@ inline int try_launch_stream3d(const Params& p, int dtype, cudaStream_t st, T3La
   if (dtype == 0 && p.fm != kS3FloatPattern) return MVR_STREAM3D_NOT_APPLICABLE;
   // small outputs (detection heads) are better served one element per thread
   if (p.ovol < 4096 || p.ow < 8) return MVR_STREAM3D_NOT_APPLICABLE;
-  if (p.vol >= 0x7fffffffLL) return MVR_STREAM3D_NOT_APPLICABLE;           // 32-bit offsets inside a volume
-  if (dtype == 1 && (p.D > 2048 || p.H > 2048 || p.W > 2048)) return MVR_STREAM3D_NOT_APPLICABLE;  // sizes as half values
+  // 32-bit byte offsets inside a volume (float volumes of 2^30 elements and more go to the flat kernel)
+  if (!pair_taps_applicable(3, p.D, p.H, p.W, p.vol, dtype == 0 ? 4 : 2)) return MVR_STREAM3D_NOT_APPLICABLE;
 
   T3Maps maps;
   const bool tma = t3_make_maps(p, dtype, maps);
@@ -588,31 +588,21 @@ inline int try_launch_stream3d(const Params& p, int dtype, cudaStream_t st, T3La
   G.chunks = (p.od + G.chunk - 1) / G.chunk;
   G.vec_store = ((p.ow & 1) == 0) && (((uintptr_t)p.out) % (2 * esz) == 0);
   G.filter = 0;
+  G.pair = make_pair_const(3, p.D, p.H, p.W, esz);
   const long long g_ctas = g_per_depth * G.chunks;
   if (g_ctas > 0x7fffffffLL) return MVR_STREAM3D_NOT_APPLICABLE;
-  if (!tma) {
-    if (dtype == 0) resample_fwd_stream3d<float><<<(unsigned)g_ctas, kS3Threads, 0, st>>>(p, G);
-    else resample_fwd_stream3d<__half><<<(unsigned)g_ctas, kS3Threads, 0, st>>>(p, G);
-    return cudaGetLastError() == cudaSuccess ? 0 : -8;
-  }
-
-  // ---- geometry of the plane-streaming kernel: 32 x 16*pairs tiles, long depth chunks.
-  // The set-up of a CTA costs about as much as five depths, so: the fewest chunks that still give
-  // every SM about five CTAs.  Measured on Resize 4 x (160,512,512) -> (128,256,256): 43 depths
-  // per CTA 83 us, 26: 84, 64: 87, 16: 91; on 96^3 crops one chunk of 96 beats two of 48 by 9 %.
+  // ---- geometry of the plane walk: 32 x 16*pairs tiles for the plane-streaming kernel, 32 x 16 without a tensor map; long
+  // depth chunks (s3_pick_chunk: measured on Resize 4 x (160,512,512) -> (128,256,256), 43 depths per CTA 83 us, 26: 84,
+  // 64: 87, 16: 91; on 96^3 crops one chunk of 96 beats two of 48 by 9 %).
+  const int rows_per_tile = kS3TileH * (tma ? pairs : 1);
   S3Launch L;
   L.tiles_w = G.tiles_w;
-  L.tiles_h = (p.oh + kS3TileH * pairs - 1) / (kS3TileH * pairs);
+  L.tiles_h = (p.oh + rows_per_tile - 1) / rows_per_tile;
   const long long per_depth_ctas = (long long)p.R * p.C * L.tiles_w * L.tiles_h;
-  {
-    long long want = (148LL * 5 + per_depth_ctas - 1) / per_depth_ctas;
-    want = std::max<long long>(want, (p.od + kS3MaxChunk - 1) / kS3MaxChunk);
-    want = std::min<long long>(want, std::max(1, p.od / 8));
-    int chunk = (int)((p.od + want - 1) / want);
-    L.chunk = chunk;
-  }
+  L.chunk = s3_pick_chunk(per_depth_ctas, p.od, 148 * (!tma && dtype == 1 ? 4 : 3), 6);
   L.chunks = (p.od + L.chunk - 1) / L.chunk;
   L.vec_store = G.vec_store;
+  L.pair = G.pair;
   const long long ctas = per_depth_ctas * L.chunks;
   if (ctas > 0x7fffffffLL) return MVR_STREAM3D_NOT_APPLICABLE;
   L.skip_plane = g_t3_selftest_skip_plane.load();
@@ -676,6 +666,11 @@ inline int try_launch_stream3d(const Params& p, int dtype, cudaStream_t st, T3La
   cfg.attrs = attr;
   cfg.numAttrs = overlap ? 1 : 0;
   cudaError_t err = cudaSuccess;
+  if (!tma) {
+    cfg.blockDim = dim3(kS3Threads);
+    err = dtype == 0 ? cudaLaunchKernelEx(&cfg, resample_fwd_stream3d<float>, p, L) : cudaLaunchKernelEx(&cfg, resample_fwd_stream3d<__half>, p, L);
+    return err == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -8;
+  }
   // more dynamic shared memory than the default limit: opt in (per function and device)
 #define T3_LAUNCH_V(TYPE, NP, VEC)                                                                           \
   {                                                                                                          \

@@ -253,17 +253,27 @@ at::Tensor label_forward(RoiOp op, const at::Tensor& labels, const at::Tensor& r
   return affine_forward(op, labels.to(at::kFloat), rois).to(at::kInt);
 }
 
-// An image field and its label field in one go (3D, one sample per voxel, orders 0 and 1).
-void fields_into(const RoiOp& op, const at::Tensor& image, const at::Tensor& image_rois, const at::Tensor& image_out,
+// An image field and its label field in one go (one sample per voxel, orders 0 and 1); false: rois too small for the label
+// kernels.
+bool fields_into(const RoiOp& op, const at::Tensor& image, const at::Tensor& image_rois, const at::Tensor& image_out,
                  const at::Tensor& labels, const at::Tensor& label_rois, const at::Tensor& label_out) {
   const int index = image.device().index();
   c10::cuda::CUDAGuard guard(image.device());
   void* stream = (void*)c10::cuda::getCurrentCUDAStream(index).stream();
-  check_rc(mvr_affine_fields_3d(image.data_ptr(), dtype_code(image.scalar_type()), image_rois.data_ptr(), image_out.data_ptr(),
-                                image.size(1), labels.data_ptr(), label_code(labels.scalar_type()),
-                                (const float*)label_rois.data_ptr(), (int32_t*)label_out.data_ptr(), labels.size(1), image.size(0),
-                                image.size(2), image.size(3), image.size(4), image_rois.size(0), 10, (int)op.out[0], (int)op.out[1],
-                                (int)op.out[2], op.scale, op.aligned, op.order, status_ptr(index), stream));
+  int* status = status_ptr(index);
+  const int code = dtype_code(image.scalar_type()), lcode = label_code(labels.scalar_type());
+  const int rc = op.ndim == 3
+      ? mvr_affine_fields_3d(image.data_ptr(), code, image_rois.data_ptr(), image_out.data_ptr(), image.size(1), labels.data_ptr(), lcode,
+                             (const float*)label_rois.data_ptr(), (int32_t*)label_out.data_ptr(), labels.size(1), image.size(0),
+                             image.size(2), image.size(3), image.size(4), image_rois.size(0), 10, (int)op.out[0], (int)op.out[1],
+                             (int)op.out[2], op.scale, op.aligned, op.order, status, stream)
+      : mvr_affine_fields_2d(image.data_ptr(), code, image_rois.data_ptr(), image_out.data_ptr(), image.size(1), labels.data_ptr(), lcode,
+                             (const float*)label_rois.data_ptr(), (int32_t*)label_out.data_ptr(), labels.size(1), image.size(0),
+                             image.size(2), image.size(3), image_rois.size(0), 6, (int)op.out[1], (int)op.out[2], op.scale,
+                             op.aligned, op.order, status, stream);
+  if (rc == MVR_ERR_UNSUPPORTED) return false;
+  check_rc(rc);
+  return true;
 }
 
 // ---- upload of a call's parameters ------------------------------------------------------------------
@@ -386,7 +396,7 @@ void resample_fields(RoiOp op, const Tensors& images, const Tensors& labels, con
   };
   const int64_t R = src.size(0);
   size_t fused = 0;
-  if (op.ndim == 3 && op.sampling == 1 && (op.order == 0 || op.order == 1)) {
+  if (op.sampling == 1 && (op.order == 0 || op.order == 1)) {
     // pairs of (image field, label field): one call each
     for (; fused < images.size() && fused < labels.size(); ++fused) {
       const at::Tensor &im = images[fused], &lb = labels[fused];
@@ -396,7 +406,7 @@ void resample_fields(RoiOp op, const Tensors& images, const Tensors& labels, con
       const at::Tensor i = im.contiguous(), l = lb.contiguous();
       at::Tensor io = at::empty(result_shape(op, R, i.size(1)), i.options().requires_grad(false));
       at::Tensor lo = at::empty(result_shape(op, R, l.size(1)), l.options().dtype(at::kInt));
-      fields_into(op, i, rois_for(i), io, l, staged.f32, lo);
+      if (!fields_into(op, i, rois_for(i), io, l, staged.f32, lo)) lo = label_forward(op, l, staged.f32);
       images_out.push_back(io);
       labels_out.push_back(lo);
     }
@@ -730,7 +740,8 @@ PyObject* py_fields_call(PyObject*, PyObject* const* a, Py_ssize_t n) {
     TORCH_CHECK(image_out.sizes() == at::IntArrayRef(result_shape(op, R, image.size(1))) &&
                     label_out.sizes() == at::IntArrayRef(result_shape(op, R, labels.size(1))) && image_out.is_contiguous() && label_out.is_contiguous(),
                 "affine_fields_3d: the results must be contiguous (R, C, *out_size) tensors");
-    fields_into(op, image.contiguous(), image_rois.contiguous(), image_out, labels.contiguous(), label_rois.contiguous(), label_out);
+    TORCH_CHECK(fields_into(op, image.contiguous(), image_rois.contiguous(), image_out, labels.contiguous(), label_rois.contiguous(), label_out),
+                mvr_strerror(MVR_ERR_UNSUPPORTED));
   }
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
