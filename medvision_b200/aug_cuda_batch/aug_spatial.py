@@ -32,15 +32,13 @@ def _resample_fields(result, dim, rois, out_size, sampling_ratio, order):
     result.update(zip(seg_keys, labels))
 
 
-def _affine_rois(index, center, shape, shifts, scales, rotate, dim):
-    """[index, center - shape * shifts / scales, shape / scales, angles] in float32; rotation about z in 3D."""
-    scales = scales.astype(np.float32)
-    rois = np.zeros((len(scales), 2 * dim + (2 if dim == 2 else 4)), dtype=np.float32)
-    rois[:, 0] = index
-    rois[:, 1:1 + dim] = center - shape * shifts.astype(np.float32) / scales
-    rois[:, 1 + dim:1 + 2 * dim] = shape / scales
-    rois[:, -1:] = rotate
-    return torch.from_numpy(rois)
+def _affine_rois(t, n_images, image_shape, start=None, end=None):
+    """[image, center - shape * shifts / scales, shape / scales, angles] of every sample of the transform ``t`` in float32
+    (rotation about z in 3D): over the whole image, or over the patches start..end (xyz)."""
+    p = [np.ascontiguousarray(t.params[k], dtype=np.float64) for k in ("scales", "shifts", "rotate")]
+    if start is not None:
+        start, end = (np.ascontiguousarray(v, dtype=np.int64) for v in (start, end))
+    return _C._native.affine_rois(len(p[0]), t.dim, n_images, *p, None if image_shape is None else tuple(image_shape), start, end)
 
 
 def _whole_image(image_shape):
@@ -136,9 +134,7 @@ class BatchCudaRandomAffine(BatchCudaAugBase):
             self.params = {"scales": 1 / params["scales"], "shifts": -params["shifts"], "rotate": -params["rotate"]}
 
     def _rois(self):
-        center, shape = _whole_image(self.image_shape)
-        return _affine_rois(np.arange(self.batch), center, shape, self.params["shifts"], self.params["scales"],
-                            self.params["rotate"], self.dim)
+        return _affine_rois(self, self.batch, self.image_shape)
 
     def apply_to_img(self, result: dict):
         _resample_fields(result, self.dim, self._rois(), self.image_shape, self.sampling_ratio, self.order)
@@ -286,15 +282,16 @@ class BatchCudaCropRandomWithAffine(BatchCudaAugBase):
 
     def _forward_crop_params(self, result: dict):
         # one draw per patch and axis (d, h, w), as _random_start() makes them
-        start = np.random.randint(0, np.tile(np.subtract(self.image_shape, self.patch_size) + 1, (self.batch, 1)))
-        return start[:, ::-1], (start + np.array(self.patch_size))[:, ::-1]
+        start = np.empty((self.batch, self.dim), dtype=np.int64)
+        end = np.empty_like(start)
+        generator = np.random.get_bit_generator()
+        with generator.lock:
+            _C._native.draw_starts(generator.capsule, self.batch, tuple(self.image_shape), tuple(self.patch_size), start, end)
+        return start, end
 
     def _rois(self):
-        start = self.params["start"].astype(np.float32)
-        end = self.params["end"].astype(np.float32)
         # patch r*B + b is cut from image b
-        return _affine_rois(np.arange(self.batch) % self.n_images, (start + end) / 2, end - start, self.params["shifts"],
-                            self.params["scales"], self.params["rotate"], self.dim)
+        return _affine_rois(self, self.n_images, None, self.params["start"], self.params["end"])
 
     def apply_to_img(self, result: dict):
         _resample_fields(result, self.dim, self._rois(), self.patch_size, self.sampling_ratio, self.order)

@@ -12,7 +12,6 @@ of the random draws are the interface a pipeline relies on; the bodies are this 
 * ``backward`` pops that log entry and, for a transform with ``canBackward``, applies the inverse
   parameters (``_backward_params``) through the same ``apply_to_*`` hooks.
 """
-import math
 import random
 import time
 from datetime import datetime
@@ -71,18 +70,16 @@ class BatchCudaAugBase(object):
         return bias + np.random.uniform(lo, hi)
 
     def _draw_affine(self, n):
-        """Scale, shifts and rotation (radians) of ``n`` samples: the values that :meth:`get_range` draws sample by sample
-        -- scale, one shift per axis, rotation -- from one array of uniform numbers (numpy's ``uniform(lo, hi)`` is
-        ``lo + (hi - lo) * random_sample()``, one number per draw).  Returns (n, dim), (n, dim) and (n, 1) arrays."""
+        """Scale, shifts and rotation (radians) of ``n`` samples -- (n, dim), (n, dim) and (n, 1) arrays: the values that
+        :meth:`get_range` draws sample by sample (scale, one shift per axis, rotation in degrees), drawn natively from numpy's
+        global generator."""
         dim = self.dim
-        u = np.random.random_sample((n, dim + 2))
-        lo, hi = self._bounds(self.scale)
-        scales = np.empty((n, dim))
-        scales[:] = 1 + (lo + (hi - lo) * u[:, :1])
-        lo, hi = self._bounds(self.shift)
-        shifts = 0 + (lo + (hi - lo) * u[:, 1:-1])
-        lo, hi = self._bounds(self.rotate)
-        return scales, shifts, math.pi * (0 + (lo + (hi - lo) * u[:, -1:])) / 180
+        scales, shifts, rotate = np.empty((n, dim)), np.empty((n, dim)), np.empty((n, 1))
+        generator = np.random.get_bit_generator()
+        with generator.lock:
+            _C._native.draw_affine(generator.capsule, n, dim, self._bounds(self.scale), self._bounds(self.shift),
+                                   self._bounds(self.rotate), scales, shifts, rotate)
+        return scales, shifts, rotate
 
     @staticmethod
     def to_tuple(value: Union[int, float, Iterable[int], Iterable[float]], length: int = 1) \
@@ -150,7 +147,8 @@ class BatchCudaAugBase(object):
         for key in _LOG_KEYS:
             result.setdefault(key, [])
         took = time.time() - self._tic_
-        began = datetime.fromtimestamp(self._tic_).strftime('%H:%M:%S.%f')
+        t = datetime.fromtimestamp(self._tic_)
+        began = f'{t.hour:02d}:{t.minute:02d}:{t.second:02d}.{t.microsecond:06d}'
         # the reference logs the allocator's peak divided by 1024 * 1024 * 8 under the label "MB"; kept as is
         peak = _C._native.peak_allocated() / (1024 * 1024 * 8) if torch.cuda.is_initialized() else 0.0
         result['history'].append(self.name)

@@ -33,12 +33,11 @@ class ElasticField:
         ``num_locked_borders`` control points of every axis zero."""
         grid = self.to_tuple(self.num_control_points, self.dim)
         reach = self.max_displacement * (np.array(self.image_shape) / (np.array(grid) - 1)) / 2
-        drawn = 2 * np.random.rand(*batch, *grid, self.dim).astype(np.float32) - 1  # [-1, 1)
-        drawn *= reach.astype(np.float32)
-        coarse = np.zeros_like(drawn)
-        n = self.num_locked_borders
-        inner = (Ellipsis,) + (slice(n, -n),) * self.dim + (slice(None),)
-        coarse[inner] = drawn[inner]
+        coarse = np.empty((*batch, *grid, self.dim), dtype=np.float32)
+        generator = np.random.get_bit_generator()
+        with generator.lock:  # 2 * rand(*grid, dim).astype(float32) - 1 per sample, in [-1, 1)
+            _C._native.draw_coarse(generator.capsule, batch[0] if batch else 1, grid, reach.astype(np.float32),
+                                   self.num_locked_borders, coarse)
         return coarse
 
     def _batched_params(self):

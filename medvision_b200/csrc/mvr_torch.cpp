@@ -7,6 +7,7 @@
 // took 18 us per forward, 98 us per forward + backward of a head and about 300 us per augmentation call.
 #include <Python.h>
 
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -155,6 +156,17 @@ at::Tensor roi_forward(const RoiOp& op, const at::Tensor& features, const at::Te
   return out;
 }
 
+// at::zeros without its tensor iterator: one memset on the current stream.
+at::Tensor zero_filled(at::IntArrayRef size, const at::TensorOptions& options) {
+  at::Tensor t = at::empty(size, options);
+  if (!t.is_cuda()) return t.zero_();
+  if (t.numel() > 0) {
+    c10::cuda::CUDAGuard guard(t.device());
+    C10_CUDA_CHECK(cudaMemsetAsync(t.data_ptr(), 0, t.nbytes(), c10::cuda::getCurrentCUDAStream(t.device().index()).stream()));
+  }
+  return t;
+}
+
 // Gradient of the features.  The roi kernels add into a zero-filled tensor.
 struct RoiBackward : public torch::autograd::Node {
   RoiOp op;
@@ -168,7 +180,7 @@ struct RoiBackward : public torch::autograd::Node {
     const at::Tensor r = rois.unpack();
     if (!task_should_compute_output(0)) return result;
     at::NoGradGuard no_grad;
-    at::Tensor gin = at::zeros(feature_size, options);
+    at::Tensor gin = zero_filled(feature_size, options);
     if (grads[0].defined()) {
       const at::Tensor g = grads[0].contiguous();
       check_roi_tensors(op, g, r, &gin);
@@ -504,6 +516,34 @@ bool elastic(const at::Tensor& coarse, int border, const std::vector<int64_t>& s
   return true;
 }
 
+// ---- parameter draws --------------------------------------------------------------------------------------
+// numpy's global generator, drawn from natively through the C interface that numpy documents for extensions (the capsule of
+// a BitGenerator).  The order and the arithmetic of the draws are numpy's: uniform(lo, hi) is lo + (hi - lo) * next_double,
+// randint(0, n) masks 32-bit numbers and rejects those above n - 1 (and draws nothing for n = 1).
+
+struct BitGen {
+  void* state;
+  uint64_t (*next_uint64)(void*);
+  uint32_t (*next_uint32)(void*);
+  double (*next_double)(void*);
+  uint64_t (*next_raw)(void*);
+};
+
+// A C-contiguous numpy array of 8-byte (double / int64) or 4-byte (float) items.
+struct Buffer {
+  Py_buffer view;
+  Buffer(PyObject* o, int itemsize, Py_ssize_t items, bool writable) {
+    if (PyObject_GetBuffer(o, &view, PyBUF_C_CONTIGUOUS | (writable ? PyBUF_WRITABLE : 0)) != 0) throw python_error();
+    if (view.itemsize != itemsize || view.len != items * itemsize) {
+      PyBuffer_Release(&view);
+      raise(PyExc_ValueError, "unexpected array size");
+    }
+  }
+  ~Buffer() { PyBuffer_Release(&view); }
+  Buffer(const Buffer&) = delete;
+  template <typename T> T* as() { return (T*)view.buf; }
+};
+
 // ---- Python bindings ----------------------------------------------------------------------------------
 
 const at::Tensor& tensor_arg(PyObject* o, const char* name) {
@@ -800,6 +840,142 @@ PyObject* py_resample_fields(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+BitGen* bitgen_arg(PyObject* capsule) {
+  BitGen* g = (BitGen*)PyCapsule_GetPointer(capsule, "BitGenerator");
+  if (!g) throw python_error();
+  return g;
+}
+
+// draw_affine(capsule, n, dim, (scale lo, hi), (shift lo, hi), (rotate lo, hi), scales, shifts, rotate): per sample scale, one
+// shift per axis, rotation in degrees; fills float64 arrays (n, dim), (n, dim), (n, 1)
+PyObject* py_draw_affine(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  HANDLE_TH_ERRORS
+  need(n_args, 9, 9);
+  BitGen* g = bitgen_arg(a[0]);
+  const Py_ssize_t n = int_arg(a[1]), dim = int_arg(a[2]);
+  double lo[3], span[3];
+  for (int k = 0; k < 3; ++k) {
+    lo[k] = float_arg(PyTuple_GET_ITEM(a[3 + k], 0));
+    span[k] = float_arg(PyTuple_GET_ITEM(a[3 + k], 1)) - lo[k];
+  }
+  Buffer scales(a[6], 8, n * dim, true), shifts(a[7], 8, n * dim, true), rotate(a[8], 8, n, true);
+  double *sc = scales.as<double>(), *sh = shifts.as<double>(), *ro = rotate.as<double>();
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    const double s = 1 + (lo[0] + span[0] * g->next_double(g->state));
+    for (Py_ssize_t d = 0; d < dim; ++d) sc[i * dim + d] = s;
+    for (Py_ssize_t d = 0; d < dim; ++d) sh[i * dim + d] = 0 + (lo[1] + span[1] * g->next_double(g->state));
+    ro[i] = 3.141592653589793 * (0 + (lo[2] + span[2] * g->next_double(g->state))) / 180;
+  }
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+// draw_starts(capsule, n, image_shape, patch_size, start, end): randint(0, image - patch + 1) per patch and axis (d, h, w);
+// fills int64 arrays (n, dim) in x, y, z order
+PyObject* py_draw_starts(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  HANDLE_TH_ERRORS
+  need(n_args, 6, 6);
+  BitGen* g = bitgen_arg(a[0]);
+  const Py_ssize_t n = int_arg(a[1]), dim = PyTuple_GET_SIZE(a[2]);
+  if (dim > 3 || PyTuple_GET_SIZE(a[3]) != dim) raise(PyExc_ValueError, "unexpected shape");
+  int64_t patch[3];
+  uint32_t range[3], mask[3];
+  for (Py_ssize_t d = 0; d < dim; ++d) {
+    patch[d] = int_arg(PyTuple_GET_ITEM(a[3], d));
+    const int64_t room = int_arg(PyTuple_GET_ITEM(a[2], d)) - patch[d];
+    if (room < 0 || room >= 0xffffffffll) raise(PyExc_ValueError, "low >= high");
+    range[d] = mask[d] = (uint32_t)room;
+    for (int s = 1; s < 32; s <<= 1) mask[d] |= mask[d] >> s;
+  }
+  Buffer start(a[4], 8, n * dim, true), end(a[5], 8, n * dim, true);
+  int64_t *st = start.as<int64_t>(), *en = end.as<int64_t>();
+  for (Py_ssize_t i = 0; i < n; ++i)
+    for (Py_ssize_t d = 0; d < dim; ++d) {
+      uint32_t v = 0;
+      if (range[d])
+        while ((v = g->next_uint32(g->state) & mask[d]) > range[d]) {}
+      st[i * dim + dim - 1 - d] = v;
+      en[i * dim + dim - 1 - d] = v + patch[d];
+    }
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+// draw_coarse(capsule, batch, grid, reach, border, out): 2 * float32(rand) - 1 times reach per component, the `border`
+// outermost points of every axis zero; fills a float32 array (batch, *grid, dim).  reach: float32 array (dim).
+PyObject* py_draw_coarse(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  HANDLE_TH_ERRORS
+  need(n_args, 6, 6);
+  BitGen* g = bitgen_arg(a[0]);
+  const Py_ssize_t batch = int_arg(a[1]), dim = PyTuple_GET_SIZE(a[2]);
+  const int border = (int)int_arg(a[4]);
+  if (dim != 2 && dim != 3) raise(PyExc_ValueError, "unexpected shape");
+  Py_ssize_t grid[3] = {1, 1, 1}, points = 1;
+  for (Py_ssize_t d = 0; d < dim; ++d) points *= grid[3 - dim + d] = int_arg(PyTuple_GET_ITEM(a[2], d));
+  Buffer reach(a[3], 4, dim, false), out(a[5], 4, batch * points * dim, true);
+  const float* r = reach.as<float>();
+  float* o = out.as<float>();
+  auto locked = [&](Py_ssize_t i, int axis) { return i < border || i >= grid[axis] - border; };
+  for (Py_ssize_t b = 0; b < batch; ++b)
+    for (Py_ssize_t z = 0; z < grid[0]; ++z)
+      for (Py_ssize_t y = 0; y < grid[1]; ++y) {
+        const bool row_locked = (dim == 3 && locked(z, 0)) || locked(y, 1);
+        for (Py_ssize_t x = 0; x < grid[2]; ++x) {
+          const bool lock = row_locked || locked(x, 2);
+          for (Py_ssize_t c = 0; c < dim; ++c) {
+            const float u = (float)g->next_double(g->state);
+            *o++ = lock ? 0.0f : (2 * u - 1) * r[c];
+          }
+        }
+      }
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+// affine_rois(n, dim, images, scales, shifts, rotate, image_shape | None, start | None, end | None) -> CPU float32 (n, K):
+// [i % images, center - shape * shifts / scales, shape / scales, angles], every step one float32 operation; centre and shape
+// are the whole image's or the patch's (start + end) / 2 and end - start
+PyObject* py_affine_rois(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  HANDLE_TH_ERRORS
+  need(n_args, 9, 9);
+  const Py_ssize_t n = int_arg(a[0]), dim = int_arg(a[1]), images = int_arg(a[2]);
+  if (dim != 2 && dim != 3) raise(PyExc_ValueError, "unexpected shape");
+  Buffer scales(a[3], 8, n * dim, false), shifts(a[4], 8, n * dim, false), rotate(a[5], 8, n, false);
+  const double *sc = scales.as<double>(), *sh = shifts.as<double>(), *ro = rotate.as<double>();
+  const bool whole = a[6] != Py_None;
+  float image[3] = {0, 0, 0};
+  if (whole)
+    for (Py_ssize_t d = 0; d < dim; ++d) image[d] = (float)int_arg(PyTuple_GET_ITEM(a[6], dim - 1 - d));
+  std::unique_ptr<Buffer> start, end;
+  if (!whole) {
+    start.reset(new Buffer(a[7], 8, n * dim, false));
+    end.reset(new Buffer(a[8], 8, n * dim, false));
+  }
+  const Py_ssize_t K = dim == 2 ? 6 : 10;
+  at::Tensor out = at::zeros({n, K}, at::kFloat);
+  float* o = (float*)out.data_ptr();
+  for (Py_ssize_t i = 0; i < n; ++i, o += K) {
+    o[0] = (float)(i % images);
+    for (Py_ssize_t d = 0; d < dim; ++d) {
+      float centre, shape;
+      if (whole) {
+        shape = image[d];
+        centre = shape / 2;
+      } else {
+        const float s = (float)start->as<int64_t>()[i * dim + d], e = (float)end->as<int64_t>()[i * dim + d];
+        centre = (s + e) / 2;
+        shape = e - s;
+      }
+      const float scale = (float)sc[i * dim + d], moved = shape * (float)sh[i * dim + d];
+      o[1 + d] = centre - moved / scale;
+      o[1 + dim + d] = shape / scale;
+    }
+    o[K - 1] = (float)ro[i];
+  }
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
 // apply_offset(input, offset, order)
 PyObject* py_apply_offset(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -902,6 +1078,10 @@ PyMethodDef methods[] = {
     {"label_call", FAST(py_label_call), nullptr},
     {"fields_call", FAST(py_fields_call), nullptr},
     {"resample_fields", FAST(py_resample_fields), nullptr},
+    {"draw_affine", FAST(py_draw_affine), nullptr},
+    {"draw_starts", FAST(py_draw_starts), nullptr},
+    {"draw_coarse", FAST(py_draw_coarse), nullptr},
+    {"affine_rois", FAST(py_affine_rois), nullptr},
     {"elastic", FAST(py_elastic), nullptr},
     {"apply_offset", FAST(py_apply_offset), nullptr},
     {"status_word", py_status_word, METH_O, nullptr},
