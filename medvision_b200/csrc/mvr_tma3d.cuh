@@ -49,14 +49,14 @@ struct T3Maps {
   int n;
 };
 
-// per output depth, for the consumers
+// per output depth, for the consumers: the z weights in both lanes of a pair
 template <typename T>
-struct __align__(8) T3Ent {
-  T h, l;               // z weights
+struct __align__(16) T3Ent {
+  typename P2<T>::V h, l;
   unsigned short adv;   // new planes to take from the ring before this depth (0, 1 or 2)
   unsigned short flags; // T3_INSIDE
 };
-enum { T3_INSIDE = 1 };
+enum { T3_INSIDE = 1, T3_PAIR = 2 };  // T3_PAIR: this depth and the next one are inside and take one new plane each
 
 template <typename T>
 struct T3Shared {
@@ -69,6 +69,8 @@ struct T3Shared {
   int box[4];                              // xmin, xmax, ymin, ymax over the tile's inside voxels
   volatile int abort_flag;
 };
+
+constexpr unsigned kT3EmptyOff = kT3MaxStages * 8;  // bytes from a slot's "full" to its "empty" barrier
 
 __device__ __forceinline__ unsigned t3_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
@@ -114,23 +116,21 @@ __device__ __forceinline__ void t3_tma_load_3d(unsigned dst, const CUtensorMap* 
       : "memory");
 }
 
-// Two elements from two 32-bit shared-memory addresses, as the two lanes of a pair.
-template <typename T>
-__device__ __forceinline__ typename P2<T>::V t3_lds_pair(unsigned addr_a, unsigned addr_b);
-template <>
-__device__ __forceinline__ __half2 t3_lds_pair<__half>(unsigned addr_a, unsigned addr_b) {
-  unsigned va, vb;
-  asm volatile("ld.shared.u16 %0, [%1];" : "=r"(va) : "r"(addr_a) : "memory");
-  asm volatile("ld.shared.u16 %0, [%1];" : "=r"(vb) : "r"(addr_b) : "memory");
-  const unsigned packed = __byte_perm(va, vb, 0x5410);
-  return *reinterpret_cast<const __half2*>(&packed);
-}
-template <>
-__device__ __forceinline__ Float2Lanes t3_lds_pair<float>(unsigned addr_a, unsigned addr_b) {
-  Float2Lanes v;
-  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v.a) : "r"(addr_a) : "memory");
-  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v.b) : "r"(addr_b) : "memory");
-  return v;
+// Two elements from two 32-bit shared-memory addresses (plus OFF bytes), as the two lanes of a pair.
+template <typename T, unsigned OFF>
+__device__ __forceinline__ typename P2<T>::V t3_lds_pair(unsigned addr_a, unsigned addr_b) {
+  if constexpr (sizeof(T) == 2) {
+    unsigned va, vb;
+    asm volatile("ld.shared.u16 %0, [%1+%2];" : "=r"(va) : "r"(addr_a), "n"(OFF) : "memory");
+    asm volatile("ld.shared.u16 %0, [%1+%2];" : "=r"(vb) : "r"(addr_b), "n"(OFF) : "memory");
+    const unsigned packed = __byte_perm(va, vb, 0x5410);
+    return *reinterpret_cast<const __half2*>(&packed);
+  } else {
+    Float2Lanes v;
+    asm volatile("ld.shared.f32 %0, [%1+%2];" : "=f"(v.a) : "r"(addr_a), "n"(OFF) : "memory");
+    asm volatile("ld.shared.f32 %0, [%1+%2];" : "=f"(v.b) : "r"(addr_b), "n"(OFF) : "memory");
+    return v;
+  }
 }
 
 // Bounded wait written as one PTX loop (no divergence bookkeeping around it): up to `tries` tries, each
@@ -156,14 +156,14 @@ __device__ __forceinline__ bool t3_mbar_wait_ptx(unsigned bar, unsigned parity, 
       : "memory");
   return ok != 0;
 }
-// lane 0 of the warp arrives; the others fall through (predicated, no branch)
-__device__ __forceinline__ void t3_mbar_arrive_lane0(unsigned bar, int lane) {
+// one lane of the (converged) warp arrives; the others fall through (predicated, no branch)
+__device__ __forceinline__ void t3_mbar_arrive_one(unsigned bar) {
   asm volatile(
       "{\n"
       "  .reg .pred p;\n"
-      "  setp.eq.s32 p, %1, 0;\n"
+      "  elect.sync _|p, 0xffffffff;\n"
       "  @p mbarrier.arrive.shared::cta.b64 _, [%0];\n"
-      "}\n" ::"r"(bar), "r"(lane)
+      "}\n" ::"r"(bar)
       : "memory");
 }
 
@@ -178,6 +178,120 @@ __device__ __forceinline__ void t3_fallback(const Params& p, const S3Launch& L, 
     k2.th = k.th * np + q;
     if (k2.th * kS3TileH < p.oh) s3_body_l1<T>(p, L, k2, sh);
   }
+}
+
+// The depth loop of a consumer warp.  BW: box width in elements.
+template <typename T, int NP, bool VEC, int BW>
+__device__ __forceinline__ void t3_consume(const Params& p, T3Shared<T>& sh, unsigned tries, int npd, bool any_inside, unsigned stride,
+                                           int nst, unsigned full_s, const unsigned* oa, const unsigned* ob,
+                                           const typename P2<T>::V* lx2, const typename P2<T>::V* hx2, const typename P2<T>::V* ly2,
+                                           const typename P2<T>::V* hy2, const typename P2<T>::M* mask, const bool* act, bool has_b,
+                                           T* o, long long plane_o) {
+  typedef Ar<T> A;
+  typedef P2<T> Q;
+  typedef typename Q::V V;
+  constexpr unsigned esz = sizeof(T), row = BW * sizeof(T);
+  const long long sub_o = (long long)kS3TileH * p.ow;  // output offset between a thread's pairs
+  const V zero2 = Q::dup(A::fi(0));
+  unsigned soff = 0;                      // byte offset of the current ring slot
+  unsigned fa = full_s;                   // its "full" mbarrier; the "empty" one lies kT3EmptyOff behind it
+  const unsigned ring_end = stride * nst;
+  unsigned par = 0;
+  // Tap values of the two planes held in registers (lanes = the two voxels): x0y0, x1y0, x0y1,
+  // x1y1.  Which of the two sets is the newest plane alternates with every fetch; `b_newest`
+  // tracks it, and the code below exists once per role assignment, so no register is ever moved.
+  V ra[NP][4], rb[NP][4];
+#pragma unroll
+  for (int q = 0; q < NP; ++q)
+#pragma unroll
+    for (int t = 0; t < 4; ++t) ra[q][t] = rb[q][t] = zero2;
+  bool b_newest = true;
+
+// take the next plane of the schedule out of the ring into register set R
+#define T3_FETCH(R)                                                                       \
+  {                                                                                       \
+    if (!t3_mbar_wait_ptx(fa, par, tries)) {                                              \
+      sh.abort_flag = 1;                                                                  \
+      if (p.status) atomicOr(p.status, STATUS_TMA_TIMEOUT);                               \
+      return; /* no barrier follows: leaving is safe, the producer drains its copies */   \
+    }                                                                                     \
+    _Pragma("unroll") for (int q = 0; q < NP; ++q) {                                      \
+      const unsigned ua = oa[q] + soff, ub = ob[q] + soff;                                \
+      R[q][0] = t3_lds_pair<T, 0>(ua, ub);                                                \
+      R[q][1] = t3_lds_pair<T, esz>(ua, ub);                                              \
+      R[q][2] = t3_lds_pair<T, row>(ua, ub);                                              \
+      R[q][3] = t3_lds_pair<T, row + esz>(ua, ub);                                        \
+    }                                                                                     \
+    __syncwarp();                                                                         \
+    t3_mbar_arrive_one(fa + kT3EmptyOff); /* this warp is done with the slot */           \
+    soff += stride; fa += 8u;                                                             \
+    if (soff == ring_end) { soff = 0; fa = full_s; par ^= 1u; }                           \
+  }
+
+// the reference's tap sum: older plane OLD supplies taps 1-4, newest plane NEW taps 5-8
+#define T3_COMPUTE(E, OLD, NEW)                                                           \
+  {                                                                                       \
+    const V hz2 = E.h, lz2 = E.l;                                                         \
+    _Pragma("unroll") for (int q = 0; q < NP; ++q) {                                      \
+      const V hzhy = Q::mul(hz2, hy2[q]), hzly = Q::mul(hz2, ly2[q]);                     \
+      const V lzhy = Q::mul(lz2, hy2[q]), lzly = Q::mul(lz2, ly2[q]);                     \
+      V acc = Q::tap_first(Q::mul(hzhy, hx2[q]), OLD[q][0], Q::mul(hzhy, lx2[q]), OLD[q][1]); \
+      acc = Q::tap_next(acc, Q::mul(hzly, hx2[q]), OLD[q][2]);                            \
+      acc = Q::tap_next(acc, Q::mul(hzly, lx2[q]), OLD[q][3]);                            \
+      acc = Q::tap_next(acc, Q::mul(lzhy, hx2[q]), NEW[q][0]);                            \
+      acc = Q::tap_next(acc, Q::mul(lzhy, lx2[q]), NEW[q][1]);                            \
+      acc = Q::tap_next(acc, Q::mul(lzly, hx2[q]), NEW[q][2]);                            \
+      acc = Q::tap_next(acc, Q::mul(lzly, lx2[q]), NEW[q][3]);                            \
+      /* output_val = 0 + val (normalises -0), then /count with count == 1 */             \
+      val[q] = Q::apply(Q::add(zero2, acc), mask[q]);                                     \
+    }                                                                                     \
+  }
+
+#define T3_STORE()                                                                        \
+  _Pragma("unroll") for (int q = 0; q < NP; ++q) {                                        \
+    if (act[q]) {                                                                         \
+      T* oq = o + q * sub_o;                                                              \
+      if (VEC) {                                                                          \
+        Q::store2(oq, val[q]);                                                            \
+      } else {                                                                            \
+        oq[0] = Q::lo(val[q]);                                                            \
+        if (has_b) oq[1] = Q::hi(val[q]);                                                 \
+      }                                                                                   \
+    }                                                                                     \
+  }                                                                                       \
+  o += plane_o;
+
+  int i = 0;
+  while (i < npd) {
+    const T3Ent<T> e = sh.ent[i];
+    V val[NP];
+    if ((e.flags & T3_PAIR) && b_newest && any_inside) { /* uniform: the usual walk, two depths without a decision */
+      const T3Ent<T> e2 = sh.ent[i + 1];
+      T3_FETCH(ra);
+      T3_COMPUTE(e, rb, ra);
+      T3_STORE();
+      T3_FETCH(rb);
+      T3_COMPUTE(e2, ra, rb);
+      T3_STORE();
+      i += 2;
+      continue;
+    }
+    _Pragma("unroll") for (int q = 0; q < NP; ++q) val[q] = zero2;
+    if (e.flags && any_inside) { /* uniform */
+      if (b_newest) {
+        if (e.adv == 1) { T3_FETCH(ra); b_newest = false; T3_COMPUTE(e, rb, ra); }
+        else { if (e.adv == 2) { T3_FETCH(ra); T3_FETCH(rb); } T3_COMPUTE(e, ra, rb); }
+      } else {
+        if (e.adv == 1) { T3_FETCH(rb); b_newest = true; T3_COMPUTE(e, ra, rb); }
+        else { if (e.adv == 2) { T3_FETCH(rb); T3_FETCH(ra); } T3_COMPUTE(e, rb, ra); }
+      }
+    }
+    T3_STORE();
+    ++i;
+  }
+#undef T3_STORE
+#undef T3_COMPUTE
+#undef T3_FETCH
 }
 
 // NP = voxel pairs per thread: pair q sits 16*q output rows below pair 0, so a CTA covers a
@@ -284,20 +398,25 @@ __device__ __forceinline__ void t3_body(const Params& p, const S3Launch& L, cons
   {
     const int i = threadIdx.x;
     int adv = 0, z_first = 0, z_second = 0;
+    auto planes_of = [&](int k) {  // new planes of depth k
+      const S3ZTap<T> e = sh.s3.zt[k];
+      if (e.z0 < 0) return 0;
+      if (k > 0 && sh.s3.zt[k - 1].z0 >= 0) {
+        const int pz0 = sh.s3.zt[k - 1].z0, pz1 = sh.s3.zt[k - 1].z1;
+        if (e.z0 == pz0 && e.z1 == pz1) return 0;
+        if (e.z0 == pz1) return 1;
+      }
+      return 2;
+    };
     if (i < npd) {
       const S3ZTap<T> e = sh.s3.zt[i];
       T3Ent<T> t;
-      t.h = e.h; t.l = e.l; t.flags = 0;
+      t.h = P2<T>::dup(e.h); t.l = P2<T>::dup(e.l); t.flags = 0;
       if (e.z0 >= 0) {
-        adv = 2;
-        if (i > 0 && sh.s3.zt[i - 1].z0 >= 0) {
-          const int pz0 = sh.s3.zt[i - 1].z0, pz1 = sh.s3.zt[i - 1].z1;
-          if (e.z0 == pz0 && e.z1 == pz1) adv = 0;
-          else if (e.z0 == pz1) adv = 1;
-        }
+        adv = planes_of(i);
         z_first = (adv == 2) ? e.z0 : e.z1;
         z_second = e.z1;
-        t.flags = T3_INSIDE;
+        t.flags = T3_INSIDE | (adv == 1 && i + 1 < npd && planes_of(i + 1) == 1 ? T3_PAIR : 0);
       }
       t.adv = (unsigned short)adv;
       sh.ent[i] = t;
@@ -382,7 +501,7 @@ __device__ __forceinline__ void t3_body(const Params& p, const S3Launch& L, cons
   }
 
   // ================= consumer warps =================
-  const unsigned row = (unsigned)(bw * esz);
+  // (a copy of the loop per box width: the row pitch is then an immediate of the shared-memory loads)
   unsigned oa[NP], ob[NP];  // shared-memory addresses of the base taps in ring slot 0
   typename Q::M mask[NP];
 #pragma unroll
@@ -391,93 +510,14 @@ __device__ __forceinline__ void t3_body(const Params& p, const S3Launch& L, cons
     ob[q] = ring_s + (inb[q] ? (unsigned)(((y0b[q] - by0) * bw + (x0b[q] - bx0)) * esz) : 0u);
     mask[q] = Q::make_mask(ina[q], inb[q]);
   }
-
   const long long plane_o = (long long)p.oh * p.ow;
-  const long long sub_o = (long long)kS3TileH * p.ow;  // output offset between a thread's pairs
-  T* o = (T*)p.out + k.nc * p.ovol + (long long)k.pd0 * plane_o +
-         (long long)(act[0] ? ph0 : 0) * p.ow + (col_ok ? pw0 : 0);
-  const V zero2 = Q::dup(A::fi(0));
-
-  unsigned soff = 0;                      // byte offset of the current ring slot
-  unsigned fa = full_s, ea = empty_s;     // its two mbarriers
-  const unsigned ring_end = stride * nst;
-  unsigned par = 0;
-  // Tap values of the two planes held in registers (lanes = the two voxels): x0y0, x1y0, x0y1,
-  // x1y1.  Which of the two sets is the newest plane alternates with every fetch; `b_newest`
-  // tracks it, and the code below exists once per role assignment, so no register is ever moved.
-  V ra[NP][4], rb[NP][4];
-#pragma unroll
-  for (int q = 0; q < NP; ++q)
-#pragma unroll
-    for (int t = 0; t < 4; ++t) ra[q][t] = rb[q][t] = zero2;
-  bool b_newest = true;
-  const unsigned tries = L.wait_tries;
-
-// take the next plane of the schedule out of the ring into register set R
-#define T3_FETCH(R)                                                                       \
-  {                                                                                       \
-    if (!t3_mbar_wait_ptx(fa, par, tries)) {                                              \
-      sh.abort_flag = 1;                                                                  \
-      if (p.status && lane == 0) atomicOr(p.status, STATUS_TMA_TIMEOUT);                  \
-      return; /* no barrier follows: leaving is safe, the producer drains its copies */   \
-    }                                                                                     \
-    _Pragma("unroll") for (int q = 0; q < NP; ++q) {                                      \
-      const unsigned ua = oa[q] + soff, ub = ob[q] + soff;                                \
-      R[q][0] = t3_lds_pair<T>(ua, ub);                                                   \
-      R[q][1] = t3_lds_pair<T>(ua + esz, ub + esz);                                       \
-      R[q][2] = t3_lds_pair<T>(ua + row, ub + row);                                       \
-      R[q][3] = t3_lds_pair<T>(ua + row + esz, ub + row + esz);                           \
-    }                                                                                     \
-    __syncwarp();                                                                         \
-    t3_mbar_arrive_lane0(ea, lane); /* this warp is done with the slot */                 \
-    soff += stride; fa += 8u; ea += 8u;                                                   \
-    if (soff == ring_end) { soff = 0; fa = full_s; ea = empty_s; par ^= 1u; }             \
-  }
-
-// the reference's tap sum: older plane OLD supplies taps 1-4, newest plane NEW taps 5-8
-#define T3_COMPUTE(OLD, NEW)                                                              \
-  {                                                                                       \
-    const V hz2 = Q::dup(e.h), lz2 = Q::dup(e.l);                                         \
-    _Pragma("unroll") for (int q = 0; q < NP; ++q) {                                      \
-      const V hzhy = Q::mul(hz2, hy2[q]), hzly = Q::mul(hz2, ly2[q]);                     \
-      const V lzhy = Q::mul(lz2, hy2[q]), lzly = Q::mul(lz2, ly2[q]);                     \
-      V acc = Q::tap_first(Q::mul(hzhy, hx2[q]), OLD[q][0], Q::mul(hzhy, lx2[q]), OLD[q][1]); \
-      acc = Q::tap_next(acc, Q::mul(hzly, hx2[q]), OLD[q][2]);                            \
-      acc = Q::tap_next(acc, Q::mul(hzly, lx2[q]), OLD[q][3]);                            \
-      acc = Q::tap_next(acc, Q::mul(lzhy, hx2[q]), NEW[q][0]);                            \
-      acc = Q::tap_next(acc, Q::mul(lzhy, lx2[q]), NEW[q][1]);                            \
-      acc = Q::tap_next(acc, Q::mul(lzly, hx2[q]), NEW[q][2]);                            \
-      acc = Q::tap_next(acc, Q::mul(lzly, lx2[q]), NEW[q][3]);                            \
-      /* output_val = 0 + val (normalises -0), then /count with count == 1 */             \
-      val[q] = Q::apply(Q::add(zero2, acc), mask[q]);                                     \
-    }                                                                                     \
-  }
-
-#define T3_DEPTH_LOOP(STORE)                                                              \
-  for (int i = 0; i < npd; ++i, o += plane_o) {                                           \
-    const T3Ent<T> e = sh.ent[i];                                                         \
-    V val[NP];                                                                            \
-    _Pragma("unroll") for (int q = 0; q < NP; ++q) val[q] = zero2;                        \
-    if (e.flags && any_inside) { /* uniform */                                            \
-      if (b_newest) {                                                                     \
-        if (e.adv == 1) { T3_FETCH(ra); b_newest = false; T3_COMPUTE(rb, ra); }           \
-        else { if (e.adv == 2) { T3_FETCH(ra); T3_FETCH(rb); } T3_COMPUTE(ra, rb); }      \
-      } else {                                                                            \
-        if (e.adv == 1) { T3_FETCH(rb); b_newest = true; T3_COMPUTE(ra, rb); }            \
-        else { if (e.adv == 2) { T3_FETCH(rb); T3_FETCH(ra); } T3_COMPUTE(rb, ra); }      \
-      }                                                                                   \
-    }                                                                                     \
-    _Pragma("unroll") for (int q = 0; q < NP; ++q) { STORE }                              \
-  }
-
-  if (VEC) {
-    T3_DEPTH_LOOP(if (act[q]) Q::store2(o + q * sub_o, val[q]);)
-  } else {
-    T3_DEPTH_LOOP(if (act[q]) { T* oq = o + q * sub_o; oq[0] = Q::lo(val[q]); if (has_b) oq[1] = Q::hi(val[q]); })
-  }
-#undef T3_DEPTH_LOOP
-#undef T3_COMPUTE
-#undef T3_FETCH
+  T* o = (T*)p.out + k.nc * p.ovol + (long long)k.pd0 * plane_o + (long long)(act[0] ? ph0 : 0) * p.ow + (col_ok ? pw0 : 0);
+#define T3_CONSUME(BW) \
+  t3_consume<T, NP, VEC, BW>(p, sh, L.wait_tries, npd, any_inside, stride, nst, full_s, oa, ob, lx2, hx2, ly2, hy2, mask, act, has_b, o, plane_o)
+  if (bw == (sizeof(T) == 2 ? 112 : 72)) T3_CONSUME((sizeof(T) == 2 ? 112 : 72));
+  else if (bw == (sizeof(T) == 2 ? 80 : 56)) T3_CONSUME((sizeof(T) == 2 ? 80 : 56));
+  else T3_CONSUME((sizeof(T) == 2 ? 48 : 40));
+#undef T3_CONSUME
 }
 
 template <typename T, int NP, bool VEC>
@@ -569,7 +609,7 @@ inline int try_launch_stream3d(const Params& p, int dtype, cudaStream_t st, T3La
 
   T3Maps maps;
   const bool tma = t3_make_maps(p, dtype, maps);
-  const int pairs = kT3Pairs;
+  constexpr int pairs = kT3Pairs;
   const size_t esz = dtype == 0 ? 4 : 2;
 
   // ---- geometry of the gather kernel (plain loads through L1): 32 x 16 tiles, short depth chunks.
@@ -599,7 +639,7 @@ inline int try_launch_stream3d(const Params& p, int dtype, cudaStream_t st, T3La
   L.tiles_w = G.tiles_w;
   L.tiles_h = (p.oh + rows_per_tile - 1) / rows_per_tile;
   const long long per_depth_ctas = (long long)p.R * p.C * L.tiles_w * L.tiles_h;
-  L.chunk = s3_pick_chunk(per_depth_ctas, p.od, 148 * (!tma && dtype == 1 ? 4 : 3), 6);
+  L.chunk = s3_pick_chunk(per_depth_ctas, p.od, 148 * (!tma && dtype == 1 ? 4 : 3), 9);
   L.chunks = (p.od + L.chunk - 1) / L.chunk;
   L.vec_store = G.vec_store;
   L.pair = G.pair;
@@ -683,11 +723,7 @@ inline int try_launch_stream3d(const Params& p, int dtype, cudaStream_t st, T3La
   {                                                                                                          \
     if (L.vec_store) T3_LAUNCH_V(TYPE, NP, true) else T3_LAUNCH_V(TYPE, NP, false)                           \
   }
-  if (dtype == 0) {
-    if (pairs == 2) T3_LAUNCH(float, 2) else T3_LAUNCH(float, 1)
-  } else {
-    if (pairs == 2) T3_LAUNCH(__half, 2) else T3_LAUNCH(__half, 1)
-  }
+  if (dtype == 0) T3_LAUNCH(float, kT3Pairs) else T3_LAUNCH(__half, kT3Pairs)
 #undef T3_LAUNCH
 #undef T3_LAUNCH_V
   if (err != cudaSuccess) return -8;
