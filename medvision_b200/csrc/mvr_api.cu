@@ -272,7 +272,7 @@ int mvr_roi_resample_bwd_noalloc(const void* grad_out, const void* rois, void* g
   long long ctas = 0;
   if (bwd_stream3d_applicable(p, dtype, L, ctas)) {
     if (dtype == MVR_F32) {  // float gradients are reduced straight into grad_in: no scratch at all
-      resample_bwd_stream3d<float><<<(unsigned)ctas, kS3Threads, 0, st>>>(p, L, (float*)p.out);
+      launch_bwd_kernel<float>(p, L, ctas, (float*)p.out, st);
       return cudaGetLastError() == cudaSuccess ? MVR_OK : MVR_ERR_LAUNCH;
     }
     // half: the float accumulator volume is the library's own static array

@@ -28,8 +28,50 @@ __device__ __forceinline__ void bwd_red_row(float* p0, float* p1, float v0, floa
   atomic_add_pair(p0, p1, v0, v1, lo, hi);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kS3Threads)
+// Float rows of one channel's volume, addressed by byte offsets below 2^32 from the 16-byte boundary at or below its start.
+struct BwdRows {
+  char* base;
+  unsigned shift;        // bytes from the boundary to the volume's first element
+  unsigned lo, span;     // 16-byte windows that lie inside the tensor start at lo .. lo + span
+};
+__device__ __forceinline__ BwdRows bwd_rows(float* vol, long long elements, const float* tensor_lo, const float* tensor_hi) {
+  BwdRows r;
+  r.shift = (unsigned)reinterpret_cast<unsigned long long>(vol) & 15u;
+  r.base = reinterpret_cast<char*>(vol) - r.shift;
+  const unsigned end = r.shift + (unsigned)(elements * 4);
+  const bool last = vol + elements == tensor_hi;
+  r.lo = vol == tensor_lo && r.shift ? 16u : 0u;
+  const unsigned hi = last ? (end - 16u) & ~15u : end & ~15u;
+  r.span = hi - r.lo;
+  if (last && end < r.lo + 16u) {  // no window fits
+    r.lo = 0xffffffffu;
+    r.span = 0u;
+  }
+  return r;
+}
+// Two neighbouring elements as one 16-byte reduction to the window of the lower one (see atomic_add_pair); the upper one
+// alone where it falls into the next window.
+__device__ __forceinline__ void bwd_send_row(const BwdRows& r, unsigned at, float v0, float v1) {
+  const unsigned win = at & ~15u, k = at & 15u;
+  char* const w = r.base + win;
+  if (win - r.lo > r.span) {  // would reach beyond the tensor
+    atomicAdd(reinterpret_cast<float*>(r.base + at), v0);
+    atomicAdd(reinterpret_cast<float*>(r.base + at) + 1, v1);
+    return;
+  }
+  const bool k0 = k == 0u, k1 = k == 4u, k2 = k == 8u, k3 = k == 12u;
+  const float a = k0 ? v0 : 0.0f;
+  const float b = k1 ? v0 : (k0 ? v1 : 0.0f);
+  const float c = k2 ? v0 : (k1 ? v1 : 0.0f);
+  const float d = k3 ? v0 : (k2 ? v1 : 0.0f);
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(w), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+  if (k3) atomicAdd(reinterpret_cast<float*>(w + 16), v1);
+}
+
+// PAIR: both voxels of a thread share their instructions and offsets are 32-bit bytes (mvr_stream3d.cuh, pair taps; sizes of
+// at least two, float volumes below 4 GiB); the other form takes every other shape.
+template <typename T, bool PAIR>
+__global__ void __launch_bounds__(kS3Threads, PAIR ? 3 : 1)
 resample_bwd_stream3d(const Params p, const S3Launch L, typename BwdAcc<T>::type* __restrict__ acc_base) {
   typedef Ar<T> A;
   typedef P2<T> Q;
@@ -157,6 +199,83 @@ resample_bwd_stream3d(const Params p, const S3Launch L, typename BwdAcc<T>::type
   for (int r = 0; r < 3; ++r)
     sxy[r] = Q::row_xy(Q::dup(g.rot[3 * r]), x2, Q::dup(A::mul(g.rot[3 * r + 1], y)));
   const V c2[3] = {Q::dup(g.centre[0]), Q::dup(g.centre[1]), Q::dup(g.centre[2])};
+  if (PAIR) {
+    // Consecutive depths often share tap rows (the upper z rows of one sample are the lower ones of the next half of the
+    // time): the two upper rows of a voxel's last sample are held back and summed with the next sample's row of the same
+    // place, and leave alone only when there is none.  3.4 reductions per voxel instead of 5 on rotations of up to 30 degrees.
+    const BwdRows rows = bwd_rows(acc, p.vol, acc_lo, acc_hi);
+    const unsigned sy = L.pair.sy, sz = L.pair.sz;
+    const typename Q::M lanes = Q::make_mask(true, has_b);
+    unsigned held[2] = {0u, 0u};                // byte offset of the last sample's lowest tap
+    float hv[2][4];                             // its upper z rows: (y0, z1) and (y1, z1), two taps each
+    bool holds[2] = {false, false};
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int t = 0; t < 4; ++t) hv[s][t] = 0.0f;
+    for (int i = 0; i < k.npd; ++i) {
+      const S3ZProd<T> e = sh.zp[i];
+      const V rx2 = Q::add(Q::add(sxy[0], Q::dup(e.p[0])), c2[0]);
+      const V ry2 = Q::add(Q::add(sxy[1], Q::dup(e.p[1])), c2[1]);
+      const V rz2 = Q::add(Q::add(sxy[2], Q::dup(e.p[2])), c2[2]);
+      const V g2 = Q::make(go[i * plane_o], has_b ? go[i * plane_o + 1] : A::fi(0));
+      const typename Q::M mask = lanes & ~(Q::outside(rx2, L.pair, 0) | Q::outside(ry2, L.pair, 1) | Q::outside(rz2, L.pair, 2));
+      if (!mask) continue;
+      AxisTap2<T> tx, ty, tz;
+      axis_tap2<T, 0>(rx2, L.pair, p.order, tx);
+      axis_tap2<T, 1>(ry2, L.pair, p.order, ty);
+      axis_tap2<T, 2>(rz2, L.pair, p.order, tz);
+      V w[8];
+      pair_weights<T, 3>(tx, ty, tz, w);
+#pragma unroll
+      for (int t = 0; t < 8; ++t) w[t] = Q::mul(g2, w[t]);  // grad * w_k, each product rounded
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        if (!(s ? Q::lane_b(mask) : Q::lane_a(mask))) continue;
+        const unsigned at = (s ? tx.rb : tx.ra) * 4u + (s ? ty.rb : ty.ra) * sy + ((s ? tz.rb : tz.ra) * sz + L.pair.bias) + rows.shift;
+        float c[8];
+#pragma unroll
+        for (int t = 0; t < 8; ++t) c[t] = s ? Q::hi_float(w[t]) : Q::lo_float(w[t]);
+        const bool clamped[3] = {s ? tx.cb : tx.ca, s ? ty.cb : ty.ca, s ? tz.cb : tz.ca};
+        if (clamped[0] || clamped[1] || clamped[2]) {  // both taps of the axis are the upper one
+#pragma unroll
+          for (int a = 0; a < 3; ++a)
+            if (clamped[a]) {
+#pragma unroll
+              for (int t = 0; t < 8; ++t)
+                if (!((t >> a) & 1)) {
+                  c[t | (1 << a)] += c[t];
+                  c[t] = 0.0f;
+                }
+            }
+        }
+        // which of the new rows (y0,z0) (y1,z0) (y0,z1) (y1,z1) lies where a held row does
+        const unsigned d = at - held[s];
+        const bool same = d == 0u, up = d == sz, dn_y = d == sz - sy, up_y = d == sz + sy, only_y = d == sy, back_y = d == 0u - sy;
+        if (up) { c[0] += hv[s][0]; c[1] += hv[s][1]; c[2] += hv[s][2]; c[3] += hv[s][3]; }
+        if (same) { c[4] += hv[s][0]; c[5] += hv[s][1]; c[6] += hv[s][2]; c[7] += hv[s][3]; }
+        if (dn_y) { c[2] += hv[s][0]; c[3] += hv[s][1]; }
+        if (back_y) { c[6] += hv[s][0]; c[7] += hv[s][1]; }
+        if (up_y) { c[0] += hv[s][2]; c[1] += hv[s][3]; }
+        if (only_y) { c[4] += hv[s][2]; c[5] += hv[s][3]; }
+        if (holds[s] && !(up || same || dn_y || back_y)) bwd_send_row(rows, held[s] + sz, hv[s][0], hv[s][1]);
+        if (holds[s] && !(up || same || up_y || only_y)) bwd_send_row(rows, held[s] + sz + sy, hv[s][2], hv[s][3]);
+        bwd_send_row(rows, at, c[0], c[1]);
+        bwd_send_row(rows, at + sy, c[2], c[3]);
+        held[s] = at;
+        holds[s] = true;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) hv[s][t] = c[4 + t];
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+      if (holds[s]) {
+        bwd_send_row(rows, held[s] + sz, hv[s][0], hv[s][1]);
+        bwd_send_row(rows, held[s] + sz + sy, hv[s][2], hv[s][3]);
+      }
+    return;
+  }
   for (int i = 0; i < k.npd; ++i) {
     const S3ZProd<T> e = sh.zp[i];
     const V rx2 = Q::add(Q::add(sxy[0], Q::dup(e.p[0])), c2[0]);
@@ -216,8 +335,15 @@ inline bool bwd_stream3d_applicable(const Params& p, int dtype, S3Launch& L, lon
   L.chunks = (p.od + chunk - 1) / chunk;
   L.vec_store = 0;
   L.filter = 0;
+  L.pair = make_pair_const(3, p.D, p.H, p.W, 4);  // offsets in the float accumulator
   ctas = per_depth_ctas * L.chunks;
   return ctas <= 0x7fffffffLL;
+}
+
+template <typename T>
+inline void launch_bwd_kernel(const Params& p, const S3Launch& L, long long ctas, float* acc, cudaStream_t st) {
+  if (pair_taps_applicable(3, p.D, p.H, p.W, p.vol + 8, 4)) resample_bwd_stream3d<T, true><<<(unsigned)ctas, kS3Threads, 0, st>>>(p, L, acc);
+  else resample_bwd_stream3d<T, false><<<(unsigned)ctas, kS3Threads, 0, st>>>(p, L, acc);
 }
 
 // Half backward through a float scratch volume of n = N*C*D*H*W elements that the caller of this
@@ -226,7 +352,7 @@ inline int launch_bwd_stream3d_half(const Params& p, const S3Launch& L, long lon
                                     cudaStream_t st) {
   const long long n = (long long)p.N * p.C * p.vol;
   cudaMemsetAsync(scratch, 0, (size_t)n * sizeof(float), st);
-  resample_bwd_stream3d<__half><<<(unsigned)ctas, kS3Threads, 0, st>>>(p, L, scratch);
+  launch_bwd_kernel<__half>(p, L, ctas, scratch, st);
   const long long blocks = (n + 8 * 256 - 1) / (8 * 256);
   bwd_fold_half<<<(unsigned)blocks, 256, 0, st>>>((__half*)p.out, scratch, n);
   return cudaGetLastError() == cudaSuccess ? 0 : -8;
@@ -279,7 +405,7 @@ inline int try_launch_bwd_stream3d(const Params& p, int dtype, cudaStream_t st) 
   long long ctas = 0;
   if (!bwd_stream3d_applicable(p, dtype, L, ctas)) return MVR_STREAM3D_NOT_APPLICABLE;
   if (dtype == 0) {
-    resample_bwd_stream3d<float><<<(unsigned)ctas, kS3Threads, 0, st>>>(p, L, (float*)p.out);
+    launch_bwd_kernel<float>(p, L, ctas, (float*)p.out, st);
     return cudaGetLastError() == cudaSuccess ? 0 : -8;
   }
   const long long n = (long long)p.N * p.C * p.vol;
