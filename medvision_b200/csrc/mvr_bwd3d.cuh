@@ -232,15 +232,16 @@ resample_bwd_stream3d(const Params p, const S3Launch L, typename BwdAcc<T>::type
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
         if (!(s ? Q::lane_b(mask) : Q::lane_a(mask))) continue;
-        const unsigned at = (s ? tx.rb : tx.ra) * 4u + (s ? ty.rb : ty.ra) * sy + ((s ? tz.rb : tz.ra) * sz + L.pair.bias) + rows.shift;
+        unsigned at = (s ? tx.rb : tx.ra) * 4u + (s ? ty.rb : ty.ra) * sy + ((s ? tz.rb : tz.ra) * sz + L.pair.bias) + rows.shift;
         float c[8];
 #pragma unroll
         for (int t = 0; t < 8; ++t) c[t] = s ? Q::hi_float(w[t]) : Q::lo_float(w[t]);
-        const bool clamped[3] = {s ? tx.cb : tx.ca, s ? ty.cb : ty.ca, s ? tz.cb : tz.ca};
-        if (clamped[0] || clamped[1] || clamped[2]) {  // both taps of the axis are the upper one
+        const bool clamped[3] = {(s ? tx.db : tx.da) == 0u, (s ? ty.db : ty.da) == 0u, (s ? tz.db : tz.da) == 0u};
+        if (clamped[0] || clamped[1] || clamped[2]) {  // both taps of the axis are the last voxel: the upper one of a row here
 #pragma unroll
           for (int a = 0; a < 3; ++a)
             if (clamped[a]) {
+              at -= a == 0 ? 4u : a == 1 ? sy : sz;
 #pragma unroll
               for (int t = 0; t < 8; ++t)
                 if (!((t >> a) & 1)) {
@@ -342,7 +343,8 @@ inline bool bwd_stream3d_applicable(const Params& p, int dtype, S3Launch& L, lon
 
 template <typename T>
 inline void launch_bwd_kernel(const Params& p, const S3Launch& L, long long ctas, float* acc, cudaStream_t st) {
-  if (pair_taps_applicable(3, p.D, p.H, p.W, p.vol + 8, 4)) resample_bwd_stream3d<T, true><<<(unsigned)ctas, kS3Threads, 0, st>>>(p, L, acc);
+  if (p.D >= 2 && p.H >= 2 && p.W >= 2 && pair_taps_applicable(p.D, p.H, p.W, p.vol + 8, 4))
+    resample_bwd_stream3d<T, true><<<(unsigned)ctas, kS3Threads, 0, st>>>(p, L, acc);
   else resample_bwd_stream3d<T, false><<<(unsigned)ctas, kS3Threads, 0, st>>>(p, L, acc);
 }
 

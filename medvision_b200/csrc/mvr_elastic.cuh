@@ -217,7 +217,7 @@ elastic_warp_kernel(const ElasticParams p) {
 #pragma unroll 1
         for (int ch = 0; ch < p.C; ++ch, img += vol, out += vol) {
           V v[1 << NDIM];
-          taps.load(img, p.pair, v);
+          taps.load(img, v);
           const V val = Q::apply(pair_sum<T, (1 << NDIM)>(w, v), mask);
           if (p.vec_img) {
             Q::store2(out, val);
@@ -232,9 +232,8 @@ elastic_warp_kernel(const ElasticParams p) {
         unsigned oa = taps.a, ob = taps.b;
 #pragma unroll
         for (int a = 0; a < NDIM; ++a) {
-          const unsigned step = a == 0 ? (unsigned)sizeof(T) : a == 1 ? p.pair.sy : p.pair.sz;
-          if (t[a].ca || !Ar<T>::ge_half(Q::lo(t[a].h))) oa += step;
-          if (t[a].cb || !Ar<T>::ge_half(Q::hi(t[a].h))) ob += step;
+          if (!Ar<T>::ge_half(Q::lo(t[a].h))) oa += t[a].da;
+          if (!Ar<T>::ge_half(Q::hi(t[a].h))) ob += t[a].db;
         }
         const unsigned ia = oa / (unsigned)sizeof(T), ib = ob / (unsigned)sizeof(T);
         const bool ina = Q::lane_a(mask), inb = Q::lane_b(mask);
@@ -255,14 +254,13 @@ elastic_warp_kernel(const ElasticParams p) {
   }
 }
 
-// 0 launched, 1 not applicable (grid too large for the tables, a single voxel along an axis, volume too large for 32-bit offsets), -8 launch failed
+// 0 launched, 1 not applicable (grid too large for the tables, volume too large for 32-bit offsets), -8 launch failed
 inline int launch_elastic(ElasticParams p, int ndim, int dtype, int label_dtype, cudaStream_t st) {
-  if (!pair_taps_applicable(ndim, p.D, p.H, p.W, (long long)p.D * p.H * p.W, dtype == 0 ? 4 : 2) || elastic_smem(ndim, p.gw, p.gh) > (size_t)kElasticMaxSmem) return 1;
+  if (!pair_taps_applicable(p.D, p.H, p.W, (long long)p.D * p.H * p.W, dtype == 0 ? 4 : 2) || elastic_smem(ndim, p.gw, p.gh) > (size_t)kElasticMaxSmem) return 1;
   if (p.B == 0) return 0;
   p.pair = make_pair_const(ndim, p.D, p.H, p.W, dtype == 0 ? 4 : 2);
-  // A CTA's contraction along z costs about as much as a row: as many rows per CTA as leave six CTAs per SM.
-  p.rows = 64;
-  while (p.rows > 8 && (long long)p.B * p.D * ((p.H + p.rows - 1) / p.rows) < 148LL * 6) p.rows >>= 1;
+  // a CTA's set-up costs about as much as two rounds of its eight warps' rows
+  p.rows = 8 * s3_pick_chunk((long long)p.B * p.D, (p.H + 7) / 8, 148 * 3, 2);
   p.blocks_h = (p.H + p.rows - 1) / p.rows;
   const long long ctas = (long long)p.B * p.D * p.blocks_h;
   if (ctas > 0x7fffffffLL) return 1;

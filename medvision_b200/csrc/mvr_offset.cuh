@@ -142,7 +142,7 @@ __device__ __forceinline__ void apply_offset_pair(const OffsetParams& p, int b, 
     V val = Q::dup(zero);
     if (mask) {
       V v[1 << NDIM];
-      taps.load(img, p.pair, v);
+      taps.load(img, v);
       // a sample outside the image gives the literal 0; inside, the reference returns the sum as it is
       val = Q::apply(pair_sum<T, (1 << NDIM)>(w, v), mask);
     }
@@ -179,7 +179,7 @@ inline int launch_apply_offset(OffsetParams p, int dtype, cudaStream_t st) {
   if (per_sample == 0 || p.B == 0 || p.C == 0) return 0;
   const dim3 grid((unsigned)((per_sample + kOffsetThreads - 1) / kOffsetThreads), (unsigned)min(p.B, 65535));
   p.pair = make_pair_const(NDIM, p.D, p.H, p.W, dtype == 0 ? 4 : 2);
-  const bool voxels = p.order == 3 || !pair_taps_applicable(NDIM, p.D, p.H, p.W, (long long)p.D * p.H * p.W, dtype == 0 ? 4 : 2);
+  const bool voxels = p.order == 3 || !pair_taps_applicable(p.D, p.H, p.W, (long long)p.D * p.H * p.W, dtype == 0 ? 4 : 2);
   if (dtype == 0) {
     if (voxels) apply_offset_kernel<float, NDIM, true><<<grid, kOffsetThreads, 0, st>>>(p);
     else apply_offset_kernel<float, NDIM, false><<<grid, kOffsetThreads, 0, st>>>(p);

@@ -157,7 +157,7 @@ resample_fwd_plane2d(const Params p, const PairConst pc, const Plane2dLabel lab,
       V val = zero2;
       if (mask) {
         V v[4];
-        taps.load(plane, pc, v);
+        taps.load(plane, v);
         // output_val = 0 + val (normalises -0), then / count with count == 1
         val = Q::apply(Q::add(zero2, pair_sum<T, 4>(w, v)), mask);
       }
@@ -178,7 +178,7 @@ inline int try_launch_plane2d(const Params& p, int dtype, cudaStream_t st, const
   if ((dtype == 0 || label) && p.fm != kS3FloatPattern) return 1;
   if (p.ovol < 4096 || p.ow < 8) return 1;
   const size_t esz = dtype == 0 ? 4 : 2;
-  if (!pair_taps_applicable(2, 1, p.H, p.W, p.vol, esz) || p.vol >= 0x7fffffffLL) return 1;
+  if (!pair_taps_applicable(1, p.H, p.W, p.vol, esz) || p.vol >= 0x7fffffffLL) return 1;
   const int tiles_w = (p.ow + kS3TileW - 1) / kS3TileW, row_blocks = (p.oh + kS3TileH - 1) / kS3TileH;
   // a CTA's set-up costs about two row blocks; five CTAs per SM
   const int blocks = s3_pick_chunk((long long)p.R * tiles_w, std::min(row_blocks, 4096), 148 * 5, 2);

@@ -169,46 +169,45 @@ __device__ __forceinline__ void nearest_axis(T& l, T& h) {
 //   * the truncation c -> i0 is one addition: for 0 <= c <= size - 1 < 2^22, c + 2^23 rounded towards zero carries i0 in
 //     its low mantissa bits (conversion instructions run at a sixteenth of the rate of an addition); the bias of the raw
 //     bits is part of the address constant;
-//   * the eight taps are read at FIXED distances from one address per lane: the lower tap of an axis is taken from
-//     [0, size - 2], and in the rare case that a coordinate sits on the last index (where the reference clamps the upper
-//     tap onto the lower one and the upper weight is 0) the values are put right afterwards, behind a branch;
 //   * everything that depends on the sizes only comes from the host, in the kernel's parameters.
-// Sizes of at least 2 on every axis; byte offsets inside a channel's volume below 2^32.
+// Byte offsets inside a channel's volume below 2^32.  (Reading the taps at fixed distances from one address, and putting the
+// values right behind a branch where a coordinate sits on the last index, costs fewer instructions but more time: the branch
+// stands between the loads and the sum.  Elastic warp 2 x 128 x 256 x 256: 180 us, with the steps selected 152 us.)
 constexpr unsigned kTapMagic = 0x4B000000u;   // bits of 2^23
 constexpr int kTapMaxSize = 1 << 22;
 
 struct PairConst {
   float last[3];          // size - 1                                  (axis 0 = w, 1 = h, 2 = d)
-  unsigned base_max[3];   // kTapMagic + size - 2
+  unsigned last_raw[3];   // kTapMagic + size - 1
   float size[3];
   unsigned size_floor2[3], size_ceil2[3];  // half2 of the largest half <= size and of the smallest half >= size
-  unsigned sy, sz, bias;  // byte strides, and -kTapMagic * (sx + sy + sz) modulo 2^32
+  unsigned sx, sy, sz, bias;  // byte strides, and -kTapMagic * (sx + sy + sz) modulo 2^32
 };
 inline PairConst make_pair_const(int ndim, int D, int H, int W, size_t esz) {
   PairConst k;
   const int size[3] = {W, H, D};
   for (int a = 0; a < 3; ++a) {
     k.last[a] = (float)(size[a] - 1);
-    k.base_max[a] = kTapMagic + (unsigned)(size[a] - 2);
+    k.last_raw[a] = kTapMagic + (unsigned)(size[a] - 1);
     k.size[a] = (float)size[a];
     const unsigned lo = __half_as_ushort(__float2half_rd(k.size[a])), hi = __half_as_ushort(__float2half_ru(k.size[a]));
     k.size_floor2[a] = lo | (lo << 16);
     k.size_ceil2[a] = hi | (hi << 16);
   }
+  k.sx = (unsigned)esz;
   k.sy = (unsigned)((size_t)W * esz);
   k.sz = ndim == 3 ? (unsigned)((size_t)H * W * esz) : 0u;
   k.bias = 0u - kTapMagic * ((unsigned)esz + k.sy + k.sz);
   return k;
 }
-inline bool pair_taps_applicable(int ndim, int D, int H, int W, long long vol, size_t esz) {
-  return D <= kTapMaxSize && H <= kTapMaxSize && W <= kTapMaxSize && H >= 2 && W >= 2 && (ndim == 2 || D >= 2) &&
-         (unsigned long long)vol * esz <= 0xffffffffull;
+inline bool pair_taps_applicable(int D, int H, int W, long long vol, size_t esz) {
+  return D <= kTapMaxSize && H <= kTapMaxSize && W <= kTapMaxSize && (unsigned long long)vol * esz <= 0xffffffffull;
 }
 
 template <typename T>
 struct AxisTap2 {
-  unsigned ra, rb;             // kTapMagic + index of the lower of the two taps read, per lane
-  bool ca, cb;                 // coordinate on the last index: both taps are the upper one
+  unsigned ra, rb;             // kTapMagic + lower tap index, per lane
+  unsigned da, db;             // byte step to the upper tap; 0: clamped onto the lower one, the last
   typename P2<T>::V l, h;
 };
 
@@ -232,10 +231,11 @@ __device__ __forceinline__ void axis_tap2(typename P2<T>::V c, const PairConst& 
   // `if (c <= 0) c = 0`; at and beyond the last index: c = last, hence l = 0
   const float fa = min_nan(max_nan(Q::lo_float(c), 0.0f), k.last[AXIS]), fb = min_nan(max_nan(Q::hi_float(c), 0.0f), k.last[AXIS]);
   const float ma = __fadd_rz(fa, magic), mb = __fadd_rz(fb, magic);
-  t.ra = min(__float_as_uint(ma), k.base_max[AXIS]);
-  t.rb = min(__float_as_uint(mb), k.base_max[AXIS]);
-  t.ca = fa >= k.last[AXIS];
-  t.cb = fb >= k.last[AXIS];
+  t.ra = min(__float_as_uint(ma), k.last_raw[AXIS]);
+  t.rb = min(__float_as_uint(mb), k.last_raw[AXIS]);
+  const unsigned step = AXIS == 0 ? k.sx : AXIS == 1 ? k.sy : k.sz;
+  t.da = t.ra < k.last_raw[AXIS] ? step : 0u;
+  t.db = t.rb < k.last_raw[AXIS] ? step : 0u;
   // c - i0 is exact in the element type, so forming it in float and narrowing it changes nothing
   t.l = Q::from_floats(__fsub_rn(fa, __fsub_rn(ma, magic)), __fsub_rn(fb, __fsub_rn(mb, magic)));
   t.h = Q::sub(Q::dup(A::fi(1)), t.l);
@@ -246,41 +246,34 @@ __device__ __forceinline__ void axis_tap2(typename P2<T>::V c, const PairConst& 
 template <typename T, int NDIM>
 struct PairTaps {
   typedef typename P2<T>::V V;
-  unsigned a, b;               // byte offsets of the lowest taps
-  bool ca[3], cb[3], any;
+  unsigned a, b, dxa, dxb, dya, dyb, dza, dzb;  // byte offsets of the lowest taps, steps
   __device__ __forceinline__ PairTaps(const AxisTap2<T>& tx, const AxisTap2<T>& ty, const AxisTap2<T>& tz, const PairConst& k) {
     a = tx.ra * (unsigned)sizeof(T) + (ty.ra * k.sy + k.bias);
     b = tx.rb * (unsigned)sizeof(T) + (ty.rb * k.sy + k.bias);
-    ca[0] = tx.ca; cb[0] = tx.cb;
-    ca[1] = ty.ca; cb[1] = ty.cb;
-    any = tx.ca || tx.cb || ty.ca || ty.cb;
+    dxa = tx.da; dxb = tx.db; dya = ty.da; dyb = ty.db;
+    dza = dzb = 0u;
     if (NDIM == 3) {
       a += tz.ra * k.sz;
       b += tz.rb * k.sz;
-      ca[2] = tz.ca; cb[2] = tz.cb;
-      any = any || tz.ca || tz.cb;
+      dza = tz.da;
+      dzb = tz.db;
     }
   }
-  __device__ __forceinline__ void load(const T* vol, const PairConst& k, V* v) const {
+  __device__ __forceinline__ static T ld(const char* base, unsigned off) { return __ldg(reinterpret_cast<const T*>(base + off)); }
+  __device__ __forceinline__ void load(const T* vol, V* v) const {
     typedef P2<T> Q;
-    const char* pa = reinterpret_cast<const char*>(vol) + a;
-    const char* pb = reinterpret_cast<const char*>(vol) + b;
-#pragma unroll
-    for (int r = 0; r < (NDIM == 3 ? 4 : 2); ++r) {
-      const size_t step = (r & 1 ? k.sy : 0u) + (size_t)(r & 2 ? k.sz : 0u);
-      const T* ra = reinterpret_cast<const T*>(pa + step);
-      const T* rb = reinterpret_cast<const T*>(pb + step);
-      v[2 * r] = Q::make(__ldg(ra), __ldg(rb));
-      v[2 * r + 1] = Q::make(__ldg(ra + 1), __ldg(rb + 1));
-    }
-    if (any) {
-#pragma unroll
-      for (int ax = 0; ax < NDIM; ++ax) {
-        const typename Q::M m = Q::make_mask(ca[ax], cb[ax]);
-#pragma unroll
-        for (int t = 0; t < (1 << NDIM); ++t)
-          if (!((t >> ax) & 1)) v[t] = Q::blend(v[t], v[t | (1 << ax)], m);
-      }
+    const char* p = reinterpret_cast<const char*>(vol);
+    const unsigned ya = a + dya, yb = b + dyb;
+    v[0] = Q::make(ld(p, a), ld(p, b));
+    v[1] = Q::make(ld(p, a + dxa), ld(p, b + dxb));
+    v[2] = Q::make(ld(p, ya), ld(p, yb));
+    v[3] = Q::make(ld(p, ya + dxa), ld(p, yb + dxb));
+    if (NDIM == 3) {
+      const unsigned za = a + dza, zb = b + dzb, wa = ya + dza, wb = yb + dzb;
+      v[4] = Q::make(ld(p, za), ld(p, zb));
+      v[5] = Q::make(ld(p, za + dxa), ld(p, zb + dxb));
+      v[6] = Q::make(ld(p, wa), ld(p, wb));
+      v[7] = Q::make(ld(p, wa + dxa), ld(p, wb + dxb));
     }
   }
 };
@@ -390,7 +383,7 @@ __device__ __forceinline__ void s3_full_depth_loop(const Params& p, const S3Laun
       V val = zero2;
       if (mask) {  // a lane outside keeps valid (clamped) addresses; its value is dropped
         V v[8], w[8];
-        PairTaps<T, 3>(tx, ty, tz, pc).load(vol, pc, v);
+        PairTaps<T, 3>(tx, ty, tz, pc).load(vol, v);
         pair_weights<T, 3>(tx, ty, tz, w);
         val = Q::apply(Q::add(zero2, pair_sum<T, 8>(w, v)), mask);
       }
@@ -576,7 +569,7 @@ __device__ void s3_body_l1(const Params& p, const S3Launch& L, const S3Cta& k, S
     V q0[4], q1[4], qn[4];
     int at0 = -1, at1 = -1, atn = -1;
     const int HW = p.H * p.W;
-    auto load = [&](V* q, int plane) { taps.load(vol + (long long)plane * HW, L.pair, q); };
+    auto load = [&](V* q, int plane) { taps.load(vol + (long long)plane * HW, q); };
     auto prefetch = [&](const S3ZTap<T>& e) {
       if (e.z0 >= 0 && e.z1 != at1 && e.z1 != atn) {
         load(qn, e.z1);

@@ -605,7 +605,7 @@ inline int try_launch_stream3d(const Params& p, int dtype, cudaStream_t st, T3La
   // small outputs (detection heads) are better served one element per thread
   if (p.ovol < 4096 || p.ow < 8) return MVR_STREAM3D_NOT_APPLICABLE;
   // 32-bit byte offsets inside a volume (float volumes of 2^30 elements and more go to the flat kernel)
-  if (!pair_taps_applicable(3, p.D, p.H, p.W, p.vol, dtype == 0 ? 4 : 2)) return MVR_STREAM3D_NOT_APPLICABLE;
+  if (!pair_taps_applicable(p.D, p.H, p.W, p.vol, dtype == 0 ? 4 : 2)) return MVR_STREAM3D_NOT_APPLICABLE;
 
   T3Maps maps;
   const bool tma = t3_make_maps(p, dtype, maps);
