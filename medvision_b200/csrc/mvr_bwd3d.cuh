@@ -68,6 +68,40 @@ __device__ __forceinline__ void bwd_send_row(const BwdRows& r, unsigned at, floa
   if (k3) atomicAdd(reinterpret_cast<float*>(w + 16), v1);
 }
 
+// Two such pairs in one row of the volume: one operation where they share a window.
+__device__ __forceinline__ void bwd_send_two(const BwdRows& r, unsigned at_p, float p0, float p1, unsigned at_q, float q0, float q1) {
+  if (at_q < at_p) {  // p to the left
+    const unsigned u = at_p; at_p = at_q; at_q = u;
+    float f = p0; p0 = q0; q0 = f;
+    f = p1; p1 = q1; q1 = f;
+  }
+  const unsigned win = at_p & ~15u, kp = at_p & 15u, kq = at_q - win;  // kq: 0..12 in p's window, 16 the next one's first slot
+  if (kq > 16u || win - r.lo > r.span) {
+    bwd_send_row(r, at_p, p0, p1);
+    bwd_send_row(r, at_q, q0, q1);
+    return;
+  }
+  char* const w = r.base + win;
+  if (kq == 16u) {
+    if (kp == 12u) {  // p's upper element is q's lower one
+      q0 += p1;
+      atomicAdd(reinterpret_cast<float*>(w + 12), p0);
+    } else {
+      bwd_send_row(r, at_p, p0, p1);
+    }
+    bwd_send_row(r, at_q, q0, q1);
+    return;
+  }
+  const bool k0 = kp == 0u, k1 = kp == 4u, k2 = kp == 8u, k3 = kp == 12u;
+  const bool m0 = kq == 0u, m1 = kq == 4u, m2 = kq == 8u, m3 = kq == 12u;
+  const float a = (k0 ? p0 : 0.0f) + (m0 ? q0 : 0.0f);
+  const float b = (k1 ? p0 : (k0 ? p1 : 0.0f)) + (m1 ? q0 : (m0 ? q1 : 0.0f));
+  const float c = (k2 ? p0 : (k1 ? p1 : 0.0f)) + (m2 ? q0 : (m1 ? q1 : 0.0f));
+  const float d = (k3 ? p0 : (k2 ? p1 : 0.0f)) + (m3 ? q0 : (m2 ? q1 : 0.0f));
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(w), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+  if (m3) atomicAdd(reinterpret_cast<float*>(w + 16), k3 ? p1 + q1 : q1);
+}
+
 // PAIR: both voxels of a thread share their instructions and offsets are 32-bit bytes (mvr_stream3d.cuh, pair taps; sizes of
 // at least two, float volumes below 4 GiB); the other form takes every other shape.
 template <typename T, bool PAIR>
@@ -139,17 +173,58 @@ resample_bwd_stream3d(const Params p, const S3Launch L, typename BwdAcc<T>::type
 #pragma unroll
     for (int t = 0; t < 8; ++t) acc0[t] = acc1[t] = 0.0f;
     int held0 = -1, held1 = -1;  // planes of acc0 / acc1, -1: nothing held
-    auto flush = [&](const float* a, int plane) {
+    // The two voxels of a thread are neighbours, so their rows mostly coincide and leave together: 3.3 operations per thread
+    // and plane instead of 5 on rotations of up to 30 degrees.
+    const BwdRows rows = PAIR ? bwd_rows(acc, p.vol, acc_lo, acc_hi) : BwdRows();
+    const unsigned sy = L.pair.sy;
+    // rows of two: base one voxel below where a coordinate sits on the last index
+    const unsigned ra = (unsigned)(min(txa.i0, p.W - 2) * 4) + (unsigned)min(tya.i0, p.H - 2) * sy + rows.shift;
+    const unsigned rb = (unsigned)(min(txb.i0, p.W - 2) * 4) + (unsigned)min(tyb.i0, p.H - 2) * sy + rows.shift;
+    const bool clamps = txa.i0 == txa.i1 || txb.i0 == txb.i1 || tya.i0 == tya.i1 || tyb.i0 == tyb.i1;
+    const int dy = min(tyb.i0, p.H - 2) - min(tya.i0, p.H - 2);
+    const int mode = !(ina && inb) || dy < -1 || dy > 1 ? 2 : dy;  // rows shared: all (0), one (+-1), none (2)
+    auto flush = [&](const float* v, int plane) {
       if (plane < 0) return;
-      Acc* pl = acc + plane * HW;
-      if (ina) {
-        bwd_red_row(pl + oa[0], pl + oa[1], a[0], a[1], acc_lo, acc_hi);
-        bwd_red_row(pl + oa[2], pl + oa[3], a[2], a[3], acc_lo, acc_hi);
+      if (!PAIR) {
+        Acc* pl = acc + plane * HW;
+        if (ina) {
+          bwd_red_row(pl + oa[0], pl + oa[1], v[0], v[1], acc_lo, acc_hi);
+          bwd_red_row(pl + oa[2], pl + oa[3], v[2], v[3], acc_lo, acc_hi);
+        }
+        if (inb) {
+          bwd_red_row(pl + ob[0], pl + ob[1], v[4], v[5], acc_lo, acc_hi);
+          bwd_red_row(pl + ob[2], pl + ob[3], v[6], v[7], acc_lo, acc_hi);
+        }
+        return;
       }
-      if (inb) {
-        bwd_red_row(pl + ob[0], pl + ob[1], a[4], a[5], acc_lo, acc_hi);
-        bwd_red_row(pl + ob[2], pl + ob[3], a[6], a[7], acc_lo, acc_hi);
+      float c[8];
+#pragma unroll
+      for (int t = 0; t < 8; ++t) c[t] = v[t];
+      if (clamps) {  // both taps of the axis are the last voxel
+        if (txa.i0 == txa.i1) { c[1] += c[0]; c[3] += c[2]; c[0] = c[2] = 0.0f; }
+        if (txb.i0 == txb.i1) { c[5] += c[4]; c[7] += c[6]; c[4] = c[6] = 0.0f; }
+        if (tya.i0 == tya.i1) { c[2] += c[0]; c[3] += c[1]; c[0] = c[1] = 0.0f; }
+        if (tyb.i0 == tyb.i1) { c[6] += c[4]; c[7] += c[5]; c[4] = c[5] = 0.0f; }
       }
+      const unsigned at = (unsigned)plane * L.pair.sz, a0 = at + ra, b0 = at + rb;
+      if (mode == 2) {
+        if (ina) {
+          bwd_send_row(rows, a0, c[0], c[1]);
+          bwd_send_row(rows, a0 + sy, c[2], c[3]);
+        }
+        if (inb) {
+          bwd_send_row(rows, b0, c[4], c[5]);
+          bwd_send_row(rows, b0 + sy, c[6], c[7]);
+        }
+        return;
+      }
+      // b's row that lies in a's first row, in a's second row, and the row(s) left
+      const bool up = mode == 1, down = mode == -1;
+      if (mode == 0) bwd_send_two(rows, a0, c[0], c[1], b0, c[4], c[5]);
+      else bwd_send_row(rows, up ? a0 : b0, up ? c[0] : c[4], up ? c[1] : c[5]);
+      bwd_send_two(rows, down ? a0 : a0 + sy, down ? c[0] : c[2], down ? c[1] : c[3], up ? b0 : b0 + sy, up ? c[4] : c[6],
+                   up ? c[5] : c[7]);
+      if (mode != 0) bwd_send_row(rows, (up ? b0 : a0) + sy, up ? c[6] : c[2], up ? c[7] : c[3]);
     };
     for (int i = 0; i < k.npd; ++i) {
       const S3ZTap<T> e = sh.zt[i];
@@ -170,26 +245,30 @@ resample_bwd_stream3d(const Params p, const S3Launch L, typename BwdAcc<T>::type
         c0[t] = A::tof(Q::lo(lo)); c0[4 + t] = A::tof(Q::hi(lo));
         c1[t] = A::tof(Q::lo(hi)); c1[4 + t] = A::tof(Q::hi(hi));
       }
-      if (e.z0 == held0 && e.z1 == held1) {  // CTA-uniform
-#pragma unroll
-        for (int t = 0; t < 8; ++t) { acc0[t] += c0[t]; acc1[t] += c1[t]; }
-      } else if (e.z0 == held1) {
+      // CTA-uniform: planes that this depth leaves behind
+      const int leave = e.z0 == held0 && e.z1 == held1 ? 0 : e.z0 == held1 ? 1 : 2;
+#pragma unroll 1
+      for (int f = 0; f < leave; ++f) {
         flush(acc0, held0);
 #pragma unroll
-        for (int t = 0; t < 8; ++t) { acc0[t] = acc1[t] + c0[t]; acc1[t] = c1[t]; }
+        for (int t = 0; t < 8; ++t) acc0[t] = acc1[t];
         held0 = held1;
-        held1 = e.z1;
-      } else {
-        flush(acc0, held0);
-        flush(acc1, held1);
-#pragma unroll
-        for (int t = 0; t < 8; ++t) { acc0[t] = c0[t]; acc1[t] = c1[t]; }
-        held0 = e.z0;
-        held1 = e.z1;
       }
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        acc0[t] = leave == 2 ? c0[t] : acc0[t] + c0[t];
+        acc1[t] = leave == 0 ? acc1[t] + c1[t] : c1[t];
+      }
+      held0 = e.z0;
+      held1 = e.z1;
     }
-    flush(acc0, held0);
-    flush(acc1, held1);
+#pragma unroll 1
+    for (int f = 0; f < 2; ++f) {
+      flush(acc0, held0);
+#pragma unroll
+      for (int t = 0; t < 8; ++t) acc0[t] = acc1[t];
+      held0 = held1;
+    }
     return;
   }
 
