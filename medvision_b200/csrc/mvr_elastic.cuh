@@ -179,7 +179,7 @@ __device__ __forceinline__ int elastic_label(const IT* p) {
 }
 
 template <typename T, typename IT, int NDIM>
-__global__ void __launch_bounds__(kElasticThreads, 3)
+__global__ void __launch_bounds__(kElasticThreads, sizeof(T) == 2 ? 4 : 3)
 elastic_warp_kernel(const ElasticParams p) {
   typedef P2<T> Q;
   typedef typename Q::V V;
@@ -259,8 +259,10 @@ inline int launch_elastic(ElasticParams p, int ndim, int dtype, int label_dtype,
   if (!pair_taps_applicable(p.D, p.H, p.W, (long long)p.D * p.H * p.W, dtype == 0 ? 4 : 2) || elastic_smem(ndim, p.gw, p.gh) > (size_t)kElasticMaxSmem) return 1;
   if (p.B == 0) return 0;
   p.pair = make_pair_const(ndim, p.D, p.H, p.W, dtype == 0 ? 4 : 2);
-  // a CTA's set-up costs about as much as two rounds of its eight warps' rows
-  p.rows = 8 * s3_pick_chunk((long long)p.B * p.D, (p.H + 7) / 8, 148 * 3, 2);
+  // 64 rows spread a CTA's set-up over eight rounds of its warps; fewer where that would leave less than six CTAs per SM
+  // (longer columns, as many as still fill the chip, measured 190 against 166 us on 2 x 96 x 160 x 160: an uneven last wave)
+  p.rows = 64;
+  while (p.rows > 8 && (long long)p.B * p.D * ((p.H + p.rows - 1) / p.rows) < 148 * 6) p.rows >>= 1;
   p.blocks_h = (p.H + p.rows - 1) / p.rows;
   const long long ctas = (long long)p.B * p.D * p.blocks_h;
   if (ctas > 0x7fffffffLL) return 1;

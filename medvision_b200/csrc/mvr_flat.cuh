@@ -72,23 +72,100 @@ template <> struct FlatWide<double> {
   __device__ __forceinline__ static double narrow(double v) { return v; }
 };
 
+// Taps of a sample in few instructions (the truncation by one addition, see axis_tap2 in mvr_stream3d.cuh); same taps and
+// weights as make_taps.  Sizes up to kTapMaxSize.  Taken for run-time grids, whose loops are bound by the instructions of a
+// sample: with the table of offsets and one reciprocal per output, rotated 3D heads of 583 000 outputs and 27 samples, half
+// backward 893 -> 727 us, 151 000 in float 122 -> 86; rotated 2D, 317 000 outputs, adaptive, half backward 170 -> 145 (forwards
+// equal).  The fixed grids keep make_taps: their half 3D backward measured 71 against 91 us.
+template <typename T>
+struct FlatAxis {
+  int i0, d;   // lower tap, distance to the upper one (0: clamped)
+  T l, h;
+};
+template <typename T>
+__device__ __forceinline__ bool flat_axis(T c, int size, FlatAxis<T>& t) {
+  typedef Ar<T> A;
+  const float magic = 8388608.0f, last = (float)(size - 1);
+  const float v = A::tof(c);
+  const float f = min_nan(max_nan(v, 0.0f), last);
+  const float m = __fadd_rz(f, magic);
+  t.i0 = (int)(min(__float_as_uint(m), kTapMagic + (unsigned)(size - 1)) - kTapMagic);
+  t.d = t.i0 < size - 1 ? 1 : 0;
+  t.l = A::ff(__fsub_rn(f, __fsub_rn(m, magic)));  // exact
+  t.h = A::sub(A::fi(1), t.l);
+  return !(v < -1.0f || v > (float)size);
+}
+// double, and volumes too large for 32-bit offsets, form their taps the long way
+template <typename T, int NDIM, typename OFF>
+__device__ __forceinline__ bool flat_taps(const Params& p, T z, T y, T x, T* w, OFF* off) {
+  typedef Ar<T> A;
+  if constexpr (sizeof(T) == 8 || sizeof(OFF) == 8) {
+    return make_taps<T, NDIM, OFF>(p.D, p.H, p.W, z, y, x, p.order, w, off);
+  } else {
+    FlatAxis<T> t[3];
+    bool in = flat_axis<T>(x, p.W, t[0]);
+    in = flat_axis<T>(y, p.H, t[1]) && in;
+    if (NDIM == 3) in = flat_axis<T>(z, p.D, t[2]) && in;
+    if (!in) return false;
+    const int dy = t[1].d * p.W;
+    off[0] = t[1].i0 * p.W + t[0].i0;
+    if (NDIM == 3) off[0] += t[2].i0 * (p.H * p.W);
+    off[1] = off[0] + t[0].d;
+    off[2] = off[0] + dy;
+    off[3] = off[1] + dy;
+    if (NDIM == 3) {
+      const int dz = t[2].d * (p.H * p.W);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) off[4 + k] = off[k] + dz;
+    }
+    if (p.order == 0) {
+      AxisTap<T> n[3];
+#pragma unroll
+      for (int a = 0; a < NDIM; ++a) {
+        n[a].l = t[a].l;
+        n[a].h = t[a].h;
+      }
+      nearest_pick<T, NDIM>(n, w);
+    } else if (NDIM == 2) {
+      w[0] = A::mul(t[1].h, t[0].h);
+      w[1] = A::mul(t[1].h, t[0].l);
+      w[2] = A::mul(t[1].l, t[0].h);
+      w[3] = A::mul(t[1].l, t[0].l);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; k += 2) {
+        const T zy = A::mul((k & 4) ? t[2].l : t[2].h, (k & 2) ? t[1].l : t[1].h);
+        w[k] = A::mul(zy, t[0].h);
+        w[k + 1] = A::mul(zy, t[0].l);
+      }
+    }
+    return true;
+  }
+}
+
+constexpr int kFlatSubs = 16;  // sub-sample offsets per axis kept in shared memory (run-time grids)
+
 // SR: compile-time sampling ratio per axis (1 or 2), or 0 = taken from the roi at run time
 // (any fixed ratio, or the adaptive ceil(bin) grid).
 // OFF: type of the tap offsets inside one channel's volume (int when D*H*W < 2^31).
+// SR == 0: 2^lg lanes share an output (a roi's outputs are few, its samples many): in the forward they take consecutive
+// samples and every lane adds the values up in the reference's order; in the backward they take the sample lines in turn.
 template <typename T, int NDIM, int SR, bool BWD, typename OFF>
 // (the 2D half backward is the one instantiation that gains from a full single wave of 16 CTAs per SM: 22.6 against
 // 26.7 us on the rotated 2D head; the float kernels lose more to the 32-register limit than the wave gives)
 __global__ void __launch_bounds__(kFlatThreads, (NDIM == 2 && BWD && sizeof(T) == 2 && SR != 0) ? 16 : 1)
-resample_flat(const Params p, const FlatDivs fd, int total) {
+resample_flat(const Params p, const FlatDivs fd, int total, int lg) {
   typedef Ar<T> A;
   constexpr int fm = kFlatFm;
   flat_grid_dependency();
   __shared__ RoiGeom<T> geo[kFlatMaxRois];
+  __shared__ T subs[SR ? 1 : kFlatMaxRois][SR ? 1 : NDIM][SR ? 1 : kFlatSubs];
+  if (SR) lg = 0;
   const int per_roi = (int)fd.per_roi.d;
-  const int e0 = (int)blockIdx.x * kFlatThreads;
+  const int e0 = (int)blockIdx.x * (kFlatThreads >> lg);
   const int n0 = flat_div(e0, fd.per_roi);
   const int rem0 = e0 - n0 * per_roi;
-  const int e_last = min(e0 + kFlatThreads, total) - 1;
+  const int e_last = min(e0 + (kFlatThreads >> lg), total) - 1;
   const int n_rois = flat_div(e_last, fd.per_roi) - n0 + 1;
   if ((int)threadIdx.x < n_rois) {
     const int osz[3] = {p.ow, p.oh, p.od};
@@ -96,9 +173,19 @@ resample_flat(const Params p, const FlatDivs fd, int total) {
                   fm, geo[threadIdx.x]);
   }
   __syncthreads();
-  const int e = e0 + (int)threadIdx.x;
-  if (e >= total) return;
-  const int t = rem0 + (int)threadIdx.x;
+  if (SR == 0) {  // the in-bin offsets of the sub-samples: the only divisions of the lattice
+    for (int i = threadIdx.x; i < n_rois * NDIM * kFlatSubs; i += kFlatThreads) {
+      const int k = i % kFlatSubs, a = i / kFlatSubs % NDIM, q = i / (kFlatSubs * NDIM);
+      if (k < geo[q].grid[a]) subs[q][a][k] = lattice_sub<T>(geo[q].bin[a], k, geo[q].grid[a]);
+    }
+    __syncthreads();
+  }
+  const int slot = (int)threadIdx.x >> lg, part = (int)threadIdx.x & ((1 << lg) - 1);
+  const int e = e0 + slot;
+  // lanes that share an output stay together (shuffles below)
+  const bool beyond = e >= total;
+  if (beyond && (SR || BWD)) return;
+  const int t = beyond ? 0 : rem0 + slot;
   const int r = flat_div(t, fd.per_roi);
   const int rem = t - r * per_roi;
   const RoiGeom<T>& g = geo[r];
@@ -112,24 +199,29 @@ resample_flat(const Params p, const FlatDivs fd, int total) {
   // count of samples per output when the sampling ratio is fixed at compile time: a power of two
   constexpr float inv_count = 1.0f / (float)((SR ? SR : 1) * (SR ? SR : 1) * ((NDIM == 3 && SR) ? SR : 1));
 
-  if (g.batch < 0 || g.batch >= p.N) {
-    if (p.status && rem == 0) atomicOr(p.status, STATUS_BAD_BATCH_INDEX);
-    if (!BWD) ((T*)p.out)[e] = zero;
-    return;
+  const bool bad = g.batch < 0 || g.batch >= p.N;
+  if (bad) {
+    if (p.status && rem == 0 && !beyond) atomicOr(p.status, STATUS_BAD_BATCH_INDEX);
+    if (SR || BWD) {
+      if (!BWD) ((T*)p.out)[e] = zero;
+      return;
+    }
   }
   // fwd: the volume read; bwd: the gradient volume accumulated into
-  const T* vol = (const T*)(BWD ? p.out : p.in) + ((long long)g.batch * p.C + c) * p.vol;
+  const T* vol = (const T*)(BWD ? p.out : p.in) + ((long long)(bad ? 0 : g.batch) * p.C + c) * p.vol;
   T* gvol = (T*)p.out + ((long long)g.batch * p.C + c) * p.vol;
   const T* const glo = (const T*)p.out;                                // the whole gradient tensor
   const T* const ghi = glo + (long long)p.N * p.C * p.vol;
   const T go = BWD ? ((const T*)p.in)[e] : zero;
+  // run-time grids: one reciprocal per output instead of a division per tap
+  const float inv_n = (BWD && SR == 0) ? 1.0f / A::tof(g.count_bwd) : 0.0f;
 
   const T bx = lattice_base<T>(g.start[0], pw, g.bin[0], fm);
   const T by = lattice_base<T>(g.start[1], ph, g.bin[1], fm);
   const T bz = (NDIM == 3) ? lattice_base<T>(g.start[2], pd, g.bin[2], fm) : zero;
   const int gx = SR ? SR : g.grid[0], gy = SR ? SR : g.grid[1], gz = (NDIM == 3) ? (SR ? SR : g.grid[2]) : 1;
 
-  T acc = zero;
+  T acc = zero, value = zero;
   // backward: the cell of the volume whose contributions are being summed.  Always for half gradients (the sums are
   // what keeps the small addends of an up-sampling roi); for float and double only with a run-time sample grid, where
   // consecutive samples share cells often enough for the saved reductions to pay for the bookkeeping (on the
@@ -151,7 +243,8 @@ resample_flat(const Params p, const FlatDivs fd, int total) {
     to_volume<T, NDIM>(g, p.kind, fm, x, y, z, sx, sy, sz);
     T w[1 << NDIM];
     OFF off[1 << NDIM];
-    const bool in = make_taps<T, NDIM, OFF>(p.D, p.H, p.W, sz, sy, sx, p.order, w, off);
+    const bool in = SR ? make_taps<T, NDIM, OFF>(p.D, p.H, p.W, sz, sy, sx, p.order, w, off)
+                       : flat_taps<T, NDIM, OFF>(p, sz, sy, sx, w, off);
     if (BWD) {
       if (!in) return;
       if (kCellSums) {
@@ -168,7 +261,9 @@ resample_flat(const Params p, const FlatDivs fd, int total) {
         }
 #pragma unroll
         for (int k = 0; k < (1 << NDIM); ++k)
-          cell_sum[k] += (Wide)A::tof(SR ? A::scale_pow2(A::mul(go, w[k]), inv_count) : A::div(A::mul(go, w[k]), g.count_bwd));
+          if (SR) cell_sum[k] += (Wide)A::tof(A::scale_pow2(A::mul(go, w[k]), inv_count));
+          else if (sizeof(T) == 8) cell_sum[k] += (Wide)A::div(A::mul(go, w[k]), g.count_bwd);
+          else cell_sum[k] += (Wide)(A::tof(A::mul(go, w[k])) * inv_n);
       } else {
 #pragma unroll
         for (int k = 0; k < (1 << NDIM); k += 2) {
@@ -179,14 +274,14 @@ resample_flat(const Params p, const FlatDivs fd, int total) {
         }
       }
     } else {
-      T val = zero;
+      value = zero;
       if (in) {
         T tap[1 << NDIM];
 #pragma unroll
         for (int k = 0; k < (1 << NDIM); ++k) tap[k] = __ldg(vol + off[k]);
-        val = tap_sum<T, (1 << NDIM)>(w, tap, fm);
+        value = tap_sum<T, (1 << NDIM)>(w, tap, fm);
       }
-      acc = A::add(acc, val);
+      if (SR) acc = A::add(acc, value);
     }
   };
 
@@ -210,16 +305,71 @@ resample_flat(const Params p, const FlatDivs fd, int total) {
       }
     }
   } else {
-    for (int iz = 0; iz < gz; ++iz) {
-      const T z = (NDIM == 3) ? A::add(bz, lattice_sub<T>(g.bin[2], iz, gz)) : zero;
-      for (int iy = 0; iy < gy; ++iy) {
-        const T y = A::add(by, lattice_sub<T>(g.bin[1], iy, gy));
-        for (int ix = 0; ix < gx; ++ix) sample(A::add(bx, lattice_sub<T>(g.bin[0], ix, gx)), y, z);
+    auto sub = [&](int a, int i) { return i < kFlatSubs ? subs[r][a][i] : lattice_sub<T>(g.bin[a], i, g.grid[a]); };
+    if (BWD) {
+      // an up-sampling roi (in half) keeps its samples in one lane: they share cells, whose sums are formed before they are
+      // rounded
+      int lanes = 1 << lg;
+      if (sizeof(T) == 2 && lanes > 1) {
+        bool wide = true;
+#pragma unroll
+        for (int a = 0; a < NDIM; ++a) wide = wide && A::tof(g.bin[a]) >= 2.0f;
+        if (!wide) {
+          if (part) return;
+          lanes = 1;
+        }
       }
+      int iz = 0, iy = lanes == 1 ? 0 : part;
+      for (;; iy += lanes) {
+        while (iy >= gy && iz < gz) {
+          iy -= gy;
+          ++iz;
+        }
+        if (iz >= gz) break;
+        const T z = (NDIM == 3) ? A::add(bz, sub(NDIM - 1, iz)) : zero;
+        const T y = A::add(by, sub(1, iy));
+        for (int ix = 0; ix < gx; ++ix) sample(A::add(bx, sub(0, ix)), y, z);
+      }
+    } else if (lg == 0) {
+      if (!bad && !beyond)
+        for (int iz = 0; iz < gz; ++iz) {
+          const T z = (NDIM == 3) ? A::add(bz, sub(NDIM - 1, iz)) : zero;
+          for (int iy = 0; iy < gy; ++iy) {
+            const T y = A::add(by, sub(1, iy));
+#pragma unroll 2
+            for (int ix = 0; ix < gx; ++ix) {
+              sample(A::add(bx, sub(0, ix)), y, z);
+              acc = A::add(acc, value);
+            }
+          }
+        }
+    } else {
+      const int lanes = 1 << lg, n = bad || beyond ? 0 : gx * gy * gz;
+      const int rounds = __reduce_max_sync(0xffffffffu, (n + lanes - 1) >> lg);
+      int ix = part, iy = 0, iz = 0;
+      for (int k = 0; k < rounds; ++k, ix += lanes) {
+        const int left = n - (k << lg);  // samples from this round on
+        value = zero;
+        if (part < left) {
+          while (ix >= gx) {
+            ix -= gx;
+            if (++iy == gy) {
+              iy = 0;
+              ++iz;
+            }
+          }
+          sample(A::add(bx, sub(0, ix)), A::add(by, sub(1, iy)), (NDIM == 3) ? A::add(bz, sub(NDIM - 1, iz)) : zero);
+        }
+        for (int j = 0; j < lanes; ++j) {
+          const T v = __shfl_sync(0xffffffffu, value, j, lanes);
+          if (j < left) acc = A::add(acc, v);
+        }
+      }
+      if (part || beyond) return;
     }
   }
   if (BWD && kCellSums) flush_cell();
-  if (!BWD) ((T*)p.out)[e] = SR ? A::scale_pow2(acc, inv_count) : A::div(acc, g.count_fwd);
+  if (!BWD && !beyond) ((T*)p.out)[e] = SR ? A::scale_pow2(acc, inv_count) : bad ? zero : A::div(acc, g.count_fwd);
 }
 
 // Forward for axis-aligned boxes (RoIAlign) with a fixed sampling ratio of 1 or 2.  Without a
@@ -337,8 +487,8 @@ resample_flat_box_fwd(const Params p, const FlatDivs fd, int total) {
   ((T*)p.out)[e] = A::scale_pow2(acc, inv_count);
 }
 
-template <typename K>
-inline void flat_launch(K kernel, unsigned grid, cudaStream_t st, const Params& p, const FlatDivs& fd, int total) {
+template <typename K, typename... More>
+inline void flat_launch(K kernel, unsigned grid, cudaStream_t st, const Params& p, const FlatDivs& fd, int total, More... more) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -348,7 +498,7 @@ inline void flat_launch(K kernel, unsigned grid, cudaStream_t st, const Params& 
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, p, fd, total);
+  cudaLaunchKernelEx(&cfg, kernel, p, fd, total, more...);
 }
 
 // 0 launched, 1 not applicable
@@ -367,7 +517,7 @@ inline int launch_flat(const Params& p, bool fwd, cudaStream_t st) {
   fd.oh = make_flat_div((unsigned)p.oh);
   const int tot = (int)total;
   const int sr = (p.sampling_ratio == 1 || p.sampling_ratio == 2) ? p.sampling_ratio : 0;
-  const bool small = p.vol < 0x7fffffffLL;
+  const bool small = p.vol < 0x7fffffffLL && p.D <= kTapMaxSize && p.H <= kTapMaxSize && p.W <= kTapMaxSize;
   if (fwd && p.kind == KIND_BOX && sr > 0) {
 #define MVR_BOX(ND, SRV)                                                                             \
   {                                                                                                  \
@@ -382,14 +532,20 @@ inline int launch_flat(const Params& p, bool fwd, cudaStream_t st) {
 #undef MVR_BOX
     return 0;
   }
+  // Lanes per output with a run-time grid: more than one only where the outputs would leave most of the chip idle
+  // (measured: 6 500 outputs of 27 samples 15.4 -> 7.9 us, 65 000 of 9 samples 7.9 -> 13.5 us).
+  int lg = 0;
+  if (sr == 0)
+    while (lg < 3 && (total << (lg + 1)) <= 148LL * 384) ++lg;
+  const unsigned lanes_grid = (unsigned)((total + (kFlatThreads >> lg) - 1) / (kFlatThreads >> lg));
 #define MVR_FLAT(ND, SRV)                                                                            \
   {                                                                                                  \
     if (small) {                                                                                     \
-      if (fwd) flat_launch(resample_flat<T, ND, SRV, false, int>, grid, st, p, fd, tot);          \
-      else flat_launch(resample_flat<T, ND, SRV, true, int>, grid, st, p, fd, tot);               \
+      if (fwd) flat_launch(resample_flat<T, ND, SRV, false, int>, lanes_grid, st, p, fd, tot, lg); \\
+      else flat_launch(resample_flat<T, ND, SRV, true, int>, lanes_grid, st, p, fd, tot, lg); \\
     } else {                                                                                         \
-      if (fwd) flat_launch(resample_flat<T, ND, SRV, false, long long>, grid, st, p, fd, tot);    \
-      else flat_launch(resample_flat<T, ND, SRV, true, long long>, grid, st, p, fd, tot);         \
+      if (fwd) flat_launch(resample_flat<T, ND, SRV, false, long long>, lanes_grid, st, p, fd, tot, lg); \\
+      else flat_launch(resample_flat<T, ND, SRV, true, long long>, lanes_grid, st, p, fd, tot, lg); \\
     }                                                                                                \
   }
   if (p.ndim == 2) {

@@ -1,0 +1,69 @@
+"""Sampling kernels with a run-time sample grid (csrc/mvr_flat.cuh) where few outputs are shared by several lanes: eight, four
+and two lanes and one, counts that leave the last block partly empty, grids beyond the table of sub-sample offsets, a roi with a
+bad batch index.  Forward bit for bit, backward against the wide-accumulator restatement."""
+import math
+
+import pytest
+import torch
+
+import cases
+from oracle import port
+from util import BWD_TOL, assert_close, n_mismatch
+
+pytestmark = pytest.mark.gpu
+REF_FM = 1 | (1 << 1) | (1 << 2) | (1 << 3) | (1 << 5) | (1 << 7) | (1 << 10) | (1 << 13) | \
+    (1 << 16) | (1 << 18) | (2 << 20) | (1 << 22)
+
+CASES = [
+    # spatial,        channels, rois, output,    sampling, order
+    ((37, 41),        3, 9,   (5, 7),    3, 1),
+    ((70, 53),        1, 8,   (3, 3),    0, 1),    # up to 20 samples per axis
+    ((37, 41),        5, 37,  (7, 7),    3, 0),
+    ((70, 53),        9, 31,  (7, 7),    0, 1),
+    ((37, 41),        9, 51,  (7, 7),    3, 1),
+    ((70, 53),        12, 61, (7, 7),    3, 1),    # one lane again
+    ((9, 14, 17),     1, 8,   (3, 2, 5), 3, 1),
+    ((19, 23, 29),    3, 9,   (7, 7, 7), 0, 1),
+    ((9, 14, 17),     7, 11,  (5, 5, 5), 3, 0),
+]
+
+
+def _rois(spatial, R, g):
+    nd = len(spatial)
+    ext = torch.tensor(spatial[::-1], dtype=torch.float32)
+    b = torch.randint(0, 2, (R, 1), generator=g).float()
+    c = torch.rand(R, nd, generator=g) * ext
+    s = torch.rand(R, nd, generator=g) * ext * 0.4 + 4.0
+    s[1] = ext                        # the whole map
+    c[2] = ext * 3                    # outside
+    c[3] = ext - 0.5                  # over the border
+    a = (torch.rand(R, 1 if nd == 2 else 3, generator=g) * 2 - 1) * math.pi
+    return torch.cat([b, c, s, a], 1)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16], ids=["float32", "float16"])
+@pytest.mark.parametrize("spatial,C,R,out,sr,order", CASES,
+                         ids=["%s-c%d-%s-s%d-o%d" % ("x".join(map(str, c[0])), c[1], "x".join(map(str, c[3])), c[4], c[5]) for c in CASES])
+def test_shared_outputs_match_the_restatement(spatial, C, R, out, sr, order, dtype):
+    from medvision_b200 import _C
+    nd = len(spatial)
+    g = torch.Generator().manual_seed(sum(spatial) + R)
+    feat = (torch.rand((2, C) + spatial, generator=g) * 2 - 0.5).to(dtype)
+    rois = _rois(spatial, R, g).to(dtype)
+    bad = rois.clone()
+    bad[6, 0] = 5                     # batch index outside the batch
+    fwd, bwd = ((_C.roi_align_rotated_2d_forward, _C.roi_align_rotated_2d_backward) if nd == 2 else
+                (_C.roi_align_rotated_3d_forward, _C.roi_align_rotated_3d_backward))
+    keep = [i for i in range(R) if i != 6]
+    kw = dict(spatial_scale=1.0, sampling_ratio=sr, aligned=True, order=order, trig=port.device_trig(rois[keep]),
+              fma_mode=REF_FM if dtype == torch.float32 else 0)
+    got = torch.full((R, C) + out, float("nan"), dtype=dtype, device="cuda")
+    fwd(feat.cuda(), bad.cuda(), got, *out, 1.0, sr, True, order)
+    assert not bool(got[6].any())
+    assert n_mismatch(got[keep], port.forward(feat, rois[keep], out, cases.KIND_ROTATED, **kw)) == 0
+    grad = torch.randn((R, C) + out, generator=g).to(dtype)
+    want = port.backward(grad[keep], rois[keep], feat.shape, cases.KIND_ROTATED, wide_acc=True, **kw)
+    gin = torch.zeros(feat.shape, dtype=dtype, device="cuda")
+    bwd(grad.cuda(), bad.cuda(), gin, *out, 1.0, sr, True, order)
+    assert_close(gin, want, 1e-5 if dtype == torch.float32 else BWD_TOL[dtype], "gradient")
+    _C.last_status()
