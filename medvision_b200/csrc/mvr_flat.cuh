@@ -541,11 +541,11 @@ inline int launch_flat(const Params& p, bool fwd, cudaStream_t st) {
 #define MVR_FLAT(ND, SRV)                                                                            \
   {                                                                                                  \
     if (small) {                                                                                     \
-      if (fwd) flat_launch(resample_flat<T, ND, SRV, false, int>, lanes_grid, st, p, fd, tot, lg); \\
-      else flat_launch(resample_flat<T, ND, SRV, true, int>, lanes_grid, st, p, fd, tot, lg); \\
+      if (fwd) flat_launch(resample_flat<T, ND, SRV, false, int>, lanes_grid, st, p, fd, tot, lg); \
+      else flat_launch(resample_flat<T, ND, SRV, true, int>, lanes_grid, st, p, fd, tot, lg); \
     } else {                                                                                         \
-      if (fwd) flat_launch(resample_flat<T, ND, SRV, false, long long>, lanes_grid, st, p, fd, tot, lg); \\
-      else flat_launch(resample_flat<T, ND, SRV, true, long long>, lanes_grid, st, p, fd, tot, lg); \\
+      if (fwd) flat_launch(resample_flat<T, ND, SRV, false, long long>, lanes_grid, st, p, fd, tot, lg); \
+      else flat_launch(resample_flat<T, ND, SRV, true, long long>, lanes_grid, st, p, fd, tot, lg); \
     }                                                                                                \
   }
   if (p.ndim == 2) {
