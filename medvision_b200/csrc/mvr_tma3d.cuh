@@ -615,14 +615,14 @@ inline int try_launch_stream3d(const Params& p, int dtype, cudaStream_t st, T3La
   // ---- geometry of the gather kernel (plain loads through L1): 32 x 16 tiles, short depth chunks.
   // Rois under a general rotation are bound by load latency and want many CTAs.  Measured on
   // RandomAffine 16 x 128^3 with three-axis rotations: 8 depths per CTA 329 us, 16: 365, 32: 430,
-  // 64: 725.
+  // 64: 725.  The work items are dealt out in turn to CTAs that stay, so a short launch wants many of them.
   S3Launch G;
   G.tiles_w = (p.ow + kS3TileW - 1) / kS3TileW;
   G.tiles_h = (p.oh + kS3TileH - 1) / kS3TileH;
   const long long g_per_depth = (long long)p.R * p.C * G.tiles_w * G.tiles_h;
   {
     int chunk = kS3MaxChunk;
-    while (chunk > 8 && g_per_depth * ((p.od + chunk - 1) / chunk) < 148LL * 16) chunk >>= 1;
+    while (chunk > 8 && g_per_depth * ((p.od + chunk - 1) / chunk) < 148LL * 32) chunk >>= 1;
     G.chunk = min(chunk, p.od);
   }
   G.chunks = (p.od + G.chunk - 1) / G.chunk;
@@ -633,13 +633,22 @@ inline int try_launch_stream3d(const Params& p, int dtype, cudaStream_t st, T3La
   if (g_ctas > 0x7fffffffLL) return MVR_STREAM3D_NOT_APPLICABLE;
   // ---- geometry of the plane walk: 32 x 16*pairs tiles for the plane-streaming kernel, 32 x 16 without a tensor map; long
   // depth chunks (s3_pick_chunk: measured on Resize 4 x (160,512,512) -> (128,256,256), 43 depths per CTA 83 us, 26: 84,
-  // 64: 87, 16: 91; on 96^3 crops one chunk of 96 beats two of 48 by 9 %).
+  // 64: 87, 16: 91; on 96^3 crops one chunk of 96 beats two of 48 by 9 %).  Without a tensor map a CTA's set-up is cheaper
+  // (no plane schedule), and one launch takes every roi, of a general rotation or not, in chunks that suit both: 16 crops of
+  // (37, 97, 104) x 2 channels in half under three-axis rotations 136 us with the rois split over two launches, 100 with one;
+  // about z alone 24 float crops of (40, 66, 109) 50.2 -> 49.5.  Chunks of 8 at most: 57 on the latter; of 64: as for the
+  // gather.  With a label volume the gather launch carries that one's work items, so it stays.
+  const bool one = !tma && p.kind == KIND_ROTATED && !label;
   const int rows_per_tile = kS3TileH * (tma ? pairs : 1);
   S3Launch L;
   L.tiles_w = G.tiles_w;
   L.tiles_h = (p.oh + rows_per_tile - 1) / rows_per_tile;
   const long long per_depth_ctas = (long long)p.R * p.C * L.tiles_w * L.tiles_h;
-  L.chunk = s3_pick_chunk(per_depth_ctas, p.od, 148 * (!tma && dtype == 1 ? 4 : 3), 9);
+  L.chunk = s3_pick_chunk(per_depth_ctas, p.od, 148 * (!tma && dtype == 1 ? 4 : 3), tma ? 9 : 3);
+  if (one) {
+    const int parts = (L.chunk + 15) / 16;
+    L.chunk = (L.chunk + parts - 1) / parts;
+  }
   L.chunks = (p.od + L.chunk - 1) / L.chunk;
   L.vec_store = G.vec_store;
   L.pair = G.pair;
@@ -649,7 +658,7 @@ inline int try_launch_stream3d(const Params& p, int dtype, cudaStream_t st, T3La
   if (L.skip_plane >= 0) L.wait_tries = 32;  // self-test of the bounded waits: short limits
   // axis-aligned boxes have no rotation: one launch; rotated rois: this launch takes those that turn
   // about z at most, the gather launch below takes the rest
-  const bool two = (p.kind == KIND_ROTATED);
+  const bool two = p.kind == KIND_ROTATED && !one;
   L.filter = two ? 1 : 0;
   G.filter = 2;
   // The gather launch goes first and lets its dependents start as soon as its CTAs are resident
