@@ -173,7 +173,10 @@ resample_flat(const Params p, const FlatDivs fd, int total, int lg) {
                   fm, geo[threadIdx.x]);
   }
   __syncthreads();
-  if (SR == 0) {  // the in-bin offsets of the sub-samples: the only divisions of the lattice
+  // the in-bin offsets of the sub-samples: the only divisions of the lattice.  A half forward with one lane per output forms them
+  // as it goes, which costs it less than a second barrier (1 477 000 outputs of an adaptive 2D head 29.7 -> 27.0 us); for the same
+  // reason the loop over a line's few samples is not unrolled.
+  if (SR == 0 && (BWD || lg || sizeof(T) != 2)) {
     for (int i = threadIdx.x; i < n_rois * NDIM * kFlatSubs; i += kFlatThreads) {
       const int k = i % kFlatSubs, a = i / kFlatSubs % NDIM, q = i / (kFlatSubs * NDIM);
       if (k < geo[q].grid[a]) subs[q][a][k] = lattice_sub<T>(geo[q].bin[a], k, geo[q].grid[a]);
@@ -305,7 +308,7 @@ resample_flat(const Params p, const FlatDivs fd, int total, int lg) {
       }
     }
   } else {
-    auto sub = [&](int a, int i) { return i < kFlatSubs ? subs[r][a][i] : lattice_sub<T>(g.bin[a], i, g.grid[a]); };
+    auto sub = [&](int a, int i) { return (BWD || lg || sizeof(T) != 2) && i < kFlatSubs ? subs[r][a][i] : lattice_sub<T>(g.bin[a], i, g.grid[a]); };
     if (BWD) {
       // an up-sampling roi (in half) keeps its samples in one lane: they share cells, whose sums are formed before they are
       // rounded
@@ -336,7 +339,7 @@ resample_flat(const Params p, const FlatDivs fd, int total, int lg) {
           const T z = (NDIM == 3) ? A::add(bz, sub(NDIM - 1, iz)) : zero;
           for (int iy = 0; iy < gy; ++iy) {
             const T y = A::add(by, sub(1, iy));
-#pragma unroll 2
+#pragma unroll 1
             for (int ix = 0; ix < gx; ++ix) {
               sample(A::add(bx, sub(0, ix)), y, z);
               acc = A::add(acc, value);
