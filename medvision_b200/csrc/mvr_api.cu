@@ -118,7 +118,8 @@ int launch_mark(const Params& p, cudaStream_t st) {
 // the flat kernel where it applies, else the one-CTA-per-tile kernel.
 int dispatch_flat_or_generic(const Params& p, int dtype, bool fwd, cudaStream_t st) {
   if (dtype != MVR_F64) {
-    const int rc = dtype == MVR_F32 ? launch_box_head<float>(p, fwd, st) : launch_box_head<__half>(p, fwd, st);
+    int rc = dtype == MVR_F32 ? launch_box_head<float>(p, fwd, st) : launch_box_head<__half>(p, fwd, st);
+    if (rc && !fwd && dtype == MVR_F16) rc = launch_rot_head_bwd(p, st);
     if (rc == 0) return cudaGetLastError() == cudaSuccess ? MVR_OK : MVR_ERR_LAUNCH;
   }
   {

@@ -67,3 +67,32 @@ def test_shared_outputs_match_the_restatement(spatial, C, R, out, sr, order, dty
     bwd(grad.cuda(), bad.cuda(), gin, *out, 1.0, sr, True, order)
     assert_close(gin, want, 1e-5 if dtype == torch.float32 else BWD_TOL[dtype], "gradient")
     _C.last_status()
+
+
+@pytest.mark.parametrize("spatial,C,R,out,sr,order", [
+    ((19, 23, 29), 3, 9, (7, 7, 7), 2, 1),      # slabs of a roi
+    ((12, 40, 61), 5, 70, (5, 3, 4), 0, 1),     # a roi per block; boxes larger than the shared memory beside small ones
+    ((9, 14, 17), 2, 8, (3, 5, 2), 2, 0),
+    ((70, 53), 3, 8, (7, 7), 2, 1),
+    ((37, 41), 2, 170, (5, 9), 3, 1),
+], ids=["slabs", "large", "nearest", "plane", "plane-many"])
+def test_half_gradient_of_rotated_rois(spatial, C, R, out, sr, order):
+    from medvision_b200 import _C
+    nd = len(spatial)
+    g = torch.Generator().manual_seed(sum(spatial) + R)
+    rois = _rois(spatial, R, g).half()
+    rois[4, 1 + nd:1 + 2 * nd] = 0.3  # far fewer voxels than samples
+    grad = torch.randn((R, C) + out, generator=g).half()
+    shape = (2, C) + spatial
+    want = port.backward(grad, rois, shape, cases.KIND_ROTATED, spatial_scale=1.0, sampling_ratio=sr, aligned=True, order=order,
+                         trig=port.device_trig(rois), wide_acc=True, fma_mode=0)
+    n = want.numel()
+    for offset in (0, 3):             # a gradient tensor at an unaligned place inside a buffer
+        buf = torch.full((n + 32,), -0.0, dtype=torch.half, device="cuda")
+        gin = buf[16 + offset:16 + offset + n].view(shape)
+        gin.zero_()
+        (_C.roi_align_rotated_2d_backward if nd == 2 else _C.roi_align_rotated_3d_backward)(
+            grad.cuda(), rois.cuda(), gin, *out, 1.0, sr, True, order)
+        assert_close(gin, want, BWD_TOL[torch.half], "gradient")
+        around = torch.cat([buf[:16 + offset], buf[16 + offset + n:]])
+        assert bool((torch.signbit(around) & (around == 0)).all()), "something was added outside the gradient tensor"
