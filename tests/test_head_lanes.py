@@ -96,3 +96,35 @@ def test_half_gradient_of_rotated_rois(spatial, C, R, out, sr, order):
         assert_close(gin, want, BWD_TOL[torch.half], "gradient")
         around = torch.cat([buf[:16 + offset], buf[16 + offset + n:]])
         assert bool((torch.signbit(around) & (around == 0)).all()), "something was added outside the gradient tensor"
+
+
+@pytest.mark.parametrize("rotated,C,R,out,sr,order,dtype", [
+    (True, 7, 3100, (7, 7), 1, 1, torch.float32),    # a last group of three channels, a last block partly empty
+    (True, 9, 2077, (7, 7), 1, 0, torch.float16),
+    (False, 5, 3130, (7, 7), 0, 1, torch.float16),   # a last group of one
+    (False, 4, 1601, (14, 14), 3, 1, torch.float16),
+], ids=["rotated-float32", "rotated-nearest-float16", "adaptive", "three"])
+def test_channel_groups_match_the_restatement(rotated, C, R, out, sr, order, dtype):
+    from medvision_b200 import _C
+    spatial = (37, 41)
+    g = torch.Generator().manual_seed(C * R)
+    feat = (torch.rand((2, C) + spatial, generator=g) * 2 - 0.5).to(dtype)
+    rois = _rois(spatial, R, g)
+    if not rotated:
+        rois = torch.cat([rois[:, :1], rois[:, 1:3] - rois[:, 3:5] / 2, rois[:, 1:3] + rois[:, 3:5] / 2], 1)
+    rois = rois.to(dtype)
+    bad = rois.clone()
+    bad[6, 0] = 5
+    keep = [i for i in range(R) if i != 6]
+    got = torch.full((R, C) + out, float("nan"), dtype=dtype, device="cuda")
+    args = (feat.cuda(), bad.cuda(), got) + out + (1.0, sr)
+    if rotated:
+        _C.roi_align_rotated_2d_forward(*args, True, order)
+    else:
+        _C.roi_align_2d_forward(*args, order)
+    assert not bool(got[6].any())
+    want = port.forward(feat, rois[keep], out, cases.KIND_ROTATED if rotated else cases.KIND_BOX, spatial_scale=1.0, sampling_ratio=sr,
+                        aligned=True, order=order, trig=port.device_trig(rois[keep]) if rotated else None,
+                        fma_mode=REF_FM if dtype == torch.float32 else 0)
+    assert n_mismatch(got[keep], want) == 0
+    _C.last_status()
