@@ -630,12 +630,12 @@ inline int launch_flat(const Params& p, bool fwd, cudaStream_t st) {
   }
   // Four channels per thread from one full wave of threads on, in 2D (3D: 46 -> 66 us, its taps share less of the L1), where
   // that measured faster over every width of rois: one sample per bin under a rotation (2 237 000 outputs 20.8 -> 13.3 us in
-  // float, 2 080 000 in half 20.1 -> 13.3), boxes in half with a run-time grid (1 477 000 outputs, adaptive, 28.3 -> 16.8 and, of
-  // up to 96 voxels, 113 -> 71).  Rotated rois of more samples lose up to 14 % where their bins are wide.
+  // float, 2 080 000 in half 20.1 -> 13.3), boxes with a run-time grid (half, 1 477 000 outputs, adaptive, 28.3 -> 16.8 and, of
+  // up to 96 voxels, 113 -> 71; float, 1 872 000 outputs 39 -> 26).  Rotated rois of more samples lose up to 14 % where their bins are wide.
   if constexpr (sizeof(T) != 8) {
     const int groups = (p.C + kFlatGroup - 1) / kFlatGroup;
     const long long threads = (long long)p.R * groups * p.ovol;
-    const bool one = p.kind == KIND_ROTATED && sr == 1, boxes = p.kind == KIND_BOX && sr == 0 && sizeof(T) == 2;
+    const bool one = p.kind == KIND_ROTATED && sr == 1, boxes = p.kind == KIND_BOX && sr == 0;
     if (fwd && small && p.ndim == 2 && (one || boxes) && p.C > 2 && groups * p.ovol >= kFlatMinPerRoi && threads >= 148 * 2048) {
       FlatDivs fg = fd;
       fg.per_roi = make_flat_div((unsigned)(groups * p.ovol));
@@ -644,10 +644,8 @@ inline int launch_flat(const Params& p, bool fwd, cudaStream_t st) {
         flat_launch(resample_flat_channels_fwd<T, 2, 1>, group_grid, st, p, fg, (int)threads);
         return 0;
       }
-      if constexpr (sizeof(T) == 2) {
-        flat_launch(resample_flat_channels_fwd<T, 2, 0>, group_grid, st, p, fg, (int)threads);
-        return 0;
-      }
+      flat_launch(resample_flat_channels_fwd<T, 2, 0>, group_grid, st, p, fg, (int)threads);
+      return 0;
     }
   }
   // Lanes per output with a run-time grid: more than one only where the outputs would leave most of the chip idle

@@ -103,7 +103,8 @@ def test_half_gradient_of_rotated_rois(spatial, C, R, out, sr, order):
     (True, 9, 2077, (7, 7), 1, 0, torch.float16),
     (False, 5, 3130, (7, 7), 0, 1, torch.float16),   # a last group of one
     (False, 4, 1601, (14, 14), 3, 1, torch.float16),
-], ids=["rotated-float32", "rotated-nearest-float16", "adaptive", "three"])
+    (False, 6, 3130, (7, 7), 0, 1, torch.float32),
+], ids=["rotated-float32", "rotated-nearest-float16", "adaptive", "three", "adaptive-float32"])
 def test_channel_groups_match_the_restatement(rotated, C, R, out, sr, order, dtype):
     from medvision_b200 import _C
     spatial = (37, 41)
