@@ -61,11 +61,6 @@ template <> struct P2<__half> {
   __device__ __forceinline__ static V tap_next(V acc, V w, V v) { return __hadd2_rn(acc, __hmul2_rn(w, v)); }
   __device__ __forceinline__ static __half lo(V v) { return __low2half(v); }
   __device__ __forceinline__ static __half hi(V v) { return __high2half(v); }
-  __device__ __forceinline__ static V select(V v, bool keep_a, bool keep_b) {
-    unsigned u = *reinterpret_cast<unsigned*>(&v);
-    u &= (keep_a ? 0x0000ffffu : 0u) | (keep_b ? 0xffff0000u : 0u);
-    return *reinterpret_cast<V*>(&u);
-  }
   __device__ __forceinline__ static void store2(__half* p, V v) { *reinterpret_cast<__half2*>(p) = v; }
   typedef unsigned M;  // lane mask, built once per thread
   __device__ __forceinline__ static M make_mask(bool keep_a, bool keep_b) {
@@ -126,9 +121,6 @@ template <> struct P2<float> {
   }
   __device__ __forceinline__ static float lo(V v) { return v.a; }
   __device__ __forceinline__ static float hi(V v) { return v.b; }
-  __device__ __forceinline__ static V select(V v, bool keep_a, bool keep_b) {
-    return make(keep_a ? v.a : 0.0f, keep_b ? v.b : 0.0f);
-  }
   __device__ __forceinline__ static void store2(float* p, V v) { *reinterpret_cast<float2*>(p) = make_float2(v.a, v.b); }
   typedef unsigned M;
   __device__ __forceinline__ static M make_mask(bool keep_a, bool keep_b) { return (keep_a ? 1u : 0u) | (keep_b ? 2u : 0u); }
