@@ -201,7 +201,7 @@ resample_fwd_stream3d_rest_label(const Params p, const S3Launch L, long long ite
       const S3Cta k = s3_cta(p, L, item);
       if (!((general[k.n >> 5] >> (k.n & 31)) & 1u)) continue;  // CTA-uniform
       s3_prologue<T, true>(p, k, sh.img);
-      s3_body_l1<T, true>(p, L, k, sh.img);
+      s3_body_l1<T, true, false>(p, L, k, sh.img);
       __syncthreads();  // the next item's prologue overwrites the tables
     }
   for (long long item = blockIdx.x; item < items_l; item += gridDim.x) {

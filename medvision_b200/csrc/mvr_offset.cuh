@@ -75,7 +75,7 @@ __device__ __forceinline__ void warp_taps(const typename P2<T>::V* c, const Pair
   else t[2] = t[1];  // not read
 }
 
-template <typename T, int NDIM, bool VOXELS>
+template <typename T, int NDIM, bool VOXELS, bool WIDE>
 __device__ __forceinline__ void apply_offset_pair(const OffsetParams& p, int b, int d, int h, int wp) {
   typedef Ar<T> A;
   typedef P2<T> Q;
@@ -97,7 +97,7 @@ __device__ __forceinline__ void apply_offset_pair(const OffsetParams& p, int b, 
   const T* img = (const T*)p.img + (long long)b * p.C * vol;
   T* out = (T*)p.out + (long long)b * p.C * vol + s0;
 
-  if (VOXELS) {  // Catmull-Rom, and volumes too large for the pair form's 32-bit offsets: voxel by voxel
+  if (VOXELS) {  // Catmull-Rom, and axes too long for the pair form: voxel by voxel
     const int lim[3] = {p.W, p.H, p.D};  // in float: any size
     bool ina = true, inb = has_b;
 #pragma unroll
@@ -134,7 +134,7 @@ __device__ __forceinline__ void apply_offset_pair(const OffsetParams& p, int b, 
   AxisTap2<T> t[3];
   warp_taps<T, NDIM>(c, p.pair, p.order, t);
   const typename Q::M mask = warp_inside<T, NDIM>(c, p.pair, has_b);
-  const PairTaps<T, NDIM> taps(t[0], t[1], t[2], p.pair);
+  const PairTaps<T, NDIM, WIDE> taps(t[0], t[1], t[2], p.pair);
   V w[1 << NDIM];
   pair_weights<T, NDIM>(t[0], t[1], t[2], w);
 #pragma unroll 1
@@ -155,7 +155,7 @@ __device__ __forceinline__ void apply_offset_pair(const OffsetParams& p, int b, 
   }
 }
 
-template <typename T, int NDIM, bool VOXELS>
+template <typename T, int NDIM, bool VOXELS, bool WIDE>
 __global__ void __launch_bounds__(kOffsetThreads, VOXELS ? 1 : 4)
 apply_offset_kernel(const OffsetParams p) {
   typedef Ar<T> A;
@@ -170,7 +170,7 @@ apply_offset_kernel(const OffsetParams p) {
   const unsigned row = idx / pairs_w;
   const int h = (int)(row % (unsigned)p.H);
   const int d = (int)(row / (unsigned)p.H);
-  for (int b = blockIdx.y; b < p.B; b += gridDim.y) apply_offset_pair<T, NDIM, VOXELS>(p, b, d, h, wp);
+  for (int b = blockIdx.y; b < p.B; b += gridDim.y) apply_offset_pair<T, NDIM, VOXELS, WIDE>(p, b, d, h, wp);
 }
 
 template <int NDIM>
@@ -178,15 +178,21 @@ inline int launch_apply_offset(OffsetParams p, int dtype, cudaStream_t st) {
   const long long per_sample = (long long)p.D * p.H * ((p.W + 1) / 2);
   if (per_sample == 0 || p.B == 0 || p.C == 0) return 0;
   const dim3 grid((unsigned)((per_sample + kOffsetThreads - 1) / kOffsetThreads), (unsigned)min(p.B, 65535));
-  p.pair = make_pair_const(NDIM, p.D, p.H, p.W, dtype == 0 ? 4 : 2);
-  const bool voxels = p.order == 3 || !pair_taps_applicable(p.D, p.H, p.W, (long long)p.D * p.H * p.W, dtype == 0 ? 4 : 2);
+  const long long vol = (long long)p.D * p.H * p.W;  // < 2^31
+  const size_t esz = dtype == 0 ? 4 : 2;
+  const bool voxels = p.order == 3 || !pair_taps_applicable(p.D, p.H, p.W, vol, 1);
+  const bool wide = !pair_taps_applicable(p.D, p.H, p.W, vol, esz);  // float volumes of 2^30 elements and more
+  p.pair = make_pair_const(NDIM, p.D, p.H, p.W, wide ? 1 : esz);
+#define MVR_OFFSET(T, VOXELS, WIDE) apply_offset_kernel<T, NDIM, VOXELS, WIDE><<<grid, kOffsetThreads, 0, st>>>(p)
   if (dtype == 0) {
-    if (voxels) apply_offset_kernel<float, NDIM, true><<<grid, kOffsetThreads, 0, st>>>(p);
-    else apply_offset_kernel<float, NDIM, false><<<grid, kOffsetThreads, 0, st>>>(p);
+    if (voxels) MVR_OFFSET(float, true, false);
+    else if (wide) MVR_OFFSET(float, false, true);
+    else MVR_OFFSET(float, false, false);
   } else {
-    if (voxels) apply_offset_kernel<__half, NDIM, true><<<grid, kOffsetThreads, 0, st>>>(p);
-    else apply_offset_kernel<__half, NDIM, false><<<grid, kOffsetThreads, 0, st>>>(p);
+    if (voxels) MVR_OFFSET(__half, true, false);
+    else MVR_OFFSET(__half, false, false);
   }
+#undef MVR_OFFSET
   return cudaGetLastError() == cudaSuccess ? 0 : -8;
 }
 

@@ -24,7 +24,7 @@ struct Plane2dLabel {
   int C, vec;
 };
 
-template <typename T, int ORDER, typename IT, bool IMG, bool LAB>
+template <typename T, int ORDER, typename IT, bool IMG, bool LAB, bool WIDE>
 __global__ void __launch_bounds__(kS3Threads, 5)
 resample_fwd_plane2d(const Params p, const PairConst pc, const Plane2dLabel lab, int tiles_w, int tiles_h, int blocks, int vec_store) {
   typedef Ar<T> A;
@@ -147,7 +147,7 @@ resample_fwd_plane2d(const Params p, const PairConst pc, const Plane2dLabel lab,
     axis_tap2<T, 0>(rx2, pc, ORDER, tx);
     axis_tap2<T, 1>(ry2, pc, ORDER, ty);
     const typename Q::M mask = lanes & ~(Q::outside(rx2, pc, 0) | Q::outside(ry2, pc, 1));
-    const PairTaps<T, 2> taps(tx, ty, ty, pc);
+    const PairTaps<T, 2, WIDE> taps(tx, ty, ty, pc);
     V w[4];
     pair_weights<T, 2>(tx, ty, ty, w);
     const T* plane = vol;
@@ -178,7 +178,9 @@ inline int try_launch_plane2d(const Params& p, int dtype, cudaStream_t st, const
   if ((dtype == 0 || label) && p.fm != kS3FloatPattern) return 1;
   if (p.ovol < 4096 || p.ow < 8) return 1;
   const size_t esz = dtype == 0 ? 4 : 2;
-  if (!pair_taps_applicable(1, p.H, p.W, p.vol, esz) || p.vol >= 0x7fffffffLL) return 1;
+  if (!pair_taps_applicable(1, p.H, p.W, p.vol, 1) || p.vol >= 0x7fffffffLL) return 1;
+  const bool wide = !pair_taps_applicable(1, p.H, p.W, p.vol, esz);  // float images of 2^30 pixels and more
+  if (wide && label) return 1;  // the fields get a launch each
   const int tiles_w = (p.ow + kS3TileW - 1) / kS3TileW, row_blocks = (p.oh + kS3TileH - 1) / kS3TileH;
   // a CTA's set-up costs about two row blocks; five CTAs per SM
   const int blocks = s3_pick_chunk((long long)p.R * tiles_w, std::min(row_blocks, 4096), 148 * 5, 2);
@@ -187,17 +189,17 @@ inline int try_launch_plane2d(const Params& p, int dtype, cudaStream_t st, const
   if (ctas > 0x7fffffffLL) return 1;
   const int vec_store = ((p.ow & 1) == 0) && (((uintptr_t)p.out) % (2 * esz) == 0);
   const unsigned grid = (unsigned)ctas;
-  const PairConst pc = make_pair_const(2, 1, p.H, p.W, esz);
+  const PairConst pc = make_pair_const(2, 1, p.H, p.W, wide ? 1 : esz);
   Plane2dLabel lab = {};
   if (label) lab = *label;
-#define MVR_PLANE(T, ORDER, IT, IMG, LAB) \
-  resample_fwd_plane2d<T, ORDER, IT, IMG, LAB><<<grid, kS3Threads, 0, st>>>(p, pc, lab, tiles_w, tiles_h, blocks, vec_store)
+#define MVR_PLANE(T, ORDER, IT, IMG, LAB, WIDE) \
+  resample_fwd_plane2d<T, ORDER, IT, IMG, LAB, WIDE><<<grid, kS3Threads, 0, st>>>(p, pc, lab, tiles_w, tiles_h, blocks, vec_store)
 #define MVR_PLANE_IT(T, ORDER, IMG)                                        \
   switch (label_dtype) {                                                   \
-    case LABEL_U8: MVR_PLANE(T, ORDER, unsigned char, IMG, true); break;   \
-    case LABEL_I16: MVR_PLANE(T, ORDER, short, IMG, true); break;          \
-    case LABEL_I32: MVR_PLANE(T, ORDER, int, IMG, true); break;            \
-    default: MVR_PLANE(T, ORDER, long long, IMG, true); break;             \
+    case LABEL_U8: MVR_PLANE(T, ORDER, unsigned char, IMG, true, false); break;   \
+    case LABEL_I16: MVR_PLANE(T, ORDER, short, IMG, true, false); break;          \
+    case LABEL_I32: MVR_PLANE(T, ORDER, int, IMG, true, false); break;            \
+    default: MVR_PLANE(T, ORDER, long long, IMG, true, false); break;             \
   }
   if (!p.in) {
     MVR_PLANE_IT(float, 0, false)
@@ -207,12 +209,15 @@ inline int try_launch_plane2d(const Params& p, int dtype, cudaStream_t st, const
     } else {
       if (p.order == 0) MVR_PLANE_IT(__half, 0, true) else MVR_PLANE_IT(__half, 1, true)
     }
+  } else if (wide) {
+    if (p.order == 0) MVR_PLANE(float, 0, int, true, false, true);
+    else MVR_PLANE(float, 1, int, true, false, true);
   } else if (dtype == 0) {
-    if (p.order == 0) MVR_PLANE(float, 0, int, true, false);
-    else MVR_PLANE(float, 1, int, true, false);
+    if (p.order == 0) MVR_PLANE(float, 0, int, true, false, false);
+    else MVR_PLANE(float, 1, int, true, false, false);
   } else {
-    if (p.order == 0) MVR_PLANE(__half, 0, int, true, false);
-    else MVR_PLANE(__half, 1, int, true, false);
+    if (p.order == 0) MVR_PLANE(__half, 0, int, true, false, false);
+    else MVR_PLANE(__half, 1, int, true, false, false);
   }
 #undef MVR_PLANE_IT
 #undef MVR_PLANE

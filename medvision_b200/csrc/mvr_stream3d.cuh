@@ -162,7 +162,8 @@ __device__ __forceinline__ void nearest_axis(T& l, T& h) {
 //     its low mantissa bits (conversion instructions run at a sixteenth of the rate of an addition); the bias of the raw
 //     bits is part of the address constant;
 //   * everything that depends on the sizes only comes from the host, in the kernel's parameters.
-// Byte offsets inside a channel's volume below 2^32.  (Reading the taps at fixed distances from one address, and putting the
+// Offsets inside a channel's volume are 32 bits: bytes, or elements where a volume has 4 GiB or more (WIDE; float volumes of
+// 2^30 to 2^31 elements), which costs a wider multiplication per load.  (Reading the taps at fixed distances from one address, and putting the
 // values right behind a branch where a coordinate sits on the last index, costs fewer instructions but more time: the branch
 // stands between the loads and the sum.  Elastic warp 2 x 128 x 256 x 256: 180 us, with the steps selected 152 us.)
 constexpr unsigned kTapMagic = 0x4B000000u;   // bits of 2^23
@@ -173,9 +174,10 @@ struct PairConst {
   unsigned last_raw[3];   // kTapMagic + size - 1
   float size[3];
   unsigned size_floor2[3], size_ceil2[3];  // half2 of the largest half <= size and of the smallest half >= size
-  unsigned sx, sy, sz, bias;  // byte strides, and -kTapMagic * (sx + sy + sz) modulo 2^32
+  unsigned sx, sy, sz, bias;  // strides in bytes (WIDE: elements), and -kTapMagic * (sx + sy + sz) modulo 2^32
 };
-inline PairConst make_pair_const(int ndim, int D, int H, int W, size_t esz) {
+// unit: size of an element, 1 for the WIDE form
+inline PairConst make_pair_const(int ndim, int D, int H, int W, size_t unit) {
   PairConst k;
   const int size[3] = {W, H, D};
   for (int a = 0; a < 3; ++a) {
@@ -186,20 +188,20 @@ inline PairConst make_pair_const(int ndim, int D, int H, int W, size_t esz) {
     k.size_floor2[a] = lo | (lo << 16);
     k.size_ceil2[a] = hi | (hi << 16);
   }
-  k.sx = (unsigned)esz;
-  k.sy = (unsigned)((size_t)W * esz);
-  k.sz = ndim == 3 ? (unsigned)((size_t)H * W * esz) : 0u;
-  k.bias = 0u - kTapMagic * ((unsigned)esz + k.sy + k.sz);
+  k.sx = (unsigned)unit;
+  k.sy = (unsigned)((size_t)W * unit);
+  k.sz = ndim == 3 ? (unsigned)((size_t)H * W * unit) : 0u;
+  k.bias = 0u - kTapMagic * ((unsigned)unit + k.sy + k.sz);
   return k;
 }
-inline bool pair_taps_applicable(int D, int H, int W, long long vol, size_t esz) {
-  return D <= kTapMaxSize && H <= kTapMaxSize && W <= kTapMaxSize && (unsigned long long)vol * esz <= 0xffffffffull;
+inline bool pair_taps_applicable(int D, int H, int W, long long vol, size_t unit) {
+  return D <= kTapMaxSize && H <= kTapMaxSize && W <= kTapMaxSize && (unsigned long long)vol * unit <= 0xffffffffull;
 }
 
 template <typename T>
 struct AxisTap2 {
   unsigned ra, rb;             // kTapMagic + lower tap index, per lane
-  unsigned da, db;             // byte step to the upper tap; 0: clamped onto the lower one, the last
+  unsigned da, db;             // step to the upper tap (unit of PairConst); 0: clamped onto the lower one, the last
   typename P2<T>::V l, h;
 };
 
@@ -235,13 +237,14 @@ __device__ __forceinline__ void axis_tap2(typename P2<T>::V c, const PairConst& 
 }
 
 // The 2^NDIM tap values of both lanes from one channel's volume, in the reference's tap order.
-template <typename T, int NDIM>
+template <typename T, int NDIM, bool WIDE = false>
 struct PairTaps {
   typedef typename P2<T>::V V;
-  unsigned a, b, dxa, dxb, dya, dyb, dza, dzb;  // byte offsets of the lowest taps, steps
+  unsigned a, b, dxa, dxb, dya, dyb, dza, dzb;  // offsets of the lowest taps, steps
   __device__ __forceinline__ PairTaps(const AxisTap2<T>& tx, const AxisTap2<T>& ty, const AxisTap2<T>& tz, const PairConst& k) {
-    a = tx.ra * (unsigned)sizeof(T) + (ty.ra * k.sy + k.bias);
-    b = tx.rb * (unsigned)sizeof(T) + (ty.rb * k.sy + k.bias);
+    constexpr unsigned unit = WIDE ? 1u : (unsigned)sizeof(T);
+    a = tx.ra * unit + (ty.ra * k.sy + k.bias);
+    b = tx.rb * unit + (ty.rb * k.sy + k.bias);
     dxa = tx.da; dxb = tx.db; dya = ty.da; dyb = ty.db;
     dza = dzb = 0u;
     if (NDIM == 3) {
@@ -251,7 +254,9 @@ struct PairTaps {
       dzb = tz.db;
     }
   }
-  __device__ __forceinline__ static T ld(const char* base, unsigned off) { return __ldg(reinterpret_cast<const T*>(base + off)); }
+  __device__ __forceinline__ static T ld(const char* base, unsigned off) {
+    return WIDE ? __ldg(reinterpret_cast<const T*>(base) + off) : __ldg(reinterpret_cast<const T*>(base + off));
+  }
   __device__ __forceinline__ void load(const T* vol, V* v) const {
     typedef P2<T> Q;
     const char* p = reinterpret_cast<const char*>(vol);
@@ -327,7 +332,7 @@ struct S3Launch {
 // rows below pair 0): positions change with depth, so all three axis taps are formed per voxel;
 // the x- and y-products of the rotation are formed once per thread, the z-products once per
 // depth and CTA (S3ZProd table).  Both lanes of a pair go through the same instructions.
-template <typename T, int NP>
+template <typename T, int NP, bool WIDE>
 __device__ __forceinline__ void s3_full_depth_loop(const Params& p, const S3Launch& L, const S3Shared<T>& sh, int npd, int c,
                                                    int pw0, int ph0, int row_step, bool vec_store, T* out0) {
   typedef Ar<T> A;
@@ -375,7 +380,7 @@ __device__ __forceinline__ void s3_full_depth_loop(const Params& p, const S3Laun
       V val = zero2;
       if (mask) {  // a lane outside keeps valid (clamped) addresses; its value is dropped
         V v[8], w[8];
-        PairTaps<T, 3>(tx, ty, tz, pc).load(vol, v);
+        PairTaps<T, 3, WIDE>(tx, ty, tz, pc).load(vol, v);
         pair_weights<T, 3>(tx, ty, tz, w);
         val = Q::apply(Q::add(zero2, pair_sum<T, 8>(w, v)), mask);
       }
@@ -496,7 +501,7 @@ __device__ __forceinline__ void s3_prologue(const Params& p, const S3Cta& k, S3S
 }
 
 // Everything after the prologue, gathering through L1/L2 with plain loads.
-template <typename T, bool GENERAL = false>
+template <typename T, bool GENERAL, bool WIDE>
 __device__ void s3_body_l1(const Params& p, const S3Launch& L, const S3Cta& k, S3Shared<T>& sh) {
   typedef Ar<T> A;
   typedef P2<T> Q;
@@ -551,7 +556,7 @@ __device__ void s3_body_l1(const Params& p, const S3Launch& L, const S3Cta& k, S
     axis_tap2<T, 1>(ry2, L.pair, p.order, ty);
     const typename Q::M mask = Q::make_mask(true, has_b) & ~(Q::outside(rx2, L.pair, 0) | Q::outside(ry2, L.pair, 1));
     // the pair's in-plane taps; the plane is added per depth (the z stride of the bias belongs to it)
-    PairTaps<T, 2> taps(tx, ty, ty, L.pair);
+    PairTaps<T, 2, WIDE> taps(tx, ty, ty, L.pair);
     taps.a += kTapMagic * L.pair.sz;
     taps.b += kTapMagic * L.pair.sz;
     const V lx2 = tx.l, hx2 = tx.h, ly2 = ty.l, hy2 = ty.h;
@@ -624,20 +629,20 @@ __device__ void s3_body_l1(const Params& p, const S3Launch& L, const S3Cta& k, S
   }
 
   // ---- general rotation: positions change with depth
-  s3_full_depth_loop<T, 1>(p, L, sh, npd, c, pw0, ph, kS3TileH, L.vec_store != 0, out);
+  s3_full_depth_loop<T, 1, WIDE>(p, L, sh, npd, c, pw0, ph, kS3TileH, L.vec_store != 0, out);
 }
 
 // The plane walk of the rows that no tensor map can describe (row pitch not a multiple of 16 bytes), and every roi of calls
 // with more rois than the gather launch can mark.  Like the plane-streaming kernel it may have been started before the gather
 // launch ahead of it is finished; one thread waits for that before the grid ends.
-template <typename T>
+template <typename T, bool WIDE>
 __global__ void __launch_bounds__(kS3Threads, sizeof(T) == 2 ? 4 : 3)
 resample_fwd_stream3d(const Params p, const S3Launch L) {
   __shared__ S3Shared<T> sh;
   const S3Cta k = s3_cta(p, L);
   if (!s3_filtered_out<T>(p, L, k)) {
     s3_prologue<T>(p, k, sh);
-    s3_body_l1<T>(p, L, k, sh);
+    s3_body_l1<T, false, WIDE>(p, L, k, sh);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
@@ -648,7 +653,7 @@ resample_fwd_stream3d(const Params p, const S3Launch L) {
 // whole grid is gone after a few loads -- and then strides over the (roi, channel, tile, chunk)
 // work items of the marked rois.
 constexpr int kS3RestMaxRois = 16384;
-template <typename T>
+template <typename T, bool WIDE>
 __global__ void __launch_bounds__(kS3Threads, 4)
 resample_fwd_stream3d_rest(const Params p, const S3Launch L, long long items) {
   __shared__ S3Shared<T> sh;
@@ -669,7 +674,7 @@ resample_fwd_stream3d_rest(const Params p, const S3Launch L, long long items) {
     const S3Cta k = s3_cta(p, L, item);
     if (!((general[k.n >> 5] >> (k.n & 31)) & 1u)) continue;  // CTA-uniform
     s3_prologue<T, true>(p, k, sh);
-    s3_body_l1<T, true>(p, L, k, sh);
+    s3_body_l1<T, true, WIDE>(p, L, k, sh);
     __syncthreads();  // the next item's prologue overwrites the tables
   }
 }

@@ -170,13 +170,13 @@ __device__ __forceinline__ void t3_mbar_arrive_one(unsigned bar) {
 // The rare ways out of the plane-streaming kernel (batch index outside the batch, coordinates that
 // are not finite, a tile whose footprint exceeds every box): the CTA's tile, 16 rows at a time,
 // through the gather path.
-template <typename T>
+template <typename T, bool WIDE>
 __device__ __forceinline__ void t3_fallback(const Params& p, const S3Launch& L, const S3Cta& k, S3Shared<T>& sh, int np) {
   if (threadIdx.x >= kS3Threads) return;
   for (int q = 0; q < np; ++q) {
     S3Cta k2 = k;
     k2.th = k.th * np + q;
-    if (k2.th * kS3TileH < p.oh) s3_body_l1<T>(p, L, k2, sh);
+    if (k2.th * kS3TileH < p.oh) s3_body_l1<T, false, WIDE>(p, L, k2, sh);
   }
 }
 
@@ -297,8 +297,9 @@ __device__ __forceinline__ void t3_consume(const Params& p, T3Shared<T>& sh, uns
 // NP = voxel pairs per thread: pair q sits 16*q output rows below pair 0, so a CTA covers a
 // 32 (w) x 16*NP (h) tile.  More work per thread spreads the per-depth control (table read, ring
 // hand-shake, loop) over more voxels.
-// VEC: even output width and aligned pointer, every stored pair is one vector store.
-template <typename T, int NP, bool VEC>
+// VEC: even output width and aligned pointer, every stored pair is one vector store.  WIDE: see mvr_stream3d.cuh (the boxes are
+// addressed by coordinates, so only the gather path of t3_fallback differs).
+template <typename T, int NP, bool VEC, bool WIDE>
 __device__ __forceinline__ void t3_body(const Params& p, const S3Launch& L, const T3Maps& maps) {
   typedef Ar<T> A;
   typedef P2<T> Q;
@@ -317,7 +318,7 @@ __device__ __forceinline__ void t3_body(const Params& p, const S3Launch& L, cons
   const RoiGeom<T>& g = sh.s3.g;
   const bool bad_batch = (g.batch < 0 || g.batch >= p.N);
   if (bad_batch || !sh.s3.zsep) {  // CTA-uniform: zeros and the status bit / coordinates that are not finite
-    t3_fallback<T>(p, L, k, sh.s3, NP);
+    t3_fallback<T, WIDE>(p, L, k, sh.s3, NP);
     return;
   }
 
@@ -458,7 +459,7 @@ __device__ __forceinline__ void t3_body(const Params& p, const S3Launch& L, cons
     for (int j = 0; j < maps.n; ++j)
       if (bsel < 0 && need_w <= maps.bw[j] && need_h <= maps.bh[j]) bsel = j;
     if (bsel < 0) {  // the tile's footprint exceeds every box: plain loads
-      t3_fallback<T>(p, L, k, sh.s3, NP);
+      t3_fallback<T, WIDE>(p, L, k, sh.s3, NP);
       return;
     }
   }
@@ -520,10 +521,10 @@ __device__ __forceinline__ void t3_body(const Params& p, const S3Launch& L, cons
 #undef T3_CONSUME
 }
 
-template <typename T, int NP, bool VEC>
+template <typename T, int NP, bool VEC, bool WIDE>
 __global__ void __launch_bounds__(kT3Threads, 3)
 resample_fwd_stream3d_tma(const Params p, const S3Launch L, const __grid_constant__ T3Maps maps) {
-  t3_body<T, NP, VEC>(p, L, maps);
+  t3_body<T, NP, VEC, WIDE>(p, L, maps);
   // This grid may have been started before the gather launch ahead of it in the stream has finished
   // (programmatic dependent launch).  One thread waits for that launch before the grid ends, so that
   // the completion of this grid implies the completion of both, whatever follows in the stream.
@@ -604,8 +605,10 @@ inline int try_launch_stream3d(const Params& p, int dtype, cudaStream_t st, T3La
   if (dtype == 0 && p.fm != kS3FloatPattern) return MVR_STREAM3D_NOT_APPLICABLE;
   // small outputs (detection heads) are better served one element per thread
   if (p.ovol < 4096 || p.ow < 8) return MVR_STREAM3D_NOT_APPLICABLE;
-  // 32-bit byte offsets inside a volume (float volumes of 2^30 elements and more go to the flat kernel)
-  if (!pair_taps_applicable(p.D, p.H, p.W, p.vol, dtype == 0 ? 4 : 2)) return MVR_STREAM3D_NOT_APPLICABLE;
+  // 32-bit offsets inside a volume: in bytes, and in elements for float volumes of 2^30 elements and more
+  if (p.vol >= 0x7fffffffLL || !pair_taps_applicable(p.D, p.H, p.W, p.vol, 1)) return MVR_STREAM3D_NOT_APPLICABLE;
+  const bool wide = !pair_taps_applicable(p.D, p.H, p.W, p.vol, dtype == 0 ? 4 : 2);  // never in half
+  if (wide) label = nullptr;  // its work items ride along with the narrow form only
 
   T3Maps maps;
   const bool tma = t3_make_maps(p, dtype, maps);
@@ -628,7 +631,7 @@ inline int try_launch_stream3d(const Params& p, int dtype, cudaStream_t st, T3La
   G.chunks = (p.od + G.chunk - 1) / G.chunk;
   G.vec_store = ((p.ow & 1) == 0) && (((uintptr_t)p.out) % (2 * esz) == 0);
   G.filter = 0;
-  G.pair = make_pair_const(3, p.D, p.H, p.W, esz);
+  G.pair = make_pair_const(3, p.D, p.H, p.W, wide ? 1 : esz);
   const long long g_ctas = g_per_depth * G.chunks;
   if (g_ctas > 0x7fffffffLL) return MVR_STREAM3D_NOT_APPLICABLE;
   // ---- geometry of the plane walk: 32 x 16*pairs tiles for the plane-streaming kernel, 32 x 16 without a tensor map; long
@@ -671,8 +674,8 @@ inline int try_launch_stream3d(const Params& p, int dtype, cudaStream_t st, T3La
       static int occ[2] = {0, 0};  // resident CTAs per SM of the two instantiations
       if (occ[dtype] == 0) {
         int n = 0;
-        if (dtype == 0) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, resample_fwd_stream3d_rest<float>, kS3Threads, 0);
-        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, resample_fwd_stream3d_rest<__half>, kS3Threads, 0);
+        if (dtype == 0) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, resample_fwd_stream3d_rest<float, false>, kS3Threads, 0);
+        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, resample_fwd_stream3d_rest<__half, false>, kS3Threads, 0);
         occ[dtype] = n > 0 ? n : 1;
       }
       G.filter = 0;
@@ -695,13 +698,15 @@ inline int try_launch_stream3d(const Params& p, int dtype, cudaStream_t st, T3La
         label->done = true;
       } else {
         const unsigned grid = (unsigned)std::min<long long>(g_ctas, 148LL * occ[dtype]);
-        if (dtype == 0) resample_fwd_stream3d_rest<float><<<grid, kS3Threads, 0, st>>>(p, G, g_ctas);
-        else resample_fwd_stream3d_rest<__half><<<grid, kS3Threads, 0, st>>>(p, G, g_ctas);
+        if (wide) resample_fwd_stream3d_rest<float, true><<<grid, kS3Threads, 0, st>>>(p, G, g_ctas);
+        else if (dtype == 0) resample_fwd_stream3d_rest<float, false><<<grid, kS3Threads, 0, st>>>(p, G, g_ctas);
+        else resample_fwd_stream3d_rest<__half, false><<<grid, kS3Threads, 0, st>>>(p, G, g_ctas);
       }
       overlap = true;
     } else {
-      if (dtype == 0) resample_fwd_stream3d<float><<<(unsigned)g_ctas, kS3Threads, 0, st>>>(p, G);
-      else resample_fwd_stream3d<__half><<<(unsigned)g_ctas, kS3Threads, 0, st>>>(p, G);
+      if (wide) resample_fwd_stream3d<float, true><<<(unsigned)g_ctas, kS3Threads, 0, st>>>(p, G);
+      else if (dtype == 0) resample_fwd_stream3d<float, false><<<(unsigned)g_ctas, kS3Threads, 0, st>>>(p, G);
+      else resample_fwd_stream3d<__half, false><<<(unsigned)g_ctas, kS3Threads, 0, st>>>(p, G);
     }
     if (cudaGetLastError() != cudaSuccess) return -8;
   }
@@ -717,22 +722,24 @@ inline int try_launch_stream3d(const Params& p, int dtype, cudaStream_t st, T3La
   cudaError_t err = cudaSuccess;
   if (!tma) {
     cfg.blockDim = dim3(kS3Threads);
-    err = dtype == 0 ? cudaLaunchKernelEx(&cfg, resample_fwd_stream3d<float>, p, L) : cudaLaunchKernelEx(&cfg, resample_fwd_stream3d<__half>, p, L);
+    err = wide         ? cudaLaunchKernelEx(&cfg, resample_fwd_stream3d<float, true>, p, L)
+          : dtype == 0 ? cudaLaunchKernelEx(&cfg, resample_fwd_stream3d<float, false>, p, L)
+                       : cudaLaunchKernelEx(&cfg, resample_fwd_stream3d<__half, false>, p, L);
     return err == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -8;
   }
   // more dynamic shared memory than the default limit: opt in (per function and device)
-#define T3_LAUNCH_V(TYPE, NP, VEC)                                                                           \
+#define T3_LAUNCH_V(TYPE, VEC, WIDE)                                                                         \
   {                                                                                                          \
-    cfg.dynamicSmemBytes = t3_dynamic_smem<TYPE>();                                              \
-    cudaFuncSetAttribute(resample_fwd_stream3d_tma<TYPE, NP, VEC>,                                           \
+    cfg.dynamicSmemBytes = t3_dynamic_smem<TYPE>();                                                          \
+    cudaFuncSetAttribute(resample_fwd_stream3d_tma<TYPE, kT3Pairs, VEC, WIDE>,                               \
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);            \
-    err = cudaLaunchKernelEx(&cfg, resample_fwd_stream3d_tma<TYPE, NP, VEC>, p, L, maps);                    \
+    err = cudaLaunchKernelEx(&cfg, resample_fwd_stream3d_tma<TYPE, kT3Pairs, VEC, WIDE>, p, L, maps);        \
   }
-#define T3_LAUNCH(TYPE, NP)                                                                                  \
+#define T3_LAUNCH(TYPE, WIDE)                                                                                \
   {                                                                                                          \
-    if (L.vec_store) T3_LAUNCH_V(TYPE, NP, true) else T3_LAUNCH_V(TYPE, NP, false)                           \
+    if (L.vec_store) T3_LAUNCH_V(TYPE, true, WIDE) else T3_LAUNCH_V(TYPE, false, WIDE)                       \
   }
-  if (dtype == 0) T3_LAUNCH(float, kT3Pairs) else T3_LAUNCH(__half, kT3Pairs)
+  if (wide) T3_LAUNCH(float, true) else if (dtype == 0) T3_LAUNCH(float, false) else T3_LAUNCH(__half, false)
 #undef T3_LAUNCH
 #undef T3_LAUNCH_V
   if (err != cudaSuccess) return -8;
