@@ -225,6 +225,7 @@ box_head_fwd(const Params p, int tasks, int chunks, int chunk) {
 
 constexpr int kBoxBwdThreads = 256;
 constexpr int kBoxBwdSamples = 4096;   // samples per bin and axis: larger grids go sample by sample
+constexpr int kBoxBwdMaxSmem = 200 * 1024;  // dynamic shared memory; a larger plan goes to the flat kernels
 constexpr int kBoxBwdPad = 8;          // zeros on either side of a contracted row (a window may overhang by 7)
 
 // positions that osz bins of the given size reach at most, counted from the one below the roi's start
@@ -606,13 +607,14 @@ inline int launch_box_head(const Params& p, bool fwd, cudaStream_t st) {
     return 1;
   }
   const BoxBwdPlan plan = box_bwd_plan(p);
-  if (plan.bytes > 200 * 1024 || p.ow > 0x7fff || p.oh > 0x7fff || p.od > 0x7fff || (long long)p.R * plan.chunks * plan.splits > 0x7fffffffLL) return 1;
+  if (plan.bytes > (size_t)kBoxBwdMaxSmem || p.ow > 0x7fff || p.oh > 0x7fff || p.od > 0x7fff || (long long)p.R * plan.chunks * plan.splits > 0x7fffffffLL) return 1;
   cfg.gridDim = dim3((unsigned)(p.R * plan.chunks * plan.splits));
   cfg.blockDim = dim3(kBoxBwdThreads);
   cfg.dynamicSmemBytes = plan.bytes;
+  // (the limit is the same for every call: one of this call's own size could land between another thread's setting and its launch)
 #define MVR_BOX_BWD(ND)                                                                                                   \
   {                                                                                                                       \
-    if (plan.bytes > 32 * 1024) cudaFuncSetAttribute(box_head_bwd<T, ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.bytes); \
+    if (plan.bytes > 32 * 1024) cudaFuncSetAttribute(box_head_bwd<T, ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBoxBwdMaxSmem); \
     cudaLaunchKernelEx(&cfg, box_head_bwd<T, ND>, p, plan);                                                               \
   }
   if (p.ndim == 2) MVR_BOX_BWD(2) else MVR_BOX_BWD(3)
