@@ -7,6 +7,7 @@
 // took 18 us per forward, 98 us per forward + backward of a head and about 300 us per augmentation call.
 #include <Python.h>
 
+#include <atomic>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -294,7 +295,48 @@ bool fields_into(const RoiOp& op, const at::Tensor& image, const at::Tensor& ima
 // again when the kernels that read it last are done (an event recorded behind them), so up to kSlots calls can be in
 // flight; the ring is locked for the whole call, so any number of threads and streams may use it.  It holds kSlots times
 // twice the largest call (some KB each) and goes away with release_staging().
+//
+// A call that is being captured into a CUDA graph takes no slot: a replay reads the host memory again, whatever eager calls
+// have done to the ring since.  It gets pinned memory of its own, which the graph and everything instantiated from it hold
+// as a user object, and device memory from the graph's own pool.
 constexpr int kSlots = 8;
+
+// Calls that allocate or wait must not break a capture that this or another thread has under way.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { C10_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode)); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Pinned memory of graphs that are gone.  A user object's destructor may not call CUDA, so it only leaves the address here;
+// the next eager upload and release_staging() free it.
+struct Orphans {
+  std::mutex mutex;
+  std::vector<void*> memory;
+  std::atomic<bool> any{false};
+};
+Orphans& orphans() {
+  static Orphans* o = new Orphans();  // a graph may outlive every static
+  return *o;
+}
+void CUDART_CB leave_orphan(void* memory) {
+  Orphans& o = orphans();
+  std::lock_guard<std::mutex> lock(o.mutex);
+  o.memory.push_back(memory);
+  o.any = true;
+}
+void free_orphans() {
+  Orphans& o = orphans();
+  if (!o.any) return;
+  std::vector<void*> memory;
+  {
+    std::lock_guard<std::mutex> lock(o.mutex);
+    memory.swap(o.memory);
+    o.any = false;
+  }
+  RelaxedCapture relaxed;
+  for (void* m : memory) cudaFreeHost(m);
+}
 
 struct Stage {
   std::mutex mutex;
@@ -306,6 +348,7 @@ struct Stage {
   int next = 0;
 
   void release() {
+    RelaxedCapture relaxed;
     for (int k = 0; k < kSlots; ++k) {
       if (recorded[k]) C10_CUDA_CHECK(cudaEventSynchronize(event[k]));
       recorded[k] = false;
@@ -318,6 +361,7 @@ struct Stage {
   void reserve(int64_t bytes, at::Device device) {
     if (bytes <= capacity) return;
     release();
+    RelaxedCapture relaxed;
     const int64_t want = std::max<int64_t>(8192, 2 * bytes);
     for (int k = 0; k < kSlots; ++k) {
       C10_CUDA_CHECK(cudaHostAlloc(&host[k], (size_t)want, cudaHostAllocDefault));
@@ -337,33 +381,60 @@ Stage& stage_of(int index) {
   return *g_stage[index];
 }
 
-// A slot of the ring for one call: fill host(), send(), launch the kernels that read device(); the destructor marks the
-// slot free behind them.
+// The memory of one call: fill host(), send(), launch the kernels that read device(); the destructor marks the slot free
+// behind them.
 struct Upload {
   Stage& stage;
-  std::lock_guard<std::mutex> lock;
+  std::unique_lock<std::mutex> lock;
   cudaStream_t stream;
   bool capturing;
-  int slot;
+  int slot = -1;
+  void* own_host = nullptr;  // captured calls
+  at::Tensor own_dev;
 
   Upload(int64_t bytes, at::Device device)
-      : stage(stage_of(device.index())), lock(stage.mutex), stream(c10::cuda::getCurrentCUDAStream(device.index()).stream()) {
+      : stage(stage_of(device.index())), stream(c10::cuda::getCurrentCUDAStream(device.index()).stream()) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     C10_CUDA_CHECK(cudaStreamIsCapturing(stream, &cs));
     capturing = cs != cudaStreamCaptureStatusNone;
+    if (capturing) {
+      own(std::max<int64_t>(bytes, 1), device);
+      return;
+    }
+    free_orphans();
+    lock = std::unique_lock<std::mutex>(stage.mutex);
     stage.reserve(bytes, device);
     slot = stage.next;
     stage.next = (slot + 1) % kSlots;
-    if (stage.recorded[slot] && !capturing) {
+    if (stage.recorded[slot]) {
+      RelaxedCapture relaxed;
       C10_CUDA_CHECK(cudaEventSynchronize(stage.event[slot]));
       stage.recorded[slot] = false;
     }
   }
-  void* host() { return stage.host[slot]; }
-  void* device() { return stage.dev[slot].data_ptr(); }
+  void own(int64_t bytes, at::Device device) {
+    own_dev = at::empty({bytes}, at::TensorOptions().dtype(at::kByte).device(device));
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cudaGraph_t graph = nullptr;
+    C10_CUDA_CHECK(cudaStreamGetCaptureInfo_v2(stream, &cs, nullptr, &graph, nullptr, nullptr));
+    TORCH_CHECK(cs == cudaStreamCaptureStatusActive && graph, "the capture of the current stream is invalid");
+    RelaxedCapture relaxed;
+    C10_CUDA_CHECK(cudaHostAlloc(&own_host, (size_t)bytes, cudaHostAllocDefault));
+    cudaUserObject_t object = nullptr;
+    cudaError_t err = cudaUserObjectCreate(&object, own_host, leave_orphan, 1, cudaUserObjectNoDestructorSync);
+    if (err != cudaSuccess) {
+      cudaFreeHost(own_host);
+    } else {
+      err = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
+      if (err != cudaSuccess) cudaUserObjectRelease(object, 1);
+    }
+    C10_CUDA_CHECK(err);
+  }
+  void* host() { return capturing ? own_host : stage.host[slot]; }
+  void* device() { return capturing ? own_dev.data_ptr() : stage.dev[slot].data_ptr(); }
   void send(int64_t bytes) { C10_CUDA_CHECK(cudaMemcpyAsync(device(), host(), (size_t)bytes, cudaMemcpyHostToDevice, stream)); }
   ~Upload() {
-    if (capturing) return;
+    if (capturing || slot < 0) return;
     if (cudaEventRecord(stage.event[slot], stream) == cudaSuccess) stage.recorded[slot] = true;
     else cudaStreamSynchronize(stream);
   }
@@ -385,7 +456,7 @@ struct StagedRois {
       h16[i] = at::Half(src[i]);  // round to nearest even
     }
     up.send(n * 6);
-    // views by pointer: the ring keeps the memory
+    // views by pointer: the upload (its ring, or its graph) keeps the memory
     auto none = [](void*) {};
     f32 = at::from_blob(up.device(), {R, K}, none, at::TensorOptions().dtype(at::kFloat).device(device));
     f16 = at::from_blob((char*)up.device() + 4 * n, {R, K}, none, at::TensorOptions().dtype(at::kHalf).device(device));
@@ -1059,6 +1130,7 @@ PyObject* py_release_staging(PyObject*, PyObject* index) {
   Stage& s = stage_of((int)int_arg(index));
   {
     pybind11::gil_scoped_release nogil;
+    free_orphans();
     std::lock_guard<std::mutex> lock(s.mutex);
     s.release();
   }

@@ -99,3 +99,45 @@ def test_backward_calls_of_several_threads_do_not_disturb_each_other():
     for th in threads:
         th.join()
     assert not bad, bad
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["affine", "elastic"])
+def test_captured_transforms_keep_their_parameters(kind):
+    """A replay gives what the captured call drew, whatever eager calls have done to the upload ring since -- used it over and
+    over, grown it, given it back -- and whichever of two graphs goes first."""
+    from medvision_b200 import _C
+    from medvision_b200.aug_cuda_batch import BatchCudaRandomElasticDeformation
+    img = torch.rand(2, 1, 20, 24, 32, generator=torch.Generator().manual_seed(1)).cuda()
+    t = (BatchCudaRandomAffine(1.0, scale=0.2, shift=0.1, rotate=25) if kind == "affine"
+         else BatchCudaRandomElasticDeformation(1.0, num_control_points=7))
+    src = {"img_dim": 3, "img": img, "img_fields": ["img"], "seg_fields": []}
+
+    def call(seed):
+        np.random.seed(seed)
+        return t(dict(src))["img"]
+
+    want = {seed: call(seed).clone() for seed in (1, 2)}
+    assert not torch.equal(want[1], want[2])
+    graphs = {}
+    for seed in (1, 2):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = call(seed)
+        graphs[seed] = graph, out
+    for k in range(20):
+        call(100 + k)
+    big = torch.rand(300, 1, 4, 4, 4).cuda()
+    BatchCudaRandomAffine(1.0, scale=0.2, shift=0.1, rotate=25)(dict(src, img=big))  # more rois than the ring was made for
+    _C.release_cached_memory()
+    for k in range(20):
+        call(100 + k)
+    for seed in (2, 1, 2):
+        graph, out = graphs[seed]
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want[seed])
+    del graph, out, graphs   # their memory goes back with the next call
+    assert torch.equal(call(1), want[1])
+    _C.release_cached_memory()
