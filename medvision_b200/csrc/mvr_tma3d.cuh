@@ -43,8 +43,38 @@ constexpr int kT3Pairs = 2;                   // voxel pairs per consumer thread
 constexpr int kT3RingBytes = 60 * 1024;       // plane ring of one CTA: what three resident CTAs per SM can share
 static_assert(kT3RingBytes >= 3 * ((kT3MaxBoxBytes + 127) & ~127), "the ring must hold three of the largest boxes");
 
+// Boxes in elements; a tile takes the first that holds its taps.  Their widths keep the row pitch at 8 or 24 (mod 32) four-byte words: the four rows a
+// warp reads then fall into different shared-memory banks.  Each width has a depth loop of its own (t3_consume), whose loads
+// take the row pitch as an immediate.
+constexpr int kT3Widths = 3;
+template <typename T> struct T3Boxes;
+template <> struct T3Boxes<__half> {
+  static constexpr int n = 6;
+  static constexpr int width[kT3Widths] = {48, 80, 112};
+  static constexpr int box[n][2] = {{48, 40}, {48, 48}, {80, 40}, {80, 56}, {80, 72}, {112, 56}};
+};
+template <> struct T3Boxes<float> {
+  static constexpr int n = 4;
+  static constexpr int width[kT3Widths] = {40, 56, 72};
+  static constexpr int box[n][2] = {{40, 40}, {56, 40}, {56, 56}, {72, 40}};
+};
+// every box has one of the widths that a depth loop exists for, fits a ring slot, and its rows are whole 16-byte units in
+// different banks
+template <typename T>
+constexpr bool t3_boxes_sound() {
+  typedef T3Boxes<T> B;
+  for (int j = 0; j < B::n; ++j) {
+    bool known = false;
+    for (int k = 0; k < kT3Widths; ++k) known = known || B::box[j][0] == B::width[k];
+    const int pitch = B::box[j][0] * (int)sizeof(T);
+    if (!known || pitch % 16 || (pitch / 4 % 32 != 8 && pitch / 4 % 32 != 24) || pitch * B::box[j][1] > kT3MaxBoxBytes) return false;
+  }
+  return B::n <= kT3MaxBoxes;
+}
+static_assert(t3_boxes_sound<__half>() && t3_boxes_sound<float>(), "box table");
+
 struct T3Maps {
-  CUtensorMap map[kT3MaxBoxes];  // same tensor (W, H, N*C*D), different box sizes, ascending
+  CUtensorMap map[kT3MaxBoxes];  // same tensor (W, H, N*C*D), the boxes of T3Boxes
   int bw[kT3MaxBoxes], bh[kT3MaxBoxes];
   int n;
 };
@@ -447,7 +477,7 @@ __device__ __forceinline__ void t3_body(const Params& p, const S3Launch& L, cons
   }
   __syncthreads();  // the last CTA-wide barrier: from here on warps run independently
 
-  // ---- choose the smallest box that holds the tile's taps (+1 neighbour column and row)
+  // ---- choose the first box that holds the tile's taps (+1 neighbour column and row)
   const int esz = (int)sizeof(T);
   const int xalign = 16 / esz;
   const bool any_inside = sh.box[0] <= sh.box[1];
@@ -515,9 +545,10 @@ __device__ __forceinline__ void t3_body(const Params& p, const S3Launch& L, cons
   T* o = (T*)p.out + k.nc * p.ovol + (long long)k.pd0 * plane_o + (long long)(act[0] ? ph0 : 0) * p.ow + (col_ok ? pw0 : 0);
 #define T3_CONSUME(BW) \
   t3_consume<T, NP, VEC, BW>(p, sh, L.wait_tries, npd, any_inside, stride, nst, full_s, oa, ob, lx2, hx2, ly2, hy2, mask, act, has_b, o, plane_o)
-  if (bw == (sizeof(T) == 2 ? 112 : 72)) T3_CONSUME((sizeof(T) == 2 ? 112 : 72));
-  else if (bw == (sizeof(T) == 2 ? 80 : 56)) T3_CONSUME((sizeof(T) == 2 ? 80 : 56));
-  else T3_CONSUME((sizeof(T) == 2 ? 48 : 40));
+  constexpr int w0 = T3Boxes<T>::width[0], w1 = T3Boxes<T>::width[1], w2 = T3Boxes<T>::width[2];
+  if (bw == w2) T3_CONSUME(w2);
+  else if (bw == w1) T3_CONSUME(w1);
+  else T3_CONSUME(w0);  // (or no plane at all)
 #undef T3_CONSUME
 }
 
@@ -558,20 +589,14 @@ inline bool t3_make_maps(const Params& p, int dtype, T3Maps& m) {
   const size_t esz = dtype == 0 ? 4 : 2;
   const unsigned long long planes = (unsigned long long)p.N * p.C * p.D;
   if (((uintptr_t)p.in) % 16 != 0 || ((size_t)p.W * esz) % 16 != 0 || planes > 0x7fffffffULL) return false;
-  // boxes in elements, ascending in area; every one fits kT3MaxBoxBytes
-  // Box widths keep the row pitch at 8 or 24 (mod 32) four-byte words: the four rows a warp
-  // reads then fall into different shared-memory banks.
-  static const int half_boxes[][2] = {{48, 40}, {48, 48}, {80, 40}, {80, 56}, {80, 72}, {112, 56}};
-  static const int float_boxes[][2] = {{40, 40}, {56, 40}, {56, 56}, {72, 40}};
-  const int (*boxes)[2] = dtype == 0 ? float_boxes : half_boxes;
-  const int nb = dtype == 0 ? 4 : 6;
+  const int (*boxes)[2] = dtype == 0 ? T3Boxes<float>::box : T3Boxes<__half>::box;
+  const int nb = dtype == 0 ? T3Boxes<float>::n : T3Boxes<__half>::n;
   const cuuint64_t gdim[3] = {(cuuint64_t)p.W, (cuuint64_t)p.H, (cuuint64_t)planes};
   const cuuint64_t gstride[2] = {(cuuint64_t)p.W * esz, (cuuint64_t)p.W * p.H * esz};
   const cuuint32_t estride[3] = {1, 1, 1};
   m.n = 0;
   for (int j = 0; j < nb; ++j) {
     const cuuint32_t box[3] = {(cuuint32_t)boxes[j][0], (cuuint32_t)boxes[j][1], 1};
-    if ((size_t)box[0] * box[1] * esz > (size_t)kT3MaxBoxBytes) continue;
     CUresult r = enc(&m.map[m.n], dtype == 0 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3,
                      const_cast<void*>(p.in), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
                      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
