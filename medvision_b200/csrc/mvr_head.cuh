@@ -20,7 +20,6 @@
 
 namespace mvr {
 
-constexpr int kBoxMaxEntries = 256;  // forward: table entries (bins x samples) per axis; larger grids form taps on the fly
 
 // one axis of a box: decode as decode_roi does it
 template <typename T>
@@ -86,14 +85,16 @@ __device__ __forceinline__ BoxTap<T> box_tap(const BoxAxis<T>& x, int pos, int i
 
 constexpr int kBoxFwdThreads = 256;
 constexpr int kBoxSegment = 128;     // sample values per warp and channel between two rounds of sums
+constexpr int kBoxFwdSmallMap = 96;
+constexpr int kBoxFwdTable = 31 * 1024;  // bytes of both axes' tables at most: four CTAs per SM, no opt-in to more memory
 
 // 2D forward with a run-time sample grid (adaptive sampling, three and more samples per axis), float.  A warp takes one output
 // row of G channels.  Its lanes first take SAMPLES, neighbouring samples of the row in neighbouring lanes -- a load of one
 // tap then touches one or two lines, where one output bin per lane spread it over ten -- form the weights of a sample once
 // for all channels and leave the values in shared memory; then its lanes take OUTPUTS and add the values up in the
-// reference's order.  Bound by instruction issue (70 %).  Measured on 200 boxes of 8-64 px, 32 channels of 101 x 135, 7 x 7
-// bins: 39.6 us, the flat kernel 59.3 us.  In 3D (few samples per line) and in half (loads half as wide) it does not gain:
-// those stay with the flat kernel.
+// reference's order.  The tables hold the samples of any box inside the map (up to 1980 positions on both axes together); the
+// taps of a larger grid are formed as they are used.  In 3D (few samples per line) and in half (loads half as wide) it does
+// not gain: those stay with the flat kernel.
 template <typename T>
 __device__ __forceinline__ void box_zero_task(const Params& p, T* out, int task, int group) {
   const int rows = p.od * p.oh, cg = task / rows, row = task - cg * rows, c0 = cg * group, nc = min(group, p.C - c0);
@@ -121,11 +122,12 @@ __device__ __forceinline__ T box_output_direct(const Params& p, const BoxAxis<T>
 
 template <typename T, int G>
 __global__ void __launch_bounds__(kBoxFwdThreads, 4)
-box_head_fwd(const Params p, int tasks, int chunks, int chunk) {
+box_head_fwd(const Params p, int tasks, int chunks, int chunk, int entries_x, int entries_y) {
   typedef Ar<T> A;
   constexpr int fm = kFlatFm;
-  __shared__ BoxTap<T> tab[2][kBoxMaxEntries];
+  extern __shared__ __align__(16) unsigned char box_table[];
   __shared__ T values[kBoxFwdThreads / 32][G][kBoxSegment];
+  BoxTap<T>* const tab[2] = {reinterpret_cast<BoxTap<T>*>(box_table), reinterpret_cast<BoxTap<T>*>(box_table) + entries_x};
   flat_grid_dependency();
   const int n = (int)blockIdx.x / chunks;
   const int t_begin = ((int)blockIdx.x - n * chunks) * chunk, t_end = min(t_begin + chunk, tasks);
@@ -144,8 +146,7 @@ box_head_fwd(const Params p, int tasks, int chunks, int chunk) {
   const int gx = ax[0].grid, gy = ax[1].grid;
   const T count = A::fi(max(gx * gy, 1));
   const T* const vol0 = (const T*)p.in + (long long)batch * p.C * p.vol;
-  if ((long long)p.ow * gx > kBoxMaxEntries || (long long)p.oh * gy > kBoxMaxEntries) {
-    // a grid beyond the tables: output by output, taps on the fly
+  if ((double)p.ow * gx * max(gy, 1) > 1.0e9) {  // sample numbers beyond 32 bits: output by output
     for (int t = t_begin; t < t_end; ++t) {
       const int cg = t / p.oh, ph = t - cg * p.oh, c0 = cg * G, nc = min(G, p.C - c0);
       for (int i = threadIdx.x; i < nc * p.ow; i += kBoxFwdThreads) {
@@ -155,9 +156,10 @@ box_head_fwd(const Params p, int tasks, int chunks, int chunk) {
     }
     return;
   }
+  const bool tabled = p.ow * gx <= entries_x && (long long)p.oh * gy <= entries_y;  // CTA-uniform
 #pragma unroll
   for (int a = 0; a < 2; ++a) {
-    const int g = ax[a].grid, m = (a == 0 ? p.ow : p.oh) * g;
+    const int g = ax[a].grid, m = tabled ? (a == 0 ? p.ow : p.oh) * g : 0;
     // the axes' entries start at different threads, so that they are formed in one go
     for (int e = (int)threadIdx.x ^ (a * (kBoxFwdThreads / 2)); e < m; e += kBoxFwdThreads) {
       const int pos = e / g;
@@ -171,54 +173,68 @@ box_head_fwd(const Params p, int tasks, int chunks, int chunk) {
   const int x_lo = my_pw * gx, x_hi = x_lo + gx;
   const unsigned off_mask = ~kBoxOutside;
 
-  for (int task = t_begin + warp; task < t_end; task += kBoxFwdThreads / 32) {
-    const int cg = task / p.oh, ph = task - cg * p.oh;
-    const int c0 = cg * G, nc = min(G, p.C - c0);
-    // channels beyond the last repeat it
-    const T* vol[G];
+  // a copy of the loop for grids beyond the tables: one loop with the choice inside it costs the others 15 %
+  auto rows = [&](auto tables) {
+    constexpr bool kTabled = decltype(tables)::value != 0;
+    for (int task = t_begin + warp; task < t_end; task += kBoxFwdThreads / 32) {
+      const int cg = task / p.oh, ph = task - cg * p.oh;
+      const int c0 = cg * G, nc = min(G, p.C - c0);
+      // channels beyond the last repeat it
+      const T* vol[G];
 #pragma unroll
-    for (int c = 0; c < G; ++c) vol[c] = vol0 + (long long)min(c0 + c, p.C - 1) * p.vol;
-    T acc = zero;
-    const BoxTap<T>* const ty_row = &tab[1][ph * gy];
-    for (int s0 = 0, iy0 = 0, x0s = 0; s0 < plane_samples; s0 += kBoxSegment) {
-      const int m = min(kBoxSegment, plane_samples - s0);
-      int xg = x0s + lane, iy = iy0;
-      __syncwarp();  // the sums of the segment before are done with the values
-      for (int k = lane; k < m; k += 32, xg += 32) {
-        while (xg >= row_samples) {
-          xg -= row_samples;
-          ++iy;
-        }
-        const BoxTap<T> tx = tab[0][xg], ty = ty_row[iy];
-        const bool outside = ((tx.o1 | ty.o1) & kBoxOutside) != 0;
-        const unsigned a0 = tx.o0 + ty.o0, a1 = (tx.o1 & off_mask) + ty.o0;
-        const unsigned b0 = tx.o0 + (ty.o1 & off_mask), b1 = (tx.o1 & off_mask) + (ty.o1 & off_mask);
-        T* dst = &values[warp][0][k];
-        const T w[4] = {A::mul(ty.h, tx.h), A::mul(ty.h, tx.l), A::mul(ty.l, tx.h), A::mul(ty.l, tx.l)};
+      for (int c = 0; c < G; ++c) vol[c] = vol0 + (long long)min(c0 + c, p.C - 1) * p.vol;
+      T acc = zero;
+      const BoxTap<T>* const ty_row = tab[1] + ph * gy;
+      for (int s0 = 0, iy0 = 0, x0s = 0; s0 < plane_samples; s0 += kBoxSegment) {
+        const int m = min(kBoxSegment, plane_samples - s0);
+        int xg = x0s + lane, iy = iy0;
+        __syncwarp();  // the sums of the segment before are done with the values
+        for (int k = lane; k < m; k += 32, xg += 32) {
+          while (xg >= row_samples) {
+            xg -= row_samples;
+            ++iy;
+          }
+          BoxTap<T> tx, ty;
+          if (kTabled) {
+            tx = tab[0][xg];
+            ty = ty_row[iy];
+          } else {
+            const int pw = xg / gx;
+            tx = box_tap<T>(ax[0], pw, xg - pw * gx, p.W, 1u, p.order);
+            ty = box_tap<T>(ax[1], ph, iy, p.H, (unsigned)p.W, p.order);
+          }
+          const bool outside = ((tx.o1 | ty.o1) & kBoxOutside) != 0;
+          const unsigned a0 = tx.o0 + ty.o0, a1 = (tx.o1 & off_mask) + ty.o0;
+          const unsigned b0 = tx.o0 + (ty.o1 & off_mask), b1 = (tx.o1 & off_mask) + (ty.o1 & off_mask);
+          T* dst = &values[warp][0][k];
+          const T w[4] = {A::mul(ty.h, tx.h), A::mul(ty.h, tx.l), A::mul(ty.l, tx.h), A::mul(ty.l, tx.l)};
 #pragma unroll
-        for (int c = 0; c < G; ++c) {
-          const T tap[4] = {__ldg(vol[c] + a0), __ldg(vol[c] + a1), __ldg(vol[c] + b0), __ldg(vol[c] + b1)};
-          const T sum = tap_sum<T, 4>(w, tap, fm);
-          dst[c * kBoxSegment] = outside ? zero : sum;  // a sample outside keeps valid (clamped) addresses
+          for (int c = 0; c < G; ++c) {
+            const T tap[4] = {__ldg(vol[c] + a0), __ldg(vol[c] + a1), __ldg(vol[c] + b0), __ldg(vol[c] + b1)};
+            const T sum = tap_sum<T, 4>(w, tap, fm);
+            dst[c * kBoxSegment] = outside ? zero : sum;  // a sample outside keeps valid (clamped) addresses
+          }
         }
-      }
-      __syncwarp();
-      if (my_ch < nc) {
-        const T* v = values[warp][my_ch];
-        for (int l0 = -x0s; l0 < m; l0 += row_samples) {  // start of each sample line inside the segment
-          const int hi = min(m, l0 + x_hi);
+        __syncwarp();
+        if (my_ch < nc) {
+          const T* v = values[warp][my_ch];
+          for (int l0 = -x0s; l0 < m; l0 += row_samples) {  // start of each sample line inside the segment
+            const int hi = min(m, l0 + x_hi);
 #pragma unroll 4
-          for (int k = max(0, l0 + x_lo); k < hi; ++k) acc = A::add(acc, v[k]);
+            for (int k = max(0, l0 + x_lo); k < hi; ++k) acc = A::add(acc, v[k]);
+          }
+        }
+        x0s += kBoxSegment;
+        while (x0s >= row_samples) {
+          x0s -= row_samples;
+          ++iy0;
         }
       }
-      x0s += kBoxSegment;
-      while (x0s >= row_samples) {
-        x0s -= row_samples;
-        ++iy0;
-      }
+      if (my_ch < nc) out[(long long)(c0 + my_ch) * ovol + ph * p.ow + my_pw] = A::div(acc, count);
     }
-    if (my_ch < nc) out[(long long)(c0 + my_ch) * ovol + ph * p.ow + my_pw] = A::div(acc, count);
-  }
+  };
+  if (tabled) rows(FlatCount<1>());
+  else rows(FlatCount<0>());
 }
 
 // ---- backward ----------------------------------------------------------------------------------------------------
@@ -574,8 +590,15 @@ inline int launch_box_head(const Params& p, bool fwd, cudaStream_t st) {
   if (fwd) {
     // one and two samples per axis: the flat kernel, whose unrolled samples keep more loads in flight
     if (p.ndim != 2 || sizeof(T) != 4 || p.sampling_ratio == 1 || p.sampling_ratio == 2 || p.ow > 32) return 1;
-    // calls that fill the chip with four channels per thread (resample_flat_channels_fwd): 1 538 000 outputs 48 -> 39 us
-    if (p.C > 2 && (long long)p.R * ((p.C + 3) / 4) * p.ovol >= 148 * 2048) return 1;
+    // few outputs, which the flat kernel shares among eight lanes each: 5 900 outputs of boxes of 8-64 px 12.3 us here, 7.4
+    // there, of 10-120 px 29.9 and 15.7; 25 000 outputs 13.7 and 19.1, 38.8 and 60.9
+    if ((double)p.R * per_roi * 8 <= 148.0 * 384) return 1;
+    // calls that fill the chip with four channels per thread (resample_flat_channels_fwd), on small maps: its threads take the
+    // samples of a bin one after the other, which suits small bins, and how large the boxes are the host only knows from the
+    // map.  1 606 000 outputs, adaptive, here and there: boxes of 4-29 px on 42 x 58 49 and 39 us, of 6-45 on 84 x 90
+    // 83 and 91 (four times the channels 311 and 278), of 8-64 on 101 x 135 139 and
+    // 183, of 10-120 on 200 x 336 434 and 805; three samples per axis: 46 and 38, 47 and 49, 48 and 69
+    if (p.C > 2 && std::max(p.W, p.H) <= kBoxFwdSmallMap && (long long)p.R * ((p.C + 3) / 4) * p.ovol >= 148 * 2048) return 1;
     const int group = p.C >= 3 && p.ow <= 8 ? 4 : p.C >= 2 && p.ow <= 16 ? 2 : 1;  // group * ow lanes hold outputs
     const int tasks = ((p.C + group - 1) / group) * p.oh;
     // CTAs of a roi: sixteen per SM in total (rois differ in size by two orders of magnitude in samples, so short CTAs
@@ -587,9 +610,14 @@ inline int launch_box_head(const Params& p, bool fwd, cudaStream_t st) {
     if ((long long)p.R * chunks > 0x7fffffffLL) return 1;
     cfg.gridDim = dim3((unsigned)(p.R * chunks));
     cfg.blockDim = dim3(kBoxFwdThreads);
-    if (group == 4) cudaLaunchKernelEx(&cfg, box_head_fwd<float, 4>, p, tasks, (int)chunks, chunk);
-    else if (group == 2) cudaLaunchKernelEx(&cfg, box_head_fwd<float, 2>, p, tasks, (int)chunks, chunk);
-    else cudaLaunchKernelEx(&cfg, box_head_fwd<float, 1>, p, tasks, (int)chunks, chunk);
+    // samples per axis of a box as large as the map, an axis that does not fit going without
+    const long long room = kBoxFwdTable / (long long)sizeof(BoxTap<float>);
+    auto samples = [&](int bins, int size) { return (long long)bins * (p.sampling_ratio > 0 ? p.sampling_ratio : (size + bins - 1) / bins); };
+    const int ex = (int)std::min(samples(p.ow, p.W), room), ey = (int)std::min(samples(p.oh, p.H), room - ex);
+    cfg.dynamicSmemBytes = (size_t)(ex + ey) * sizeof(BoxTap<float>);
+    if (group == 4) cudaLaunchKernelEx(&cfg, box_head_fwd<float, 4>, p, tasks, (int)chunks, chunk, ex, ey);
+    else if (group == 2) cudaLaunchKernelEx(&cfg, box_head_fwd<float, 2>, p, tasks, (int)chunks, chunk, ex, ey);
+    else cudaLaunchKernelEx(&cfg, box_head_fwd<float, 1>, p, tasks, (int)chunks, chunk, ex, ey);
     return 0;
   }
   // Forming the tables costs 5-8 us, which the flat kernels do not spend: they are faster where few reductions leave.

@@ -19,6 +19,10 @@ CASES = [
     ((64, 97),        2, 40, (14, 14),  3, 1, torch.float32),   # groups of two
     ((50, 63),        3, 9,  (3, 33),   0, 1, torch.float32),   # rows wider than a warp
     ((37, 41),        4, 12, (7, 7),    0, 0, torch.float32),   # nearest
+    ((37, 41),        5, 40, (7, 7),    0, 1, torch.float32),   # enough outputs for a row per warp
+    ((37, 41),        4, 40, (7, 7),    0, 0, torch.float32),
+    ((600, 530),      2, 90, (7, 7),    0, 1, torch.float32),
+    ((70, 2100),      4, 40, (7, 7),    0, 1, torch.float32),   # samples beyond the forward's tables
     ((33, 27),        3, 60, (7, 7),    0, 1, torch.float16),
     ((64, 97),        6, 90, (14, 14),  2, 1, torch.float16),
     ((19, 23, 29),    7, 80, (7, 6, 5), 3, 1, torch.float32),
