@@ -10,9 +10,8 @@
 // x, and writes the touched rows of the volume, four (eight for half) consecutive elements per reduction, neighbouring lanes
 // on neighbouring windows.  One reduction per window and roi instead of 1.25 per sample and tap row: the reduction path of
 // this GPU charges per operation (mvr_generic.cuh), and that was the whole cost of these kernels.  The sums are formed in
-// float for every element type.  Measured (us, flat kernel -> here): 200 boxes of 8-64 px, adaptive, 32 x 101 x 135 float
-// 145 -> 35; 790 boxes of 4-29, adaptive, 2 x 58 x 42 x 88 float 314 -> 53; 169 boxes, 2 samples, 5 x 35 x 65 x 48 half
-// 69 -> 18.  Bound by instruction issue (forming the windows, about 60 per 16 bytes), the tables' latency on small calls.
+// float for every element type.  A box whose samples lie too far apart for that, or that exceeds the tables, goes sample by
+// sample in the same CTA.
 //
 // Launched as programmatic dependents like the flat kernels (mvr_flat.cuh).
 #pragma once
@@ -278,9 +277,10 @@ inline BoxBwdPlan box_bwd_plan(const Params& p) {
     while (q.channels < 8 && q.channels * 2 <= p.C && (long long)p.R * ((p.C + 2 * q.channels - 1) / (2 * q.channels)) >= 148LL * 4) q.channels *= 2;
   while (q.channels > 1 && (words + per_channel * q.channels) * 4 > 64 * 1024) q.channels /= 2;
   q.chunks = (p.C + q.channels - 1) / q.channels;
-  // 3D: with few (roi, channel) pairs, several CTAs per pair, each a share of the planes (every one forms the tables)
+  // With few (roi, channel) pairs, several CTAs per pair: each a share of the planes in 3D (every one forms the tables), or of the
+  // samples of a box beyond the tables
   q.splits = 1;
-  if (p.ndim == 3)
+  if (p.ndim == 3 || std::max(p.W, p.H) > most)
     while (q.splits < 8 && (long long)p.R * q.chunks * q.splits < 148LL * 2) q.splits *= 2;
   if (p.ndim == 3) words += (size_t)(kBoxBwdThreads / 32) * p.oh * q.row;  // a plane's rows per warp
   q.bytes = (words + per_channel * q.channels) * 4;
@@ -305,9 +305,121 @@ __device__ __forceinline__ void box_red_window(__half* base, const float* v) {
 // n / d for 0 <= n < 2^20, d >= 1, inv = 1 / d: the float quotient is off by less than one half of 1 / d
 __device__ __forceinline__ int box_div(int n, float inv) { return __float2int_rz(((float)n + 0.5f) * inv); }
 
+// A roi's channels sample by sample: boxes beyond the tables, and boxes whose samples lie so far apart that most windows of a
+// row would be empty.  Threads take (sample line, output) items; the samples of a line that fall into the same cell are summed
+// in float and leave together, as in the flat kernel.  The taps of an axis are tabled where the shared memory holds them.
+// part of parts: this CTA's share of the items.
 template <typename T, int NDIM>
-__global__ void __launch_bounds__(kBoxBwdThreads)
-box_head_bwd(const Params p, const BoxBwdPlan plan) {
+struct BoxAxes {
+  BoxAxis<T> ax[NDIM];
+};
+template <typename T, int NDIM>
+__device__ __noinline__ void box_bwd_samples(const Params& p, const BoxAxes<T, NDIM> roi_axes, T* grad, const T* go, int nc, float inv_count, int part,
+                                             int parts, size_t smem_bytes, const T* tensor_lo, const T* tensor_hi) {
+  typedef Ar<T> A;
+  constexpr int kRows = 1 << (NDIM - 1);
+  extern __shared__ __align__(16) float box_smem[];
+  const BoxAxis<T>* const ax = roi_axes.ax;
+  const int size[3] = {p.W, p.H, p.D}, osz[3] = {p.ow, p.oh, p.od};
+  const unsigned stride[3] = {1u, (unsigned)p.W, (unsigned)(p.W * p.H)};
+  BoxTap<T>* tab[NDIM];
+  BoxTap<T>* next = reinterpret_cast<BoxTap<T>*>(box_smem);
+  long long room = (long long)(smem_bytes / sizeof(BoxTap<T>));
+#pragma unroll
+  for (int a = 0; a < NDIM; ++a) {
+    const long long m = (long long)osz[a] * ax[a].grid;
+    tab[a] = m <= room ? next : nullptr;
+    if (m > room) continue;
+    next += m;
+    room -= m;
+  }
+  __syncthreads();  // whoever used the shared memory before is done
+#pragma unroll
+  for (int a = 0; a < NDIM; ++a)
+    if (tab[a])
+      for (int e = threadIdx.x; e < osz[a] * ax[a].grid; e += kBoxBwdThreads) {
+        const int bin = e / ax[a].grid;
+        tab[a][e] = box_tap<T>(ax[a], bin, e - bin * ax[a].grid, size[a], stride[a], p.order);
+      }
+  __syncthreads();
+  auto tap = [&](int a, int bin, int i) {
+    return tab[a] ? tab[a][bin * ax[a].grid + i] : box_tap<T>(ax[a], bin, i, size[a], stride[a], p.order);
+  };
+  const int gx = ax[0].grid, gy = ax[1].grid, outputs = nc * (int)p.ovol;  // outputs: below 2^20
+  const long long items = (long long)outputs * gy * (NDIM == 3 ? ax[NDIM - 1].grid : 1);
+  const float inv_out = 1.0f / (float)outputs, inv_vol = 1.0f / (float)p.ovol, inv_w = 1.0f / (float)p.ow, inv_h = 1.0f / (float)p.oh,
+              inv_gy = 1.0f / (float)gy;
+  auto walk = [&](auto tables) {
+    constexpr bool kTabled = decltype(tables)::value != 0;
+    for (long long item = part * kBoxBwdThreads + threadIdx.x; item < items; item += parts * kBoxBwdThreads) {
+      int iy, iz = 0, o;
+      if (items < (1 << 20)) {
+        const int line = box_div((int)item, inv_out);
+        o = (int)item - line * outputs;
+        if (NDIM == 3) iz = box_div(line, inv_gy);
+        iy = line - iz * gy;
+      } else {
+        const long long line = item / outputs;
+        o = (int)(item - line * outputs);
+        if (NDIM == 3) iz = (int)(line / gy);
+        iy = (int)(line - (long long)iz * gy);
+      }
+      const int c = box_div(o, inv_vol), v = o - c * (int)p.ovol;
+      const int row = box_div(v, inv_w), pw = v - row * p.ow, pd = NDIM == 3 ? box_div(row, inv_h) : 0, ph = row - pd * p.oh;
+      const BoxTap<T> ty = tap(1, ph, iy);
+      BoxTap<T> tz = {};
+      if (NDIM == 3) tz = tap(NDIM - 1, pd, iz);
+      if ((ty.o1 | tz.o1) & kBoxOutside) continue;
+      T* const vol = grad + (long long)c * p.vol;
+      const T g = __ldg(go + o);
+      T w[kRows];
+      unsigned off[kRows];
+#pragma unroll
+      for (int r = 0; r < kRows; ++r) {
+        w[r] = (r & 1) ? ty.l : ty.h;
+        off[r] = (r & 1) ? ty.o1 : ty.o0;
+        if (NDIM == 3) {
+          w[r] = A::mul((r & 2) ? tz.l : tz.h, w[r]);
+          off[r] += (r & 2) ? tz.o1 : tz.o0;
+        }
+      }
+      unsigned x0 = 0, x1 = 0;   // the cell whose contributions are being summed
+      bool held = false;
+      float sum[kRows][2];
+      auto flush = [&]() {
+        if (!held) return;
+#pragma unroll
+        for (int r = 0; r < kRows; ++r)
+          atomic_add_pair(vol + (off[r] + x0), vol + (off[r] + x1), FlatWide<T>::narrow(sum[r][0]), FlatWide<T>::narrow(sum[r][1]), tensor_lo,
+                          tensor_hi);
+      };
+      for (int ix = 0; ix < gx; ++ix) {
+        const BoxTap<T> tx = kTabled ? tab[0][pw * gx + ix] : box_tap<T>(ax[0], pw, ix, p.W, 1u, p.order);
+        if (tx.o1 & kBoxOutside) continue;
+        if (!held || tx.o0 != x0) {
+          flush();
+          held = true;
+          x0 = tx.o0;
+          x1 = tx.o1;
+#pragma unroll
+          for (int r = 0; r < kRows; ++r) sum[r][0] = sum[r][1] = 0.0f;
+        }
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+          sum[r][0] += A::tof(A::mul(g, A::mul(w[r], tx.h))) * inv_count;
+          sum[r][1] += A::tof(A::mul(g, A::mul(w[r], tx.l))) * inv_count;
+        }
+      }
+      flush();
+    }
+  };
+  if (tab[0]) walk(FlatCount<1>());
+  else walk(FlatCount<0>());
+}
+
+template <typename T, int NDIM>
+__global__ void __launch_bounds__(kBoxBwdThreads, 4)
+box_head_bwd(const __grid_constant__ Params p, const BoxBwdPlan plan) {
   typedef Ar<T> A;
   constexpr int kWin = 16 / (int)sizeof(T);
   extern __shared__ __align__(16) float box_smem[];
@@ -334,6 +446,7 @@ box_head_bwd(const Params p, const BoxBwdPlan plan) {
 #pragma unroll
   for (int a = 0; a < NDIM; ++a) count *= ax[a].grid;
   if (count == 0) return;  // no samples
+  const float inv_count = 1.0f / A::tof(A::fi(count));  // the count in the element type, as the reference divides by it
 
   // shared memory: weights and bin ranges per axis and position, contracted rows, gradients
   float* wmat[NDIM];
@@ -357,6 +470,26 @@ box_head_bwd(const Params p, const BoxBwdPlan plan) {
     span[a] = min(size[a] - base[a], box_span(A::tof(ax[a].bin), osz[a]));
     fits = fits && span[a] <= plan.positions[a] && span[a] * kb[a] <= plan.weights[a] && ax[a].grid <= kBoxBwdSamples;
   }
+  // Samples far apart leave most windows of a row empty, and an empty window costs what a full one does: then by samples.
+  // What a channel takes either way, in units of one sampled row pair, fitted to the times of 512 x 64 boxes in 2D and 300 x 32
+  // in 3D: its windows, the row elements it contracts, and the difference of what is fixed.  Windows / samples, us, 7 bins: 2D
+  // float, three samples, boxes of 8-64 px 90 / 129, of 10-120 178 / 142; half, two samples, 8-64 73 / 142, 30-180 153 / 145, 60-358
+  // 351 / 156; 3D float, two samples, 8-48 354 / 376, one sample, 10-67 266 / 127; half, three, 10-67 418 / 1803
+  constexpr bool kHalf = sizeof(T) == 2;
+  constexpr float kWindowCost = NDIM == 2 ? (kHalf ? 0.37f : 0.74f) : (kHalf ? 0.50f : 0.87f);
+  constexpr float kElementCost = NDIM == 2 ? (kHalf ? 0.42f : 1.0f) : (kHalf ? 0.23f : 1.4f);
+  constexpr float kSetupCost = NDIM == 2 ? (kHalf ? -73.0f : -40.0f) : (kHalf ? 1500.0f : 800.0f);
+  float items = (float)(span[0] / kWin + 2), elements = (float)span[0], pairs = (float)osz[0] * (float)ax[0].grid;
+#pragma unroll
+  for (int a = 1; a < NDIM; ++a) {
+    const float lines = 2.0f * (float)osz[a] * (float)ax[a].grid;
+    items *= fminf((float)span[a], lines);
+    elements *= (float)osz[a];
+    pairs *= lines;
+  }
+  // a call that leaves the chip idle waits for its slowest box, and a box takes longer by samples
+  const float idle = kHalf && gridDim.x < 148 * 4 ? 0.6f : 1.0f;
+  fits = fits && idle * (kWindowCost * items + kElementCost * elements) + kSetupCost < pairs;
   float* const abuf = next;                                   // [channel][row][row_s]
   float* const gbuf = next + plan.channels * (NDIM == 3 ? p.od * p.oh : p.oh) * plan.row; // [channel][row][ow]
   if (threadIdx.x < 3) {
@@ -373,7 +506,6 @@ box_head_bwd(const Params p, const BoxBwdPlan plan) {
         last_bin[a][i] = -1;
       }
     }
-    const float inv_count = 1.0f / (float)count;
     for (int i = threadIdx.x; i < nc * ovol; i += kBoxBwdThreads) gbuf[i] = A::tof(__ldg(go + i)) * inv_count;
   }
   __syncthreads();
@@ -419,37 +551,10 @@ box_head_bwd(const Params p, const BoxBwdPlan plan) {
     fits = overflow == 0;
   }
   if (!fits) {
-    // a grid or an extent beyond the tables: output by output, sample by sample (by the first of the pair's CTAs)
-    if (((int)blockIdx.x % plan.splits) != 0) return;
-    const T cnt = A::fi(count);
-    for (int o = threadIdx.x; o < nc * ovol; o += kBoxBwdThreads) {
-      const int c = o / ovol, v = o - c * ovol;
-      const int pw = v % p.ow, ph = (v / p.ow) % p.oh, pd = v / (p.ow * p.oh);
-      T* vol = grad + (long long)c * p.vol;
-      const T g = go[o];
-      for (int iz = 0; iz < (NDIM == 3 ? ax[NDIM - 1].grid : 1); ++iz) {
-        BoxTap<T> tz = {};
-        if (NDIM == 3) tz = box_tap<T>(ax[NDIM - 1], pd, iz, p.D, (unsigned)(p.H * p.W), p.order);
-        for (int iy = 0; iy < ax[1].grid; ++iy) {
-          const BoxTap<T> ty = box_tap<T>(ax[1], ph, iy, p.H, (unsigned)p.W, p.order);
-          for (int ix = 0; ix < ax[0].grid; ++ix) {
-            const BoxTap<T> tx = box_tap<T>(ax[0], pw, ix, p.W, 1u, p.order);
-            if ((tx.o1 | ty.o1 | (NDIM == 3 ? tz.o1 : 0u)) & kBoxOutside) continue;
+    BoxAxes<T, NDIM> axes;
 #pragma unroll
-            for (int r = 0; r < (NDIM == 3 ? 4 : 2); ++r) {
-              T wr = (r & 1) ? ty.l : ty.h;
-              unsigned off = (r & 1) ? ty.o1 : ty.o0;
-              if (NDIM == 3) {
-                wr = A::mul((r & 2) ? tz.l : tz.h, wr);
-                off += (r & 2) ? tz.o1 : tz.o0;
-              }
-              atomic_add_pair(vol + off + tx.o0, vol + off + tx.o1, A::div(A::mul(g, A::mul(wr, tx.h)), cnt),
-                              A::div(A::mul(g, A::mul(wr, tx.l)), cnt), tensor_lo, tensor_hi);
-            }
-          }
-        }
-      }
-    }
+    for (int a = 0; a < NDIM; ++a) axes.ax[a] = ax[a];
+    box_bwd_samples<T, NDIM>(p, axes, grad, go, nc, inv_count, (int)blockIdx.x % plan.splits, plan.splits, plan.bytes, tensor_lo, tensor_hi);
     return;
   }
 
@@ -527,6 +632,7 @@ box_head_bwd(const Params p, const BoxBwdPlan plan) {
     return block - kWin >= tensor_lo && block + (long long)(span[1] - 1) * p.W + nx + kWin <= tensor_hi;
   };
   if (NDIM == 2) {
+    if ((int)blockIdx.x % plan.splits) return;
     const float inv_ny = 1.0f / (float)n_y;
     for (int i = threadIdx.x; i < nc * n_y * windows; i += kBoxBwdThreads) {
       const int q = box_div(i, inv_win), win = i - q * windows;
@@ -620,19 +726,28 @@ inline int launch_box_head(const Params& p, bool fwd, cudaStream_t st) {
     else cudaLaunchKernelEx(&cfg, box_head_fwd<float, 1>, p, tasks, (int)chunks, chunk, ex, ey);
     return 0;
   }
-  // Forming the tables costs 5-8 us, which the flat kernels do not spend: they are faster where few reductions leave.
-  // Measured crossings, in samples; a run-time grid makes the flat kernel's samples four times dearer, and its half gradients
-  // (summed per cell first) ten times dearer than its float ones.  Adaptive grids: the number of samples is not known here,
-  // only that of the outputs.
+  // Measured, here / flat, in us.  One sample per bin is too little to share: half, 512 x 64 boxes 50-284 / 24-31, float 52-302 /
+  // 18-43.  So are, in float, less than 16 x 16 samples on a 2D box (7 x 7 bins of 2 x 2: 56 / 55 at best, 66-160 / 51-123 else; 14 x
+  // 14 bins 85 / 234), and small calls, where the set-up of 5-8 us does not pay: 2D, three samples, 39 000 outputs 9.2 / 7.6,
+  // 314 000 16 / 27; 3D, two samples, 55 000 outputs 14 / 13, 176 000 20-36 / 25-30, three samples, 2 700 outputs 10 / 7.4, 22 000
+  // 15-21 / 18; adaptive, 2 700 outputs 8.7-18 / 7.9-65, 22 000 16 / 16-56.  The flat kernel's half gradients (summed per cell first)
+  // are so much dearer that no call is too small: 2 700 outputs in 3D 8.5-14 / 32-185.  With less than 16 x 16 samples the size of
+  // the boxes decides, and the host knows that of the map: 512 x 64 boxes of 4-29 px on 42 x 58 55 / 101, of 8-64 on 101 x 135
+  // 73 / 91, of 10-120 on 200 x 336 143 / 82, of 60-358 on 512 x 512 202 / 83; 200 x 4 of 10-120 10.9 / 14.
   const double outputs = (double)p.R * per_roi;
-  if (p.sampling_ratio > 0) {
-    double samples = outputs;
-    for (int a = 0; a < p.ndim; ++a) samples *= p.sampling_ratio;
-    double least = sizeof(T) == 2 ? 1.0e5 : p.ndim == 3 ? 1.6e6 : 4.0e6;
-    if (p.sampling_ratio > 2) least /= 4;
-    if (samples < least) return 1;
-  } else if (p.ndim == 3 && outputs < (sizeof(T) == 2 ? 2.0e4 : 1.0e5)) {
-    return 1;
+  const int sr = p.sampling_ratio;
+  if (sr == 1) return 1;
+  const bool few_samples = p.ndim == 2 && sr > 0 && (double)p.ow * sr * p.oh * sr < 256.0;
+  if (sizeof(T) == 2) {
+    if (few_samples && std::max(p.W, p.H) > 160 && outputs > 2.0e5) return 1;
+  } else {
+    if (sr > 0) {
+      if (few_samples) return 1;
+      const double samples = outputs * sr * sr * (p.ndim == 3 ? sr : 1);
+      if (samples < (p.ndim == 3 ? 1.6e6 : 4.0e6) / (sr > 2 ? 4 : 1)) return 1;
+    } else if (p.ndim == 3 && outputs < 5.0e3) {
+      return 1;
+    }
   }
   const BoxBwdPlan plan = box_bwd_plan(p);
   if (plan.bytes > (size_t)kBoxBwdMaxSmem || p.ow > 0x7fff || p.oh > 0x7fff || p.od > 0x7fff || (long long)p.R * plan.chunks * plan.splits > 0x7fffffffLL) return 1;

@@ -29,6 +29,11 @@ CASES = [
     ((19, 23, 29),    9, 60, (7, 6, 5), 0, 1, torch.float32),   # enough outputs for the 3D tables
     ((12, 40, 170),   2, 30, (5, 5, 5), 0, 1, torch.float16),   # an axis beyond the tables of positions
     ((19, 23, 29),    3, 40, (7, 7, 7), 2, 0, torch.float16),
+    ((640, 700),      2, 30, (5, 4),    0, 1, torch.float16),   # maps beyond the tables: several blocks per box, some idle
+    ((200, 336),      5, 30, (7, 7),    2, 1, torch.float16),   # samples far apart beside samples close together
+    ((200, 336),      4, 60, (14, 14),  3, 1, torch.float32),
+    ((40, 60, 70),    12, 50, (7, 7, 7), 2, 1, torch.float32),  # the same in 3D
+    ((64, 80, 96),    2, 20, (4, 5, 6), 2, 0, torch.float16),
 ]
 
 
@@ -78,3 +83,16 @@ def test_box_heads_match_the_restatement(spatial, C, R, out, sr, order, dtype):
         around = torch.cat([buf[:16 + offset], buf[16 + offset + n:]])
         assert bool((torch.signbit(around) & (around == 0)).all()), "something was added outside the gradient tensor"
     _C.last_status()
+
+
+def test_half_gradient_divides_by_the_count_in_half():
+    """A bin of more than 255 pixels a side has more samples than half can count: the reference divides by infinity."""
+    from medvision_b200 import _C
+    rois = torch.tensor([[0, 10, 12, 310, 312], [0, 10, 12, 110, 132]]).half()
+    grad = torch.randn(2, 3, 1, 1, generator=torch.Generator().manual_seed(2)).half()
+    want = port.backward(grad, rois, (1, 3, 330, 340), cases.KIND_BOX, spatial_scale=1.0, sampling_ratio=0, aligned=True, order=1,
+                         wide_acc=True, fma_mode=0)
+    assert bool(want[0, :, 50, 50].any()) and not bool(want[0, :, 200, 200].any())
+    gin = torch.zeros(want.shape, dtype=torch.half, device="cuda")
+    _C.roi_align_2d_backward(grad.cuda(), rois.cuda(), gin, 1, 1, 1.0, 0, 1)
+    assert_close(gin, want, 2e-3, "gradient")
