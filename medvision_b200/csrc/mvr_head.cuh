@@ -771,23 +771,166 @@ inline int launch_box_head(const Params& p, bool fwd, cudaStream_t st) {
 // per sample and tap row, and half reductions to the same few addresses wait for one another.  Here a CTA sums the gradient of
 // a roi's channel, or of a slab of its outputs where the rois are few, in float in shared memory and sends every 16-byte window
 // of the box once.  The samples of a line that fall into the same cell are summed in registers first.  A slab whose box exceeds
-// the shared memory, or has more voxels than it has taps, is sent sample by sample.  Bound by the shared-memory additions and,
-// on small rois, by the walk of the sample lines.
+// the shared memory, or has more voxels than it has taps, is sent sample by sample or cell by cell.  Bound by the shared-memory
+// additions and, on small rois, by the walk of the sample lines.
 // The flat kernel -> this one: 3D, 583 000 outputs of 27 samples 727 -> 530 us; 2 103 000 of 8 1080 -> 435; 31 000 of 27, one
 // channel, 310 -> 71; 1 250 of 27 in ten rois 73 -> 32; 2D adaptive, 317 000 outputs 145 -> 86.
 constexpr int kRotThreads = 256;
-constexpr int kRotCells = 13 * 1024;   // floats of the patch: four CTAs per SM
+constexpr int kRotPatchFloats = 13 * 1024;   // four CTAs per SM
+
+// How the contributions of a slab's samples leave: through the patch in shared memory; summed per cell of the volume over consecutive
+// samples; or each by itself.
+enum { kRotPatch, kRotCells, kRotSamples };
+
+// What the walks over a slab's samples share.
+template <typename T, int NDIM>
+struct RotSlab {
+  const RoiGeom<T>* g;
+  const T (*subs)[kFlatSubs];
+  T* grad;                              // the channel's gradient
+  const T *go, *tensor_lo, *tensor_hi;  // the slab's output gradients; the whole gradient tensor
+  int first, outputs, lines, part, parts;
+  int lo[3], ext[3], sy, sz;            // the patch
+};
+
+// The sample lines of the slab's outputs, a line and output at a time per thread.
+template <typename T, int NDIM, int HOW>
+__device__ __forceinline__ void rot_walk(const Params& p, const RotSlab<T, NDIM>& s, float* patch) {
+  typedef Ar<T> A;
+  constexpr int fm = kFlatFm, kWin = 16 / (int)sizeof(T), kTaps = 1 << NDIM;
+  const RoiGeom<T>& g = *s.g;
+  const int gx = g.grid[0], gy = g.grid[1], outputs = s.outputs, sy = s.sy, sz = s.sz;
+  const float inv_n = 1.0f / A::tof(g.count_bwd);
+  auto sub = [&](int a, int i) { return i < kFlatSubs ? s.subs[a][i] : lattice_sub<T>(g.bin[a], i, g.grid[a]); };
+  // one sample's contributions straight to the gradient
+  auto send = [&](const FlatAxis<T>* t, const T* w, T gv) {
+    T* const q = s.grad + ((NDIM == 3 ? (long long)t[2].i0 * p.H * p.W : 0) + (long long)t[1].i0 * p.W + t[0].i0);
+#pragma unroll
+    for (int k = 0; k < kTaps; k += 2) {
+      T* row_p = q + ((k & 2) ? t[1].d * p.W : 0);
+      if (NDIM == 3 && (k & 4)) row_p += (long long)t[2].d * p.H * p.W;
+      atomic_add_pair(row_p, row_p + t[0].d, A::ff(A::tof(A::mul(gv, w[k])) * inv_n), A::ff(A::tof(A::mul(gv, w[k + 1])) * inv_n), s.tensor_lo,
+                      s.tensor_hi);
+    }
+  };
+  const int parts = HOW == kRotPatch ? 1 : s.parts, part = HOW == kRotPatch ? 0 : s.part;
+  for (long long item = part * kRotThreads + threadIdx.x; item < (long long)outputs * s.lines; item += parts * kRotThreads) {
+    const int line = (int)(item / outputs), o = (int)(item - (long long)line * outputs);
+    const int iz = line / gy, iy = line - iz * gy;
+    const int pw = o % p.ow, row = o / p.ow + s.first * (NDIM == 3 ? p.oh : 1), pd = NDIM == 3 ? row / p.oh : 0, ph = row - pd * p.oh;
+    const T bx = lattice_base<T>(g.start[0], pw, g.bin[0], fm);
+    const T y = A::add(lattice_base<T>(g.start[1], ph, g.bin[1], fm), sub(1, iy));
+    const T z = NDIM == 3 ? A::add(lattice_base<T>(g.start[2], pd, g.bin[2], fm), sub(NDIM - 1, iz)) : A::fi(0);
+    const T gv = __ldg(s.go + o);
+    int held = -1;               // cell whose contributions are being summed: of the patch, or of the channel's volume
+    int hx = 0, hy = 0, hz = 0;  // (volume) steps to its upper taps
+    float sum[kTaps];
+    auto flush = [&]() {
+      if (held < 0) return;
+      if (HOW == kRotPatch) {
+        float* const q = patch + held;
+#pragma unroll
+        for (int t = 0; t < kTaps; ++t)
+          if (sum[t] != 0.0f) atomicAdd(q + (t & 1) + (t & 2 ? sy : 0) + (t & 4 ? sz : 0), sum[t]);
+      } else {
+#pragma unroll
+        for (int t = 0; t < kTaps; t += 2) {
+          T* const row_p = s.grad + held + (t & 2 ? hy : 0) + (t & 4 ? hz : 0);
+          atomic_add_pair(row_p, row_p + hx, FlatWide<T>::narrow(sum[t]), FlatWide<T>::narrow(sum[t + 1]), s.tensor_lo, s.tensor_hi);
+        }
+      }
+    };
+    auto hold = [&](int cell) {
+      if (cell == held) return;
+      flush();
+      held = cell;
+#pragma unroll
+      for (int k = 0; k < kTaps; ++k) sum[k] = 0.0f;
+    };
+    for (int ix = 0; ix < gx; ++ix) {
+      T px, py, pz;
+      to_volume<T, NDIM>(g, KIND_ROTATED, fm, A::add(bx, sub(0, ix)), y, z, px, py, pz);
+      FlatAxis<T> t[3];
+      bool in = flat_axis<T>(px, p.W, t[0]);
+      in = flat_axis<T>(py, p.H, t[1]) && in;
+      if (NDIM == 3) in = flat_axis<T>(pz, p.D, t[2]) && in;
+      if (!in) continue;
+      T w[kTaps];
+      if (p.order == 0) {
+        AxisTap<T> m[3];
+#pragma unroll
+        for (int a = 0; a < NDIM; ++a) {
+          m[a].l = t[a].l;
+          m[a].h = t[a].h;
+        }
+        nearest_pick<T, NDIM>(m, w);
+      } else {
+#pragma unroll
+        for (int k = 0; k < kTaps; k += 2) {
+          T zy = (k & 2) ? t[1].l : t[1].h;
+          if (NDIM == 3) zy = A::mul((k & 4) ? t[2].l : t[2].h, zy);
+          w[k] = A::mul(zy, t[0].h);
+          w[k + 1] = A::mul(zy, t[0].l);
+        }
+      }
+      if constexpr (HOW == kRotSamples) {
+        send(t, w, gv);
+      } else if constexpr (HOW == kRotCells) {
+        hold((NDIM == 3 ? t[2].i0 * p.H * p.W : 0) + t[1].i0 * p.W + t[0].i0);
+        hx = t[0].d;
+        hy = t[1].d * p.W;
+        hz = NDIM == 3 ? t[2].d * p.H * p.W : 0;
+#pragma unroll
+        for (int k = 0; k < kTaps; ++k) sum[k] += A::tof(A::mul(gv, w[k])) * inv_n;
+      } else {
+        const int rx = t[0].i0 - s.lo[0], ry = t[1].i0 - s.lo[1], rz = NDIM == 3 ? t[2].i0 - s.lo[2] : 0;
+        const bool inside = rx >= 0 && rx + t[0].d < s.ext[0] && ry >= 0 && ry + t[1].d < s.ext[1] &&
+                            (NDIM == 2 || (rz >= 0 && rz + t[2].d < s.ext[2]));
+        if (inside) {
+          const int cell = rz * sz + ry * sy + rx + kWin;
+          hold(cell);
+          // a clamped upper tap lies on the lower one, with weight 0: its (zero) product goes there
+#pragma unroll
+          for (int k = 0; k < kTaps; ++k) {
+            const float v = A::tof(A::mul(gv, w[k])) * inv_n;
+            int at = k;
+            if (!t[0].d) at &= ~1;
+            if (!t[1].d) at &= ~2;
+            if (NDIM == 3 && !t[2].d) at &= ~4;
+            if (at == k) sum[k] += v;
+            else if (v != 0.0f) atomicAdd(patch + cell + (at & 1) + (at & 2 ? sy : 0) + (at & 4 ? sz : 0), v);
+          }
+        } else {  // (the room for rounding is generous: hardly ever)
+          send(t, w, gv);
+        }
+      }
+    }
+    flush();
+  }
+}
+
+// The walks without a patch, in a function of their own, which leaves the walk of the patch more registers (all three in the kernel:
+// 10 % slower).  The samples of a line share cells only where they lie less than a voxel apart.  There they are summed per cell
+// first, as in the flat kernel, or the half result would be less exact (14^3 bins of 4^3 samples in 24-30 voxels: error of the
+// gradient 2.1e-3 sample by sample, 1.7e-3 by cells, flat kernel 1.8e-3).
+template <typename T, int NDIM>
+__device__ __noinline__ void rot_without_patch(const Params& p, const RotSlab<T, NDIM> s) {
+  __builtin_assume(__isShared(s.g));
+  __builtin_assume(__isShared(s.subs));
+  if (Ar<T>::tof(s.g->bin[0]) < (float)s.g->grid[0]) rot_walk<T, NDIM, kRotCells>(p, s, nullptr);
+  else rot_walk<T, NDIM, kRotSamples>(p, s, nullptr);
+}
 
 template <typename T, int NDIM>
-__global__ void __launch_bounds__(kRotThreads)
-rot_head_bwd(const Params p, int slabs) {
+__global__ void __launch_bounds__(kRotThreads, 4)
+rot_head_bwd(const __grid_constant__ Params p, int slabs, int parts) {
   typedef Ar<T> A;
   constexpr int fm = kFlatFm, kWin = 16 / (int)sizeof(T), kTaps = 1 << NDIM;
   extern __shared__ __align__(16) float rot_patch[];
   __shared__ RoiGeom<T> g;
   __shared__ T subs[NDIM][kFlatSubs];
   flat_grid_dependency();
-  const int nc = (int)blockIdx.x / slabs, slab = (int)blockIdx.x - nc * slabs;
+  const int part = (int)blockIdx.x % parts, nc = (int)blockIdx.x / parts / slabs, slab = (int)blockIdx.x / parts - nc * slabs;
   const int n = nc / p.C, c = nc - n * p.C;
   if (threadIdx.x == 0) {
     const int osz[3] = {p.ow, p.oh, p.od};
@@ -836,7 +979,8 @@ rot_head_bwd(const Params p, int slabs) {
   const int sy = ext[0] + kWin;
   const long long cells = (long long)sy * ext[1] * ext[2] + kWin;
   const int lines = gy * gz;  // sample lines of an output
-  const bool patch = box && cells <= kRotCells && cells <= 2LL * outputs * lines * gx * kTaps;
+  const bool patch = box && cells <= kRotPatchFloats && cells <= 2LL * outputs * lines * gx * kTaps;
+  if (patch && part) return;  // one CTA sums a patch; CTA-uniform
   T* const grad = (T*)p.out + ((long long)g.batch * p.C + c) * p.vol;
   const T* const tensor_lo = (const T*)p.out;
   const T* const tensor_hi = tensor_lo + (long long)p.N * p.C * p.vol;
@@ -845,90 +989,30 @@ rot_head_bwd(const Params p, int slabs) {
   if (patch)
     for (int i = threadIdx.x; i < (int)cells; i += kRotThreads) rot_patch[i] = 0.0f;
   __syncthreads();
-  const float inv_n = 1.0f / A::tof(g.count_bwd);
-  auto sub = [&](int a, int i) { return i < kFlatSubs ? subs[a][i] : lattice_sub<T>(g.bin[a], i, g.grid[a]); };
-
-  for (long long item = threadIdx.x; item < (long long)outputs * lines; item += kRotThreads) {
-    const int line = (int)(item / outputs), o = (int)(item - (long long)line * outputs);
-    const int iz = line / gy, iy = line - iz * gy;
-    const int pw = o % p.ow, row = o / p.ow + first * (NDIM == 3 ? p.oh : 1), pd = NDIM == 3 ? row / p.oh : 0, ph = row - pd * p.oh;
-    const T bx = lattice_base<T>(g.start[0], pw, g.bin[0], fm);
-    const T y = A::add(lattice_base<T>(g.start[1], ph, g.bin[1], fm), sub(1, iy));
-    const T z = NDIM == 3 ? A::add(lattice_base<T>(g.start[2], pd, g.bin[2], fm), sub(NDIM - 1, iz)) : A::fi(0);
-    const T gv = __ldg(go + o);
-    int held = -1;            // cell whose contributions are being summed
-    float sum[kTaps];
-    auto flush = [&]() {
-      if (held < 0) return;
-      float* const q = rot_patch + held;
+  RotSlab<T, NDIM> work;
+  work.g = &g;
+  work.subs = subs;
+  work.grad = grad;
+  work.go = go;
+  work.tensor_lo = tensor_lo;
+  work.tensor_hi = tensor_hi;
+  work.first = first;
+  work.outputs = outputs;
+  work.lines = lines;
+  work.part = part;
+  work.parts = parts;
 #pragma unroll
-      for (int t = 0; t < kTaps; ++t)
-        if (sum[t] != 0.0f) atomicAdd(q + (t & 1) + (t & 2 ? sy : 0) + (t & 4 ? sz : 0), sum[t]);
-    };
-    for (int ix = 0; ix < gx; ++ix) {
-      T px, py, pz;
-      to_volume<T, NDIM>(g, KIND_ROTATED, fm, A::add(bx, sub(0, ix)), y, z, px, py, pz);
-      FlatAxis<T> t[3];
-      bool in = flat_axis<T>(px, p.W, t[0]);
-      in = flat_axis<T>(py, p.H, t[1]) && in;
-      if (NDIM == 3) in = flat_axis<T>(pz, p.D, t[2]) && in;
-      if (!in) continue;
-      T w[kTaps];
-      if (p.order == 0) {
-        AxisTap<T> m[3];
-#pragma unroll
-        for (int a = 0; a < NDIM; ++a) {
-          m[a].l = t[a].l;
-          m[a].h = t[a].h;
-        }
-        nearest_pick<T, NDIM>(m, w);
-      } else {
-#pragma unroll
-        for (int k = 0; k < kTaps; k += 2) {
-          T zy = (k & 2) ? t[1].l : t[1].h;
-          if (NDIM == 3) zy = A::mul((k & 4) ? t[2].l : t[2].h, zy);
-          w[k] = A::mul(zy, t[0].h);
-          w[k + 1] = A::mul(zy, t[0].l);
-        }
-      }
-      const int rx = t[0].i0 - lo[0], ry = t[1].i0 - lo[1], rz = NDIM == 3 ? t[2].i0 - lo[2] : 0;
-      // (the room for rounding is generous: a sample outside the box is sent directly, like every sample without a patch)
-      const bool inside = patch && rx >= 0 && rx + t[0].d < ext[0] && ry >= 0 && ry + t[1].d < ext[1] &&
-                          (NDIM == 2 || (rz >= 0 && rz + t[2].d < ext[2]));
-      if (inside) {
-        const int cell = rz * sz + ry * sy + rx + kWin;
-        if (cell != held) {
-          flush();
-          held = cell;
-#pragma unroll
-          for (int k = 0; k < kTaps; ++k) sum[k] = 0.0f;
-        }
-        // a clamped upper tap lies on the lower one, with weight 0: its (zero) product goes there
-#pragma unroll
-        for (int k = 0; k < kTaps; ++k) {
-          const float v = A::tof(A::mul(gv, w[k])) * inv_n;
-          int at = k;
-          if (!t[0].d) at &= ~1;
-          if (!t[1].d) at &= ~2;
-          if (NDIM == 3 && !t[2].d) at &= ~4;
-          if (at == k) sum[k] += v;
-          else if (v != 0.0f) atomicAdd(rot_patch + cell + (at & 1) + (at & 2 ? sy : 0) + (at & 4 ? sz : 0), v);
-        }
-      } else {
-        const long long at = (NDIM == 3 ? (long long)t[2].i0 * p.H * p.W : 0) + (long long)t[1].i0 * p.W + t[0].i0;
-        const long long dy = (long long)t[1].d * p.W, dz = NDIM == 3 ? (long long)t[2].d * p.H * p.W : 0;
-        T* const q = grad + at;
-#pragma unroll
-        for (int k = 0; k < kTaps; k += 2) {
-          T* const row_p = q + ((k & 2) ? dy : 0) + ((k & 4) ? dz : 0);
-          atomic_add_pair(row_p, row_p + t[0].d, A::ff(A::tof(A::mul(gv, w[k])) * inv_n), A::ff(A::tof(A::mul(gv, w[k + 1])) * inv_n),
-                          tensor_lo, tensor_hi);
-        }
-      }
-    }
-    flush();
+  for (int a = 0; a < 3; ++a) {
+    work.lo[a] = lo[a];
+    work.ext[a] = ext[a];
   }
-  if (!patch) return;
+  work.sy = sy;
+  work.sz = sz;
+  if (!patch) {
+    rot_without_patch<T, NDIM>(p, work);
+    return;
+  }
+  rot_walk<T, NDIM, kRotPatch>(p, work, rot_patch);
   __syncthreads();
   // every window of the box with something in it, once
   const int windows = (ext[0] + 2 * kWin - 2) / kWin, rows = ext[1] * ext[2];
@@ -960,32 +1044,39 @@ rot_head_bwd(const Params p, int slabs) {
 
 // 0 launched, 1 not applicable (then the flat kernel).
 // Half only: the float sums of the flat kernel do not wait for one another that long and are faster there (2D, 301 000 outputs
-// 29 against 37 us, 3D, 2 100 000 outputs 368 against 488).  In 2D two samples per axis are few for the patch: from some 57 000
-// outputs on the flat kernel is as fast or faster (3 channels of 512 rois 25 against 42 us; 13 000 outputs 15 against 7).
+// 29 against 37 us, 3D, 2 100 000 outputs 368 against 488).  In 2D few samples per bin are few for the patch: two per axis from
+// some 57 000 outputs on (3 channels of 512 rois 25 us there, 42 here; 13 000 outputs 15 and 7), three from a million on (512 x
+// 64 rois of 4-20 px 290 and 314, of 8-64 292 and 353, of 16-256 258 and 467; 200 x 32: 78 and 65, 73 and 73, 64 and 99).
+// Four: 457 and 392, 491 and 407, 438 and 609.
 inline int launch_rot_head_bwd(const Params& p, cudaStream_t st) {
   if (p.kind != KIND_ROTATED || p.order > 1 || p.fm != kFlatFm || p.vol >= 0x7fffffffLL || p.sampling_ratio == 1) return 1;
   if (p.D > kTapMaxSize || p.H > kTapMaxSize || p.W > kTapMaxSize || p.ovol > 4096) return 1;
   const long long channels = (long long)p.R * p.C;
   if (p.ndim == 2 && p.sampling_ratio == 2 && channels * p.ovol > 148 * 384) return 1;
+  if (p.ndim == 2 && p.sampling_ratio == 3 && channels * p.ovol > 1000000) return 1;
   // few rois are cut into slabs of outputs until there are two CTAs per SM
   const int slow = p.ndim == 3 ? p.od : p.oh;
   int slabs = 1;
   while (slabs * 2 <= slow && channels * slabs * 2 <= 148 * 2) slabs *= 2;
+  // CTAs that share the lines of a slab without a patch.  With a patch all but one leave at once, which is no loss as long as all of
+  // them find a place beside one another (up to four per SM the call on 60 x 4 small rois took 240-280 instead of 157 us)
+  int parts = 1;
+  while (parts < 8 && channels * slabs * parts * 2 <= 148 * 2) parts *= 2;
   if (channels * slabs > 0x7fffffffLL) return 1;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(channels * slabs));
+  cfg.gridDim = dim3((unsigned)(channels * slabs * parts));
   cfg.blockDim = dim3(kRotThreads);
-  cfg.dynamicSmemBytes = (size_t)kRotCells * 4;
+  cfg.dynamicSmemBytes = (size_t)kRotPatchFloats * 4;
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
 #define MVR_ROT(ND)                                                                                                          \
   {                                                                                                                          \
     cudaFuncSetAttribute(rot_head_bwd<__half, ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes); \
-    cudaLaunchKernelEx(&cfg, rot_head_bwd<__half, ND>, p, slabs);                                                            \
+    cudaLaunchKernelEx(&cfg, rot_head_bwd<__half, ND>, p, slabs, parts);                                                     \
   }
   if (p.ndim == 2) MVR_ROT(2) else MVR_ROT(3)
 #undef MVR_ROT

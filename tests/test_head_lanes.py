@@ -75,7 +75,10 @@ def test_shared_outputs_match_the_restatement(spatial, C, R, out, sr, order, dty
     ((9, 14, 17), 2, 8, (3, 5, 2), 2, 0),
     ((70, 53), 3, 8, (7, 7), 2, 1),
     ((37, 41), 2, 170, (5, 9), 3, 1),
-], ids=["slabs", "large", "nearest", "plane", "plane-many"])
+    ((60, 70, 80), 1, 8, (5, 5, 5), 0, 1),      # several blocks per slab
+    ((60, 70, 80), 1, 8, (3, 4, 5), 2, 0),
+    ((300, 260), 2, 8, (7, 6), 0, 1),
+], ids=["slabs", "large", "nearest", "plane", "plane-many", "parts", "parts-sparse", "parts-plane"])
 def test_half_gradient_of_rotated_rois(spatial, C, R, out, sr, order):
     from medvision_b200 import _C
     nd = len(spatial)
@@ -96,6 +99,22 @@ def test_half_gradient_of_rotated_rois(spatial, C, R, out, sr, order):
         assert_close(gin, want, BWD_TOL[torch.half], "gradient")
         around = torch.cat([buf[:16 + offset], buf[16 + offset + n:]])
         assert bool((torch.signbit(around) & (around == 0)).all()), "something was added outside the gradient tensor"
+
+
+def test_half_gradient_beyond_the_patch_is_as_exact_as_the_flat_kernels():
+    """Dense samples in rois larger than the shared-memory patch: summed per cell before they leave.  Against the wide-accumulator
+    restatement the flat kernel's error is 1.80e-3 of the gradient's norm, sample by sample it is 2.12e-3."""
+    from medvision_b200 import _C
+    g = torch.Generator().manual_seed(5)
+    R, out = 30, (14, 14, 14)
+    rois = torch.cat([torch.zeros(R, 1), torch.rand(R, 3, generator=g) * 48, torch.rand(R, 3, generator=g) * 6 + 24,
+                      (torch.rand(R, 3, generator=g) * 2 - 1) * math.pi], 1).half()
+    grad = torch.randn((R, 2) + out, generator=g).half()
+    want = port.backward(grad, rois, (1, 2, 48, 48, 48), cases.KIND_ROTATED, spatial_scale=1.0, sampling_ratio=4, aligned=True, order=1,
+                         trig=port.device_trig(rois), wide_acc=True, fma_mode=0).double()
+    gin = torch.zeros((1, 2, 48, 48, 48), dtype=torch.half, device="cuda")
+    _C.roi_align_rotated_3d_backward(grad.cuda(), rois.cuda(), gin, *out, 1.0, 4, True, 1)
+    assert float((gin.cpu().double() - want).norm() / want.norm()) < 1.9e-3
 
 
 @pytest.mark.parametrize("rotated,C,R,out,sr,order,dtype", [
