@@ -7,20 +7,37 @@ Same public surface as medvision/ops/roi_align_nd.py: ``RoIAlign2DFunction``,
 import torch.nn as nn
 
 from .. import _C
+from ._common import RoiFunction
 
 # features, rois, output_size, spatial_scale, sampling_ratio=0, order=1; differentiable in the features
 roi_align_2d = _C._native.roi_align_2d
 roi_align_3d = _C._native.roi_align_3d
 
 
-class RoIAlign2DFunction:
-    """``apply`` is the differentiable operation; its autograd node is native (csrc/mvr_torch.cpp)."""
-    apply = staticmethod(roi_align_2d)
+class RoIAlign2DFunction(RoiFunction):
+    ndim, call = 2, staticmethod(roi_align_2d)
+    kernels = _C.roi_align_2d_forward, _C.roi_align_2d_backward
+
+    @staticmethod
+    def forward(ctx, features, rois, output_size, spatial_scale, sampling_ratio=0, order=1):
+        return RoIAlign2DFunction._forward(ctx, features, rois, output_size, spatial_scale, sampling_ratio, order)
+
+    @staticmethod
+    def backward(ctx, grad_output):
+        return RoIAlign2DFunction._backward(ctx, grad_output)
 
 
-class RoIAlign3DFunction:
-    """See :class:`RoIAlign2DFunction`."""
-    apply = staticmethod(roi_align_3d)
+class RoIAlign3DFunction(RoiFunction):
+    ndim, call = 3, staticmethod(roi_align_3d)
+    kernels = _C.roi_align_3d_forward, _C.roi_align_3d_backward
+
+    @staticmethod
+    def forward(ctx, features, rois, output_size, spatial_scale, sampling_ratio=0, order=1):
+        return RoIAlign3DFunction._forward(ctx, features, rois, output_size, spatial_scale, sampling_ratio, order)
+
+    @staticmethod
+    def backward(ctx, grad_output):
+        return RoIAlign3DFunction._backward(ctx, grad_output)
 
 
 class RoIAlign(nn.Module):

@@ -8,20 +8,37 @@ Same public surface as medvision/ops/roi_align_rotated_nd.py: ``RoIAlignRotated2
 import torch.nn as nn
 
 from .. import _C
+from ._common import RoiFunction
 
 # features, rois, output_size, spatial_scale, sampling_ratio=0, aligned=True, order=1; differentiable in the features
 roi_align_rotated_2d = _C._native.roi_align_rotated_2d
 roi_align_rotated_3d = _C._native.roi_align_rotated_3d
 
 
-class RoIAlignRotated2DFunction:
-    """``apply`` is the differentiable operation; its autograd node is native (csrc/mvr_torch.cpp)."""
-    apply = staticmethod(roi_align_rotated_2d)
+class RoIAlignRotated2DFunction(RoiFunction):
+    ndim, call = 2, staticmethod(roi_align_rotated_2d)
+    kernels = _C.roi_align_rotated_2d_forward, _C.roi_align_rotated_2d_backward
+
+    @staticmethod
+    def forward(ctx, features, rois, output_size, spatial_scale, sampling_ratio=0, aligned=True, order=1):
+        return RoIAlignRotated2DFunction._forward(ctx, features, rois, output_size, spatial_scale, sampling_ratio, aligned, order)
+
+    @staticmethod
+    def backward(ctx, grad_output):
+        return RoIAlignRotated2DFunction._backward(ctx, grad_output)
 
 
-class RoIAlignRotated3DFunction:
-    """See :class:`RoIAlignRotated2DFunction`."""
-    apply = staticmethod(roi_align_rotated_3d)
+class RoIAlignRotated3DFunction(RoiFunction):
+    ndim, call = 3, staticmethod(roi_align_rotated_3d)
+    kernels = _C.roi_align_rotated_3d_forward, _C.roi_align_rotated_3d_backward
+
+    @staticmethod
+    def forward(ctx, features, rois, output_size, spatial_scale, sampling_ratio=0, aligned=True, order=1):
+        return RoIAlignRotated3DFunction._forward(ctx, features, rois, output_size, spatial_scale, sampling_ratio, aligned, order)
+
+    @staticmethod
+    def backward(ctx, grad_output):
+        return RoIAlignRotated3DFunction._backward(ctx, grad_output)
 
 
 class RoIAlignRotated(nn.Module):
