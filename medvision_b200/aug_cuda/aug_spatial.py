@@ -220,16 +220,6 @@ class CudaRandomElasticDeformation(ElasticField, CudaAugBase):
     def elastic_transform(self, image: torch.Tensor, order=1):
         return self._warp_with_dense_field(image, self.dense_field(image.device), order)
 
-    def apply_to_img(self, result):
-        # image and label fields together
-        img_keys, seg_keys = list(result.get('img_fields', ())), list(result.get('seg_fields', ()))
-        images, labels = self._warp_fields([result[k] for k in img_keys], [result[k] for k in seg_keys])
-        result.update(zip(img_keys, images))
-        result.update(zip(seg_keys, labels))
-
-    def apply_to_seg(self, result):
-        pass  # done together with the images
-
     def apply_to_det(self, result):
         for _ in result.get('det_fields', []):
             raise NotImplementedError

@@ -15,7 +15,7 @@ from typing import Union
 import numpy as np
 import torch
 
-from .base import BatchCudaAugBase
+from .base import BatchCudaAugBase, global_bit_generator, overrides
 from .elastic_field import ElasticField
 from .. import _C
 
@@ -210,16 +210,6 @@ class BatchCudaRandomElasticDeformation(ElasticField, BatchCudaAugBase):
         """One field (B, C, *image_shape) by the dense field."""
         return self._warp_with_dense_field(image, self.dense_field(image.device), order)
 
-    def apply_to_img(self, result):
-        # image and label fields together
-        img_keys, seg_keys = list(result.get('img_fields', ())), list(result.get('seg_fields', ()))
-        images, labels = self._warp_fields([result[k] for k in img_keys], [result[k] for k in seg_keys])
-        result.update(zip(img_keys, images))
-        result.update(zip(seg_keys, labels))
-
-    def apply_to_seg(self, result):
-        pass  # done together with the images
-
     def apply_to_det(self, result):
         for key in result.get('det_fields', []):
             raise NotImplementedError
@@ -281,10 +271,12 @@ class BatchCudaCropRandomWithAffine(BatchCudaAugBase):
         return np.array(batch_start), np.array(batch_end)
 
     def _forward_crop_params(self, result: dict):
+        if overrides(self, BatchCudaCropRandomWithAffine, '_random_start'):
+            return self._collect([self._random_start() for _ in range(self.batch)])
         # one draw per patch and axis (d, h, w), as _random_start() makes them
         start = np.empty((self.batch, self.dim), dtype=np.int64)
         end = np.empty_like(start)
-        generator = np.random.get_bit_generator()
+        generator = global_bit_generator()
         with generator.lock:
             _C._native.draw_starts(generator.capsule, self.batch, tuple(self.image_shape), tuple(self.patch_size), start, end)
         return start, end

@@ -27,6 +27,21 @@ _HOOKS = ('apply_to_img', 'apply_to_cls', 'apply_to_seg', 'apply_to_det')
 _LOG_KEYS = ('history', 'time', 'memory')
 
 
+def global_bit_generator():
+    """The bit generator behind ``np.random``'s functions."""
+    get = getattr(np.random, 'get_bit_generator', None)  # numpy 1.24
+    return get() if get is not None else np.random.mtrand._rand._bit_generator
+
+
+def overrides(obj, cls, *names):
+    """Whether ``obj`` has another of the named methods than ``cls`` -- a hook of a subclass, or of the object itself."""
+    for name in names:
+        own = getattr(obj, name)
+        if getattr(own, '__func__', own) is not getattr(cls, name):
+            return True
+    return False
+
+
 class BatchCudaAugBase(object):
     def __init__(self):
         cls_name = type(self).__name__
@@ -72,10 +87,14 @@ class BatchCudaAugBase(object):
     def _draw_affine(self, n):
         """Scale, shifts and rotation (radians) of ``n`` samples -- (n, dim), (n, dim) and (n, 1) arrays: the values that
         :meth:`get_range` draws sample by sample (scale, one shift per axis, rotation in degrees), drawn natively from numpy's
-        global generator."""
+        global generator, or by :meth:`get_range` itself where a subclass has its own."""
         dim = self.dim
+        if overrides(self, BatchCudaAugBase, 'get_range'):
+            draws = [([self.get_range(self.scale, 1)] * dim, [self.get_range(self.shift, 0) for _ in range(dim)],
+                      [np.pi * self.get_range(self.rotate, 0) / 180]) for _ in range(n)]
+            return tuple(np.array(v) for v in zip(*draws))
         scales, shifts, rotate = np.empty((n, dim)), np.empty((n, dim)), np.empty((n, 1))
-        generator = np.random.get_bit_generator()
+        generator = global_bit_generator()
         with generator.lock:
             _C._native.draw_affine(generator.capsule, n, dim, self._bounds(self.scale), self._bounds(self.shift),
                                    self._bounds(self.rotate), scales, shifts, rotate)

@@ -8,6 +8,7 @@ types take the two-step form: one ``affine_*`` blow-up, one ``apply_offset_*`` p
 import numpy as np
 import torch
 
+from .base import global_bit_generator, overrides
 from .. import _C
 from ..ops.cuda_fun_tools import affine_2d, affine_3d, apply_offset_2d, apply_offset_3d
 
@@ -34,7 +35,7 @@ class ElasticField:
         grid = self.to_tuple(self.num_control_points, self.dim)
         reach = self.max_displacement * (np.array(self.image_shape) / (np.array(grid) - 1)) / 2
         coarse = np.empty((*batch, *grid, self.dim), dtype=np.float32)
-        generator = np.random.get_bit_generator()
+        generator = global_bit_generator()
         with generator.lock:  # 2 * rand(*grid, dim).astype(float32) - 1 per sample, in [-1, 1)
             _C._native.draw_coarse(generator.capsule, batch[0] if batch else 1, grid, reach.astype(np.float32),
                                    self.num_locked_borders, coarse)
@@ -91,3 +92,24 @@ class ElasticField:
         field = self.dense_field((images + labels)[0].device)
         return ([self._warp_with_dense_field(t, field.to(t.device), 1) for t in images],
                 [self._warp_with_dense_field(t, field.to(t.device), 0) for t in labels])
+
+    def _warp_in_place(self, result, img_keys, seg_keys):
+        own = next(c for c in type(self).__mro__ if ElasticField in c.__bases__)  # the transform that a subclass derives from
+        if overrides(self, own, 'elastic_transform', 'dense_field'):
+            result.update({k: self.elastic_transform(result[k]) for k in img_keys})
+            result.update({k: self.elastic_transform(result[k], order=0).int() for k in seg_keys})
+            return
+        images, labels = self._warp_fields([result[k] for k in img_keys], [result[k] for k in seg_keys])
+        result.update(zip(img_keys, images))
+        result.update(zip(seg_keys, labels))
+
+    # image and label fields go together, unless a subclass has its own say in either
+    def _together(self):
+        return not overrides(self, ElasticField, 'apply_to_img', 'apply_to_seg')
+
+    def apply_to_img(self, result):
+        self._warp_in_place(result, result.get('img_fields', ()), result.get('seg_fields', ()) if self._together() else ())
+
+    def apply_to_seg(self, result):
+        if not self._together():
+            self._warp_in_place(result, (), result.get('seg_fields', ()))

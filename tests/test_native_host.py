@@ -141,3 +141,75 @@ def test_captured_transforms_keep_their_parameters(kind):
     del graph, out, graphs   # their memory goes back with the next call
     assert torch.equal(call(1), want[1])
     _C.release_cached_memory()
+
+
+def test_draws_go_through_the_hooks_of_a_subclass(monkeypatch):
+    from medvision_b200.aug_cuda_batch import BatchCudaRandomScale
+
+    class Corner(BatchCudaCropRandomWithAffine):
+        def _random_start(self):
+            return (1, 2, 3)
+
+        @staticmethod
+        def get_range(val_range, bias=0, always_pos=False):
+            return bias + 0.25
+
+    res = {"img_dim": 3, "img": torch.zeros(2, 1, 8, 10, 12), "img_fields": ["img"], "seg_fields": []}
+    t = Corner((4, 5, 6), scale=0.1, shift=0.1, rotate=10, times=3)
+    t._forward_params(dict(res))
+    assert np.array_equal(t.params["start"], [(3, 2, 1)] * 6) and np.array_equal(t.params["end"], [(9, 7, 5)] * 6)
+    assert np.array_equal(t.params["scales"], np.full((6, 3), 1.25)) and np.array_equal(t.params["shifts"], np.full((6, 3), 0.25))
+    assert np.array_equal(t.params["rotate"], np.full((6, 1), np.pi * 0.25 / 180))
+    t = BatchCudaRandomScale(1.0, 0.1)
+    t.get_range = lambda val_range, bias=0, always_pos=False: bias + 0.5  # of the object itself
+    t._forward_params(dict(res))
+    assert np.array_equal(t.params["scales"], np.full((2, 3), 1.5))
+    # numpy before 1.24 has no get_bit_generator
+    plain = BatchCudaCropRandomWithAffine((4, 5, 6), scale=0.1, shift=0.1, rotate=10)
+    params = []
+    for k in range(2):
+        if k:
+            monkeypatch.delattr(np.random, "get_bit_generator", raising=False)
+        np.random.seed(4)
+        plain._forward_params(dict(res))
+        params.append(plain.params)
+    assert all(np.array_equal(params[0][k], params[1][k]) for k in params[0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("batched", [True, False])
+def test_elastic_deformation_goes_through_the_hooks_of_a_subclass(batched):
+    from medvision_b200.aug_cuda import CudaRandomElasticDeformation
+    from medvision_b200.aug_cuda_batch import BatchCudaRandomElasticDeformation
+    cls = BatchCudaRandomElasticDeformation if batched else CudaRandomElasticDeformation
+    shape = (2, 1, 12, 20, 24) if batched else (1, 12, 20, 24)
+
+    class Still(cls):
+        def dense_field(self, device):
+            return torch.zeros_like(super().dense_field(device))
+
+    class ImageOnly(cls):
+        def apply_to_seg(self, result):
+            pass
+
+    class Brighter(cls):
+        def apply_to_img(self, result):
+            super().apply_to_img(result)
+            result["img"] = result["img"] + 1
+
+    g = torch.Generator().manual_seed(3)
+    img, seg = torch.rand(shape, generator=g).cuda(), torch.randint(0, 4, shape, generator=g, dtype=torch.int32).cuda()
+
+    def call(c):
+        np.random.seed(6)
+        return c(1.0, num_control_points=7, max_displacement=0.9)({"img_dim": 3, "img": img, "gt_seg": seg, "img_fields": ["img"],
+                                                                    "seg_fields": ["gt_seg"]})
+
+    want = call(cls)
+    assert not torch.equal(want["img"], img) and not torch.equal(want["gt_seg"], seg)
+    got = call(Still)
+    assert torch.equal(got["img"], img) and torch.equal(got["gt_seg"], seg)
+    got = call(ImageOnly)
+    assert torch.equal(got["img"], want["img"]) and got["gt_seg"] is seg
+    got = call(Brighter)
+    assert torch.equal(got["img"], want["img"] + 1) and torch.equal(got["gt_seg"], want["gt_seg"])
