@@ -185,7 +185,7 @@ resample_bwd_stream3d(const Params p, const S3Launch L, typename BwdAcc<T>::type
     const int mode = !(ina && inb) || dy < -1 || dy > 1 ? 2 : dy;  // rows shared: all (0), one (+-1), none (2)
     auto flush = [&](const float* v, int plane) {
       if (plane < 0) return;
-      if (!PAIR) {
+      if constexpr (!PAIR) {
         Acc* pl = acc + plane * HW;
         if (ina) {
           bwd_red_row(pl + oa[0], pl + oa[1], v[0], v[1], acc_lo, acc_hi);
@@ -195,36 +195,36 @@ resample_bwd_stream3d(const Params p, const S3Launch L, typename BwdAcc<T>::type
           bwd_red_row(pl + ob[0], pl + ob[1], v[4], v[5], acc_lo, acc_hi);
           bwd_red_row(pl + ob[2], pl + ob[3], v[6], v[7], acc_lo, acc_hi);
         }
-        return;
-      }
-      float c[8];
+      } else {
+        float c[8];
 #pragma unroll
-      for (int t = 0; t < 8; ++t) c[t] = v[t];
-      if (clamps) {  // both taps of the axis are the last voxel
-        if (txa.i0 == txa.i1) { c[1] += c[0]; c[3] += c[2]; c[0] = c[2] = 0.0f; }
-        if (txb.i0 == txb.i1) { c[5] += c[4]; c[7] += c[6]; c[4] = c[6] = 0.0f; }
-        if (tya.i0 == tya.i1) { c[2] += c[0]; c[3] += c[1]; c[0] = c[1] = 0.0f; }
-        if (tyb.i0 == tyb.i1) { c[6] += c[4]; c[7] += c[5]; c[4] = c[5] = 0.0f; }
-      }
-      const unsigned at = (unsigned)plane * L.pair.sz, a0 = at + ra, b0 = at + rb;
-      if (mode == 2) {
-        if (ina) {
-          bwd_send_row(rows, a0, c[0], c[1]);
-          bwd_send_row(rows, a0 + sy, c[2], c[3]);
+        for (int t = 0; t < 8; ++t) c[t] = v[t];
+        if (clamps) {  // both taps of the axis are the last voxel
+          if (txa.i0 == txa.i1) { c[1] += c[0]; c[3] += c[2]; c[0] = c[2] = 0.0f; }
+          if (txb.i0 == txb.i1) { c[5] += c[4]; c[7] += c[6]; c[4] = c[6] = 0.0f; }
+          if (tya.i0 == tya.i1) { c[2] += c[0]; c[3] += c[1]; c[0] = c[1] = 0.0f; }
+          if (tyb.i0 == tyb.i1) { c[6] += c[4]; c[7] += c[5]; c[4] = c[5] = 0.0f; }
         }
-        if (inb) {
-          bwd_send_row(rows, b0, c[4], c[5]);
-          bwd_send_row(rows, b0 + sy, c[6], c[7]);
+        const unsigned at = (unsigned)plane * L.pair.sz, a0 = at + ra, b0 = at + rb;
+        if (mode == 2) {
+          if (ina) {
+            bwd_send_row(rows, a0, c[0], c[1]);
+            bwd_send_row(rows, a0 + sy, c[2], c[3]);
+          }
+          if (inb) {
+            bwd_send_row(rows, b0, c[4], c[5]);
+            bwd_send_row(rows, b0 + sy, c[6], c[7]);
+          }
+          return;
         }
-        return;
+        // b's row that lies in a's first row, in a's second row, and the row(s) left
+        const bool up = mode == 1, down = mode == -1;
+        if (mode == 0) bwd_send_two(rows, a0, c[0], c[1], b0, c[4], c[5]);
+        else bwd_send_row(rows, up ? a0 : b0, up ? c[0] : c[4], up ? c[1] : c[5]);
+        bwd_send_two(rows, down ? a0 : a0 + sy, down ? c[0] : c[2], down ? c[1] : c[3], up ? b0 : b0 + sy, up ? c[4] : c[6],
+                     up ? c[5] : c[7]);
+        if (mode != 0) bwd_send_row(rows, (up ? b0 : a0) + sy, up ? c[6] : c[2], up ? c[7] : c[3]);
       }
-      // b's row that lies in a's first row, in a's second row, and the row(s) left
-      const bool up = mode == 1, down = mode == -1;
-      if (mode == 0) bwd_send_two(rows, a0, c[0], c[1], b0, c[4], c[5]);
-      else bwd_send_row(rows, up ? a0 : b0, up ? c[0] : c[4], up ? c[1] : c[5]);
-      bwd_send_two(rows, down ? a0 : a0 + sy, down ? c[0] : c[2], down ? c[1] : c[3], up ? b0 : b0 + sy, up ? c[4] : c[6],
-                   up ? c[5] : c[7]);
-      if (mode != 0) bwd_send_row(rows, (up ? b0 : a0) + sy, up ? c[6] : c[2], up ? c[7] : c[3]);
     };
     for (int i = 0; i < k.npd; ++i) {
       const S3ZTap<T> e = sh.zt[i];
@@ -278,7 +278,7 @@ resample_bwd_stream3d(const Params p, const S3Launch L, typename BwdAcc<T>::type
   for (int r = 0; r < 3; ++r)
     sxy[r] = Q::row_xy(Q::dup(g.rot[3 * r]), x2, Q::dup(A::mul(g.rot[3 * r + 1], y)));
   const V c2[3] = {Q::dup(g.centre[0]), Q::dup(g.centre[1]), Q::dup(g.centre[2])};
-  if (PAIR) {
+  if constexpr (PAIR) {
     // Consecutive depths often share tap rows (the upper z rows of one sample are the lower ones of the next half of the
     // time): the two upper rows of a voxel's last sample are held back and summed with the next sample's row of the same
     // place, and leave alone only when there is none.  3.4 reductions per voxel instead of 5 on rotations of up to 30 degrees.
@@ -354,25 +354,25 @@ resample_bwd_stream3d(const Params p, const S3Launch L, typename BwdAcc<T>::type
         bwd_send_row(rows, held[s] + sz, hv[s][0], hv[s][1]);
         bwd_send_row(rows, held[s] + sz + sy, hv[s][2], hv[s][3]);
       }
-    return;
-  }
-  for (int i = 0; i < k.npd; ++i) {
-    const S3ZProd<T> e = sh.zp[i];
-    const V rx2 = Q::add(Q::add(sxy[0], Q::dup(e.p[0])), c2[0]);
-    const V ry2 = Q::add(Q::add(sxy[1], Q::dup(e.p[1])), c2[1]);
-    const V rz2 = Q::add(Q::add(sxy[2], Q::dup(e.p[2])), c2[2]);
-    const T rx[2] = {Q::lo(rx2), Q::hi(rx2)}, ry[2] = {Q::lo(ry2), Q::hi(ry2)}, rz[2] = {Q::lo(rz2), Q::hi(rz2)};
-    const T gv[2] = {go[i * plane_o], has_b ? go[i * plane_o + 1] : A::fi(0)};
+  } else {
+    for (int i = 0; i < k.npd; ++i) {
+      const S3ZProd<T> e = sh.zp[i];
+      const V rx2 = Q::add(Q::add(sxy[0], Q::dup(e.p[0])), c2[0]);
+      const V ry2 = Q::add(Q::add(sxy[1], Q::dup(e.p[1])), c2[1]);
+      const V rz2 = Q::add(Q::add(sxy[2], Q::dup(e.p[2])), c2[2]);
+      const T rx[2] = {Q::lo(rx2), Q::hi(rx2)}, ry[2] = {Q::lo(ry2), Q::hi(ry2)}, rz[2] = {Q::lo(rz2), Q::hi(rz2)};
+      const T gv[2] = {go[i * plane_o], has_b ? go[i * plane_o + 1] : A::fi(0)};
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      if (s == 1 && !has_b) continue;
-      T w[8];
-      long long off[8];
-      if (!make_taps<T, 3>(p.D, p.H, p.W, rz[s], ry[s], rx[s], p.order, w, off)) continue;
+      for (int s = 0; s < 2; ++s) {
+        if (s == 1 && !has_b) continue;
+        T w[8];
+        long long off[8];
+        if (!make_taps<T, 3>(p.D, p.H, p.W, rz[s], ry[s], rx[s], p.order, w, off)) continue;
 #pragma unroll
-      for (int t = 0; t < 8; t += 2)
-        bwd_red_row(acc + off[t], acc + off[t + 1], A::tof(A::mul(gv[s], w[t])), A::tof(A::mul(gv[s], w[t + 1])), acc_lo,
-                    acc_hi);
+        for (int t = 0; t < 8; t += 2)
+          bwd_red_row(acc + off[t], acc + off[t + 1], A::tof(A::mul(gv[s], w[t])), A::tof(A::mul(gv[s], w[t + 1])), acc_lo,
+                      acc_hi);
+      }
     }
   }
 }

@@ -375,12 +375,11 @@ resample_flat(const Params p, const FlatDivs fd, int total, int lg) {
   if (!BWD && !beyond) ((T*)p.out)[e] = SR ? A::scale_pow2(acc, inv_count) : bad ? zero : A::div(acc, g.count_fwd);
 }
 
-// Forward of many outputs: a thread forms the taps of an output position once and
-// applies them to kFlatGroup channels.  Bound by the instructions of the taps (position, weights, offsets) where the channels
+// 2D forward of many outputs: a thread forms the taps of an output position once and applies them to kFlatGroup channels.  Bound by the instructions of the taps (position, weights, offsets) where the channels
 // are alone, by the scattered loads here.
 constexpr int kFlatGroup = 4;
 template <int N> struct FlatCount { static constexpr int value = N; };
-template <typename T, int NDIM, int SR>
+template <typename T, int SR>
 __global__ void __launch_bounds__(kFlatThreads)
 resample_flat_channels_fwd(const Params p, const FlatDivs fd, int total) {
   typedef Ar<T> A;
@@ -392,8 +391,8 @@ resample_flat_channels_fwd(const Params p, const FlatDivs fd, int total) {
   const int n0 = flat_div(e0, fd.per_roi);
   const int n_rois = flat_div(min(e0 + kFlatThreads, total) - 1, fd.per_roi) - n0 + 1;
   if ((int)threadIdx.x < n_rois) {
-    const int osz[3] = {p.ow, p.oh, p.od};
-    decode_roi<T>((const T*)p.rois, n0 + threadIdx.x, NDIM, p.kind, osz, p.spatial_scale, p.sampling_ratio, p.aligned, fm,
+    const int osz[3] = {p.ow, p.oh, 1};
+    decode_roi<T>((const T*)p.rois, n0 + threadIdx.x, 2, p.kind, osz, p.spatial_scale, p.sampling_ratio, p.aligned, fm,
                   geo[threadIdx.x]);
   }
   __syncthreads();
@@ -405,12 +404,9 @@ resample_flat_channels_fwd(const Params p, const FlatDivs fd, int total) {
   const RoiGeom<T>& g = geo[r];
   const int group = flat_div(rem, fd.ovol);
   const int v = rem - group * (int)fd.ovol.d;
-  const int row = flat_div(v, fd.ow);
-  const int pw = v - row * p.ow;
-  const int pd = (NDIM == 3) ? flat_div(row, fd.oh) : 0;
-  const int ph = (NDIM == 3) ? row - pd * p.oh : row;
+  const int ph = flat_div(v, fd.ow), pw = v - ph * p.ow;
   const int c0 = group * kFlatGroup, nc = min(kFlatGroup, p.C - c0);
-  constexpr float inv_count = 1.0f / (float)((SR ? SR : 1) * (SR ? SR : 1) * ((NDIM == 3 && SR) ? SR : 1));
+  constexpr float inv_count = 1.0f / (float)((SR ? SR : 1) * (SR ? SR : 1));
   T* const out = (T*)p.out + ((long long)(n0 + r) * p.C + c0) * p.ovol + v;
   const bool bad = g.batch < 0 || g.batch >= p.N;
   if (bad) {
@@ -421,8 +417,7 @@ resample_flat_channels_fwd(const Params p, const FlatDivs fd, int total) {
   const T* const vol = (const T*)p.in + ((long long)g.batch * p.C + c0) * p.vol;
   const T bx = lattice_base<T>(g.start[0], pw, g.bin[0], fm);
   const T by = lattice_base<T>(g.start[1], ph, g.bin[1], fm);
-  const T bz = (NDIM == 3) ? lattice_base<T>(g.start[2], pd, g.bin[2], fm) : A::fi(0);
-  const int gx = SR ? SR : g.grid[0], gy = SR ? SR : g.grid[1], gz = (NDIM == 3) ? (SR ? SR : g.grid[2]) : 1;
+  const int gx = SR ? SR : g.grid[0], gy = SR ? SR : g.grid[1];
   // N channels from `first` on
   auto channels = [&](auto count, int first) {
     constexpr int N = decltype(count)::value;
@@ -430,37 +425,34 @@ resample_flat_channels_fwd(const Params p, const FlatDivs fd, int total) {
 #pragma unroll
     for (int c = 0; c < N; ++c) acc[c] = A::fi(0);
 #pragma unroll 1
-    for (int iz = 0; iz < gz; ++iz) {
-      const T z = (NDIM == 3) ? A::add(bz, lattice_sub<T>(g.bin[NDIM - 1], iz, gz)) : A::fi(0);
-#pragma unroll 1
-      for (int iy = 0; iy < gy; ++iy) {
-        const T y = A::add(by, lattice_sub<T>(g.bin[1], iy, gy));
+    for (int iy = 0; iy < gy; ++iy) {
+      const T y = A::add(by, lattice_sub<T>(g.bin[1], iy, gy));
 #pragma unroll(SR ? SR : 1)
-        for (int ix = 0; ix < gx; ++ix) {
-          T sx, sy, sz;
-          to_volume<T, NDIM>(g, p.kind, fm, A::add(bx, lattice_sub<T>(g.bin[0], ix, gx)), y, z, sx, sy, sz);
-          T w[1 << NDIM];
-          int off[1 << NDIM];
-          if (!flat_taps<T, NDIM, int>(p, sz, sy, sx, w, off)) continue;  // adds zero
-          // (the last group of a roi reads its last channel again for those it lacks: no branch between the loads)
-          T tap[N][1 << NDIM];
+      for (int ix = 0; ix < gx; ++ix) {
+        T sx, sy, sz;
+        to_volume<T, 2>(g, p.kind, fm, A::add(bx, lattice_sub<T>(g.bin[0], ix, gx)), y, A::fi(0), sx, sy, sz);
+        T w[4];
+        int off[4];
+        if (!flat_taps<T, 2, int>(p, sz, sy, sx, w, off)) continue;  // adds zero
+        // (the last group of a roi reads its last channel again for those it lacks: no branch between the loads)
+        T tap[N][4];
 #pragma unroll
-          for (int c = 0; c < N; ++c) {
-            const T* const q = vol + (long long)min(first + c, nc - 1) * p.vol;
+        for (int c = 0; c < N; ++c) {
+          const T* const q = vol + (long long)min(first + c, nc - 1) * p.vol;
 #pragma unroll
-            for (int k = 0; k < (1 << NDIM); ++k) tap[c][k] = __ldg(q + off[k]);
-          }
-#pragma unroll
-          for (int c = 0; c < N; ++c) acc[c] = A::add(acc[c], tap_sum<T, (1 << NDIM)>(w, tap[c], fm));
+          for (int k = 0; k < 4; ++k) tap[c][k] = __ldg(q + off[k]);
         }
+#pragma unroll
+        for (int c = 0; c < N; ++c) acc[c] = A::add(acc[c], tap_sum<T, 4>(w, tap[c], fm));
       }
     }
 #pragma unroll
     for (int c = 0; c < N; ++c)
       if (first + c < nc) out[(long long)(first + c) * p.ovol] = SR ? A::scale_pow2(acc[c], inv_count) : A::div(acc[c], g.count_fwd);
   };
-  // the bins of a wide roi under a rotation share few lines of the L1, which four channels at once would overrun
-  // (adaptive rois with bins of up to 7 voxels a side, half: 241 us together, 189 channel by channel)
+  // the bins of a wide roi under a rotation share few lines of the L1, which four channels at once would overrun (one sample per
+  // bin, channel by channel / together, us: 512 x 64 rois of 40-140 px, float 17.0 / 18.6, half 16.5 / 17.6; 800 x 32, float 14.5 /
+  // 16.4; of 60-358 px 28.9 / 29.5)
   if (p.kind == KIND_ROTATED && A::tof(g.bin[0]) * A::tof(g.bin[1]) > 9.0f) {
     for (int c = 0; c < nc; ++c) channels(FlatCount<1>(), c);
   } else {
@@ -641,10 +633,10 @@ inline int launch_flat(const Params& p, bool fwd, cudaStream_t st) {
       fg.per_roi = make_flat_div((unsigned)(groups * p.ovol));
       const unsigned group_grid = (unsigned)((threads + kFlatThreads - 1) / kFlatThreads);
       if (one) {
-        flat_launch(resample_flat_channels_fwd<T, 2, 1>, group_grid, st, p, fg, (int)threads);
+        flat_launch(resample_flat_channels_fwd<T, 1>, group_grid, st, p, fg, (int)threads);
         return 0;
       }
-      flat_launch(resample_flat_channels_fwd<T, 2, 0>, group_grid, st, p, fg, (int)threads);
+      flat_launch(resample_flat_channels_fwd<T, 0>, group_grid, st, p, fg, (int)threads);
       return 0;
     }
   }
