@@ -6,34 +6,32 @@ import torch
 
 import cases
 from oracle import port
-from util import BWD_TOL, assert_close, n_mismatch
+from util import REF_FM, assert_close, assert_half_sums, n_mismatch
 
 pytestmark = pytest.mark.gpu
-REF_FM = 1 | (1 << 1) | (1 << 2) | (1 << 3) | (1 << 5) | (1 << 7) | (1 << 10) | (1 << 13) | \
-    (1 << 16) | (1 << 18) | (2 << 20) | (1 << 22)
 
 CASES = [
-    # spatial,        channels, rois, output,    sampling, order, dtype
-    ((37, 41),        5, 12, (7, 7),    0, 1, torch.float32),
-    ((600, 530),      1, 9,  (7, 5),    0, 1, torch.float32),   # boxes wider than the tables of positions and of taps
-    ((64, 97),        2, 40, (14, 14),  3, 1, torch.float32),   # groups of two
-    ((50, 63),        3, 9,  (3, 33),   0, 1, torch.float32),   # rows wider than a warp
-    ((37, 41),        4, 12, (7, 7),    0, 0, torch.float32),   # nearest
-    ((37, 41),        5, 40, (7, 7),    0, 1, torch.float32),   # enough outputs for a row per warp
-    ((37, 41),        4, 40, (7, 7),    0, 0, torch.float32),
-    ((600, 530),      2, 90, (7, 7),    0, 1, torch.float32),
-    ((70, 2100),      4, 40, (7, 7),    0, 1, torch.float32),   # samples beyond the forward's tables
-    ((33, 27),        3, 60, (7, 7),    0, 1, torch.float16),
-    ((64, 97),        6, 90, (14, 14),  2, 1, torch.float16),
-    ((19, 23, 29),    7, 80, (7, 6, 5), 3, 1, torch.float32),
-    ((19, 23, 29),    9, 60, (7, 6, 5), 0, 1, torch.float32),   # enough outputs for the 3D tables
-    ((12, 40, 170),   2, 30, (5, 5, 5), 0, 1, torch.float16),   # an axis beyond the tables of positions
-    ((19, 23, 29),    3, 40, (7, 7, 7), 2, 0, torch.float16),
-    ((640, 700),      2, 30, (5, 4),    0, 1, torch.float16),   # maps beyond the tables: several blocks per box, some idle
-    ((200, 336),      5, 30, (7, 7),    2, 1, torch.float16),   # samples far apart beside samples close together
-    ((200, 336),      4, 60, (14, 14),  3, 1, torch.float32),
-    ((40, 60, 70),    12, 50, (7, 7, 7), 2, 1, torch.float32),  # the same in 3D
-    ((64, 80, 96),    2, 20, (4, 5, 6), 2, 0, torch.float16),
+    # spatial,        channels, rois, output,    sampling, order, dtype, half additions per roi and voxel
+    ((37, 41),        5, 12, (7, 7),    0, 1, torch.float32, 0),
+    ((600, 530),      1, 9,  (7, 5),    0, 1, torch.float32, 0),   # boxes wider than the tables of positions and of taps
+    ((64, 97),        2, 40, (14, 14),  3, 1, torch.float32, 0),   # groups of two
+    ((50, 63),        3, 9,  (3, 33),   0, 1, torch.float32, 0),   # rows wider than a warp
+    ((37, 41),        4, 12, (7, 7),    0, 0, torch.float32, 0),   # nearest
+    ((37, 41),        5, 40, (7, 7),    0, 1, torch.float32, 0),   # enough outputs for a row per warp
+    ((37, 41),        4, 40, (7, 7),    0, 0, torch.float32, 0),
+    ((600, 530),      2, 90, (7, 7),    0, 1, torch.float32, 0),
+    ((70, 2100),      4, 40, (7, 7),    0, 1, torch.float32, 0),   # samples beyond the forward's tables
+    ((33, 27),        3, 60, (7, 7),    0, 1, torch.float16, 1),
+    ((64, 97),        6, 90, (14, 14),  2, 1, torch.float16, 4),
+    ((19, 23, 29),    7, 80, (7, 6, 5), 3, 1, torch.float32, 0),
+    ((19, 23, 29),    9, 60, (7, 6, 5), 0, 1, torch.float32, 0),   # enough outputs for the 3D tables
+    ((12, 40, 170),   2, 30, (5, 5, 5), 0, 1, torch.float16, 64),   # an axis beyond the tables of positions
+    ((19, 23, 29),    3, 40, (7, 7, 7), 2, 0, torch.float16, 8),
+    ((640, 700),      2, 30, (5, 4),    0, 1, torch.float16, 16),   # maps beyond the tables: several blocks per box, some idle
+    ((200, 336),      5, 30, (7, 7),    2, 1, torch.float16, 4),   # samples far apart beside samples close together
+    ((200, 336),      4, 60, (14, 14),  3, 1, torch.float32, 0),
+    ((40, 60, 70),    12, 50, (7, 7, 7), 2, 1, torch.float32, 0),  # the same in 3D
+    ((64, 80, 96),    2, 20, (4, 5, 6), 2, 0, torch.float16, 8),
 ]
 
 
@@ -53,9 +51,9 @@ def _rois(spatial, R, g):
     return torch.cat([b, c - s / 2, c + s / 2], 1)
 
 
-@pytest.mark.parametrize("spatial,C,R,out,sr,order,dtype", CASES,
+@pytest.mark.parametrize("spatial,C,R,out,sr,order,dtype,adds", CASES,
                          ids=["%s-%s-s%d-o%d-%s" % ("x".join(map(str, c[0])), "x".join(map(str, c[3])), c[4], c[5], str(c[6])[6:]) for c in CASES])
-def test_box_heads_match_the_restatement(spatial, C, R, out, sr, order, dtype):
+def test_box_heads_match_the_restatement(spatial, C, R, out, sr, order, dtype, adds):
     from medvision_b200 import _C
     nd = len(spatial)
     g = torch.Generator().manual_seed(sum(spatial) + R)
@@ -79,7 +77,10 @@ def test_box_heads_match_the_restatement(spatial, C, R, out, sr, order, dtype):
         gin = buf[16 + offset:16 + offset + n].view(feat.shape)
         gin.zero_()
         bwd(grad.cuda(), bad.cuda(), gin, *out, 1.0, sr, order)
-        assert_close(gin, want, 1e-5 if dtype == torch.float32 else BWD_TOL[dtype], "gradient")
+        if dtype == torch.float32:
+            assert_close(gin, want, 1e-5, "gradient")
+        else:
+            assert_half_sums(gin, want, grad[keep], rois[keep], cases.KIND_BOX, adds, **kw)
         around = torch.cat([buf[:16 + offset], buf[16 + offset + n:]])
         assert bool((torch.signbit(around) & (around == 0)).all()), "something was added outside the gradient tensor"
     _C.last_status()

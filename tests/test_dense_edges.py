@@ -6,11 +6,9 @@ import torch
 
 import cases
 from oracle import port
-from util import assert_close, n_mismatch
+from util import REF_FM, assert_close, n_mismatch
 
 pytestmark = pytest.mark.gpu
-REF_FM = 1 | (1 << 1) | (1 << 2) | (1 << 3) | (1 << 5) | (1 << 7) | (1 << 10) | (1 << 13) | \
-    (1 << 16) | (1 << 18) | (2 << 20) | (1 << 22)
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.float32])

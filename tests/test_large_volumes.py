@@ -6,10 +6,9 @@ import torch
 
 import cases
 from oracle import port
+from util import REF_FM
 
 pytestmark = pytest.mark.gpu
-REF_FM = 1 | (1 << 1) | (1 << 2) | (1 << 3) | (1 << 5) | (1 << 7) | (1 << 10) | (1 << 13) | \
-    (1 << 16) | (1 << 18) | (2 << 20) | (1 << 22)
 
 
 @pytest.fixture(scope="module")
