@@ -15,7 +15,7 @@ from typing import Union
 import numpy as np
 import torch
 
-from .base import BatchCudaAugBase, global_bit_generator, overrides
+from .base import BatchCudaAugBase, global_bit_generator
 from .elastic_field import ElasticField
 from .. import _C
 
@@ -271,7 +271,7 @@ class BatchCudaCropRandomWithAffine(BatchCudaAugBase):
         return np.array(batch_start), np.array(batch_end)
 
     def _forward_crop_params(self, result: dict):
-        if overrides(self, BatchCudaCropRandomWithAffine, '_random_start'):
+        if getattr(self._random_start, '__func__', None) is not BatchCudaCropRandomWithAffine._random_start:
             return self._collect([self._random_start() for _ in range(self.batch)])
         # one draw per patch and axis (d, h, w), as _random_start() makes them
         start = np.empty((self.batch, self.dim), dtype=np.int64)

@@ -27,10 +27,12 @@ _HOOKS = ('apply_to_img', 'apply_to_cls', 'apply_to_seg', 'apply_to_det')
 _LOG_KEYS = ('history', 'time', 'memory')
 
 
-def global_bit_generator():
-    """The bit generator behind ``np.random``'s functions."""
-    get = getattr(np.random, 'get_bit_generator', None)  # numpy 1.24
-    return get() if get is not None else np.random.mtrand._rand._bit_generator
+def _bit_generator_of_old_numpy():
+    return np.random.mtrand._rand._bit_generator
+
+
+# the bit generator behind np.random's functions; numpy has a function for it since 1.24
+global_bit_generator = getattr(np.random, 'get_bit_generator', _bit_generator_of_old_numpy)
 
 
 def overrides(obj, cls, *names):
@@ -89,7 +91,7 @@ class BatchCudaAugBase(object):
         :meth:`get_range` draws sample by sample (scale, one shift per axis, rotation in degrees), drawn natively from numpy's
         global generator, or by :meth:`get_range` itself where a subclass has its own."""
         dim = self.dim
-        if overrides(self, BatchCudaAugBase, 'get_range'):
+        if self.get_range is not BatchCudaAugBase.get_range:
             draws = [([self.get_range(self.scale, 1)] * dim, [self.get_range(self.shift, 0) for _ in range(dim)],
                       [np.pi * self.get_range(self.rotate, 0) / 180]) for _ in range(n)]
             return tuple(np.array(v) for v in zip(*draws))

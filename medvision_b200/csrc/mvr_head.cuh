@@ -11,7 +11,9 @@
 // on neighbouring windows.  One reduction per window and roi instead of 1.25 per sample and tap row: the reduction path of
 // this GPU charges per operation (mvr_generic.cuh), and that was the whole cost of these kernels.  The sums are formed in
 // float for every element type.  A box whose samples lie too far apart for that, or that exceeds the tables, goes sample by
-// sample in the same CTA.
+// sample in the same CTA.  Bound by instruction issue (67 % of the slots on the first call below) and the barriers between the
+// tables, 5-8 us of which no call is free.  Flat kernel -> here, us: 200 boxes of 8-64 px, adaptive, 32 x 101 x 135 float 96 -> 27;
+// 128 of 5-24, adaptive, 16 x 48^3 float 214 -> 53; 128 of 8-48, two samples, 16 x 64^3 half 202 -> 61.
 //
 // Launched as programmatic dependents like the flat kernels (mvr_flat.cuh).
 #pragma once
@@ -93,7 +95,9 @@ constexpr int kBoxFwdTable = 31 * 1024;  // bytes of both axes' tables at most: 
 // for all channels and leave the values in shared memory; then its lanes take OUTPUTS and add the values up in the
 // reference's order.  The tables hold the samples of any box inside the map (up to 1980 positions on both axes together); the
 // taps of a larger grid are formed as they are used.  In 3D (few samples per line) and in half (loads half as wide) it does
-// not gain: those stay with the flat kernel.
+// not gain: those stay with the flat kernel.  Bound by instruction issue while its CTAs run (23 M warp instructions, 70 % of the
+// slots), and a third of the time by the uneven end of boxes of 4 to 100 samples per bin.  200 boxes x 32 channels on 101 x 135, 7 x 7
+// bins, flat kernel -> here: of 8-64 px 43 -> 34 us; of 10-120 px on 200 x 336 133 -> 102; 64 x 8 of 60-358 px on 512 x 512 571 -> 331.
 template <typename T>
 __device__ __forceinline__ void box_zero_task(const Params& p, T* out, int task, int group) {
   const int rows = p.od * p.oh, cg = task / rows, row = task - cg * rows, c0 = cg * group, nc = min(group, p.C - c0);

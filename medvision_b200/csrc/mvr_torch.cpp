@@ -200,9 +200,10 @@ struct RoiBackward : public torch::autograd::Node {
   }
 };
 
+bool has_tangent(const at::Tensor& t) { return torch::autograd::impl::get_autograd_meta(t) && t._fw_grad(/*level=*/0).defined(); }
+
 at::Tensor roi_module_forward(const RoiOp& op, const at::Tensor& features, const at::Tensor& rois) {
-  TORCH_CHECK_NOT_IMPLEMENTED(!torch::autograd::isFwGradDefined(features) && !torch::autograd::isFwGradDefined(rois), op.what(),
-                              " has no forward-mode derivative");
+  TORCH_CHECK_NOT_IMPLEMENTED(!has_tangent(features) && !has_tangent(rois), op.what(), " has no forward-mode derivative");
   at::Tensor out = roi_forward(op, features, rois);
   if (torch::autograd::compute_requires_grad(features, rois)) {
     auto node = std::shared_ptr<RoiBackward>(new RoiBackward(), torch::autograd::deleteNode);

@@ -143,7 +143,7 @@ def test_captured_transforms_keep_their_parameters(kind):
     _C.release_cached_memory()
 
 
-def test_draws_go_through_the_hooks_of_a_subclass(monkeypatch):
+def test_draws_go_through_the_hooks_of_a_subclass():
     from medvision_b200.aug_cuda_batch import BatchCudaRandomScale
 
     class Corner(BatchCudaCropRandomWithAffine):
@@ -164,15 +164,25 @@ def test_draws_go_through_the_hooks_of_a_subclass(monkeypatch):
     t.get_range = lambda val_range, bias=0, always_pos=False: bias + 0.5  # of the object itself
     t._forward_params(dict(res))
     assert np.array_equal(t.params["scales"], np.full((2, 3), 1.5))
-    # numpy before 1.24 has no get_bit_generator
-    plain = BatchCudaCropRandomWithAffine((4, 5, 6), scale=0.1, shift=0.1, rotate=10)
+    t = BatchCudaCropRandomWithAffine((4, 5, 6), scale=0.1, shift=0.1, rotate=10)
+    t._random_start = lambda: (1, 2, 3)
+    t._forward_params(dict(res))
+    assert np.array_equal(t.params["start"], [(3, 2, 1)] * 2)
+
+
+def test_draws_without_numpys_get_bit_generator(monkeypatch):
+    """numpy before 1.24"""
+    from medvision_b200.aug_cuda_batch import aug_spatial, base
+    res = {"img_dim": 3, "img": torch.zeros(2, 1, 8, 10, 12), "img_fields": ["img"], "seg_fields": []}
+    t = BatchCudaCropRandomWithAffine((4, 5, 6), scale=0.1, shift=0.1, rotate=10)
     params = []
     for k in range(2):
         if k:
-            monkeypatch.delattr(np.random, "get_bit_generator", raising=False)
+            for module in (base, aug_spatial):
+                monkeypatch.setattr(module, "global_bit_generator", base._bit_generator_of_old_numpy)
         np.random.seed(4)
-        plain._forward_params(dict(res))
-        params.append(plain.params)
+        t._forward_params(dict(res))
+        params.append(t.params)
     assert all(np.array_equal(params[0][k], params[1][k]) for k in params[0])
 
 
