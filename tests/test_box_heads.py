@@ -97,3 +97,36 @@ def test_half_gradient_divides_by_the_count_in_half():
     gin = torch.zeros(want.shape, dtype=torch.half, device="cuda")
     _C.roi_align_2d_backward(grad.cuda(), rois.cuda(), gin, 1, 1, 1.0, 0, 1)
     assert_close(gin, want, 2e-3, "gradient")
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("spatial,C,R,out,sr,rotated", [
+    ((64, 97), 3, 90, (14, 14), 2, False),
+    ((64, 97), 2, 60, (7, 7), 0, False),
+    ((600, 530), 1, 40, (7, 7), 0, False),
+    ((19, 23, 29), 7, 80, (7, 6, 5), 3, False),
+    ((19, 23, 29), 3, 12, (5, 5, 5), 2, True),
+    ((60, 70, 80), 1, 8, (5, 5, 5), 0, True),
+], ids=["boxes", "adaptive", "wide", "boxes3d", "rotated", "rotated-large"])
+def test_gradients_that_are_not_finite_stay_where_they_belong(spatial, C, R, out, sr, rotated, dtype):
+    from medvision_b200 import _C
+    nd = len(spatial)
+    g = torch.Generator().manual_seed(R)
+    rois = _rois(spatial, R, g)
+    if rotated:
+        lo, hi = rois[:, 1:1 + nd], rois[:, 1 + nd:]
+        rois = torch.cat([rois[:, :1], (lo + hi) / 2, hi - lo, torch.rand(R, 1 if nd == 2 else 3, generator=g)], 1)
+    rois = rois.to(dtype)
+    grad = torch.randn((R, C) + out, generator=g).to(dtype)
+    flat = grad.view(-1)
+    flat[::997] = float("inf")
+    flat[500::1999] = float("nan")
+    kw = dict(spatial_scale=1.0, sampling_ratio=sr, aligned=True, order=1, fma_mode=REF_FM if dtype == torch.float32 else 0)
+    if rotated:
+        kw["trig"] = port.device_trig(rois)
+    want = port.backward(grad, rois, (2, C) + spatial, cases.KIND_ROTATED if rotated else cases.KIND_BOX, wide_acc=True, **kw)
+    gin = torch.zeros(want.shape, dtype=dtype, device="cuda")
+    name = "roi_align_%s%dd_backward" % ("rotated_" if rotated else "", nd)
+    getattr(_C, name)(grad.cuda(), rois.cuda(), gin, *out, 1.0, sr, *((True,) if rotated else ()), 1)
+    bad = ~torch.isfinite(want)
+    assert 0 < int(bad.sum()) < bad.numel() and torch.equal(~torch.isfinite(gin.cpu()), bad)
