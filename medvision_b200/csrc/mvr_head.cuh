@@ -817,7 +817,8 @@ __device__ __forceinline__ void rot_walk(const Params& p, const RotSlab<T, NDIM>
                       s.tensor_hi);
     }
   };
-  const int parts = HOW == kRotPatch ? 1 : s.parts, part = HOW == kRotPatch ? 0 : s.part;
+  constexpr bool kShared = HOW != kRotPatch;  // the lines are shared by several CTAs
+  const int parts = kShared ? s.parts : 1, part = kShared ? s.part : 0;
   for (long long item = part * kRotThreads + threadIdx.x; item < (long long)outputs * s.lines; item += parts * kRotThreads) {
     const int line = (int)(item / outputs), o = (int)(item - (long long)line * outputs);
     const int iz = line / gy, iy = line - iz * gy;
@@ -925,7 +926,8 @@ __device__ __noinline__ void rot_without_patch(const Params& p, const RotSlab<T,
   else rot_walk<T, NDIM, kRotSamples>(p, s, nullptr);
 }
 
-template <typename T, int NDIM>
+// CELLS: slabs without a patch by the walks of their own above; otherwise in the walk of the patch, each sample by itself.
+template <typename T, int NDIM, bool CELLS>
 __global__ void __launch_bounds__(kRotThreads, 4)
 rot_head_bwd(const __grid_constant__ Params p, int slabs, int parts) {
   typedef Ar<T> A;
@@ -993,30 +995,118 @@ rot_head_bwd(const __grid_constant__ Params p, int slabs, int parts) {
   if (patch)
     for (int i = threadIdx.x; i < (int)cells; i += kRotThreads) rot_patch[i] = 0.0f;
   __syncthreads();
-  RotSlab<T, NDIM> work;
-  work.g = &g;
-  work.subs = subs;
-  work.grad = grad;
-  work.go = go;
-  work.tensor_lo = tensor_lo;
-  work.tensor_hi = tensor_hi;
-  work.first = first;
-  work.outputs = outputs;
-  work.lines = lines;
-  work.part = part;
-  work.parts = parts;
+  if constexpr (CELLS) {
+    RotSlab<T, NDIM> work;
+    work.g = &g;
+    work.subs = subs;
+    work.grad = grad;
+    work.go = go;
+    work.tensor_lo = tensor_lo;
+    work.tensor_hi = tensor_hi;
+    work.first = first;
+    work.outputs = outputs;
+    work.lines = lines;
+    work.part = part;
+    work.parts = parts;
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    work.lo[a] = lo[a];
-    work.ext[a] = ext[a];
+    for (int a = 0; a < 3; ++a) {
+      work.lo[a] = lo[a];
+      work.ext[a] = ext[a];
+    }
+    work.sy = sy;
+    work.sz = sz;
+    if (!patch) {
+      rot_without_patch<T, NDIM>(p, work);
+      return;
+    }
+    rot_walk<T, NDIM, kRotPatch>(p, work, rot_patch);
+  } else {
+    // through the patch, or each sample by itself (written out here: through rot_walk the registers do not suffice, 8-20 % slower)
+    const float inv_n = 1.0f / A::tof(g.count_bwd);
+    auto sub = [&](int a, int i) { return i < kFlatSubs ? subs[a][i] : lattice_sub<T>(g.bin[a], i, g.grid[a]); };
+
+    for (long long item = threadIdx.x; item < (long long)outputs * lines; item += kRotThreads) {
+      const int line = (int)(item / outputs), o = (int)(item - (long long)line * outputs);
+      const int iz = line / gy, iy = line - iz * gy;
+      const int pw = o % p.ow, row = o / p.ow + first * (NDIM == 3 ? p.oh : 1), pd = NDIM == 3 ? row / p.oh : 0, ph = row - pd * p.oh;
+      const T bx = lattice_base<T>(g.start[0], pw, g.bin[0], fm);
+      const T y = A::add(lattice_base<T>(g.start[1], ph, g.bin[1], fm), sub(1, iy));
+      const T z = NDIM == 3 ? A::add(lattice_base<T>(g.start[2], pd, g.bin[2], fm), sub(NDIM - 1, iz)) : A::fi(0);
+      const T gv = __ldg(go + o);
+      int held = -1;            // cell whose contributions are being summed
+      float sum[kTaps];
+      auto flush = [&]() {
+        if (held < 0) return;
+        float* const q = rot_patch + held;
+#pragma unroll
+        for (int t = 0; t < kTaps; ++t)
+          if (sum[t] != 0.0f) atomicAdd(q + (t & 1) + (t & 2 ? sy : 0) + (t & 4 ? sz : 0), sum[t]);
+      };
+      for (int ix = 0; ix < gx; ++ix) {
+        T px, py, pz;
+        to_volume<T, NDIM>(g, KIND_ROTATED, fm, A::add(bx, sub(0, ix)), y, z, px, py, pz);
+        FlatAxis<T> t[3];
+        bool in = flat_axis<T>(px, p.W, t[0]);
+        in = flat_axis<T>(py, p.H, t[1]) && in;
+        if (NDIM == 3) in = flat_axis<T>(pz, p.D, t[2]) && in;
+        if (!in) continue;
+        T w[kTaps];
+        if (p.order == 0) {
+          AxisTap<T> m[3];
+#pragma unroll
+          for (int a = 0; a < NDIM; ++a) {
+            m[a].l = t[a].l;
+            m[a].h = t[a].h;
+          }
+          nearest_pick<T, NDIM>(m, w);
+        } else {
+#pragma unroll
+          for (int k = 0; k < kTaps; k += 2) {
+            T zy = (k & 2) ? t[1].l : t[1].h;
+            if (NDIM == 3) zy = A::mul((k & 4) ? t[2].l : t[2].h, zy);
+            w[k] = A::mul(zy, t[0].h);
+            w[k + 1] = A::mul(zy, t[0].l);
+          }
+        }
+        const int rx = t[0].i0 - lo[0], ry = t[1].i0 - lo[1], rz = NDIM == 3 ? t[2].i0 - lo[2] : 0;
+        // (the room for rounding is generous: a sample outside the box is sent directly, like every sample without a patch)
+        const bool inside = patch && rx >= 0 && rx + t[0].d < ext[0] && ry >= 0 && ry + t[1].d < ext[1] &&
+                            (NDIM == 2 || (rz >= 0 && rz + t[2].d < ext[2]));
+        if (inside) {
+          const int cell = rz * sz + ry * sy + rx + kWin;
+          if (cell != held) {
+            flush();
+            held = cell;
+#pragma unroll
+            for (int k = 0; k < kTaps; ++k) sum[k] = 0.0f;
+          }
+          // a clamped upper tap lies on the lower one, with weight 0: its (zero) product goes there
+#pragma unroll
+          for (int k = 0; k < kTaps; ++k) {
+            const float v = A::tof(A::mul(gv, w[k])) * inv_n;
+            int at = k;
+            if (!t[0].d) at &= ~1;
+            if (!t[1].d) at &= ~2;
+            if (NDIM == 3 && !t[2].d) at &= ~4;
+            if (at == k) sum[k] += v;
+            else if (v != 0.0f) atomicAdd(rot_patch + cell + (at & 1) + (at & 2 ? sy : 0) + (at & 4 ? sz : 0), v);
+          }
+        } else {
+          const long long at = (NDIM == 3 ? (long long)t[2].i0 * p.H * p.W : 0) + (long long)t[1].i0 * p.W + t[0].i0;
+          const long long dy = (long long)t[1].d * p.W, dz = NDIM == 3 ? (long long)t[2].d * p.H * p.W : 0;
+          T* const q = grad + at;
+#pragma unroll
+          for (int k = 0; k < kTaps; k += 2) {
+            T* const row_p = q + ((k & 2) ? dy : 0) + ((k & 4) ? dz : 0);
+            atomic_add_pair(row_p, row_p + t[0].d, A::ff(A::tof(A::mul(gv, w[k])) * inv_n), A::ff(A::tof(A::mul(gv, w[k + 1])) * inv_n),
+                            tensor_lo, tensor_hi);
+          }
+        }
+      }
+      flush();
+    }
+    if (!patch) return;
   }
-  work.sy = sy;
-  work.sz = sz;
-  if (!patch) {
-    rot_without_patch<T, NDIM>(p, work);
-    return;
-  }
-  rot_walk<T, NDIM, kRotPatch>(p, work, rot_patch);
   __syncthreads();
   // every window of the box with something in it, once
   const int windows = (ext[0] + 2 * kWin - 2) / kWin, rows = ext[1] * ext[2];
@@ -1077,12 +1167,19 @@ inline int launch_rot_head_bwd(const Params& p, cudaStream_t st) {
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-#define MVR_ROT(ND)                                                                                                          \
-  {                                                                                                                          \
-    cudaFuncSetAttribute(rot_head_bwd<__half, ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes); \
-    cudaLaunchKernelEx(&cfg, rot_head_bwd<__half, ND>, p, slabs, parts);                                                     \
+  // Two and three samples per bin seldom share cells where the box exceeds the patch (error as the flat kernel's), and go without the
+  // walks of their own, which cost 5-17 % (300 x 32 rois of 40-64 voxels, two samples: 968 us without, 1134 with), unless CTAs would idle.
+  const bool by_cells = p.sampling_ratio <= 0 || p.sampling_ratio > 3 || parts > 1;
+#define MVR_ROT(ND, CELLS)                                                                                                          \
+  {                                                                                                                                 \
+    cudaFuncSetAttribute(rot_head_bwd<__half, ND, CELLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes); \
+    cudaLaunchKernelEx(&cfg, rot_head_bwd<__half, ND, CELLS>, p, slabs, parts);                                                     \
   }
-  if (p.ndim == 2) MVR_ROT(2) else MVR_ROT(3)
+  if (p.ndim == 2) {
+    if (by_cells) MVR_ROT(2, true) else MVR_ROT(2, false)
+  } else {
+    if (by_cells) MVR_ROT(3, true) else MVR_ROT(3, false)
+  }
 #undef MVR_ROT
   return 0;
 }
