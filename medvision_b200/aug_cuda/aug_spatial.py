@@ -229,6 +229,9 @@ class CudaRandomElasticDeformation(ElasticField, CudaAugBase):
         return both and tuple([t.squeeze(0) for t in v] for v in both)
 
 
+CudaRandomElasticDeformation._transform = CudaRandomElasticDeformation
+
+
 class CudaCropRandomWithAffine(CudaAugBase):
     """A ``patch_size`` crop at a random position with a random scale / shift / z-rotation, in one
     resample; ``times`` > 1 turns one sample into ``times`` crops (a list of results)."""

@@ -215,6 +215,9 @@ class BatchCudaRandomElasticDeformation(ElasticField, BatchCudaAugBase):
             raise NotImplementedError
 
 
+BatchCudaRandomElasticDeformation._transform = BatchCudaRandomElasticDeformation
+
+
 class BatchCudaCropRandomWithAffine(BatchCudaAugBase):
     def __init__(self, patch_size, scale: Union[float, list, tuple], shift: Union[float, list, tuple],
                  rotate: Union[float, list, tuple], sampling_ratio=1, order=1, times=1):

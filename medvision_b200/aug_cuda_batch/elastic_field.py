@@ -16,6 +16,7 @@ from ..ops.cuda_fun_tools import affine_2d, affine_3d, apply_offset_2d, apply_of
 class ElasticField:
     """Mixin; the class provides ``dim``, ``image_shape``, ``img_type``, ``num_control_points``, ``max_displacement``,
     ``num_locked_borders``, ``params`` and ``_field_order`` (interpolation of the blow-up)."""
+    _transform = None  # the transform itself, which a subclass may override
     _dense = None    # the dense field, once it has been asked for
     _device = None   # where the fields of the current parameters were warped
 
@@ -94,8 +95,7 @@ class ElasticField:
                 [self._warp_with_dense_field(t, field.to(t.device), 0) for t in labels])
 
     def _warp_in_place(self, result, img_keys, seg_keys):
-        own = next(c for c in type(self).__mro__ if ElasticField in c.__bases__)  # the transform that a subclass derives from
-        if overrides(self, own, 'elastic_transform', 'dense_field'):
+        if overrides(self, self._transform, 'elastic_transform', 'dense_field'):
             result.update({k: self.elastic_transform(result[k]) for k in img_keys})
             result.update({k: self.elastic_transform(result[k], order=0).int() for k in seg_keys})
             return
