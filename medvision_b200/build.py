@@ -12,7 +12,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libmvr.so")
 NATIVE = os.path.join(HERE, "_native.so")
 SOURCES = ["mvr_api.cu"]
-HEADERS = ["mvr_arith.cuh", "mvr_geom.cuh", "mvr_generic.cuh", "mvr_stream3d.cuh", "mvr_tma3d.cuh", "mvr_bwd3d.cuh", "mvr_offset.cuh", "mvr_cubic3d.cuh", "mvr_flat.cuh", "mvr_label.cuh", "mvr_plane2d.cuh", "mvr_elastic.cuh", "mvr_head.cuh",
+HEADERS = ["mvr_arith.cuh", "mvr_geom.cuh", "mvr_generic.cuh", "mvr_stream3d.cuh", "mvr_tma3d.cuh", "mvr_brick3d.cuh", "mvr_bwd3d.cuh", "mvr_offset.cuh", "mvr_cubic3d.cuh", "mvr_flat.cuh", "mvr_label.cuh", "mvr_plane2d.cuh", "mvr_elastic.cuh", "mvr_head.cuh",
            os.path.join("..", "..", "include", "mvr.h")]
 NATIVE_SOURCES = ["mvr_torch.cpp"]
 NATIVE_HEADERS = [os.path.join("..", "..", "include", "mvr.h")]

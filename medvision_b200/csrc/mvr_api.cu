@@ -281,7 +281,7 @@ int mvr_roi_resample_bwd_noalloc(const void* grad_out, const void* rois, void* g
     float* scratch = nullptr;
     rc = noalloc_scratch_of_current_device(&scratch);
     if (rc != MVR_OK) return rc;
-    return launch_bwd_stream3d_half(p, L, ctas, scratch, st) == 0 ? MVR_OK : MVR_ERR_LAUNCH;
+    return launch_bwd_stream3d_half(p, L, ctas, scratch, nullptr, st) == 0 ? MVR_OK : MVR_ERR_LAUNCH;
   }
   // every other shape goes where the regular entry point sends it: kernels that accumulate with
   // element-type atomics straight into grad_in and use no scratch

@@ -15,7 +15,7 @@
 #pragma once
 #include <mutex>
 
-#include "mvr_stream3d.cuh"
+#include "mvr_brick3d.cuh"
 
 namespace mvr {
 
@@ -105,14 +105,12 @@ __device__ __forceinline__ void bwd_send_two(const BwdRows& r, unsigned at_p, fl
 // PAIR: both voxels of a thread share their instructions and offsets are 32-bit bytes (mvr_stream3d.cuh, pair taps; sizes of
 // at least two, float volumes below 4 GiB); the other form takes every other shape.
 template <typename T, bool PAIR>
-__global__ void __launch_bounds__(kS3Threads, PAIR ? 3 : 1)
-resample_bwd_stream3d(const Params p, const S3Launch L, typename BwdAcc<T>::type* __restrict__ acc_base) {
+__device__ __forceinline__ void bwd_scatter(const Params& p, const S3Launch& L, typename BwdAcc<T>::type* __restrict__ acc_base, const S3Cta& k,
+                                            S3Shared<T>& sh) {
   typedef Ar<T> A;
   typedef P2<T> Q;
   typedef typename Q::V V;
   typedef typename BwdAcc<T>::type Acc;
-  __shared__ S3Shared<T> sh;
-  const S3Cta k = s3_cta(p, L);
   s3_prologue<T>(p, k, sh);
   const RoiGeom<T>& g = sh.g;
   const int fm = kS3FloatPattern;
@@ -377,24 +375,68 @@ resample_bwd_stream3d(const Params p, const S3Launch L, typename BwdAcc<T>::type
   }
 }
 
-// grad_in (half) += scratch (float), rounded once
-__global__ void bwd_fold_half(__half* __restrict__ grad_in, const float* __restrict__ scratch, long long n) {
-  const long long i0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
-  if (i0 + 8 <= n && ((uintptr_t)(grad_in + i0) % 16 == 0)) {
-    const float4 s0 = *reinterpret_cast<const float4*>(scratch + i0);
-    const float4 s1 = *reinterpret_cast<const float4*>(scratch + i0 + 4);
-    uint4 gv = *reinterpret_cast<const uint4*>(grad_in + i0);
-    __half2* h = reinterpret_cast<__half2*>(&gv);
-    const float s[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+template <typename T, bool PAIR>
+__global__ void __launch_bounds__(kS3Threads, PAIR ? 3 : 1)
+resample_bwd_stream3d(const Params p, const S3Launch L, typename BwdAcc<T>::type* __restrict__ acc_base) {
+  __shared__ S3Shared<T> sh;
+  bwd_scatter<T, PAIR>(p, L, acc_base, s3_cta(p, L), sh);
+}
+
+// What bwd_brick3d_half leaves: the bricks that need two words per voxel, and by the `scatter` CTAs behind those the rois that the
+// bricks do not take.  Mostly there is neither, and the grid is gone after a look at the plan.
+template <bool PAIR>
+__global__ void __launch_bounds__(kS3Threads, PAIR ? 3 : 1)
+bwd_brick3d_rest(const Params p, const PairConst pc, const BrickPlan plan, const BrickGrid G, unsigned bricks, const S3Launch L,
+                 float* __restrict__ acc_base, long long items) {
+  extern __shared__ __align__(16) unsigned char brick_smem[];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (blockIdx.x < bricks) {
+    brick_body<true>(p, pc, plan, G, brick_smem);
+    return;
+  }
+  if (blockIdx.x == bricks && p.status) {
+    for (int n = threadIdx.x; n < p.R; n += kS3Threads)
+      if (__ldcg(plan.volume + n) == INT_MIN) atomicOr(p.status, STATUS_BAD_BATCH_INDEX);
+  }
+  if (!brick_leaves_any(p, plan)) return;
+  S3Shared<__half>& sh = *reinterpret_cast<S3Shared<__half>*>(brick_smem);
+  BrickLeft& left = *reinterpret_cast<BrickLeft*>(brick_smem + ((sizeof(S3Shared<__half>) + 15) & ~size_t(15)));
+  static_assert(sizeof(S3Shared<__half>) + 16 + sizeof(BrickLeft) <= sizeof(BrickSharedTwo), "shared memory of the launch");
+  brick_left(p, plan, left);
+  for (long long item = blockIdx.x - bricks; item < items; item += gridDim.x - bricks) {
+    const S3Cta k = s3_cta(p, L, item);
+    if (!((left.mask[k.n >> 5] >> (k.n & 31)) & 1u)) continue;  // CTA-uniform
+    bwd_scatter<__half, PAIR>(p, L, acc_base, k, sh);
+    __syncthreads();  // the next item's prologue overwrites the tables
+  }
+}
+
+// grad_in (half) += scratch (float), rounded once.  IF_LEFT: only where the bricks left a roi to the scattering kernel.
+template <bool IF_LEFT>
+__global__ void __launch_bounds__(256) bwd_fold_half(const Params p, const BrickPlan plan, const float* scratch, long long n) {
+  if (IF_LEFT) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!brick_leaves_any(p, plan)) return;
+  }
+  __half* const grad_in = (__half*)p.out;
+  for (long long i0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8; i0 < n; i0 += (long long)gridDim.x * blockDim.x * 8) {
+    if (i0 + 8 <= n && ((uintptr_t)(grad_in + i0) % 16 == 0)) {
+      const float4 s0 = __ldcg(reinterpret_cast<const float4*>(scratch + i0));
+      const float4 s1 = __ldcg(reinterpret_cast<const float4*>(scratch + i0 + 4));
+      uint4 gv = *reinterpret_cast<const uint4*>(grad_in + i0);
+      __half2* h = reinterpret_cast<__half2*>(&gv);
+      const float s[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 f = __half22float2(h[j]);
-      h[j] = __floats2half2_rn(f.x + s[2 * j], f.y + s[2 * j + 1]);
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = __half22float2(h[j]);
+        h[j] = __floats2half2_rn(f.x + s[2 * j], f.y + s[2 * j + 1]);
+      }
+      *reinterpret_cast<uint4*>(grad_in + i0) = gv;
+    } else {
+      for (long long i = i0; i < n && i < i0 + 8; ++i)
+        grad_in[i] = __float2half_rn(__half2float(grad_in[i]) + scratch[i]);
     }
-    *reinterpret_cast<uint4*>(grad_in + i0) = gv;
-  } else {
-    for (long long i = i0; i < n && i < i0 + 8; ++i)
-      grad_in[i] = __float2half_rn(__half2float(grad_in[i]) + scratch[i]);
   }
 }
 
@@ -420,22 +462,83 @@ inline bool bwd_stream3d_applicable(const Params& p, int dtype, S3Launch& L, lon
   return ctas <= 0x7fffffffLL;
 }
 
+inline bool bwd_pair_form(const Params& p) {
+  return p.D >= 2 && p.H >= 2 && p.W >= 2 && pair_taps_applicable(p.D, p.H, p.W, p.vol + 8, 4);
+}
 template <typename T>
 inline void launch_bwd_kernel(const Params& p, const S3Launch& L, long long ctas, float* acc, cudaStream_t st) {
-  if (p.D >= 2 && p.H >= 2 && p.W >= 2 && pair_taps_applicable(p.D, p.H, p.W, p.vol + 8, 4))
-    resample_bwd_stream3d<T, true><<<(unsigned)ctas, kS3Threads, 0, st>>>(p, L, acc);
+  if (bwd_pair_form(p)) resample_bwd_stream3d<T, true><<<(unsigned)ctas, kS3Threads, 0, st>>>(p, L, acc);
   else resample_bwd_stream3d<T, false><<<(unsigned)ctas, kS3Threads, 0, st>>>(p, L, acc);
 }
 
-// Half backward through a float scratch volume of n = N*C*D*H*W elements that the caller of this
-// function owns: clear it, scatter into it, fold it into grad_in.  Allocates nothing.
-inline int launch_bwd_stream3d_half(const Params& p, const S3Launch& L, long long ctas, float* scratch,
-                                    cudaStream_t st) {
+// Whether the gradient is summed brick by brick.  Few rois per volume, as the dense calls have them: a brick looks at every roi of
+// its volume.
+inline bool bwd_brick3d_applicable(const Params& p, int dtype) {
+  if (dtype != 1 || p.R > kBrickMaxRois || p.R > 4LL * p.N || p.D > kTapMaxSize || p.H > kTapMaxSize || p.W > kTapMaxSize) return false;
+  if (p.ovol >= 0x7fffffffLL || p.ow >= (1 << 23) || (long long)p.R * p.C * kBrickMaxParts > 0x7ffffff0LL - p.R) return false;
+  const long long bw = (p.W + kBrick - 1) / kBrick, bh = (p.H + kBrick - 1) / kBrick, bd = (p.D + kBrick - 1) / kBrick;
+  const long long bricks = (long long)p.N * p.C * bw * bh * bd;
+  return bricks >= kBrickMinBricks && bricks <= 0x7fffff00LL;
+}
+
+template <bool PAIR>
+inline cudaError_t launch_bwd_brick3d(const Params& p, const S3Launch& L, long long ctas, float* scratch, const BrickPlan& plan, cudaStream_t st) {
+  const long long n = (long long)p.N * p.C * p.vol;
+  const size_t smem1 = sizeof(BrickShared), smem2 = sizeof(BrickSharedTwo);
+  // more dynamic shared memory than the default limit: opt in (per function and device; smem1 lies below it)
+  static_assert(sizeof(BrickShared) <= 48 * 1024, "default limit");
+  cudaFuncSetAttribute(bwd_brick3d_rest<PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
+  const PairConst pc = make_pair_const(3, p.D, p.H, p.W, 2);
+  BrickGrid G;
+  G.bricks_w = (p.W + kBrick - 1) / kBrick;
+  G.bricks_h = (p.H + kBrick - 1) / kBrick;
+  const int bd = (p.D + kBrick - 1) / kBrick;
+  const long long columns = (long long)p.N * p.C * G.bricks_w * G.bricks_h;
+  // bricks per CTA: as many as leave six CTAs per place (16 x 128^3: two 280 us, one and four 290, eight 330)
+  G.run = 1;
+  while (G.run < 4 && columns * ((bd + 2 * G.run - 1) / (2 * G.run)) >= 148 * 4 * 6) G.run *= 2;
+  G.runs = (bd + G.run - 1) / G.run;
+  BrickGrid T = G;  // a CTA per column where hardly any has work
+  T.run = bd;
+  T.runs = 1;
+  // each of the launches that follow may become resident while the one before ends
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.blockDim = dim3(256);
+  cfg.gridDim = dim3((unsigned)((long long)p.R * p.C * plan.parts + p.R));
+  cudaError_t e = cudaLaunchKernelEx(&cfg, bwd_brick3d_plan, p, plan, scratch, n);
+  cfg.numAttrs = 1;
+  cfg.gridDim = dim3((unsigned)(columns * G.runs));
+  cfg.dynamicSmemBytes = smem1;
+  if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, bwd_brick3d_half, p, pc, plan, G);
+  cfg.gridDim = dim3((unsigned)(columns + std::min(ctas, 148LL * 2)));
+  cfg.dynamicSmemBytes = smem2;
+  if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, bwd_brick3d_rest<PAIR>, p, pc, plan, T, (unsigned)columns, L, scratch, ctas);
+  cfg.gridDim = dim3(148 * 2);
+  cfg.dynamicSmemBytes = 0;
+  if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, bwd_fold_half<true>, p, plan, (const float*)scratch, n);
+  return e;
+}
+
+// Half backward through a float scratch volume of n = N*C*D*H*W elements that the caller of this function owns: clear it, scatter
+// into it, fold it into grad_in.  With memory for a plan (16-byte aligned, brick_plan_bytes; null: none) the rois that the
+// bricks take need none of that, and where they take all of them, which only the device knows, the scratch volume is not
+// touched.  Allocates nothing.
+inline int launch_bwd_stream3d_half(const Params& p, const S3Launch& L, long long ctas, float* scratch, void* plan_memory, cudaStream_t st) {
+  if (plan_memory) {
+    const BrickPlan plan = brick_plan(p, plan_memory);
+    const cudaError_t e = bwd_pair_form(p) ? launch_bwd_brick3d<true>(p, L, ctas, scratch, plan, st)
+                                           : launch_bwd_brick3d<false>(p, L, ctas, scratch, plan, st);
+    return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -8;
+  }
   const long long n = (long long)p.N * p.C * p.vol;
   cudaMemsetAsync(scratch, 0, (size_t)n * sizeof(float), st);
   launch_bwd_kernel<__half>(p, L, ctas, scratch, st);
-  const long long blocks = (n + 8 * 256 - 1) / (8 * 256);
-  bwd_fold_half<<<(unsigned)blocks, 256, 0, st>>>((__half*)p.out, scratch, n);
+  bwd_fold_half<false><<<(unsigned)((n + 8 * 256 - 1) / (8 * 256)), 256, 0, st>>>(p, BrickPlan(), scratch, n);
   return cudaGetLastError() == cudaSuccess ? 0 : -8;
 }
 
@@ -490,13 +593,15 @@ inline int try_launch_bwd_stream3d(const Params& p, int dtype, cudaStream_t st) 
     return cudaGetLastError() == cudaSuccess ? 0 : -8;
   }
   const long long n = (long long)p.N * p.C * p.vol;
+  const bool bricks = bwd_brick3d_applicable(p, dtype);
+  const size_t volume_bytes = ((size_t)n * sizeof(float) + 255) & ~(size_t)255;
   float* scratch = nullptr;
   cudaMemPool_t pool = bwd_pool_of_current_device(true);
-  if (!pool || cudaMallocFromPoolAsync((void**)&scratch, (size_t)n * sizeof(float), pool, st) != cudaSuccess) {
+  if (!pool || cudaMallocFromPoolAsync((void**)&scratch, volume_bytes + (bricks ? brick_plan_bytes(p) : 0), pool, st) != cudaSuccess) {
     cudaGetLastError();
     return MVR_STREAM3D_NOT_APPLICABLE;  // no memory for the scratch volume: element-type atomics instead
   }
-  const int rc = launch_bwd_stream3d_half(p, L, ctas, scratch, st);
+  const int rc = launch_bwd_stream3d_half(p, L, ctas, scratch, bricks ? (char*)scratch + volume_bytes : nullptr, st);
   cudaFreeAsync(scratch, st);
   return rc;
 }

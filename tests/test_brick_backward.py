@@ -1,0 +1,94 @@
+"""Half gradients of dense 3D calls, summed brick by brick of the gradient volume: bricks cut by the volume's ends, rois that
+overlap, magnify, or lie beyond the kernel's range, gradients that need one word per voxel, two, or flags.  Against the
+restatement with a wide accumulator.
+
+The contributions are the restatement's own, and their sum is exact or, in units of 2^-22 at the coarsest, off by half a unit per
+contribution (at most 64 of them here): one rounding to half on either side, 2^-11 of the value each, and 64 * 2^-23."""
+import pytest
+import torch
+
+import cases
+from oracle import port
+
+pytestmark = pytest.mark.gpu
+
+SHAPE = (4, 2, 56, 70, 75)  # 800 bricks, cut on every axis
+
+
+def make_rois(g, n, zoom, tilt=0.9):
+    ext = torch.tensor(SHAPE[:1:-1], dtype=torch.float32)
+    b = torch.arange(n).remainder(SHAPE[0]).float().view(-1, 1)
+    centre = ext / 2 + (torch.rand(n, 3, generator=g) - 0.5) * ext * 0.3
+    size = ext * zoom * (0.85 + 0.3 * torch.rand(n, 3, generator=g))
+    return torch.cat([b, centre, size, (torch.rand(n, 3, generator=g) - 0.5) * 2 * tilt], 1).half()
+
+
+CASES = {
+    # rois, zoom, out, order, gradient size, kind
+    "one word": dict(n=3, zoom=1.0, out=(48, 70, 66), size=1.0),
+    "coarser units": dict(n=3, zoom=1.0, out=(48, 70, 67), size=2.5),
+    "two words": dict(n=3, zoom=1.0, out=(48, 66, 71), size=3000.0),
+    "tiny": dict(n=3, zoom=1.0, out=(48, 66, 70), size=3e-5),
+    "turned anyhow": dict(n=3, zoom=1.0, out=(50, 61, 70), size=1.0, tilt=3.1),
+    "overlapping": dict(n=8, zoom=0.8, out=(40, 60, 64), size=1.0),
+    "large": dict(n=3, zoom=2.4, out=(24, 33, 40), size=1.0),
+    "magnified": dict(n=6, zoom=0.8, out=(44, 60, 70), size=1.0, mixed=True),  # a volume with a roi whose steps are below 0.4 voxels
+    "nearest": dict(n=3, zoom=1.0, out=(48, 70, 66), size=1.0, order=0),
+    "boxes": dict(n=3, zoom=0.9, out=(48, 70, 65), size=1.0, box=True),
+}
+
+
+@pytest.mark.parametrize("name", CASES)
+def test_gradient(name):
+    from medvision_b200 import _C
+    k = dict(dict(order=1, box=False, tilt=0.9, mixed=False), **CASES[name])
+    g = torch.Generator().manual_seed(len(name))
+    rois = make_rois(g, k["n"], k["zoom"], k["tilt"])
+    if k["mixed"]:
+        rois[0, 4:7] *= 0.4
+    if k["box"]:
+        rois = torch.cat([rois[:, :1], rois[:, 1:4] - rois[:, 4:7] / 2, rois[:, 1:4] + rois[:, 4:7] / 2], 1)
+    kind = cases.KIND_BOX if k["box"] else cases.KIND_ROTATED
+    out = k["out"]
+    grad = (torch.randn((k["n"], SHAPE[1]) + out, generator=g).clamp_(-4, 4) * k["size"]).half()
+    kw = dict(spatial_scale=1.0, sampling_ratio=1, aligned=not k["box"], order=k["order"], trig=None if k["box"] else port.device_trig(rois))
+    # unaligned gradient memory, a result that is added to
+    dev = torch.empty(grad.numel() + 1, dtype=torch.half, device="cuda")[1:].view(grad.shape).copy_(grad)
+    before = torch.randint(-2, 3, SHAPE, generator=g).half() * k["size"]
+    got = before.cuda()
+    if k["box"]:
+        _C.roi_align_3d_backward(dev, rois.cuda(), got, *out, 1.0, 1, k["order"])
+    else:
+        _C.roi_align_rotated_3d_backward(dev, rois.cuda(), got, *out, 1.0, 1, True, k["order"])
+    want = port.backward(grad, rois, SHAPE, kind, wide_acc=True, **kw).double()
+    err = (got.cpu().double() - before.double() - want).abs()
+    bound = 2.0 ** -11 * (2 * want.abs() + 2 * (want + before.double()).abs()) + 64 * 2.0 ** -23 * min(k["size"], 1.0) + 2.0 ** -24
+    assert not bool((err > bound).any()), float((err - bound).max())
+
+
+def test_infinities_nan_and_bad_batch_index():
+    from medvision_b200 import _C
+    g = torch.Generator().manual_seed(5)
+    rois = make_rois(g, 4, 1.0)
+    out = (48, 66, 70)
+    grad = torch.randn((4, SHAPE[1]) + out, generator=g).half()
+    for r, c, v in ((0, 0, float("inf")), (1, 1, float("-inf")), (2, 0, float("nan")), (2, 1, 60000.0)):
+        at = [torch.randint(0, s, (40,), generator=g) for s in out]
+        grad[r, c, at[0], at[1], at[2]] = v
+    grad[0, 0, 24, 30:33, 35] = torch.tensor([float("inf"), float("-inf"), float("inf")]).half()
+    kw = dict(spatial_scale=1.0, sampling_ratio=1, aligned=True, order=1)
+    want = port.backward(grad[:3], rois[:3], SHAPE, cases.KIND_ROTATED, wide_acc=True, trig=port.device_trig(rois[:3]), **kw)
+    rois[3, 0] = 7
+    _C.last_status()
+    got = torch.zeros(SHAPE, dtype=torch.half, device="cuda")
+    _C.roi_align_rotated_3d_backward(grad.cuda(), rois.cuda(), got, *out, 1.0, 1, True, 1)
+    assert _C.last_status() & 1
+    got = got.cpu()
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isposinf(), want.isposinf()) and torch.equal(got.isneginf(), want.isneginf())
+    fin = want.isfinite()
+    assert bool(((got - want)[fin].abs().double() <= 2.0 ** -10 * want[fin].abs().double() + 2.0 ** -18).all())
+    # the sum does not depend on any order
+    again = torch.zeros(SHAPE, dtype=torch.half, device="cuda")
+    _C.roi_align_rotated_3d_backward(grad.cuda(), rois.cuda(), again, *out, 1.0, 1, True, 1)
+    assert torch.equal(again.cpu().view(torch.int16), got.view(torch.int16))
+    _C.last_status()
