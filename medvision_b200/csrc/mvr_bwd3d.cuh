@@ -515,10 +515,10 @@ inline cudaError_t launch_bwd_brick3d(const Params& p, const S3Launch& L, long l
   cfg.gridDim = dim3((unsigned)(columns * G.runs));
   cfg.dynamicSmemBytes = smem1;
   if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, bwd_brick3d_half, p, pc, plan, G);
-  cfg.gridDim = dim3((unsigned)(columns + std::min(ctas, 148LL * 2)));
+  cfg.gridDim = dim3((unsigned)(columns + std::min(ctas, 148LL * 3 * 8)));
   cfg.dynamicSmemBytes = smem2;
   if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, bwd_brick3d_rest<PAIR>, p, pc, plan, T, (unsigned)columns, L, scratch, ctas);
-  cfg.gridDim = dim3(148 * 2);
+  cfg.gridDim = dim3(148 * 8);
   cfg.dynamicSmemBytes = 0;
   if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, bwd_fold_half<true>, p, plan, (const float*)scratch, n);
   return e;

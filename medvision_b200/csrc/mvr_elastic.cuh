@@ -11,8 +11,10 @@
 // float (3 fused multiply-adds).  Positions, taps, weights and sums of the warp itself are those of mvr_offset.cuh,
 // operation by operation.
 //
-// What bounds it: instruction issue.  On image and label of 2 x 128 x 256 x 256 (151 us) 235 instructions per voxel keep the issue
-// slots 78 % busy with 42 % of the warps resident; traffic is image and label read and written once (165 MB, 1.1 TB/s).
+// What bounds it: the loads (16 two-byte gathers per voxel pair keep the data pipe of L1 67 % busy) and instruction issue (67 %)
+// alike.  2 x 128 x 256 x 256: 134 us, where cells, indices and addresses formed per voxel and tap (235 instructions per voxel
+// of image and label) took 150; 2 x 96 x 160 x 160 66.5 -> 58.5; the first in float 183 -> 172.  Five CTAs per SM: 138; six
+// 147; three 167.
 #pragma once
 #include "mvr_label.cuh"
 #include "mvr_offset.cuh"
@@ -58,16 +60,25 @@ __device__ __forceinline__ void elastic_weights(float u, double* w) {
   w[3] = 0.5 * u3 - 0.5 * u2;
 }
 
+// What the voxels 2 * wp and 2 * wp + 1 of every row share: offsets inside their cells of the grid, the cells (16 bits each), the
+// indices as half2.
+struct __align__(16) ElasticX {
+  float ua, ub;
+  unsigned cells, w2;
+};
+
 // Displacement rows of one (sample, depth): tables in dynamic shared memory.
 template <int NDIM>
 struct ElasticTables {
   double* g;     // [NDIM][gh][gw]: the grid contracted along z
   float4* coef;  // this warp's [NDIM][gw] cubics along x
+  ElasticX* x;   // [(W + 1) / 2], where there is room
 
   __device__ __forceinline__ ElasticTables(const ElasticParams& p, unsigned char* smem) {
     g = reinterpret_cast<double*>(smem);
     const size_t n = ((size_t)NDIM * p.gw * p.gh * sizeof(double) + 15) & ~(size_t)15;
     coef = reinterpret_cast<float4*>(smem + n) + (threadIdx.x >> 5) * NDIM * p.gw;
+    x = reinterpret_cast<ElasticX*>(reinterpret_cast<float4*>(smem + n) + (kElasticThreads / 32) * NDIM * p.gw);
   }
   // all threads; the caller synchronises the CTA afterwards
   __device__ __forceinline__ void contract_z(const ElasticParams& p, int b, int d) {
@@ -111,11 +122,36 @@ struct ElasticTables {
     }
     __syncwarp();
   }
-  // displacement of voxels w0 and w0 + 1 of the row: da/db[c], c = channel of the field
-  __device__ __forceinline__ void eval_pair(const ElasticParams& p, int w0, float* da, float* db) const {
+  // all threads: what every row needs of a voxel pair
+  __device__ __forceinline__ void fill_x(const ElasticParams& p) {
+    for (int wp = threadIdx.x; wp < (p.W + 1) >> 1; wp += kElasticThreads) {
+      ElasticX e;
+      const int xa = elastic_cell(p.start[0], p.bin[0], p.centre[0], 2 * wp, p.gw, e.ua);
+      const int xb = elastic_cell(p.start[0], p.bin[0], p.centre[0], 2 * wp + 1, p.gw, e.ub);
+      e.cells = (unsigned)xa | (unsigned)xb << 16;
+      const __half2 w = __halves2half2(Ar<__half>::fi(2 * wp), Ar<__half>::fi(2 * wp + 1));
+      e.w2 = *reinterpret_cast<const unsigned*>(&w);
+      x[wp] = e;
+    }
+  }
+  // displacement of the voxels 2 * wp and 2 * wp + 1 of the row: da/db[c], c = channel of the field; x2: their indices
+  template <typename T, bool TABLE>
+  __device__ __forceinline__ void eval_pair(const ElasticParams& p, int wp, float* da, float* db, typename P2<T>::V& x2) const {
     float ua, ub;
-    const int xa = elastic_cell(p.start[0], p.bin[0], p.centre[0], w0, p.gw, ua);
-    const int xb = elastic_cell(p.start[0], p.bin[0], p.centre[0], w0 + 1, p.gw, ub);
+    int xa, xb;
+    if (TABLE) {
+      const ElasticX e = x[wp];
+      ua = e.ua;
+      ub = e.ub;
+      xa = (int)(e.cells & 0xffffu);
+      xb = (int)(e.cells >> 16);
+      if constexpr (sizeof(T) == 2) x2 = *reinterpret_cast<const __half2*>(&e.w2);
+    } else {
+      xa = elastic_cell(p.start[0], p.bin[0], p.centre[0], 2 * wp, p.gw, ua);
+      xb = elastic_cell(p.start[0], p.bin[0], p.centre[0], 2 * wp + 1, p.gw, ub);
+      if constexpr (sizeof(T) == 2) x2 = P2<T>::make(Ar<T>::fi(2 * wp), Ar<T>::fi(2 * wp + 1));
+    }
+    if constexpr (sizeof(T) == 4) x2 = P2<T>::make(Ar<T>::fi(2 * wp), Ar<T>::fi(2 * wp + 1));
 #pragma unroll
     for (int c = 0; c < NDIM; ++c) {
       const float4 ka = coef[c * p.gw + xa];
@@ -157,7 +193,8 @@ elastic_field_kernel(const ElasticParams p) {
     float* row = p.field + (long long)k.b * NDIM * vol + ((long long)k.d * p.H + h) * p.W;
     for (int wp = threadIdx.x & 31; wp < pairs; wp += 32) {
       float da[NDIM], db[NDIM];
-      tab.eval_pair(p, 2 * wp, da, db);
+      Float2Lanes index;
+      tab.template eval_pair<float, false>(p, wp, da, db, index);
 #pragma unroll
       for (int c = 0; c < NDIM; ++c) {
         float* o = row + c * vol + 2 * wp;
@@ -177,71 +214,126 @@ template <typename T, typename IT>
 __device__ __forceinline__ int elastic_label(const IT* p) {
   return Ar<T>::toi(Ar<T>::ff((float)__ldg(p)));
 }
+// The same for half without a wait between the load and its use: whole numbers up to 2048 are halves.
+template <typename IT>
+__device__ __forceinline__ int elastic_label_half(IT v) {
+  if constexpr (sizeof(IT) == 1) {
+    return (int)v;
+  } else {
+    if (v >= (IT)-2048 && v <= (IT)2048) return (int)v;
+    return Ar<__half>::toi(Ar<__half>::ff((float)v));
+  }
+}
 
-template <typename T, typename IT, int NDIM>
+// ROWS: half volumes whose sizes PairRows takes.  TABLE: what depends on w alone is tabulated, and
+// there is one channel each (no loop over them: 134 instead of 143 us on 2 x 128 x 256 x 256).
+template <typename T, typename IT, int NDIM, bool ROWS, bool TABLE>
 __global__ void __launch_bounds__(kElasticThreads, sizeof(T) == 2 ? 4 : 3)
 elastic_warp_kernel(const ElasticParams p) {
   typedef P2<T> Q;
   typedef typename Q::V V;
+  constexpr int NT = 1 << NDIM;
   extern __shared__ __align__(16) unsigned char elastic_smem_[];
   ElasticTables<NDIM> tab(p, elastic_smem_);
   const ElasticCta k = elastic_cta(p);
   tab.contract_z(p, k.b, k.d);
+  if (TABLE) tab.fill_x(p);
   __syncthreads();
   const int vol = p.D * p.H * p.W;  // < 2^31
   const int pairs = (p.W + 1) >> 1;
-  const T* img0 = p.img ? (const T*)p.img + (long long)k.b * p.C * vol : nullptr;
-  const IT* lab0 = p.lab ? (const IT*)p.lab + (long long)k.b * p.CL * vol : nullptr;
+  const T* const img0 = p.img ? (const T*)p.img + (long long)k.b * p.C * vol : nullptr;
+  const IT* const lab0 = p.lab ? (const IT*)p.lab + (long long)k.b * p.CL * vol : nullptr;
+  T* const out0 = p.img ? (T*)p.out + (long long)k.b * p.C * vol : nullptr;
+  int* const lab_out0 = p.lab ? p.lab_out + (long long)k.b * p.CL * vol : nullptr;
+  const V z2 = Q::dup(Ar<T>::fi(k.d));
   for (int h = k.h0 + (threadIdx.x >> 5); h < k.h1; h += kElasticThreads / 32) {
     tab.contract_y(p, h);
     const int row = (k.d * p.H + h) * p.W;
+    const V y2 = Q::dup(Ar<T>::fi(h));
+    T* const out_row = out0 + row;
+    int* const lab_row = lab_out0 + row;
     for (int wp = threadIdx.x & 31; wp < pairs; wp += 32) {
       const int w0 = 2 * wp;
       const bool has_b = w0 + 1 < p.W;
       float da[NDIM], db[NDIM];
-      tab.eval_pair(p, w0, da, db);
-      V o2[3], c[3];
-#pragma unroll
-      for (int a = 0; a < NDIM; ++a)  // axis w, h, d <- channel d, h, w; rounded to the image's type
-        o2[a] = Q::make(Ar<T>::ff(da[NDIM - 1 - a]), Ar<T>::ff(db[NDIM - 1 - a]));
-      warp_positions<T, NDIM>(w0, h, k.d, o2, c);
-      AxisTap2<T> t[3];
-      warp_taps<T, NDIM>(c, p.pair, 1, t);
+      V x2;
+      tab.template eval_pair<T, TABLE>(p, wp, da, db, x2);
+      V c[3];
+      // axis w, h, d <- channel d, h, w; rounded to the image's type
+      c[0] = Q::add(x2, Q::make(Ar<T>::ff(da[NDIM - 1]), Ar<T>::ff(db[NDIM - 1])));
+      c[1] = Q::add(y2, Q::make(Ar<T>::ff(da[NDIM - 2]), Ar<T>::ff(db[NDIM - 2])));
+      c[2] = NDIM == 3 ? Q::add(z2, Q::make(Ar<T>::ff(da[0]), Ar<T>::ff(db[0]))) : c[1];
+      typename std::conditional<ROWS, HalfTap2, AxisTap2<T>>::type t[3];
+      if constexpr (ROWS) {
+        half_tap2<0>(c[0], p.pair, 1, t[0]);
+        half_tap2<1>(c[1], p.pair, 1, t[1]);
+        if (NDIM == 3) half_tap2<2>(c[2], p.pair, 1, t[2]);
+        else t[2] = t[1];  // not read
+      } else {
+        warp_taps<T, NDIM>(c, p.pair, 1, t);
+      }
       const typename Q::M mask = warp_inside<T, NDIM>(c, p.pair, has_b);
-      const PairTaps<T, NDIM> taps(t[0], t[1], t[2], p.pair);
-      if (img0) {
-        V w[1 << NDIM];
+      if (p.img) {
+        V w[NT];
         pair_weights<T, NDIM>(t[0], t[1], t[2], w);
-        const T* img = img0;
-        T* out = (T*)p.out + (long long)k.b * p.C * vol + row + w0;
+        auto channels = [&](auto load) {
+          const T* img = img0;
+          T* out = out_row + w0;
 #pragma unroll 1
-        for (int ch = 0; ch < p.C; ++ch, img += vol, out += vol) {
-          V v[1 << NDIM];
-          taps.load(img, v);
-          const V val = Q::apply(pair_sum<T, (1 << NDIM)>(w, v), mask);
-          if (p.vec_img) {
-            Q::store2(out, val);
-          } else {
-            out[0] = Q::lo(val);
-            if (has_b) out[1] = Q::hi(val);
+          for (int ch = 0; ch < (TABLE ? 1 : p.C); ++ch, img += vol, out += vol) {
+            V v[NT];
+            load(img, v);
+            const V val = Q::apply(pair_sum<T, NT>(w, v), mask);
+            if (p.vec_img) {
+              Q::store2(out, val);
+            } else {
+              out[0] = Q::lo(val);
+              if (has_b) out[1] = Q::hi(val);
+            }
           }
+        };
+        if constexpr (ROWS) {
+          const PairRows<NDIM> rows(t, p.pair);
+          channels([&](const T* img, V* v) { rows.load(img, t, p.pair, v); });
+        } else {
+          const PairTaps<T, NDIM> taps(t[0], t[1], t[2], p.pair);
+          channels([&](const T* img, V* v) { taps.load(img, v); });
         }
       }
-      if (lab0) {
+      if (p.lab) {
         // nearest: the lower tap of an axis where its weight is at least one half, else the upper one
-        unsigned oa = taps.a, ob = taps.b;
+        unsigned ua[3], ub[3];
 #pragma unroll
         for (int a = 0; a < NDIM; ++a) {
-          if (!Ar<T>::ge_half(Q::lo(t[a].h))) oa += t[a].da;
-          if (!Ar<T>::ge_half(Q::hi(t[a].h))) ob += t[a].db;
+          if constexpr (ROWS) {
+            const unsigned m = __hlt2_mask(t[a].h, __float2half2_rn(0.5f)) | t[a].at_end;
+            ua[a] = m & 1u;
+            ub[a] = m >> 31;
+          } else {  // (never beyond the last voxel: there the lower tap has weight one)
+            ua[a] = Ar<T>::tof(Q::lo(t[a].h)) < 0.5f ? 1u : 0u;
+            ub[a] = Ar<T>::tof(Q::hi(t[a].h)) < 0.5f ? 1u : 0u;
+          }
         }
-        const unsigned ia = oa / (unsigned)sizeof(T), ib = ob / (unsigned)sizeof(T);
+        const unsigned W = (unsigned)p.W, HW = W * (unsigned)p.H, bias = kTapMagic * (NDIM == 3 ? 1u + W + HW : 1u + W);
+        unsigned ia = (t[0].ra + ua[0]) + (t[1].ra + ua[1]) * W - bias, ib = (t[0].rb + ub[0]) + (t[1].rb + ub[1]) * W - bias;
+        if (NDIM == 3) {
+          ia += (t[2].ra + ua[2]) * HW;
+          ib += (t[2].rb + ub[2]) * HW;
+        }
         const bool ina = Q::lane_a(mask), inb = Q::lane_b(mask);
         const IT* lab = lab0;
-        int* out = p.lab_out + (long long)k.b * p.CL * vol + row + w0;
+        int* out = lab_row + w0;
 #pragma unroll 1
-        for (int ch = 0; ch < p.CL; ++ch, lab += vol, out += vol) {
-          const int va = ina ? elastic_label<T, IT>(lab + ia) : 0, vb = inb ? elastic_label<T, IT>(lab + ib) : 0;
+        for (int ch = 0; ch < (TABLE ? 1 : p.CL); ++ch, lab += vol, out += vol) {
+          int va, vb;
+          if constexpr (ROWS && TABLE) {
+            const IT la = __ldg(lab + ia), lb = __ldg(lab + ib);  // (valid addresses for lanes outside, too)
+            va = ina ? elastic_label_half(la) : 0;
+            vb = inb ? elastic_label_half(lb) : 0;
+          } else {
+            va = ina ? elastic_label<T, IT>(lab + ia) : 0;
+            vb = inb ? elastic_label<T, IT>(lab + ib) : 0;
+          }
           if (p.vec_lab) {
             *reinterpret_cast<int2*>(out) = make_int2(va, vb);
           } else {
@@ -259,25 +351,36 @@ inline int launch_elastic(ElasticParams p, int ndim, int dtype, int label_dtype,
   if (!pair_taps_applicable(p.D, p.H, p.W, (long long)p.D * p.H * p.W, dtype == 0 ? 4 : 2) || elastic_smem(ndim, p.gw, p.gh) > (size_t)kElasticMaxSmem) return 1;
   if (p.B == 0) return 0;
   p.pair = make_pair_const(ndim, p.D, p.H, p.W, dtype == 0 ? 4 : 2);
-  // 64 rows spread a CTA's set-up over eight rounds of its warps; fewer where that would leave less than six CTAs per SM.  Longer
-  // columns end in an uneven last wave: 128 rows 183 against 159 us on 2 x 128 x 256 x 256 and 110 against 70 on 2 x 96 x 160 x 160
-  // (16 rows: 157 and 65).
-  p.rows = 64;
+  // 32 rows spread a CTA's set-up over four rounds of its warps; fewer where that would leave less than six CTAs per SM.  Longer
+  // columns end in an uneven last wave (2 x 128 x 256 x 256: 64 rows 3 us more), shorter ones pay for the set-up.
+  p.rows = 32;
   while (p.rows > 8 && (long long)p.B * p.D * ((p.H + p.rows - 1) / p.rows) < 148 * 6) p.rows >>= 1;
   p.blocks_h = (p.H + p.rows - 1) / p.rows;
   const long long ctas = (long long)p.B * p.D * p.blocks_h;
   if (ctas > 0x7fffffffLL) return 1;
   const unsigned grid = (unsigned)ctas;
-  const size_t smem = elastic_smem(ndim, p.gw, p.gh);
+  size_t smem = elastic_smem(ndim, p.gw, p.gh);
+  const size_t table = (size_t)((p.W + 1) / 2) * sizeof(ElasticX);
+  // four rows per warp pay for the table along w
+  const bool x_table = !p.field && p.C <= 1 && p.CL <= 1 && p.rows >= 32 && smem + table <= (size_t)kElasticMaxSmem && p.gw <= 0xffff;
+  if (x_table) smem += table;
   if (p.field) {
     if (ndim == 2) elastic_field_kernel<2><<<grid, kElasticThreads, smem, st>>>(p);
     else elastic_field_kernel<3><<<grid, kElasticThreads, smem, st>>>(p);
     return cudaGetLastError() == cudaSuccess ? 0 : -8;
   }
-#define MVR_ELASTIC(T, IT)                                                                    \
-  {                                                                                           \
-    if (ndim == 2) elastic_warp_kernel<T, IT, 2><<<grid, kElasticThreads, smem, st>>>(p);     \
-    else elastic_warp_kernel<T, IT, 3><<<grid, kElasticThreads, smem, st>>>(p);               \
+  const bool rows = dtype == 1 && pair_rows_applicable(ndim, p.D, p.H, p.W);
+#define MVR_ELASTIC_FORM(T, IT, NDIM)                                                                                    \
+  {                                                                                                                      \
+    if (rows && x_table) elastic_warp_kernel<T, IT, NDIM, sizeof(T) == 2, true><<<grid, kElasticThreads, smem, st>>>(p); \
+    else if (rows) elastic_warp_kernel<T, IT, NDIM, sizeof(T) == 2, false><<<grid, kElasticThreads, smem, st>>>(p);      \
+    else if (x_table) elastic_warp_kernel<T, IT, NDIM, false, true><<<grid, kElasticThreads, smem, st>>>(p);             \
+    else elastic_warp_kernel<T, IT, NDIM, false, false><<<grid, kElasticThreads, smem, st>>>(p);                         \
+  }
+#define MVR_ELASTIC(T, IT)                        \
+  {                                               \
+    if (ndim == 2) MVR_ELASTIC_FORM(T, IT, 2)     \
+    else MVR_ELASTIC_FORM(T, IT, 3)               \
   }
 #define MVR_ELASTIC_T(T)                                       \
   switch (label_dtype) {                                       \
@@ -289,6 +392,7 @@ inline int launch_elastic(ElasticParams p, int ndim, int dtype, int label_dtype,
   if (dtype == 0) MVR_ELASTIC_T(float) else MVR_ELASTIC_T(__half)
 #undef MVR_ELASTIC_T
 #undef MVR_ELASTIC
+#undef MVR_ELASTIC_FORM
   return cudaGetLastError() == cudaSuccess ? 0 : -8;
 }
 

@@ -174,6 +174,7 @@ struct PairConst {
   unsigned last_raw[3];   // kTapMagic + size - 1
   float size[3];
   unsigned size_floor2[3], size_ceil2[3];  // half2 of the largest half <= size and of the smallest half >= size
+  unsigned last2[3];                       // half2 of size - 1 (sizes up to 2049)
   unsigned sx, sy, sz, bias;  // strides in bytes (WIDE: elements), and -kTapMagic * (sx + sy + sz) modulo 2^32
 };
 // unit: size of an element, 1 for the WIDE form
@@ -187,6 +188,8 @@ inline PairConst make_pair_const(int ndim, int D, int H, int W, size_t unit) {
     const unsigned lo = __half_as_ushort(__float2half_rd(k.size[a])), hi = __half_as_ushort(__float2half_ru(k.size[a]));
     k.size_floor2[a] = lo | (lo << 16);
     k.size_ceil2[a] = hi | (hi << 16);
+    const unsigned last = __half_as_ushort(__float2half_rn(k.last[a]));
+    k.last2[a] = last | (last << 16);
   }
   k.sx = (unsigned)unit;
   k.sy = (unsigned)((size_t)W * unit);
@@ -275,9 +278,68 @@ struct PairTaps {
   }
 };
 
+// The same for half pairs in volumes of 2 to 2049 voxels per axis (indices are halves): coordinates clamped and offsets inside
+// the cell formed for both lanes at once; the taps at fixed distances from one address per lane, whose index is one lower
+// where a coordinate sits on the last voxel, the lower tap's value then being taken from the upper one's -- one
+// selection per pair of values instead of the addresses of sixteen loads.
+inline bool pair_rows_applicable(int ndim, int D, int H, int W) {
+  return W >= 2 && H >= 2 && W <= 2049 && H <= 2049 && (ndim == 2 || (D >= 2 && D <= 2049));
+}
+struct HalfTap2 {
+  unsigned ra, rb;  // kTapMagic + lower tap index, at most that of the last voxel but one
+  unsigned at_end;  // lanes whose coordinate is at or beyond the last voxel
+  __half2 l, h;
+};
+template <int AXIS>
+__device__ __forceinline__ void half_tap2(__half2 c, const PairConst& k, int order, HalfTap2& t) {
+  typedef P2<__half> Q;
+  const float magic = 8388608.0f;
+  const __half2 last = *reinterpret_cast<const __half2*>(&k.last2[AXIS]);
+  t.at_end = __hge2_mask(c, last);
+  c = __hmin2_nan(__hmax2_nan(c, __float2half2_rn(0.0f)), last);
+  const float ma = __fadd_rz(Q::lo_float(c), magic), mb = __fadd_rz(Q::hi_float(c), magic);
+  t.ra = min(__float_as_uint(ma), k.last_raw[AXIS] - 1u);  // (a NaN: there)
+  t.rb = min(__float_as_uint(mb), k.last_raw[AXIS] - 1u);
+  t.l = Q::sub(c, Q::from_floats(__fsub_rn(ma, magic), __fsub_rn(mb, magic)));  // exact
+  t.h = Q::sub(Q::dup(__float2half_rn(1.0f)), t.l);
+  if (order == 0) Q::nearest(t.l, t.h);
+}
+template <int NDIM>
+struct PairRows {
+  typedef __half2 V;
+  unsigned a, b;  // offsets of the lowest taps
+  __device__ __forceinline__ PairRows(const HalfTap2* t, const PairConst& k) {
+    a = t[0].ra * 2u + (t[1].ra * k.sy + k.bias);
+    b = t[0].rb * 2u + (t[1].rb * k.sy + k.bias);
+    if (NDIM == 3) {
+      a += t[2].ra * k.sz;
+      b += t[2].rb * k.sz;
+    }
+  }
+  __device__ __forceinline__ void load(const __half* vol, const HalfTap2* t, const PairConst& k, V* v) const {
+    typedef P2<__half> Q;
+    const char* pa = reinterpret_cast<const char*>(vol) + a;
+    const char* pb = reinterpret_cast<const char*>(vol) + b;
+#pragma unroll
+    for (int r = 0; r < (1 << (NDIM - 1)); ++r) {
+      const char *ra = pa, *rb = pb;
+      if (r & 1) { ra += k.sy; rb += k.sy; }
+      if (r & 2) { ra += k.sz; rb += k.sz; }
+      const __half *ha = reinterpret_cast<const __half*>(ra), *hb = reinterpret_cast<const __half*>(rb);
+      v[2 * r] = Q::make(__ldg(ha), __ldg(hb));
+      v[2 * r + 1] = Q::make(__ldg(ha + 1), __ldg(hb + 1));
+    }
+#pragma unroll
+    for (int i = 0; i < NDIM; ++i)
+#pragma unroll
+      for (int q = 0; q < (1 << NDIM); ++q)
+        if (!((q >> i) & 1)) v[q] = Q::blend(v[q], v[q | (1 << i)], t[i].at_end);
+  }
+};
+
 // the products of the axis weights, in tap order
-template <typename T, int NDIM>
-__device__ __forceinline__ void pair_weights(const AxisTap2<T>& tx, const AxisTap2<T>& ty, const AxisTap2<T>& tz, typename P2<T>::V* w) {
+template <typename T, int NDIM, typename TAP>
+__device__ __forceinline__ void pair_weights(const TAP& tx, const TAP& ty, const TAP& tz, typename P2<T>::V* w) {
   typedef P2<T> Q;
   typedef typename Q::V V;
   if (NDIM == 3) {
