@@ -295,7 +295,6 @@ static Plane2dLabel plane2d_label_of(const Params& p) {
   lab.rois = (const float*)p.rois;
   lab.out = (int*)p.out;
   lab.C = p.C;
-  lab.vec = (p.ow & 1) == 0 && (uintptr_t)p.out % 8 == 0;
   return lab;
 }
 

@@ -361,8 +361,8 @@ inline int launch_elastic(ElasticParams p, int ndim, int dtype, int label_dtype,
   const unsigned grid = (unsigned)ctas;
   size_t smem = elastic_smem(ndim, p.gw, p.gh);
   const size_t table = (size_t)((p.W + 1) / 2) * sizeof(ElasticX);
-  // four rows per warp pay for the table along w
-  const bool x_table = !p.field && p.C <= 1 && p.CL <= 1 && p.rows >= 32 && smem + table <= (size_t)kElasticMaxSmem && p.gw <= 0xffff;
+  // (the table along w pays for itself from one row per warp on: 4 x 1024 x 300, eight rows per CTA, 17.5 -> 14.6 us)
+  const bool x_table = !p.field && p.C <= 1 && p.CL <= 1 && smem + table <= (size_t)kElasticMaxSmem && p.gw <= 0xffff;
   if (x_table) smem += table;
   if (p.field) {
     if (ndim == 2) elastic_field_kernel<2><<<grid, kElasticThreads, smem, st>>>(p);

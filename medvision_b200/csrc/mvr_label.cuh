@@ -10,7 +10,7 @@
 // axis and is the only element read.  The value goes through float, as in the reference:
 // (int32)(float)label.
 //
-// Layout of the work as in the gather path of the forward: a thread owns two w-adjacent voxels
+// Layout of the work as in the gather path of the forward: a thread owns two voxels (S3Place)
 // of a 32 x 16 tile and walks a depth chunk; for rois that turn about z at most the in-plane tap
 // is fixed along the walk and the plane comes from the per-depth table.
 #pragma once
@@ -85,38 +85,36 @@ __device__ __forceinline__ void label_item_stream3d(const Params& p, const S3Lau
     }
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int pw0 = k.tw * kS3TileW + (warp & 1) * 16 + (lane & 7) * 2;
-  const int ph = k.th * kS3TileH + (warp >> 1) * 4 + (lane >> 3);
-  if (ph >= p.oh || pw0 >= p.ow) return;
-  const bool has_b = (pw0 + 1 < p.ow);
+  const S3Place place(p, k.tw, k.th);
+  if (!place.inside) return;
+  const bool has_b = place.has_b;
   const long long plane_o = (long long)p.oh * p.ow;
-  int* out = (int*)p.out + k.nc * p.ovol + (long long)k.pd0 * plane_o + (long long)ph * p.ow + pw0;
-  const bool vec = L.vec_store && has_b;
+  const int second = kS3SecondRow * p.ow;
+  int* out = (int*)p.out + k.nc * p.ovol + (long long)k.pd0 * plane_o + (long long)place.ph * p.ow + place.pw;
 
   if (g.batch < 0 || g.batch >= p.N) {
     if (p.status && threadIdx.x == 0 && k.tw == 0 && k.th == 0 && k.ck == 0) atomicOr(p.status, STATUS_BAD_BATCH_INDEX);
     for (int i = 0; i < npd; ++i) {
       out[i * plane_o] = 0;
-      if (has_b) out[i * plane_o + 1] = 0;
+      if (has_b) out[i * plane_o + second] = 0;
     }
     return;
   }
   const IT* vol = (const IT*)p.in + ((long long)g.batch * p.C + k.c) * p.vol;
-  const float sub_x = lattice_sub<float>(g.bin[0], 0, 1), sub_y = lattice_sub<float>(g.bin[1], 0, 1);
-  const float x[2] = {A::add(lattice_base<float>(g.start[0], pw0, g.bin[0], fm), sub_x),
-                      A::add(lattice_base<float>(g.start[0], has_b ? pw0 + 1 : pw0, g.bin[0], fm), sub_x)};
-  const float y = A::add(lattice_base<float>(g.start[1], ph, g.bin[1], fm), sub_y);
+  const float sub_y = __fmul_rn(0.5f, g.bin[1]);
+  const float x = A::add(lattice_base<float>(g.start[0], place.pw, g.bin[0], fm), __fmul_rn(0.5f, g.bin[0]));
+  const float y[2] = {A::add(lattice_base<float>(g.start[1], place.ph, g.bin[1], fm), sub_y),
+                      A::add(lattice_base<float>(g.start[1], has_b ? place.ph + kS3SecondRow : place.ph, g.bin[1], fm), sub_y)};
 
   if (zsep) {
     const IT* at[2];  // the picked tap in plane 0
     bool in[2] = {true, has_b};
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
-      float rx = x[s], ry = y;
+      float rx = x, ry = y[s];
       if (rotated) {
-        rx = A::add(__fmaf_rn(g.rot[0], x[s], A::mul(g.rot[1], y)), g.centre[0]);
-        ry = A::add(__fmaf_rn(g.rot[3], x[s], A::mul(g.rot[4], y)), g.centre[1]);
+        rx = A::add(__fmaf_rn(g.rot[0], x, A::mul(g.rot[1], y[s])), g.centre[0]);
+        ry = A::add(__fmaf_rn(g.rot[3], x, A::mul(g.rot[4], y[s])), g.centre[1]);
       }
       const unsigned ix = label_pick(rx, sx, lx, in[s]), iy = label_pick(ry, sy, ly, in[s]);
       at[s] = vol + (iy * (unsigned)p.W + ix - kTapMagic * ((unsigned)p.W + 1u));
@@ -128,12 +126,8 @@ __device__ __forceinline__ void label_item_stream3d(const Params& p, const S3Lau
       int va = 0, vb = 0;
       if (pl >= 0 && in[0]) va = label_value<IT>(at[0] + pl);
       if (pl >= 0 && in[1]) vb = label_value<IT>(at[1] + pl);
-      if (vec) {
-        *reinterpret_cast<int2*>(out) = make_int2(va, vb);
-      } else {
-        out[0] = va;
-        if (has_b) out[1] = vb;
-      }
+      out[0] = va;
+      if (has_b) out[second] = vb;
     }
     return;
   }
@@ -143,7 +137,7 @@ __device__ __forceinline__ void label_item_stream3d(const Params& p, const S3Lau
 #pragma unroll
   for (int s = 0; s < 2; ++s)
 #pragma unroll
-    for (int r = 0; r < 3; ++r) sxy[s][r] = __fmaf_rn(g.rot[3 * r], x[s], A::mul(g.rot[3 * r + 1], y));
+    for (int r = 0; r < 3; ++r) sxy[s][r] = __fmaf_rn(g.rot[3 * r], x, A::mul(g.rot[3 * r + 1], y[s]));
   const unsigned bias = kTapMagic * ((unsigned)HW + (unsigned)p.W + 1u);
 #pragma unroll 4
   for (int i = 0; i < npd; ++i, out += plane_o) {
@@ -157,12 +151,8 @@ __device__ __forceinline__ void label_item_stream3d(const Params& p, const S3Lau
       const unsigned iz = label_pick(A::add(A::add(sxy[s][2], e.p[2]), g.centre[2]), sz, lz, in);
       if (in) val[s] = label_value<IT>(vol + (iz * (unsigned)HW + (iy * (unsigned)p.W + ix) - bias));
     }
-    if (vec) {
-      *reinterpret_cast<int2*>(out) = make_int2(val[0], val[1]);
-    } else {
-      out[0] = val[0];
-      if (has_b) out[1] = val[1];
-    }
+    out[0] = val[0];
+    if (has_b) out[second] = val[1];
   }
 }
 
@@ -274,7 +264,7 @@ inline bool label_stream3d_geometry(const Params& p, S3Launch& L, long long& ite
   const long long per_depth = (long long)p.R * p.C * L.tiles_w * L.tiles_h;
   L.chunk = s3_pick_chunk(per_depth, p.od, 148 * 4, 12);
   L.chunks = (p.od + L.chunk - 1) / L.chunk;
-  L.vec_store = ((p.ow & 1) == 0) && (((uintptr_t)p.out) % 8 == 0);
+  L.vec_store = 0;
   L.filter = 0;
   items = per_depth * L.chunks;
   return items <= 0x7fffffffLL;

@@ -1,8 +1,7 @@
 // Dense 2D forward (one sample per output pixel: every 2D augmentation call): the 2D counterpart
-// of the 3D gather path, for an image field, an integer label field, or both at once.  A thread owns two w-adjacent pixels
+// of the 3D gather path, for an image field, an integer label field, or both at once.  A thread owns two pixels
 // (the two lanes of half2 arithmetic), walks down a column of row blocks of its tile and applies
-// the taps and weights of a pixel pair to every channel; the roi is decoded once per CTA; stores
-// are 2-element vectors, consecutive along w within a warp row.  The arithmetic is the
+// the taps and weights of the pair to every channel; the roi is decoded once per CTA.  The arithmetic is the
 // reference's (medvision/csrc/cuda/roi_align_rotated_2d_cuda_kernel.cuh:15-90,
 // roi_align_2d_cuda_kernel.cuh:11-74, interpolation_helpers_2d.h), one rounded operation at a
 // time: only the x products of the rotation, which do not change down a column, are hoisted.
@@ -10,7 +9,7 @@
 // Labels: affine_2d(labels.float(), rois, ..., order 0).int() on the integers, as mvr_label.cuh does it; the geometry is
 // float32 and is the image's own for a float image.
 //
-// Bound by the latency of position -> loads -> sum (issue slots half busy): two channels' loads are in flight per thread.
+// Bound by the loads: L1's data pipe 70 % busy, latency of position -> loads -> sum beneath it (issue slots 52 %).
 #pragma once
 #include "mvr_label.cuh"
 
@@ -21,15 +20,19 @@ struct Plane2dLabel {
   const void* in;      // (N, C, H, W) of IT
   const float* rois;
   int* out;            // (R, C, oh, ow)
-  int C, vec;
+  int C;
 };
 
 template <typename T, int ORDER, typename IT, bool IMG, bool LAB, bool WIDE>
 __global__ void __launch_bounds__(kS3Threads, 5)
-resample_fwd_plane2d(const Params p, const PairConst pc, const Plane2dLabel lab, int tiles_w, int tiles_h, int blocks, int vec_store) {
+resample_fwd_plane2d(const Params p, const PairConst pc, const Plane2dLabel lab, int tiles_w, int tiles_h, int blocks) {
   typedef Ar<T> A;
   typedef P2<T> Q;
   typedef typename Q::V V;
+  // A warp's lanes lie on consecutive pixels, 16 x 2, and a thread's second pixel two rows below its first: a load then touches half
+  // the lines it does with the two pixels side by side.  16 x (3,512,512) float 60 -> 55 us, half 63 -> 53 (8 x 4: 59, 59;
+  // 32 x 1: 55, 53; 4 x 8: 80, 82).
+  constexpr int kLanesW = 16, kLanesH = 32 / kLanesW;
   constexpr bool kOwnLabelGeometry = LAB && (!IMG || sizeof(T) != 4);
   __shared__ RoiGeom<T> g_sh;
   __shared__ RoiGeom<float> gl_sh;
@@ -46,11 +49,10 @@ resample_fwd_plane2d(const Params p, const PairConst pc, const Plane2dLabel lab,
   const RoiGeom<T>& g = g_sh;
   const int batch = IMG ? g_sh.batch : gl_sh.batch;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int pw0 = tw * kS3TileW + (warp & 1) * 16 + (lane & 7) * 2;
-  const int row0 = th * (kS3TileH * blocks) + (warp >> 1) * 4 + (lane >> 3);
+  constexpr int kAcross = kS3TileW / kLanesW;
+  const int pw0 = tw * kS3TileW + (warp % kAcross) * kLanesW + lane % kLanesW;
+  const int row0 = th * (kS3TileH * blocks) + (warp / kAcross) * (2 * kLanesH) + lane / kLanesW;
   if (pw0 >= p.ow || row0 >= p.oh) return;
-  const bool has_b = (pw0 + 1 < p.ow);
-  const bool vec = vec_store && has_b, vec_l = LAB && lab.vec && has_b;
   const long long ovol = p.ovol, vol_e = p.vol;
   T* out = IMG ? (T*)p.out + n * p.C * ovol + pw0 : nullptr;
   int* out_l = LAB ? lab.out + n * lab.C * ovol + pw0 : nullptr;
@@ -60,17 +62,11 @@ resample_fwd_plane2d(const Params p, const PairConst pc, const Plane2dLabel lab,
   if (batch < 0 || batch >= p.N) {
     if (p.status && threadIdx.x == 0 && tw == 0 && th == 0) atomicOr(p.status, STATUS_BAD_BATCH_INDEX);
     for (int b = 0; b < blocks; ++b) {
-      const int ph = row0 + b * kS3TileH;
-      if (ph >= p.oh) break;
-      for (int c = 0; IMG && c < p.C; ++c) {
-        T* o = out + c * ovol + (long long)ph * p.ow;
-        o[0] = zero;
-        if (has_b) o[1] = zero;
-      }
-      for (int c = 0; LAB && c < lab.C; ++c) {
-        int* o = out_l + c * ovol + (long long)ph * p.ow;
-        o[0] = 0;
-        if (has_b) o[1] = 0;
+      for (int s = 0; s < 2; ++s) {
+        const int ph = row0 + b * kS3TileH + s * kLanesH;
+        if (ph >= p.oh) break;
+        for (int c = 0; IMG && c < p.C; ++c) out[c * ovol + (long long)ph * p.ow] = zero;
+        for (int c = 0; LAB && c < lab.C; ++c) out_l[c * ovol + (long long)ph * p.ow] = 0;
       }
     }
     return;
@@ -79,47 +75,42 @@ resample_fwd_plane2d(const Params p, const PairConst pc, const Plane2dLabel lab,
   const IT* vol_l = LAB ? (const IT*)lab.in + (long long)batch * lab.C * vol_e : nullptr;
   const bool rotated = (p.kind == KIND_ROTATED);
   V x2 = zero2;
-  if (IMG) {
-    const T sub_x = lattice_sub<T>(g.bin[0], 0, 1);
-    x2 = Q::make(A::add(lattice_base<T>(g.start[0], pw0, g.bin[0], fm), sub_x),
-                 A::add(lattice_base<T>(g.start[0], has_b ? pw0 + 1 : pw0, g.bin[0], fm), sub_x));
-  }
-  Float2Lanes xl = {0.0f, 0.0f};
-  if (kOwnLabelGeometry) {
-    const float sub = lattice_sub<float>(gl_sh.bin[0], 0, 1);
-    xl.a = __fadd_rn(lattice_base<float>(gl_sh.start[0], pw0, gl_sh.bin[0], fm), sub);
-    xl.b = __fadd_rn(lattice_base<float>(gl_sh.start[0], has_b ? pw0 + 1 : pw0, gl_sh.bin[0], fm), sub);
-  }
-  const typename Q::M lanes = Q::make_mask(true, has_b);
+  if (IMG) x2 = Q::dup(A::add(lattice_base<T>(g.start[0], pw0, g.bin[0], fm), A::mul(A::ff(0.5f), g.bin[0])));
+  float xl = 0.0f;
+  if (kOwnLabelGeometry) xl = __fadd_rn(lattice_base<float>(gl_sh.start[0], pw0, gl_sh.bin[0], fm), __fmul_rn(0.5f, gl_sh.bin[0]));
   const unsigned row_l = (unsigned)p.W, bias_l = kTapMagic * ((unsigned)p.W + 1u);
   const int C = p.C, oh = p.oh;
   const long long row_step = (long long)kS3TileH * p.ow;
+  const int second = kLanesH * p.ow;  // from a thread's first pixel to its second
   long long row_o = (long long)row0 * p.ow;
 
 #pragma unroll 1
   for (int b = 0, ph = row0; b < blocks && ph < oh; ++b, ph += kS3TileH, row_o += row_step) {
+    const bool has_b = ph + kLanesH < oh;
     V rx2 = zero2, ry2 = zero2;
     if (IMG) {
-      const T y = A::add(lattice_base<T>(g.start[1], ph, g.bin[1], fm), lattice_sub<T>(g.bin[1], 0, 1));
+      const T half_bin = A::mul(A::ff(0.5f), g.bin[1]);
+      const V y2 = Q::make(A::add(lattice_base<T>(g.start[1], ph, g.bin[1], fm), half_bin),
+                           A::add(lattice_base<T>(g.start[1], ph + kLanesH, g.bin[1], fm), half_bin));
       if (rotated) {
         // rx = (x*cos - y*sin) + cx ; ry = (x*sin + y*cos) + cy
-        rx2 = Q::add(Q::row_xy(Q::dup(g.rot[0]), x2, Q::dup(A::neg(A::mul(y, g.rot[1])))), Q::dup(g.centre[0]));
-        ry2 = Q::add(Q::row_xy(Q::dup(g.rot[1]), x2, Q::dup(A::mul(y, g.rot[0]))), Q::dup(g.centre[1]));
+        const V c2 = Q::dup(g.rot[0]), s2 = Q::dup(g.rot[1]);
+        rx2 = Q::add(Q::row_xy(c2, x2, Q::neg(Q::mul(y2, s2))), Q::dup(g.centre[0]));
+        ry2 = Q::add(Q::row_xy(s2, x2, Q::mul(y2, c2)), Q::dup(g.centre[1]));
       } else {
         rx2 = x2;
-        ry2 = Q::dup(y);
+        ry2 = y2;
       }
     }
     if (LAB) {
       float rx[2], ry[2];
       if (kOwnLabelGeometry) {
-        const float y = __fadd_rn(lattice_base<float>(gl_sh.start[1], ph, gl_sh.bin[1], fm), lattice_sub<float>(gl_sh.bin[1], 0, 1));
-        const float c = gl_sh.rot[0], s = gl_sh.rot[1], ys = -__fmul_rn(y, s), yc = __fmul_rn(y, c);
+        const float c = gl_sh.rot[0], s = gl_sh.rot[1];
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-          const float x = k ? xl.b : xl.a;
-          rx[k] = rotated ? __fadd_rn(__fmaf_rn(c, x, ys), gl_sh.centre[0]) : x;
-          ry[k] = rotated ? __fadd_rn(__fmaf_rn(s, x, yc), gl_sh.centre[1]) : y;
+          const float y = __fadd_rn(lattice_base<float>(gl_sh.start[1], ph + k * kLanesH, gl_sh.bin[1], fm), __fmul_rn(0.5f, gl_sh.bin[1]));
+          rx[k] = rotated ? __fadd_rn(__fmaf_rn(c, xl, -__fmul_rn(y, s)), gl_sh.centre[0]) : xl;
+          ry[k] = rotated ? __fadd_rn(__fmaf_rn(s, xl, __fmul_rn(y, c)), gl_sh.centre[1]) : y;
         }
       } else {
         rx[0] = A::tof(Q::lo(rx2)); rx[1] = A::tof(Q::hi(rx2));
@@ -134,19 +125,15 @@ resample_fwd_plane2d(const Params p, const PairConst pc, const Plane2dLabel lab,
       int* o = out_l + row_o;
       for (int c = 0; c < lab.C; ++c, v += vol_e, o += ovol) {
         const int va = in[0] ? label_value<IT>(v + at[0]) : 0, vb = in[1] ? label_value<IT>(v + at[1]) : 0;
-        if (vec_l) {
-          *reinterpret_cast<int2*>(o) = make_int2(va, vb);
-        } else {
-          o[0] = va;
-          if (has_b) o[1] = vb;
-        }
+        o[0] = va;
+        if (has_b) o[second] = vb;
       }
     }
     if (!IMG) continue;
     AxisTap2<T> tx, ty;
     axis_tap2<T, 0>(rx2, pc, ORDER, tx);
     axis_tap2<T, 1>(ry2, pc, ORDER, ty);
-    const typename Q::M mask = lanes & ~(Q::outside(rx2, pc, 0) | Q::outside(ry2, pc, 1));
+    const typename Q::M mask = Q::make_mask(true, has_b) & ~(Q::outside(rx2, pc, 0) | Q::outside(ry2, pc, 1));
     const PairTaps<T, 2, WIDE> taps(tx, ty, ty, pc);
     V w[4];
     pair_weights<T, 2>(tx, ty, ty, w);
@@ -161,12 +148,8 @@ resample_fwd_plane2d(const Params p, const PairConst pc, const Plane2dLabel lab,
         // output_val = 0 + val (normalises -0), then / count with count == 1
         val = Q::apply(Q::add(zero2, pair_sum<T, 4>(w, v)), mask);
       }
-      if (vec) {
-        Q::store2(o, val);
-      } else {
-        o[0] = Q::lo(val);
-        if (has_b) o[1] = Q::hi(val);
-      }
+      o[0] = Q::lo(val);
+      if (has_b) o[second] = Q::hi(val);
     }
   }
 }
@@ -183,17 +166,22 @@ inline int try_launch_plane2d(const Params& p, int dtype, cudaStream_t st, const
   if (wide && label) return 1;  // the fields get a launch each
   const int tiles_w = (p.ow + kS3TileW - 1) / kS3TileW, row_blocks = (p.oh + kS3TileH - 1) / kS3TileH;
   // a CTA's set-up costs about two row blocks; five CTAs per SM
-  const int blocks = s3_pick_chunk((long long)p.R * tiles_w, std::min(row_blocks, 4096), 148 * 5, 2);
+  int blocks = s3_pick_chunk((long long)p.R * tiles_w, std::min(row_blocks, 4096), 148 * 5, 2);
+  // Large calls: at least two waves, since tiles that lie outside the image end early (16 x (3,512,512): one wave 69 us, two 60;
+  // 3 x (3,900,900) 41 -> 38).  Below six row blocks per place shorter columns cost more than they level out (4 x (3,512,512)
+  // 21 -> 23).
+  const long long per_row = (long long)p.R * tiles_w;
+  if (per_row * row_blocks >= 148 * 5 * 6)
+    while (blocks > 2 && per_row * ((row_blocks + blocks - 1) / blocks) < 148 * 5 * 2) blocks = (blocks + 1) / 2;
   const int tiles_h = (row_blocks + blocks - 1) / blocks;
   const long long ctas = (long long)p.R * tiles_w * tiles_h;
   if (ctas > 0x7fffffffLL) return 1;
-  const int vec_store = ((p.ow & 1) == 0) && (((uintptr_t)p.out) % (2 * esz) == 0);
   const unsigned grid = (unsigned)ctas;
   const PairConst pc = make_pair_const(2, 1, p.H, p.W, wide ? 1 : esz);
   Plane2dLabel lab = {};
   if (label) lab = *label;
 #define MVR_PLANE(T, ORDER, IT, IMG, LAB, WIDE) \
-  resample_fwd_plane2d<T, ORDER, IT, IMG, LAB, WIDE><<<grid, kS3Threads, 0, st>>>(p, pc, lab, tiles_w, tiles_h, blocks, vec_store)
+  resample_fwd_plane2d<T, ORDER, IT, IMG, LAB, WIDE><<<grid, kS3Threads, 0, st>>>(p, pc, lab, tiles_w, tiles_h, blocks)
 #define MVR_PLANE_IT(T, ORDER, IMG)                                        \
   switch (label_dtype) {                                                   \
     case LABEL_U8: MVR_PLANE(T, ORDER, unsigned char, IMG, true, false); break;   \

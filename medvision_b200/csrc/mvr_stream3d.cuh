@@ -7,8 +7,7 @@
 //
 // Layout of the work
 //   * CTA = 256 threads = a 32 (w) x 16 (h) tile of output positions x a chunk of output depth
-//     of ONE (roi, channel).  A thread owns two w-adjacent voxels and walks the depth chunk,
-//     so output stores are 2-element vectors, contiguous along w within a warp row.
+//     of ONE (roi, channel).  A thread owns two voxels of the tile (S3Place) and walks the depth chunk.
 //   * The roi is decoded (incl. its six sin/cos) once per CTA; per-depth quantities are
 //     tabulated once per CTA in shared memory.
 //   * Every arithmetic step keeps the reference's rounding sequence (mvr_arith.cuh); what is
@@ -88,6 +87,7 @@ template <> struct P2<__half> {
   }
   __device__ __forceinline__ static V from_floats(float a, float b) { return __floats2half2_rn(a, b); }
   __device__ __forceinline__ static V sub(V a, V b) { return __hsub2_rn(a, b); }
+  __device__ __forceinline__ static V neg(V a) { return __hneg2(a); }
   // one-hot choice of an axis: prefer the lower index when h >= .5
   __device__ __forceinline__ static void nearest(V& l, V& h) {
     const __half2 half_ = __float2half2_rn(0.5f), one = __float2half2_rn(1.0f);
@@ -136,6 +136,7 @@ template <> struct P2<float> {
   }
   __device__ __forceinline__ static V from_floats(float a, float b) { return make(a, b); }
   __device__ __forceinline__ static V sub(V a, V b) { return make(__fsub_rn(a.a, b.a), __fsub_rn(a.b, b.b)); }
+  __device__ __forceinline__ static V neg(V a) { return make(-a.a, -a.b); }
   __device__ __forceinline__ static void nearest(V& l, V& h) {
     const bool ha = h.a >= 0.5f, hb = h.b >= 0.5f, la = l.a >= 0.5f, lb = l.b >= 0.5f;
     h = make(ha ? 1.0f : 0.0f, hb ? 1.0f : 0.0f);
@@ -390,70 +391,64 @@ struct S3Launch {
   unsigned wait_tries = 1u << 20;       // tries of a bounded wait on a ring slot's barrier (each may be suspended by the hardware)
 };
 
-// General-rotation depth loop for NP voxel pairs of one thread (pair q sits q*row_step output
-// rows below pair 0): positions change with depth, so all three axis taps are formed per voxel;
-// the x- and y-products of the rotation are formed once per thread, the z-products once per
-// depth and CTA (S3ZProd table).  Both lanes of a pair go through the same instructions.
-template <typename T, int NP, bool WIDE>
+// A thread's two voxels in the gather path.  A warp's lanes lie on consecutive voxels, 16 (w) x 2 (h), and the second voxel two rows
+// below the first: a load then touches fewer lines than with the two side by side and the lanes on every other voxel.  Forward of
+// 16 x 128^3 half under three axes 241 -> 203 us, float 232 -> 200; 2 x (79,165,181) 46 -> 35 (8 x 4 voxels: 249, 220, 39; 32 x 1:
+// 207, 208, 35).
+constexpr int kS3LanesW = 16, kS3SecondRow = 32 / kS3LanesW;
+struct S3Place {
+  int pw, ph;      // the first voxel
+  bool inside, has_b;
+  __device__ __forceinline__ S3Place(const Params& p, int tw, int th) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int kAcross = kS3TileW / kS3LanesW;
+    pw = tw * kS3TileW + (warp % kAcross) * kS3LanesW + lane % kS3LanesW;
+    ph = th * kS3TileH + (warp / kAcross) * (2 * kS3SecondRow) + lane / kS3LanesW;
+    inside = ph < p.oh && pw < p.ow;
+    has_b = ph + kS3SecondRow < p.oh;
+  }
+};
+
+// General-rotation depth loop: positions change with depth, so all three axis taps are formed per voxel; the x- and
+// y-products of the rotation are formed once per thread, the z-products once per depth and CTA (S3ZProd table).  Both
+// lanes of a pair go through the same instructions.
+template <typename T, bool WIDE>
 __device__ __forceinline__ void s3_full_depth_loop(const Params& p, const S3Launch& L, const S3Shared<T>& sh, int npd, int c,
-                                                   int pw0, int ph0, int row_step, bool vec_store, T* out0) {
+                                                   typename P2<T>::V x2, typename P2<T>::V y2, bool has_b, T* out0) {
   typedef Ar<T> A;
   typedef P2<T> Q;
   typedef typename Q::V V;
   const RoiGeom<T>& g = sh.g;
-  const int fm = kS3FloatPattern;
-  const bool has_b = (pw0 + 1 < p.ow);
   const T* vol = (const T*)p.in + ((long long)g.batch * p.C + c) * p.vol;
   const V zero2 = Q::dup(A::fi(0));
-  const T sub_x = lattice_sub<T>(g.bin[0], 0, 1), sub_y = lattice_sub<T>(g.bin[1], 0, 1);
-  const T xa = A::add(lattice_base<T>(g.start[0], pw0, g.bin[0], fm), sub_x);
-  const T xb = A::add(lattice_base<T>(g.start[0], has_b ? pw0 + 1 : pw0, g.bin[0], fm), sub_x);
-  const V x2 = Q::make(xa, xb);
-  V sxy[NP][3];
-  bool act[NP];
+  V sxy[3];
 #pragma unroll
-  for (int q = 0; q < NP; ++q) {
-    const int ph = ph0 + q * row_step;
-    act[q] = ph < p.oh;
-    const T y = A::add(lattice_base<T>(g.start[1], act[q] ? ph : 0, g.bin[1], fm), sub_y);
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-      sxy[q][r] = Q::row_xy(Q::dup(g.rot[3 * r]), x2, Q::dup(A::mul(g.rot[3 * r + 1], y)));
-  }
+  for (int r = 0; r < 3; ++r) sxy[r] = Q::row_xy(Q::dup(g.rot[3 * r]), x2, Q::mul(Q::dup(g.rot[3 * r + 1]), y2));
   const V c2[3] = {Q::dup(g.centre[0]), Q::dup(g.centre[1]), Q::dup(g.centre[2])};
   const PairConst& pc = L.pair;
   const typename Q::M lanes = Q::make_mask(true, has_b);
   const long long plane_o = (long long)p.oh * p.ow;
-  const long long sub_o = (long long)row_step * p.ow;
+  const int second = kS3SecondRow * p.ow;
   T* o = out0;
   for (int i = 0; i < npd; ++i, o += plane_o) {
     const S3ZProd<T> e = sh.zp[i];
-#pragma unroll
-    for (int q = 0; q < NP; ++q) {
-      if (!act[q]) continue;
-      const V rx2 = Q::add(Q::add(sxy[q][0], Q::dup(e.p[0])), c2[0]);
-      const V ry2 = Q::add(Q::add(sxy[q][1], Q::dup(e.p[1])), c2[1]);
-      const V rz2 = Q::add(Q::add(sxy[q][2], Q::dup(e.p[2])), c2[2]);
-      AxisTap2<T> tx, ty, tz;
-      axis_tap2<T, 0>(rx2, pc, p.order, tx);
-      axis_tap2<T, 1>(ry2, pc, p.order, ty);
-      axis_tap2<T, 2>(rz2, pc, p.order, tz);
-      const typename Q::M mask = lanes & ~(Q::outside(rx2, pc, 0) | Q::outside(ry2, pc, 1) | Q::outside(rz2, pc, 2));
-      V val = zero2;
-      if (mask) {  // a lane outside keeps valid (clamped) addresses; its value is dropped
-        V v[8], w[8];
-        PairTaps<T, 3, WIDE>(tx, ty, tz, pc).load(vol, v);
-        pair_weights<T, 3>(tx, ty, tz, w);
-        val = Q::apply(Q::add(zero2, pair_sum<T, 8>(w, v)), mask);
-      }
-      T* oq = o + q * sub_o;
-      if (vec_store && has_b) {
-        Q::store2(oq, val);
-      } else {
-        oq[0] = Q::lo(val);
-        if (has_b) oq[1] = Q::hi(val);
-      }
+    const V rx2 = Q::add(Q::add(sxy[0], Q::dup(e.p[0])), c2[0]);
+    const V ry2 = Q::add(Q::add(sxy[1], Q::dup(e.p[1])), c2[1]);
+    const V rz2 = Q::add(Q::add(sxy[2], Q::dup(e.p[2])), c2[2]);
+    AxisTap2<T> tx, ty, tz;
+    axis_tap2<T, 0>(rx2, pc, p.order, tx);
+    axis_tap2<T, 1>(ry2, pc, p.order, ty);
+    axis_tap2<T, 2>(rz2, pc, p.order, tz);
+    const typename Q::M mask = lanes & ~(Q::outside(rx2, pc, 0) | Q::outside(ry2, pc, 1) | Q::outside(rz2, pc, 2));
+    V val = zero2;
+    if (mask) {  // a lane outside keeps valid (clamped) addresses; its value is dropped
+      V v[8], w[8];
+      PairTaps<T, 3, WIDE>(tx, ty, tz, pc).load(vol, v);
+      pair_weights<T, 3>(tx, ty, tz, w);
+      val = Q::apply(Q::add(zero2, pair_sum<T, 8>(w, v)), mask);
     }
+    o[0] = Q::lo(val);
+    if (has_b) o[second] = Q::hi(val);
   }
 }
 
@@ -576,20 +571,18 @@ __device__ void s3_body_l1(const Params& p, const S3Launch& L, const S3Cta& k, S
   const bool rotated = (p.kind == KIND_ROTATED);
   const bool bad_batch = (g.batch < 0 || g.batch >= p.N);
   // ---- this thread's two output columns
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int pw0 = tw * kS3TileW + (warp & 1) * 16 + (lane & 7) * 2;
-  const int ph = th * kS3TileH + (warp >> 1) * 4 + (lane >> 3);
-  if (ph >= p.oh || pw0 >= p.ow) return;
-  const bool has_b = (pw0 + 1 < p.ow);
+  const S3Place at(p, tw, th);
+  if (!at.inside) return;
+  const bool has_b = at.has_b;
   const long long plane_o = (long long)p.oh * p.ow;
-  T* out = (T*)p.out + nc * p.ovol + (long long)pd0 * plane_o + (long long)ph * p.ow + pw0;
-  const bool vec = L.vec_store && has_b;
+  const int second = kS3SecondRow * p.ow;  // from the first voxel to the second
+  T* out = (T*)p.out + nc * p.ovol + (long long)pd0 * plane_o + (long long)at.ph * p.ow + at.pw;
 
   if (bad_batch) {
     if (p.status && threadIdx.x == 0 && tw == 0 && th == 0 && ck == 0) atomicOr(p.status, STATUS_BAD_BATCH_INDEX);
     for (int i = 0; i < npd; ++i) {
       out[i * plane_o] = A::fi(0);
-      if (has_b) out[i * plane_o + 1] = A::fi(0);
+      if (has_b) out[i * plane_o + second] = A::fi(0);
     }
     return;
   }
@@ -597,21 +590,20 @@ __device__ void s3_body_l1(const Params& p, const S3Launch& L, const S3Cta& k, S
   const V zero2 = Q::dup(A::fi(0));
 
   // lattice coordinates of the two voxels in the roi frame
-  const T sub_x = lattice_sub<T>(g.bin[0], 0, 1), sub_y = lattice_sub<T>(g.bin[1], 0, 1);
-  const T xa = A::add(lattice_base<T>(g.start[0], pw0, g.bin[0], fm), sub_x);
-  const T xb = A::add(lattice_base<T>(g.start[0], has_b ? pw0 + 1 : pw0, g.bin[0], fm), sub_x);
-  const T y = A::add(lattice_base<T>(g.start[1], ph, g.bin[1], fm), sub_y);
-  const V x2 = Q::make(xa, xb);
+  const T sub_y = A::mul(A::ff(0.5f), g.bin[1]);
+  const V x2 = Q::dup(A::add(lattice_base<T>(g.start[0], at.pw, g.bin[0], fm), A::mul(A::ff(0.5f), g.bin[0])));
+  const V y2 = Q::make(A::add(lattice_base<T>(g.start[1], at.ph, g.bin[1], fm), sub_y),
+                       A::add(lattice_base<T>(g.start[1], has_b ? at.ph + kS3SecondRow : at.ph, g.bin[1], fm), sub_y));
 
   if (zsep) {
     // ---- in-plane position, taps and weights: once per thread
     V rx2, ry2;
     if (rotated) {
-      rx2 = Q::add(Q::row_xy(Q::dup(g.rot[0]), x2, Q::dup(A::mul(g.rot[1], y))), Q::dup(g.centre[0]));
-      ry2 = Q::add(Q::row_xy(Q::dup(g.rot[3]), x2, Q::dup(A::mul(g.rot[4], y))), Q::dup(g.centre[1]));
+      rx2 = Q::add(Q::row_xy(Q::dup(g.rot[0]), x2, Q::mul(Q::dup(g.rot[1]), y2)), Q::dup(g.centre[0]));
+      ry2 = Q::add(Q::row_xy(Q::dup(g.rot[3]), x2, Q::mul(Q::dup(g.rot[4]), y2)), Q::dup(g.centre[1]));
     } else {
       rx2 = x2;
-      ry2 = Q::dup(y);
+      ry2 = y2;
     }
     AxisTap2<T> tx, ty;
     axis_tap2<T, 0>(rx2, L.pair, p.order, tx);
@@ -680,18 +672,14 @@ __device__ void s3_body_l1(const Params& p, const S3Launch& L, const S3Cta& k, S
       } else {
         prefetch(next);
       }
-      if (vec) {
-        Q::store2(o, val);
-      } else {
-        o[0] = Q::lo(val);
-        if (has_b) o[1] = Q::hi(val);
-      }
+      o[0] = Q::lo(val);
+      if (has_b) o[second] = Q::hi(val);
     }
     return;
   }
 
   // ---- general rotation: positions change with depth
-  s3_full_depth_loop<T, 1, WIDE>(p, L, sh, npd, c, pw0, ph, kS3TileH, L.vec_store != 0, out);
+  s3_full_depth_loop<T, WIDE>(p, L, sh, npd, c, x2, y2, has_b, out);
 }
 
 // The plane walk of the rows that no tensor map can describe (row pitch not a multiple of 16 bytes), and every roi of calls

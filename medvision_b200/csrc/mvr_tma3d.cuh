@@ -654,7 +654,7 @@ inline int try_launch_stream3d(const Params& p, int dtype, cudaStream_t st, T3La
     G.chunk = min(chunk, p.od);
   }
   G.chunks = (p.od + G.chunk - 1) / G.chunk;
-  G.vec_store = ((p.ow & 1) == 0) && (((uintptr_t)p.out) % (2 * esz) == 0);
+  G.vec_store = 0;
   G.filter = 0;
   G.pair = make_pair_const(3, p.D, p.H, p.W, wide ? 1 : esz);
   const long long g_ctas = g_per_depth * G.chunks;
@@ -678,7 +678,7 @@ inline int try_launch_stream3d(const Params& p, int dtype, cudaStream_t st, T3La
     L.chunk = (L.chunk + parts - 1) / parts;
   }
   L.chunks = (p.od + L.chunk - 1) / L.chunk;
-  L.vec_store = G.vec_store;
+  L.vec_store = ((p.ow & 1) == 0) && (((uintptr_t)p.out) % (2 * esz) == 0);
   L.pair = G.pair;
   const long long ctas = per_depth_ctas * L.chunks;
   if (ctas > 0x7fffffffLL) return MVR_STREAM3D_NOT_APPLICABLE;
