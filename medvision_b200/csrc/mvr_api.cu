@@ -443,8 +443,6 @@ int mvr_elastic(const float* coarse, int ndim, int gd, int gh, int gw, int borde
   p.field = field;
   p.B = (int)B; p.D = (int)D; p.H = (int)H; p.W = (int)W;
   const bool even = (W & 1) == 0;
-  p.vec_img = even && (uintptr_t)image_out % (dtype == MVR_F32 ? 8 : 4) == 0;
-  p.vec_lab = even && (uintptr_t)label_out % 8 == 0;
   p.vec_field = even && (uintptr_t)field % 8 == 0;
   const int rc = launch_elastic(p, ndim, dtype, label_dtype, (cudaStream_t)stream);
   return rc == 0 ? MVR_OK : (rc == 1 ? MVR_ERR_UNSUPPORTED : MVR_ERR_LAUNCH);

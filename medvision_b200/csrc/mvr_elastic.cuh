@@ -11,10 +11,10 @@
 // float (3 fused multiply-adds).  Positions, taps, weights and sums of the warp itself are those of mvr_offset.cuh,
 // operation by operation.
 //
-// What bounds it: the loads (16 two-byte gathers per voxel pair keep the data pipe of L1 67 % busy) and instruction issue (67 %)
-// alike.  2 x 128 x 256 x 256: 134 us, where cells, indices and addresses formed per voxel and tap (235 instructions per voxel
-// of image and label) took 150; 2 x 96 x 160 x 160 66.5 -> 58.5; the first in float 183 -> 172.  Five CTAs per SM: 138; six
-// 147; three 167.
+// What bounds it: instruction issue (66 %) and the loads (L1's data pipe 53-65 % busy).  2 x 128 x 256 x 256: 131 us, where cells,
+// indices and addresses formed per voxel and tap (235 instructions per voxel of image and label) took 150, and lanes on every
+// other voxel 133; 4 x 64 x 100 x 100 46 -> 42; 2 x 96 x 160 x 160 66 -> 59; the first in float 183 -> 153.  Five CTAs per SM 138;
+// six 147; three 167.
 #pragma once
 #include "mvr_label.cuh"
 #include "mvr_offset.cuh"
@@ -34,7 +34,7 @@ struct ElasticParams {
   int B, C, CL, D, H, W;
   PairConst pair;
   int rows, blocks_h;                  // rows per CTA, row blocks per plane
-  int vec_img, vec_lab, vec_field;     // two-element vector stores are aligned
+  int vec_field;                       // two-element vector stores are aligned
 };
 
 constexpr int kElasticThreads = 256;
@@ -60,19 +60,20 @@ __device__ __forceinline__ void elastic_weights(float u, double* w) {
   w[3] = 0.5 * u3 - 0.5 * u2;
 }
 
-// What the voxels 2 * wp and 2 * wp + 1 of every row share: offsets inside their cells of the grid, the cells (16 bits each), the
-// indices as half2.
-struct __align__(16) ElasticX {
-  float ua, ub;
-  unsigned cells, w2;
+// What the voxels at one w of every row share: the offset inside their cell of the grid, the cell, the index as a half.
+struct __align__(8) ElasticX {
+  float u;
+  unsigned short cell, w;
 };
+// A warp takes 64 voxels of a row at a time: a lane's two lie 32 apart, so that its lanes load from consecutive voxels.
+constexpr int kElasticStep = 64;
 
 // Displacement rows of one (sample, depth): tables in dynamic shared memory.
 template <int NDIM>
 struct ElasticTables {
   double* g;     // [NDIM][gh][gw]: the grid contracted along z
   float4* coef;  // this warp's [NDIM][gw] cubics along x
-  ElasticX* x;   // [(W + 1) / 2], where there is room
+  ElasticX* x;   // [W, rounded up to kElasticStep], where there is room
 
   __device__ __forceinline__ ElasticTables(const ElasticParams& p, unsigned char* smem) {
     g = reinterpret_cast<double*>(smem);
@@ -122,36 +123,34 @@ struct ElasticTables {
     }
     __syncwarp();
   }
-  // all threads: what every row needs of a voxel pair
+  // all threads
   __device__ __forceinline__ void fill_x(const ElasticParams& p) {
-    for (int wp = threadIdx.x; wp < (p.W + 1) >> 1; wp += kElasticThreads) {
+    const int n = (p.W + kElasticStep - 1) & ~(kElasticStep - 1);
+    for (int w = threadIdx.x; w < n; w += kElasticThreads) {
       ElasticX e;
-      const int xa = elastic_cell(p.start[0], p.bin[0], p.centre[0], 2 * wp, p.gw, e.ua);
-      const int xb = elastic_cell(p.start[0], p.bin[0], p.centre[0], 2 * wp + 1, p.gw, e.ub);
-      e.cells = (unsigned)xa | (unsigned)xb << 16;
-      const __half2 w = __halves2half2(Ar<__half>::fi(2 * wp), Ar<__half>::fi(2 * wp + 1));
-      e.w2 = *reinterpret_cast<const unsigned*>(&w);
-      x[wp] = e;
+      e.cell = (unsigned short)elastic_cell(p.start[0], p.bin[0], p.centre[0], w, p.gw, e.u);
+      e.w = __half_as_ushort(Ar<__half>::fi(w));
+      x[w] = e;
     }
   }
-  // displacement of the voxels 2 * wp and 2 * wp + 1 of the row: da/db[c], c = channel of the field; x2: their indices
+  // displacement of the voxels wa and wb of the row: da/db[c], c = channel of the field; x2: their indices
   template <typename T, bool TABLE>
-  __device__ __forceinline__ void eval_pair(const ElasticParams& p, int wp, float* da, float* db, typename P2<T>::V& x2) const {
+  __device__ __forceinline__ void eval_pair(const ElasticParams& p, int wa, int wb, float* da, float* db, typename P2<T>::V& x2) const {
     float ua, ub;
     int xa, xb;
     if (TABLE) {
-      const ElasticX e = x[wp];
-      ua = e.ua;
-      ub = e.ub;
-      xa = (int)(e.cells & 0xffffu);
-      xb = (int)(e.cells >> 16);
-      if constexpr (sizeof(T) == 2) x2 = *reinterpret_cast<const __half2*>(&e.w2);
+      const ElasticX ea = x[wa], eb = x[wb];
+      ua = ea.u;
+      ub = eb.u;
+      xa = ea.cell;
+      xb = eb.cell;
+      if constexpr (sizeof(T) == 2) x2 = __halves2half2(__ushort_as_half(ea.w), __ushort_as_half(eb.w));
     } else {
-      xa = elastic_cell(p.start[0], p.bin[0], p.centre[0], 2 * wp, p.gw, ua);
-      xb = elastic_cell(p.start[0], p.bin[0], p.centre[0], 2 * wp + 1, p.gw, ub);
-      if constexpr (sizeof(T) == 2) x2 = P2<T>::make(Ar<T>::fi(2 * wp), Ar<T>::fi(2 * wp + 1));
+      xa = elastic_cell(p.start[0], p.bin[0], p.centre[0], wa, p.gw, ua);
+      xb = elastic_cell(p.start[0], p.bin[0], p.centre[0], wb, p.gw, ub);
+      if constexpr (sizeof(T) == 2) x2 = P2<T>::make(Ar<T>::fi(wa), Ar<T>::fi(wb));
     }
-    if constexpr (sizeof(T) == 4) x2 = P2<T>::make(Ar<T>::fi(2 * wp), Ar<T>::fi(2 * wp + 1));
+    if constexpr (sizeof(T) == 4) x2 = P2<T>::make(Ar<T>::fi(wa), Ar<T>::fi(wb));
 #pragma unroll
     for (int c = 0; c < NDIM; ++c) {
       const float4 ka = coef[c * p.gw + xa];
@@ -194,7 +193,7 @@ elastic_field_kernel(const ElasticParams p) {
     for (int wp = threadIdx.x & 31; wp < pairs; wp += 32) {
       float da[NDIM], db[NDIM];
       Float2Lanes index;
-      tab.template eval_pair<float, false>(p, wp, da, db, index);
+      tab.template eval_pair<float, false>(p, 2 * wp, 2 * wp + 1, da, db, index);
 #pragma unroll
       for (int c = 0; c < NDIM; ++c) {
         float* o = row + c * vol + 2 * wp;
@@ -240,7 +239,6 @@ elastic_warp_kernel(const ElasticParams p) {
   if (TABLE) tab.fill_x(p);
   __syncthreads();
   const int vol = p.D * p.H * p.W;  // < 2^31
-  const int pairs = (p.W + 1) >> 1;
   const T* const img0 = p.img ? (const T*)p.img + (long long)k.b * p.C * vol : nullptr;
   const IT* const lab0 = p.lab ? (const IT*)p.lab + (long long)k.b * p.CL * vol : nullptr;
   T* const out0 = p.img ? (T*)p.out + (long long)k.b * p.C * vol : nullptr;
@@ -252,12 +250,11 @@ elastic_warp_kernel(const ElasticParams p) {
     const V y2 = Q::dup(Ar<T>::fi(h));
     T* const out_row = out0 + row;
     int* const lab_row = lab_out0 + row;
-    for (int wp = threadIdx.x & 31; wp < pairs; wp += 32) {
-      const int w0 = 2 * wp;
-      const bool has_b = w0 + 1 < p.W;
+    for (int w0 = threadIdx.x & 31; w0 < p.W; w0 += kElasticStep) {
+      const bool has_b = w0 + 32 < p.W;
       float da[NDIM], db[NDIM];
       V x2;
-      tab.template eval_pair<T, TABLE>(p, wp, da, db, x2);
+      tab.template eval_pair<T, TABLE>(p, w0, w0 + 32, da, db, x2);
       V c[3];
       // axis w, h, d <- channel d, h, w; rounded to the image's type
       c[0] = Q::add(x2, Q::make(Ar<T>::ff(da[NDIM - 1]), Ar<T>::ff(db[NDIM - 1])));
@@ -284,12 +281,8 @@ elastic_warp_kernel(const ElasticParams p) {
             V v[NT];
             load(img, v);
             const V val = Q::apply(pair_sum<T, NT>(w, v), mask);
-            if (p.vec_img) {
-              Q::store2(out, val);
-            } else {
-              out[0] = Q::lo(val);
-              if (has_b) out[1] = Q::hi(val);
-            }
+            out[0] = Q::lo(val);
+            if (has_b) out[32] = Q::hi(val);
           }
         };
         if constexpr (ROWS) {
@@ -334,12 +327,8 @@ elastic_warp_kernel(const ElasticParams p) {
             va = ina ? elastic_label<T, IT>(lab + ia) : 0;
             vb = inb ? elastic_label<T, IT>(lab + ib) : 0;
           }
-          if (p.vec_lab) {
-            *reinterpret_cast<int2*>(out) = make_int2(va, vb);
-          } else {
-            out[0] = va;
-            if (has_b) out[1] = vb;
-          }
+          out[0] = va;
+          if (has_b) out[32] = vb;
         }
       }
     }
@@ -360,7 +349,7 @@ inline int launch_elastic(ElasticParams p, int ndim, int dtype, int label_dtype,
   if (ctas > 0x7fffffffLL) return 1;
   const unsigned grid = (unsigned)ctas;
   size_t smem = elastic_smem(ndim, p.gw, p.gh);
-  const size_t table = (size_t)((p.W + 1) / 2) * sizeof(ElasticX);
+  const size_t table = (((size_t)p.W + kElasticStep - 1) & ~(size_t)(kElasticStep - 1)) * sizeof(ElasticX);
   // (the table along w pays for itself from one row per warp on: 4 x 1024 x 300, eight rows per CTA, 17.5 -> 14.6 us)
   const bool x_table = !p.field && p.C <= 1 && p.CL <= 1 && smem + table <= (size_t)kElasticMaxSmem && p.gw <= 0xffff;
   if (x_table) smem += table;
