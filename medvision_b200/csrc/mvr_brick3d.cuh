@@ -670,6 +670,7 @@ __global__ void __launch_bounds__(256) bwd_brick3d_plan(const Params p, const Br
   __half2 top = __float2half2_rn(0.0f);
   unsigned most = 0u;
   if (((uintptr_t)(g + first) & 15u) == 0) {
+#pragma unroll 4
     for (long long i = first + threadIdx.x * 8; i + 8 <= last; i += 256 * 8) {
       const uint4 v = __ldg(reinterpret_cast<const uint4*>(g + i));
       const unsigned u[4] = {v.x, v.y, v.z, v.w};
