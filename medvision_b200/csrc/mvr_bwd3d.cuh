@@ -12,6 +12,9 @@
 // half running sum loses the small contributions that up-sampling produces by the dozen per
 // voxel.  The result differs from any one run of the reference by less than two runs of the
 // reference differ from each other.
+//
+// Large half calls with few rois per volume are summed by bricks of the gradient instead (mvr_brick3d.cuh); this kernel then takes
+// what those leave.
 #pragma once
 #include <mutex>
 
