@@ -12,12 +12,12 @@
 // an integer.  (Float additions in shared memory are a compare-and-swap loop: 75 clocks of an SM per warp and eight taps,
 // integers 16.5, loads and stores that no two lanes may share 47.)
 //   one word per voxel   in units of 2^-24 where the largest gradient and a bound of the samples' weights at one voxel show that
-//                        the sum cannot leave 32 bits (gradients up to 3-5 without magnification): the sum is exact.  Units of
-//                        2^-23 and 2^-22 for gradients up to four times that: what is lost per contribution is below 2^-26 of
-//                        the largest gradient, and at most two units of the last place of a subnormal half.
-//   two words            above, and for volumes that several rois point into: multiples of 2^-8 and of 2^-24 below them, exact for
-//                        every half; infinities and NaN in a bit field beside them.
-// The sum is rounded to float once (the float accumulator of the scattering kernel rounds at every addition).
+//                        the sum cannot leave 32 bits.
+//   two words            elsewhere, and for volumes that several rois point into: multiples of 2^-8 and of 2^-24 below them;
+//                        infinities and NaN in a bit field beside them.
+// Either sum is exact for every half (coarser units in one word, for larger gradients, would drop the small gradients beside
+// them: with gradients of 8 among some of 1e-6, units of 2^-22 lose a fifth of the latter's sums).  It is rounded to float
+// once, where the float accumulator of the scattering kernel rounds at every addition.
 //
 // What bounds it: instruction issue (73 % of the slots) and the shared-memory reductions (72 % of the data pipe: eight per sample
 // at 2.5 clocks; rows of 21 words and planes of 384 had the fewest bank conflicts of 250 pitches tried over rotations of up to 30
@@ -73,7 +73,7 @@ struct BrickShared {
   unsigned match[kBrickMaxRois / 32];
   int warp_tot[kBrickThreads / 32];
   int special;
-  float scale;                     // units per one in a cell's single word
+  int one_word;                    // whether a cell's single word holds the roi's sums
   int rows_h, h_first, d_first, rows;  // the rectangle of output rows to look at
   float lim_lo[3], lim_hi[3];      // limits of the brick's positions
 };
@@ -251,12 +251,12 @@ __device__ __forceinline__ void brick_setup(const Params& p, const int* b0, Bric
 // The words of a tap row's two contributions, each below 2^14 in size.
 constexpr unsigned kBrickLo = sizeof(BrickShared);  // from a cell's hi word to its lo word
 constexpr unsigned kBrickStepY = kBrickSy * 4, kBrickStepZ = kBrickSz * 4;
-// TWO: hi[0], hi[1], lo[0], lo[1]; else the two in units of 1 / scale.
+// TWO: hi[0], hi[1], lo[0], lo[1]; else the two in units of 2^-24.
 template <bool TWO>
-__device__ __forceinline__ void brick_words(float f0, float f1, float scale, unsigned* w) {
+__device__ __forceinline__ void brick_words(float f0, float f1, unsigned* w) {
   if (!TWO) {
-    w[0] = (unsigned)__float2int_rn(f0 * scale);
-    w[1] = (unsigned)__float2int_rn(f1 * scale);
+    w[0] = (unsigned)__float2int_rn(f0 * 16777216.0f);
+    w[1] = (unsigned)__float2int_rn(f1 * 16777216.0f);
     return;
   }
   // both values in the halves of a 64-bit register: two operations per instruction
@@ -345,7 +345,7 @@ __device__ __forceinline__ void brick_tap(__half2 c, const PairConst& k, int axi
 // The numbered pairs.
 template <bool EDGE, bool TWO>
 __device__ __forceinline__ void brick_pairs(const Params& p, const PairConst& pc, BrickShared& sh, int n_pairs, const __half* __restrict__ go,
-                                            const int* b0, float scale) {
+                                            const int* b0) {
   typedef P2<__half> Q;
   typedef __half2 V;
   const RoiGeom<__half>& g = sh.roi.g;
@@ -379,10 +379,10 @@ __device__ __forceinline__ void brick_pairs(const Params& p, const PairConst& pc
     if (!TWO || __hblt2(__habs2(g2), __float2half2_rn(16384.0f))) {
       unsigned w[4][4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) brick_words<TWO>(Q::lo_float(v[2 * k]), Q::lo_float(v[2 * k + 1]), scale, w[k]);
+      for (int k = 0; k < 4; ++k) brick_words<TWO>(Q::lo_float(v[2 * k]), Q::lo_float(v[2 * k + 1]), w[k]);
       if (on_a) brick_add_cube<TWO>(cells + cell_a * 4u, w);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) brick_words<TWO>(Q::hi_float(v[2 * k]), Q::hi_float(v[2 * k + 1]), scale, w[k]);
+      for (int k = 0; k < 4; ++k) brick_words<TWO>(Q::hi_float(v[2 * k]), Q::hi_float(v[2 * k + 1]), w[k]);
       if (on_b) brick_add_cube<TWO>(cells + cell_b * 4u, w);
     } else {  // large, infinite or NaN
       float f[8];
@@ -454,10 +454,8 @@ __device__ __forceinline__ void brick_body(const Params& p, const PairConst& pc,
             if (lane + 32 < kBrickRoiWords) reinterpret_cast<unsigned*>(&sh.roi)[lane + 32] = second;
             top = __reduce_max_sync(0xffffffffu, top);
             __syncwarp();
-            if (lane == 0) {  // one word per voxel where the largest gradient allows it (NaN and infinity do not)
-              const float most = 1.01f * sh.roi.weights * __half2float(__ushort_as_half((unsigned short)top));
-              sh.scale = most < 127.0f ? 16777216.0f : most < 254.0f ? 8388608.0f : most < 508.0f ? 4194304.0f : 0.0f;
-            }
+            // NaN and infinity do not allow it
+            if (lane == 0) sh.one_word = 1.01f * sh.roi.weights * __half2float(__ushort_as_half((unsigned short)top)) < 127.0f;
           }
           brick_setup(p, b0, sh);
         } else if (!cleared) {  // meanwhile
@@ -466,8 +464,8 @@ __device__ __forceinline__ void brick_body(const Params& p, const PairConst& pc,
         }
         decoded = r;
         __syncthreads();
-        const float scale = sh.scale;
-        if (TWO ? scale != 0.0f && matches == 1 && p.R <= kBrickThreads : scale == 0.0f) return;  // CTA-uniform: the other form's
+        const bool one_word = sh.one_word != 0;
+        if (TWO ? one_word && matches == 1 && p.R <= kBrickThreads : !one_word) return;  // CTA-uniform: the other form's
         if (TWO && !cleared) {
           uint4* z = reinterpret_cast<uint4*>(&two.lo[0]);
           for (int i = tid; i < (kBrickWords + kBrickFlagWords) / 4; i += kBrickThreads) z[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -574,8 +572,8 @@ __device__ __forceinline__ void brick_body(const Params& p, const PairConst& pc,
             }
             __syncthreads();
             const int n_pairs = min(total - seg, kBrickPairs);
-            if (TWO || edge) brick_pairs<true, TWO>(p, pc, sh, n_pairs, go, b0, scale);
-            else brick_pairs<false, TWO>(p, pc, sh, n_pairs, go, b0, scale);
+            if (TWO || edge) brick_pairs<true, TWO>(p, pc, sh, n_pairs, go, b0);
+            else brick_pairs<false, TWO>(p, pc, sh, n_pairs, go, b0);
           }
           __syncthreads();  // rows and list are done with
         }
@@ -585,7 +583,6 @@ __device__ __forceinline__ void brick_body(const Params& p, const PairConst& pc,
 
     // ---- the brick itself, two voxels along w per thread and depth; cell 0 of an axis is voxel b0 - 1
     const bool special = TWO && sh.special != 0;
-    const float unit = TWO ? 0.0f : __frcp_rn(sh.scale);
     const int x = (tid & 7) * 2, y = (tid >> 3) & 15, nz = min(kBrick, p.D - b0[2]);
     if (x < p.W - b0[0] && y < p.H - b0[1]) {
       const long long plane = (long long)p.H * p.W;
@@ -606,9 +603,9 @@ __device__ __forceinline__ void brick_body(const Params& p, const PairConst& pc,
         if (z0 + j * kStep >= nz) break;
         float v[2];
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {  // exact but for the last rounding where the sum is one that half can hold
+        for (int k = 0; k < 2; ++k) {  // exact but for the last rounding
           if (TWO) v[k] = __fmaf_rn((float)(int)sh.hi[cell + k], 1.0f / 256.0f, (float)(int)two.lo[cell + k] * (1.0f / 16777216.0f));
-          else v[k] = (float)(int)sh.hi[cell + k] * unit;
+          else v[k] = (float)(int)sh.hi[cell + k] * (1.0f / 16777216.0f);
         }
         if (special) {
 #pragma unroll

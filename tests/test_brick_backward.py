@@ -2,8 +2,8 @@
 overlap, magnify, or lie beyond the kernel's range, gradients that need one word per voxel, two, or flags.  Against the
 restatement with a wide accumulator.
 
-The contributions are the restatement's own, and their sum is exact or, in units of 2^-22 at the coarsest, off by half a unit per
-contribution (at most 64 of them here): one rounding to half on either side, 2^-11 of the value each, and 64 * 2^-23."""
+The contributions are the restatement's own and their sum is exact, whatever the sizes of the gradients: one rounding to half on
+either side, 2^-11 of the value or half a unit of 2^-24 each, and roundings to float far below that."""
 import pytest
 import torch
 
@@ -28,6 +28,8 @@ CASES = {
     "one word": dict(n=3, zoom=1.0, out=(48, 70, 66), size=1.0),
     "coarser units": dict(n=3, zoom=1.0, out=(48, 70, 67), size=2.5),
     "two words": dict(n=3, zoom=1.0, out=(48, 66, 71), size=3000.0),
+    "peaks": dict(n=3, zoom=1.0, out=(48, 70, 66), size=2e-6, peak=8.0),  # a few large gradients among tiny ones
+    "larger peaks": dict(n=3, zoom=1.0, out=(48, 70, 66), size=1e-4, peak=500.0),
     "tiny": dict(n=3, zoom=1.0, out=(48, 66, 70), size=3e-5),
     "turned anyhow": dict(n=3, zoom=1.0, out=(50, 61, 70), size=1.0, tilt=3.1),
     "overlapping": dict(n=8, zoom=0.8, out=(40, 60, 64), size=1.0),
@@ -41,7 +43,7 @@ CASES = {
 @pytest.mark.parametrize("name", CASES)
 def test_gradient(name):
     from medvision_b200 import _C
-    k = dict(dict(order=1, box=False, tilt=0.9, mixed=False), **CASES[name])
+    k = dict(dict(order=1, box=False, tilt=0.9, mixed=False, peak=0.0), **CASES[name])
     g = torch.Generator().manual_seed(len(name))
     rois = make_rois(g, k["n"], k["zoom"], k["tilt"])
     if k["mixed"]:
@@ -51,6 +53,9 @@ def test_gradient(name):
     kind = cases.KIND_BOX if k["box"] else cases.KIND_ROTATED
     out = k["out"]
     grad = (torch.randn((k["n"], SHAPE[1]) + out, generator=g).clamp_(-4, 4) * k["size"]).half()
+    if k["peak"]:
+        at = torch.randint(0, grad[0].numel(), (40,), generator=g)
+        grad.view(k["n"], -1)[:, at] = k["peak"] * torch.randn(40, generator=g).sign().half()
     kw = dict(spatial_scale=1.0, sampling_ratio=1, aligned=not k["box"], order=k["order"], trig=None if k["box"] else port.device_trig(rois))
     # unaligned gradient memory, a result that is added to
     dev = torch.empty(grad.numel() + 1, dtype=torch.half, device="cuda")[1:].view(grad.shape).copy_(grad)
@@ -62,7 +67,7 @@ def test_gradient(name):
         _C.roi_align_rotated_3d_backward(dev, rois.cuda(), got, *out, 1.0, 1, True, k["order"])
     want = port.backward(grad, rois, SHAPE, kind, wide_acc=True, **kw).double()
     err = (got.cpu().double() - before.double() - want).abs()
-    bound = 2.0 ** -11 * (2 * want.abs() + 2 * (want + before.double()).abs()) + 64 * 2.0 ** -23 * min(k["size"], 1.0) + 2.0 ** -24
+    bound = 2.0 ** -11 * (2 * want.abs() + 2 * (want + before.double()).abs()) + 2.0 ** -24
     assert not bool((err > bound).any()), float((err - bound).max())
 
 
