@@ -385,61 +385,81 @@ resample_bwd_stream3d(const Params p, const S3Launch L, typename BwdAcc<T>::type
   bwd_scatter<T, PAIR>(p, L, acc_base, s3_cta(p, L), sh);
 }
 
-// What bwd_brick3d_half leaves: the bricks that need two words per voxel, and by the `scatter` CTAs behind those the rois that the
-// bricks do not take.  Mostly there is neither, and the grid is gone after a look at the plan.
+// What bwd_brick3d_half leaves, by resident CTAs: the bricks that need two words per voxel, then the (volume, channel)s that the
+// bricks do not take.
 template <bool PAIR>
 __global__ void __launch_bounds__(kS3Threads, PAIR ? 3 : 1)
-bwd_brick3d_rest(const Params p, const PairConst pc, const BrickPlan plan, const BrickGrid G, unsigned bricks, const S3Launch L,
-                 float* __restrict__ acc_base, long long items) {
+bwd_brick3d_rest(const Params p, const PairConst pc, const BrickPlan plan, const BrickGrid G, const S3Launch L, float* __restrict__ acc_base,
+                 long long items) {
   extern __shared__ __align__(16) unsigned char brick_smem[];
+  __shared__ BrickTurn work;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (blockIdx.x < bricks) {
-    brick_body<true>(p, pc, plan, G, brick_smem);
-    return;
-  }
-  if (blockIdx.x == bricks && p.status) {
+  if (blockIdx.x == 0 && p.status) {
     for (int n = threadIdx.x; n < p.R; n += kS3Threads)
       if (__ldcg(plan.volume + n) == INT_MIN) atomicOr(p.status, STATUS_BAD_BATCH_INDEX);
   }
-  if (!brick_leaves_any(p, plan)) return;
+  brick_listed(p, pc, plan, G, work, brick_smem);
+  const unsigned left = __ldcg(plan.number + 1);
+  if (left == 0u) return;
+  const bool all = left == (unsigned)(p.N * p.C);
   S3Shared<__half>& sh = *reinterpret_cast<S3Shared<__half>*>(brick_smem);
-  BrickLeft& left = *reinterpret_cast<BrickLeft*>(brick_smem + ((sizeof(S3Shared<__half>) + 15) & ~size_t(15)));
-  static_assert(sizeof(S3Shared<__half>) + 16 + sizeof(BrickLeft) <= sizeof(BrickSharedTwo), "shared memory of the launch");
-  brick_left(p, plan, left);
-  for (long long item = blockIdx.x - bricks; item < items; item += gridDim.x - bricks) {
+  static_assert(sizeof(S3Shared<__half>) <= sizeof(BrickSharedTwo), "shared memory of the launch");
+  unsigned turn = 0;
+  for (unsigned item = blockIdx.x; item < items; item = work.next(turn++)) {
+    work.draw(plan.number + 3, turn);
     const S3Cta k = s3_cta(p, L, item);
-    if (!((left.mask[k.n >> 5] >> (k.n & 31)) & 1u)) continue;  // CTA-uniform
-    bwd_scatter<__half, PAIR>(p, L, acc_base, k, sh);
+    const int v = all ? 0 : __ldcg(plan.volume + k.n);
+    if (all || (v != INT_MIN && __ldcg(plan.route + (long long)(v < 0 ? -2 - v : v) * p.C + k.c) == -2))  // CTA-uniform
+      bwd_scatter<__half, PAIR>(p, L, acc_base, k, sh);
     __syncthreads();  // the next item's prologue overwrites the tables
   }
 }
 
-// grad_in (half) += scratch (float), rounded once.  IF_LEFT: only where the bricks left a roi to the scattering kernel.
-template <bool IF_LEFT>
-__global__ void __launch_bounds__(256) bwd_fold_half(const Params p, const BrickPlan plan, const float* scratch, long long n) {
-  if (IF_LEFT) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (!brick_leaves_any(p, plan)) return;
-  }
-  __half* const grad_in = (__half*)p.out;
-  for (long long i0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8; i0 < n; i0 += (long long)gridDim.x * blockDim.x * 8) {
-    if (i0 + 8 <= n && ((uintptr_t)(grad_in + i0) % 16 == 0)) {
-      const float4 s0 = __ldcg(reinterpret_cast<const float4*>(scratch + i0));
-      const float4 s1 = __ldcg(reinterpret_cast<const float4*>(scratch + i0 + 4));
-      uint4 gv = *reinterpret_cast<const uint4*>(grad_in + i0);
-      __half2* h = reinterpret_cast<__half2*>(&gv);
-      const float s[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+// GROUPS groups of eight elements of grad_in (half), `step` elements apart from i0 on, += scratch (float), rounded once; those in
+// first .. last.  The loads of all groups are under way at once.
+template <int GROUPS>
+__device__ __forceinline__ void bwd_fold_groups(__half* __restrict__ grad_in, const float* __restrict__ scratch, long long i0, int step, long long first,
+                                                long long last) {
+  const long long end = i0 + (GROUPS - 1) * step + 8;
+  if (i0 >= first && end <= last && ((uintptr_t)(grad_in + i0) % 16 == 0)) {
+    float4 s0[GROUPS], s1[GROUPS];
+    uint4 gv[GROUPS];
+#pragma unroll
+    for (int g = 0; g < GROUPS; ++g) {
+      s0[g] = __ldcg(reinterpret_cast<const float4*>(scratch + i0 + g * step));
+      s1[g] = __ldcg(reinterpret_cast<const float4*>(scratch + i0 + g * step) + 1);
+      gv[g] = *reinterpret_cast<const uint4*>(grad_in + i0 + g * step);
+    }
+#pragma unroll
+    for (int g = 0; g < GROUPS; ++g) {
+      __half2* h = reinterpret_cast<__half2*>(&gv[g]);
+      const float s[8] = {s0[g].x, s0[g].y, s0[g].z, s0[g].w, s1[g].x, s1[g].y, s1[g].z, s1[g].w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float2 f = __half22float2(h[j]);
         h[j] = __floats2half2_rn(f.x + s[2 * j], f.y + s[2 * j + 1]);
       }
-      *reinterpret_cast<uint4*>(grad_in + i0) = gv;
-    } else {
-      for (long long i = i0; i < n && i < i0 + 8; ++i)
-        grad_in[i] = __float2half_rn(__half2float(grad_in[i]) + scratch[i]);
+      *reinterpret_cast<uint4*>(grad_in + i0 + g * step) = gv[g];
     }
+  } else {
+    for (int g = 0; g < GROUPS; ++g)
+      for (long long i = max(i0 + g * step, first); i < min(i0 + g * step + 8, last); ++i)
+        grad_in[i] = __float2half_rn(__half2float(grad_in[i]) + scratch[i]);
+  }
+}
+__global__ void __launch_bounds__(256) bwd_fold_half(__half* __restrict__ grad_in, const float* __restrict__ scratch, long long n) {
+  bwd_fold_groups<1>(grad_in, scratch, ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8, 0, 0, n);
+}
+// The same for the (volume, channel)s that the bricks left to the scattering kernel, by resident CTAs.
+__global__ void __launch_bounds__(256, 6) bwd_fold_left_half(const Params p, const BrickPlan plan, const float* __restrict__ scratch) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  constexpr int kGroups = 2, kStep = 256 * 8;
+  const long long piece = kStep * kGroups, pieces = (p.vol + 7 + piece - 1) / piece;  // that a volume may lie across
+  const long long all = __ldcg(plan.number + 1) * pieces;
+  for (long long t = blockIdx.x; t < all; t += gridDim.x) {
+    const long long k = t / pieces, first = __ldcg(plan.left + k) * p.vol;
+    bwd_fold_groups<kGroups>((__half*)p.out, scratch, (first & ~7LL) + (t - k * pieces) * piece + threadIdx.x * 8, kStep, first, first + p.vol);
   }
 }
 
@@ -474,19 +494,17 @@ inline void launch_bwd_kernel(const Params& p, const S3Launch& L, long long ctas
   else resample_bwd_stream3d<T, false><<<(unsigned)ctas, kS3Threads, 0, st>>>(p, L, acc);
 }
 
-// Whether the gradient is summed brick by brick.  Few rois per volume, as the dense calls have them: a brick looks at every roi of
-// its volume.
+// Whether the gradient may be summed brick by brick.  A roi per volume, as the dense calls have it.
 inline bool bwd_brick3d_applicable(const Params& p, int dtype) {
-  if (dtype != 1 || p.R > kBrickMaxRois || p.R > 4LL * p.N || p.D > kTapMaxSize || p.H > kTapMaxSize || p.W > kTapMaxSize) return false;
+  if (dtype != 1 || p.R > kBrickMaxRois || p.R > p.N || p.D > kTapMaxSize || p.H > kTapMaxSize || p.W > kTapMaxSize) return false;
   if (p.ovol >= 0x7fffffffLL || p.ow >= (1 << 23) || (long long)p.R * p.C * kBrickMaxParts > 0x7ffffff0LL - p.R) return false;
-  const long long bw = (p.W + kBrick - 1) / kBrick, bh = (p.H + kBrick - 1) / kBrick, bd = (p.D + kBrick - 1) / kBrick;
-  const long long bricks = (long long)p.N * p.C * bw * bh * bd;
+  const long long bricks = brick_count(p);
+  if (std::min({p.D, p.H, p.W}) < kBrickMinAxis || (long long)p.N * p.C * p.vol < bricks * kBrickMinFill) return false;
   return bricks >= kBrickMinBricks && bricks <= 0x7fffff00LL;
 }
 
 template <bool PAIR>
 inline cudaError_t launch_bwd_brick3d(const Params& p, const S3Launch& L, long long ctas, float* scratch, const BrickPlan& plan, cudaStream_t st) {
-  const long long n = (long long)p.N * p.C * p.vol;
   const size_t smem1 = sizeof(BrickShared), smem2 = sizeof(BrickSharedTwo);
   // more dynamic shared memory than the default limit: opt in (per function and device; smem1 lies below it)
   static_assert(sizeof(BrickShared) <= 48 * 1024, "default limit");
@@ -495,16 +513,14 @@ inline cudaError_t launch_bwd_brick3d(const Params& p, const S3Launch& L, long l
   BrickGrid G;
   G.bricks_w = (p.W + kBrick - 1) / kBrick;
   G.bricks_h = (p.H + kBrick - 1) / kBrick;
-  const int bd = (p.D + kBrick - 1) / kBrick;
+  const int bd = G.bricks_d = (p.D + kBrick - 1) / kBrick;
   const long long columns = (long long)p.N * p.C * G.bricks_w * G.bricks_h;
   // bricks per CTA: as many as leave six CTAs per place (16 x 128^3: two 280 us, one and four 290, eight 330)
   G.run = 1;
   while (G.run < 4 && columns * ((bd + 2 * G.run - 1) / (2 * G.run)) >= 148 * 4 * 6) G.run *= 2;
   G.runs = (bd + G.run - 1) / G.run;
-  BrickGrid T = G;  // a CTA per column where hardly any has work
-  T.run = bd;
-  T.runs = 1;
-  // each of the launches that follow may become resident while the one before ends
+  // each of the two launches that follow may become resident while the one before ends; not so the last, whose loads would have the
+  // little L1 that the others' shared memory leaves (2 x 128^3: 7 us instead of 12)
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -513,17 +529,18 @@ inline cudaError_t launch_bwd_brick3d(const Params& p, const S3Launch& L, long l
   cfg.attrs = attr;
   cfg.blockDim = dim3(256);
   cfg.gridDim = dim3((unsigned)((long long)p.R * p.C * plan.parts + p.R));
-  cudaError_t e = cudaLaunchKernelEx(&cfg, bwd_brick3d_plan, p, plan, scratch, n);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, bwd_brick3d_plan, p, plan, scratch);
   cfg.numAttrs = 1;
   cfg.gridDim = dim3((unsigned)(columns * G.runs));
   cfg.dynamicSmemBytes = smem1;
-  if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, bwd_brick3d_half, p, pc, plan, G);
-  cfg.gridDim = dim3((unsigned)(columns + std::min(ctas, 148LL * 3 * 8)));
+  if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, bwd_brick3d_half, p, pc, plan, G, scratch);
+  cfg.gridDim = dim3(148 * 3);
   cfg.dynamicSmemBytes = smem2;
-  if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, bwd_brick3d_rest<PAIR>, p, pc, plan, T, (unsigned)columns, L, scratch, ctas);
-  cfg.gridDim = dim3(148 * 8);
+  if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, bwd_brick3d_rest<PAIR>, p, pc, plan, G, L, scratch, ctas);
+  cfg.numAttrs = 0;
+  cfg.gridDim = dim3(148 * 6);
   cfg.dynamicSmemBytes = 0;
-  if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, bwd_fold_half<true>, p, plan, (const float*)scratch, n);
+  if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, bwd_fold_left_half, p, plan, (const float*)scratch);
   return e;
 }
 
@@ -541,7 +558,7 @@ inline int launch_bwd_stream3d_half(const Params& p, const S3Launch& L, long lon
   const long long n = (long long)p.N * p.C * p.vol;
   cudaMemsetAsync(scratch, 0, (size_t)n * sizeof(float), st);
   launch_bwd_kernel<__half>(p, L, ctas, scratch, st);
-  bwd_fold_half<false><<<(unsigned)((n + 8 * 256 - 1) / (8 * 256)), 256, 0, st>>>(p, BrickPlan(), scratch, n);
+  bwd_fold_half<<<(unsigned)((n + 8 * 256 - 1) / (8 * 256)), 256, 0, st>>>((__half*)p.out, scratch, n);
   return cudaGetLastError() == cudaSuccess ? 0 : -8;
 }
 
