@@ -478,7 +478,6 @@ inline bool bwd_stream3d_applicable(const Params& p, int dtype, S3Launch& L, lon
   if (chunk > p.od) chunk = p.od;
   L.chunk = chunk;
   L.chunks = (p.od + chunk - 1) / chunk;
-  L.vec_store = 0;
   L.filter = 0;
   L.pair = make_pair_const(3, p.D, p.H, p.W, 4);  // offsets in the float accumulator
   ctas = per_depth_ctas * L.chunks;

@@ -264,7 +264,6 @@ inline bool label_stream3d_geometry(const Params& p, S3Launch& L, long long& ite
   const long long per_depth = (long long)p.R * p.C * L.tiles_w * L.tiles_h;
   L.chunk = s3_pick_chunk(per_depth, p.od, 148 * 4, 12);
   L.chunks = (p.od + L.chunk - 1) / L.chunk;
-  L.vec_store = 0;
   L.filter = 0;
   items = per_depth * L.chunks;
   return items <= 0x7fffffffLL;

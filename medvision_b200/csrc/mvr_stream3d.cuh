@@ -383,7 +383,7 @@ struct S3Shared {
 
 struct S3Launch {
   int tiles_w, tiles_h, chunks, chunk;  // chunk = output depths per CTA
-  int vec_store;                        // 1: two-element vector stores are aligned
+  int vec_store = 0;                    // plane-streaming kernel: two-element vector stores are aligned
   int filter;                           // 0: every roi; 1: only rois that turn about z at most; 2: only the others
   PairConst pair;                       // gather kernels: constants of the pair taps
   // plane-streaming kernel only: limits of its bounded waits, and the self-test's left-out plane (-1: none)

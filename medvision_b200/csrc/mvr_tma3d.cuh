@@ -197,12 +197,12 @@ __device__ __forceinline__ void t3_mbar_arrive_one(unsigned bar) {
       : "memory");
 }
 
-// The gather path as this kernel's rare ways out use it: the two voxels of a thread side by side, stored as a vector.  (With the
-// faster placement of s3_body_l1 in their place, the kernel's own loop compiles to code that is 3 % slower: 8 x (160,256,256) about z
-// 151 us against 146.)
-template <typename T, int NP, bool WIDE>
+// The gather path as this kernel's rare ways out use it: the two voxels of a thread side by side, stored as a vector; positions, taps and
+// sums as in s3_body_l1.  A body of its own, because what stands here decides how the kernel's main loop compiles: 512 patches of 96^3
+// half about z take 650 us, with s3_body_l1 called out of line 668, with its placement as a template parameter 674-679.
+template <typename T, bool WIDE>
 __device__ __forceinline__ void t3_side_depth_loop(const Params& p, const S3Launch& L, const S3Shared<T>& sh, int npd, int c,
-                                                   int pw0, int ph0, int row_step, bool vec_store, T* out0) {
+                                                   int pw0, int ph, bool vec_store, T* out0) {
   typedef Ar<T> A;
   typedef P2<T> Q;
   typedef typename Q::V V;
@@ -215,55 +215,42 @@ __device__ __forceinline__ void t3_side_depth_loop(const Params& p, const S3Laun
   const T xa = A::add(lattice_base<T>(g.start[0], pw0, g.bin[0], fm), sub_x);
   const T xb = A::add(lattice_base<T>(g.start[0], has_b ? pw0 + 1 : pw0, g.bin[0], fm), sub_x);
   const V x2 = Q::make(xa, xb);
-  V sxy[NP][3];
-  bool act[NP];
+  V sxy[3];
+  const T y = A::add(lattice_base<T>(g.start[1], ph, g.bin[1], fm), sub_y);
 #pragma unroll
-  for (int q = 0; q < NP; ++q) {
-    const int ph = ph0 + q * row_step;
-    act[q] = ph < p.oh;
-    const T y = A::add(lattice_base<T>(g.start[1], act[q] ? ph : 0, g.bin[1], fm), sub_y);
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-      sxy[q][r] = Q::row_xy(Q::dup(g.rot[3 * r]), x2, Q::dup(A::mul(g.rot[3 * r + 1], y)));
-  }
+  for (int r = 0; r < 3; ++r) sxy[r] = Q::row_xy(Q::dup(g.rot[3 * r]), x2, Q::dup(A::mul(g.rot[3 * r + 1], y)));
   const V c2[3] = {Q::dup(g.centre[0]), Q::dup(g.centre[1]), Q::dup(g.centre[2])};
   const PairConst& pc = L.pair;
   const typename Q::M lanes = Q::make_mask(true, has_b);
   const long long plane_o = (long long)p.oh * p.ow;
-  const long long sub_o = (long long)row_step * p.ow;
   T* o = out0;
   for (int i = 0; i < npd; ++i, o += plane_o) {
     const S3ZProd<T> e = sh.zp[i];
-#pragma unroll
-    for (int q = 0; q < NP; ++q) {
-      if (!act[q]) continue;
-      const V rx2 = Q::add(Q::add(sxy[q][0], Q::dup(e.p[0])), c2[0]);
-      const V ry2 = Q::add(Q::add(sxy[q][1], Q::dup(e.p[1])), c2[1]);
-      const V rz2 = Q::add(Q::add(sxy[q][2], Q::dup(e.p[2])), c2[2]);
-      AxisTap2<T> tx, ty, tz;
-      axis_tap2<T, 0>(rx2, pc, p.order, tx);
-      axis_tap2<T, 1>(ry2, pc, p.order, ty);
-      axis_tap2<T, 2>(rz2, pc, p.order, tz);
-      const typename Q::M mask = lanes & ~(Q::outside(rx2, pc, 0) | Q::outside(ry2, pc, 1) | Q::outside(rz2, pc, 2));
-      V val = zero2;
-      if (mask) {  // a lane outside keeps valid (clamped) addresses; its value is dropped
-        V v[8], w[8];
-        PairTaps<T, 3, WIDE>(tx, ty, tz, pc).load(vol, v);
-        pair_weights<T, 3>(tx, ty, tz, w);
-        val = Q::apply(Q::add(zero2, pair_sum<T, 8>(w, v)), mask);
-      }
-      T* oq = o + q * sub_o;
-      if (vec_store && has_b) {
-        Q::store2(oq, val);
-      } else {
-        oq[0] = Q::lo(val);
-        if (has_b) oq[1] = Q::hi(val);
-      }
+    const V rx2 = Q::add(Q::add(sxy[0], Q::dup(e.p[0])), c2[0]);
+    const V ry2 = Q::add(Q::add(sxy[1], Q::dup(e.p[1])), c2[1]);
+    const V rz2 = Q::add(Q::add(sxy[2], Q::dup(e.p[2])), c2[2]);
+    AxisTap2<T> tx, ty, tz;
+    axis_tap2<T, 0>(rx2, pc, p.order, tx);
+    axis_tap2<T, 1>(ry2, pc, p.order, ty);
+    axis_tap2<T, 2>(rz2, pc, p.order, tz);
+    const typename Q::M mask = lanes & ~(Q::outside(rx2, pc, 0) | Q::outside(ry2, pc, 1) | Q::outside(rz2, pc, 2));
+    V val = zero2;
+    if (mask) {  // a lane outside keeps valid (clamped) addresses; its value is dropped
+      V v[8], w[8];
+      PairTaps<T, 3, WIDE>(tx, ty, tz, pc).load(vol, v);
+      pair_weights<T, 3>(tx, ty, tz, w);
+      val = Q::apply(Q::add(zero2, pair_sum<T, 8>(w, v)), mask);
+    }
+    if (vec_store && has_b) {
+      Q::store2(o, val);
+    } else {
+      o[0] = Q::lo(val);
+      if (has_b) o[1] = Q::hi(val);
     }
   }
 }
 
-template <typename T, bool GENERAL, bool WIDE>
+template <typename T, bool WIDE>
 __device__ void t3_side_body(const Params& p, const S3Launch& L, const S3Cta& k, S3Shared<T>& sh) {
   typedef Ar<T> A;
   typedef P2<T> Q;
@@ -272,7 +259,7 @@ __device__ void t3_side_body(const Params& p, const S3Launch& L, const S3Cta& k,
   const long long nc = k.nc;
   const int fm = kS3FloatPattern;
   const RoiGeom<T>& g = sh.g;
-  const bool zsep = !GENERAL && sh.zsep != 0;
+  const bool zsep = sh.zsep != 0;
   const bool rotated = (p.kind == KIND_ROTATED);
   const bool bad_batch = (g.batch < 0 || g.batch >= p.N);
   // ---- this thread's two output columns
@@ -391,7 +378,7 @@ __device__ void t3_side_body(const Params& p, const S3Launch& L, const S3Cta& k,
   }
 
   // ---- general rotation: positions change with depth
-  t3_side_depth_loop<T, 1, WIDE>(p, L, sh, npd, c, pw0, ph, kS3TileH, L.vec_store != 0, out);
+  t3_side_depth_loop<T, WIDE>(p, L, sh, npd, c, pw0, ph, L.vec_store != 0, out);
 }
 
 // The rare ways out of the plane-streaming kernel (batch index outside the batch, coordinates that
@@ -403,7 +390,7 @@ __device__ __forceinline__ void t3_fallback(const Params& p, const S3Launch& L, 
   for (int q = 0; q < np; ++q) {
     S3Cta k2 = k;
     k2.th = k.th * np + q;
-    if (k2.th * kS3TileH < p.oh) t3_side_body<T, false, WIDE>(p, L, k2, sh);
+    if (k2.th * kS3TileH < p.oh) t3_side_body<T, WIDE>(p, L, k2, sh);
   }
 }
 
@@ -851,7 +838,6 @@ inline int try_launch_stream3d(const Params& p, int dtype, cudaStream_t st, T3La
     G.chunk = min(chunk, p.od);
   }
   G.chunks = (p.od + G.chunk - 1) / G.chunk;
-  G.vec_store = 0;
   G.filter = 0;
   G.pair = make_pair_const(3, p.D, p.H, p.W, wide ? 1 : esz);
   const long long g_ctas = g_per_depth * G.chunks;
