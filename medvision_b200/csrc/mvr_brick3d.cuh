@@ -63,6 +63,10 @@ constexpr long long kBrickMinFill = kBrick * kBrick * kBrick / 3;
 constexpr int kBrickMinTouched = 600;
 // Steps between samples, in voxels.  16 x 128^3 magnified by 2.2: 860 us by bricks, 640 scattered (neighbouring samples add to one word).
 constexpr float kBrickMinStep = 0.5f;
+// The same for rois that turn about z at most, where the scattering kernel sums along the depth first.  16 x 128^3 magnified by 1.6: 353 us
+// by bricks, 322 scattered, 358 as left to it here; by 1.75 383, 303, 337; by 1.9 416, 295, 325.  8 x 128^3 by 1.6 197, 189, 217; by 1.9
+// 298, 174, 198.
+constexpr float kBrickMinPlanarStep = 0.6f;
 // Rois that turn about z at most in volumes with an axis beyond this: half positions are so coarse there that most bricks need two words,
 // and the scattering kernel, which sums along the depth, is at its best.  4 x (32,512,512) 423 us by bricks, 350 scattered, 379 as left
 // to it here; 4 x (64,320,320) 272, 281.
@@ -121,7 +125,7 @@ struct BrickTurn {
 static_assert((sizeof(BrickShared) + 1024) * 4 <= 228 * 1024 && (sizeof(BrickSharedTwo) + 1024) * 3 <= 228 * 1024, "four and three CTAs per SM");
 
 // How many bricks a roi's samples lie in, about; 0 where this kernel does not take the roi: finite values, coordinates up to 2048 (where
-// half still tells voxels apart), steps of at least kBrickMinStep voxels, and the sizes above.
+// half still tells voxels apart), steps of at least kBrickMinStep (kBrickMinPlanarStep) voxels, and the sizes above.
 __device__ __forceinline__ int brick_touches(const Params& p, long long n) {
   const int width = p.kind == KIND_BOX ? 7 : 10;
   const __half* r = (const __half*)p.rois + n * width;
@@ -133,7 +137,7 @@ __device__ __forceinline__ int brick_touches(const Params& p, long long n) {
   for (int a = 0; a < 3; ++a) {
     const float first = __half2float(__ldg(r + 1 + a)), second = __half2float(__ldg(r + 4 + a));
     const float size = __fmul_rn(p.kind == KIND_BOX ? __fsub_rn(second, first) : second, scale);
-    ok = ok && __fmul_rn(fabsf(first), scale) <= 2048.0f && size <= 2048.0f && size >= __fmul_rn(kBrickMinStep, (float)osz[a]);
+    ok = ok && __fmul_rn(fabsf(first), scale) <= 2048.0f && size <= 2048.0f && size >= __fmul_rn(planar ? kBrickMinPlanarStep : kBrickMinStep, (float)osz[a]);
     if (p.kind != KIND_BOX) ok = ok && isfinite(__half2float(__ldg(r + 7 + a)));
     bricks[a] = min((isz[a] + kBrick - 1) / kBrick, (int)fminf(fmaxf(size, 0.0f), 2048.0f) / kBrick + 1);
   }

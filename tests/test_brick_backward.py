@@ -50,6 +50,8 @@ CASES = {
     "740 bricks": dict(n=740, zoom=1.0, out=(15, 17, 18), size=1.0, shape=(740, 1, 16, 16, 16)),
     "eleven planes": dict(n=4, zoom=1.0, out=(11, 150, 170), size=1.0, shape=(4, 2, 11, 160, 180), flat=True),
     "one plane": dict(n=4, zoom=1.0, out=(1, 150, 170), size=1.0, shape=(4, 2, 1, 160, 180), flat=True),
+    # turning about z at most, steps on either side of the limit of 0.6 voxels in one call
+    "about z, magnified": dict(n=60, zoom=0.57, out=(48, 52, 56), size=1.0, shape=(60, 1, 64, 64, 64), flat=True),
     "small rois": dict(n=4, zoom=0.3, out=(16, 20, 20), size=1.0),
 }
 
