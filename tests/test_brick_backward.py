@@ -162,3 +162,27 @@ def test_no_call_is_much_slower_than_by_scattering(name):
             times.append(a.elapsed_time(b))
         best.append(min(times[2:]))
     assert best[0] <= 2 * best[1], best
+
+
+@pytest.mark.parametrize("order", [1, 0])
+@pytest.mark.parametrize("shape,zoom,tilt", [((2, 1, 128, 128, 128), 1.0, 0.0), ((2, 1, 128, 128, 128), 1.1, 1.0), ((4, 1, 90, 100, 110), 1.3, 0.6),
+                                             ((8, 1, 13, 180, 200), 1.0, 0.0)])
+def test_sums_of_one_sign(shape, zoom, tilt, order):
+    """Gradients that are all the same, up to and beyond what one word per voxel holds: the largest sums that the bound of the weights
+    allows, against the entry point that scatters into float.  Sums of some tens of contributions differ by 2^-18 there, so one rounding to
+    half on either side leaves them one unit apart at most, 2^-10 of the value."""
+    from medvision_b200 import _lib
+    n = shape[0]
+    g = torch.Generator().manual_seed(7)
+    ext = torch.tensor(shape[:1:-1], dtype=torch.float32).expand(n, 3)
+    angles = (torch.rand(n, 3, generator=g) - 0.5) * tilt
+    rois = torch.cat([torch.arange(n).float().view(-1, 1), ext / 2, ext / zoom, angles], 1).half().cuda()
+    for value in (2.5, 4.0, 6.0, 8.0, 10.0, 13.0, 16.0, 24.0, -12.0):
+        grad = torch.full((n,) + shape[1:], value, dtype=torch.half, device="cuda")
+        got = []
+        for fn in (_lib.lib.mvr_roi_resample_bwd, _lib.lib.mvr_roi_resample_bwd_noalloc):
+            gin = torch.zeros(shape, dtype=torch.half, device="cuda")
+            assert fn(grad.data_ptr(), rois.data_ptr(), gin.data_ptr(), _lib.MVR_F16, 3, _lib.MVR_ROI_ROTATED, *shape, n, 10, *shape[2:], 1.0, 1, 1,
+                      order, None, torch.cuda.current_stream().cuda_stream) == 0
+            got.append(gin.double())
+        assert bool(((got[0] - got[1]).abs() <= 2.0 ** -10 * got[1].abs() + 2.0 ** -24).all()), value
