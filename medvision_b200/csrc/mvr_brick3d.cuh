@@ -22,17 +22,17 @@
 //
 // What bounds it: instruction issue (73 % of the slots) and the shared-memory reductions (72 % of the data pipe: eight per sample
 // at 2.5 clocks; rows of 21 words and planes of 384 had the fewest bank conflicts of 250 pitches tried over rotations of up to 30
-// degrees).  16 x 128^3 under three axes: plan 18 us, one word 265, with two words and idle launches 292 in all, where the scattering
-// kernel takes 469 and the clear and the fold of its accumulator 63.  Gradients of 100 throughout, two words: 390.  Rows listed pair
+// degrees).  16 x 128^3 under three axes: plan 15 us, one word 274, with two words and idle launches 295 in all, where the scattering
+// kernel takes 456 and the clear and the fold of its accumulator 70.  Gradients of 100 throughout, two words: 396.  Rows listed pair
 // by pair: 8 % slower.
 //
 // Which calls: a brick's work is one CTA's, so the kernel wants as many touched bricks as the chip has places, about evenly.  Times
 // against the scattering kernel's, us, cold caches, backward alone:
-//   128^3, gradients of deviation one, three axes   2 volumes 66 / 89, 4: 100 / 157, 16: 294 / 541;  about z 64 / 66, 98 / 111, 283 / 352
-//   the same, gradients of 100                      88 / 90, 135 / 157, 392 / 540;  about z 87 / 66, 131 / 111, 381 / 352
-//   magnified by 1.5 / 1.75, 16 volumes             403 / 608, 520 / 618;  4 volumes 172 / 178 by 1.5
+//   128^3, gradients of deviation one, three axes   2 volumes 63 / 88, 4: 97 / 146, 16: 295 / 529;  about z 61 / 70, 93 / 113, 283 / 365
+//   the same, gradients of 100                      82 / 88, 129 / 146, 396 / 527;  about z 83 / 70, 123 / 113, 385 / 365
+//   magnified by 1.5 / 1.75, 16 volumes             397 / 607, 428 / 609;  4 volumes 140 / 170 by 1.5
 // What it leaves to the scattering kernel inside its own launches (strong magnification, several rois in a volume, large planes
-// about z) takes 1.05-1.2 times as long as there, by the launches that find nothing: 2 volumes magnified by 2.2 128 / 107, 16: 676 / 637.
+// about z) takes 1.05-1.25 times as long as there, by the launches that find nothing: 2 volumes magnified by 2.2 123 / 105, 16: 658 / 617.
 #pragma once
 #include <climits>
 
@@ -271,7 +271,7 @@ __device__ __forceinline__ void brick_setup_roi(const Params& p, BrickRoi& roi) 
   }
   __syncwarp();
 }
-// Lowers roi.weights (in shared memory) to what the lattice itself shows; all 256 threads of a CTA.  The weights at a voxel depend on
+// Lowers roi.weights (in shared memory) to what the lattice itself shows; all 256 threads of a CTA; best: 64 words.  The weights at a voxel depend on
 // where it lies in a cell of the lattice.  The cell is cut into 4 x 4 x 4 parts, and for each of them every lattice point's hat counts
 // with its largest value over the part and over the positions' errors.  (Without it, 16 x 128^3 with gradients of deviation one under three
 // axes take 500 us instead of 292: most bricks would need two words.)
@@ -328,17 +328,27 @@ __device__ __forceinline__ void brick_tighten_weights(const Params& p, BrickRoi&
       }
     }
   }
-  if (tid < 8) best[tid] = 0u;
-  __syncthreads();
+  float top[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) top[k] = 0.0f;
 #pragma unroll
   for (int e = 0; e < 27; ++e) {
     sum[e] += __shfl_xor_sync(0xffffffffu, sum[e], 1);
     sum[e] += __shfl_xor_sync(0xffffffffu, sum[e], 2);
-    const unsigned top = __reduce_max_sync(0xffffffffu, __float_as_uint(sum[e]));
-    if ((tid & 31) == 0) atomicMax(&best[(e % 3 != 0) + 2 * (e / 3 % 3 != 0) + 4 * (e / 9 != 0)], top);
+    const int k = (e % 3 != 0) + 2 * (e / 3 % 3 != 0) + 4 * (e / 9 != 0);
+    top[k] = fmaxf(top[k], sum[e]);
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const unsigned t = __reduce_max_sync(0xffffffffu, __float_as_uint(top[k]));
+    if ((tid & 31) == 0) best[8 * (tid >> 5) + k] = t;
   }
   __syncthreads();
-  if (tid < 8) roi.weights[tid] = fminf(roi.weights[tid], __uint_as_float(best[tid]));
+  if (tid < 8) {
+    unsigned t = 0u;
+    for (int w = 0; w < 8; ++w) t = max(t, best[8 * w + tid]);
+    roi.weights[tid] = fminf(roi.weights[tid], __uint_as_float(t));
+  }
   __syncthreads();
 }
 // Whether the sums of gradients of at most `top` (the bits of a half without its sign) are below a limit (not where that is infinite
@@ -806,7 +816,7 @@ __device__ __forceinline__ void brick_listed(const Params& p, const PairConst& p
 // without its sign), or to clear the accumulator where the roi is left to the scattering kernel.
 __global__ void __launch_bounds__(256, 4) bwd_brick3d_plan(const Params p, const BrickPlan plan, float* __restrict__ scratch) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  __shared__ unsigned warp_top[8];
+  __shared__ unsigned warp_top[64];
   __shared__ BrickRoi roi;
   const bool enough = brick_enough(p, reinterpret_cast<int*>(warp_top));
   if (blockIdx.x == 0 && threadIdx.x < 4) plan.number[threadIdx.x] = 0u;

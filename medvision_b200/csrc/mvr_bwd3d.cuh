@@ -393,14 +393,16 @@ bwd_brick3d_rest(const Params p, const PairConst pc, const BrickPlan plan, const
                  long long items) {
   extern __shared__ __align__(16) unsigned char brick_smem[];
   __shared__ BrickTurn work;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  const unsigned left = __ldcg(plan.number + 1);
+  // (the fold may come early where there is nothing to fold; else its loads would have the little L1 that this kernel's shared memory
+  // leaves: 2 x 128^3 12 us instead of 7)
+  if (left == 0u) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (blockIdx.x == 0 && p.status) {
     for (int n = threadIdx.x; n < p.R; n += kS3Threads)
       if (__ldcg(plan.volume + n) == INT_MIN) atomicOr(p.status, STATUS_BAD_BATCH_INDEX);
   }
   brick_listed(p, pc, plan, G, work, brick_smem);
-  const unsigned left = __ldcg(plan.number + 1);
   if (left == 0u) return;
   const bool all = left == (unsigned)(p.N * p.C);
   S3Shared<__half>& sh = *reinterpret_cast<S3Shared<__half>*>(brick_smem);
@@ -518,8 +520,7 @@ inline cudaError_t launch_bwd_brick3d(const Params& p, const S3Launch& L, long l
   G.run = 1;
   while (G.run < 4 && columns * ((bd + 2 * G.run - 1) / (2 * G.run)) >= 148 * 4 * 6) G.run *= 2;
   G.runs = (bd + G.run - 1) / G.run;
-  // each of the two launches that follow may become resident while the one before ends; not so the last, whose loads would have the
-  // little L1 that the others' shared memory leaves (2 x 128^3: 7 us instead of 12)
+  // each of the three launches that follow may become resident while the one before ends
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -536,7 +537,6 @@ inline cudaError_t launch_bwd_brick3d(const Params& p, const S3Launch& L, long l
   cfg.gridDim = dim3(148 * 3);
   cfg.dynamicSmemBytes = smem2;
   if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, bwd_brick3d_rest<PAIR>, p, pc, plan, G, L, scratch, ctas);
-  cfg.numAttrs = 0;
   cfg.gridDim = dim3(148 * 6);
   cfg.dynamicSmemBytes = 0;
   if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, bwd_fold_left_half, p, plan, (const float*)scratch);
