@@ -111,7 +111,8 @@ int mvr_roi_resample_fwd(const void* features, const void* rois, void* output, i
  * the feature shape, must be zero-filled by the caller (as the reference's Python does,
  * medvision/ops/roi_align_rotated_nd.py:148) and is accumulated into, like the reference
  * (medvision/csrc/cuda/roi_align_rotated_3d_cuda_kernel.cuh:251-260): with atomics in the element
- * type, except that half gradients of dense 3D calls are summed in float and rounded once.
+ * type, except that half gradients of dense 3D calls are summed in float, or exactly in whole multiples of 2^-24 (large calls), and
+ * rounded once.
  * The two x-neighbours of a tap row are added by one 16-byte reduction that carries zeros in its
  * other slots, so elements of grad_in next to a tap may have +0 added to them (a -0 becomes +0);
  * nothing outside the N*C*D*H*W elements of grad_in is touched.
@@ -124,7 +125,8 @@ int mvr_roi_resample_bwd(const void* grad_out, const void* rois, void* grad_in, 
 /* Backward for callers that must not allocate device memory.  It has no counterpart in the
  * reference.
  *
- * Same arguments, same result and same error codes as mvr_roi_resample_bwd.  The difference is
+ * Same arguments and error codes as mvr_roi_resample_bwd, and the same result but for the rounding of the sums: they are
+ * float here, where the regular entry point sums large half calls exactly.  The difference is
  * where the float accumulator of the dense 3D half-precision backward lives: the regular entry
  * point borrows it from the library's stream-ordered memory pool for the duration of the call; this one uses
  * a fixed array inside the library image and calls no cudaMalloc / cudaFree / pool routine at all

@@ -20,7 +20,7 @@
 // them: with gradients of 8 among some of 2e-6 the result was off by 7e-7, twelve times what its rounding allows).  It is rounded
 // to float once or twice, where the float accumulator of the scattering kernel rounds at every addition.
 //
-// What bounds it: instruction issue (73 % of the slots) and the shared-memory reductions (72 % of the data pipe: eight per sample
+// What bounds it: instruction issue (69 % of the slots on 4 x 128^3) and the shared-memory reductions (63 % of the data pipe: eight per sample
 // at 2.5 clocks; rows of 21 words and planes of 384 had the fewest bank conflicts of 250 pitches tried over rotations of up to 30
 // degrees).  16 x 128^3 under three axes: plan 15 us, one word 274, with two words and idle launches 295 in all, where the scattering
 // kernel takes 456 and the clear and the fold of its accumulator 70.  Gradients of 100 throughout, two words: 396.  Rows listed pair

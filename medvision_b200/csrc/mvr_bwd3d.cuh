@@ -13,7 +13,7 @@
 // voxel.  The result differs from any one run of the reference by less than two runs of the
 // reference differ from each other.
 //
-// Large half calls with few rois per volume are summed by bricks of the gradient instead (mvr_brick3d.cuh); this kernel then takes
+// Large half calls with a roi per volume are summed by bricks of the gradient instead (mvr_brick3d.cuh); this kernel then takes
 // what those leave.
 #pragma once
 #include <mutex>

@@ -11,7 +11,7 @@
 // float (3 fused multiply-adds).  Positions, taps, weights and sums of the warp itself are those of mvr_offset.cuh,
 // operation by operation.
 //
-// What bounds it: instruction issue (66 %) and the loads (L1's data pipe 53-65 % busy).  2 x 128 x 256 x 256: 131 us, where cells,
+// What bounds it: instruction issue (73 %) and the loads (L1's data pipe 59 % busy).  2 x 128 x 256 x 256: 131 us, where cells,
 // indices and addresses formed per voxel and tap (235 instructions per voxel of image and label) took 150, and lanes on every
 // other voxel 133; 4 x 64 x 100 x 100 46 -> 42; 2 x 96 x 160 x 160 66 -> 59; the first in float 183 -> 153.  Five CTAs per SM 138;
 // six 147; three 167.
